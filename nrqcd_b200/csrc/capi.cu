@@ -79,13 +79,13 @@ int ensure_red(nrq_ctx *ctx, int64_t doubles) {
   return NRQ_OK;
 }
 
-// final reduction of nq values over nb partial blocks into h_res[0..nq)
+// final reduction of nq values over nb partial blocks into h_res[0..nq): one
+// block per value, which stores it into the pinned host array itself (a
+// separate copy costs a launch as long as the reduction)
 int reduce_to_host(nrq_ctx *ctx, int64_t nb, int nq, unsigned maxmask) {
-  nrq::k_reduce_final<<<1, 256, 0, ctx->stream>>>(ctx->d_red, nb, nq, maxmask, ctx->d_res);
+  nrq::k_reduce_final<<<nq, 256, 0, ctx->stream>>>(ctx->d_red, nb, nq, maxmask, ctx->h_res);
   int rc = check_launch(ctx, "k_reduce_final");
   if (rc) return rc;
-  NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_res, ctx->d_res, sizeof(double) * nq, cudaMemcpyDeviceToHost,
-                                    ctx->stream));
   NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return NRQ_OK;
 }
@@ -234,7 +234,6 @@ extern "C" int nrq_init(const int64_t ext[3], const double a[4], int device, nrq
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) ctx->sm_count = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&ctx->d_res, sizeof(double) * 64) != cudaSuccess ||
         cudaMallocHost(&ctx->h_res, sizeof(double) * 64) != cudaSuccess)
       rc = NRQ_ERR_CUDA;
   }
@@ -252,7 +251,6 @@ extern "C" int nrq_finalize(nrq_ctx *ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   if (ctx->d_red) cudaFree(ctx->d_red);
-  if (ctx->d_res) cudaFree(ctx->d_res);
   if (ctx->h_res) cudaFreeHost(ctx->h_res);
   if (ctx->d_stage) cudaFree(ctx->d_stage);
   if (ctx->d_proj) cudaFree(ctx->d_proj);
@@ -959,13 +957,15 @@ extern "C" int nrq_heavy_norms(nrq_heavy *h, double *nq, double *na) {
   nrq_ctx *ctx = h->ctx;
   int rc = set_device(ctx);
   if (rc) return rc;
-  int64_t nb_ = nblk(ctx->lat.V, 256);
-  if ((rc = ensure_red(ctx, nb_ * 2))) return rc;
-  nrq::launch_norms(h->P, ctx->lat.V, ctx->d_red, nb_, ctx->stream);
+  // only the species asked for is read
+  const int sp0 = nq ? 0 : 1, nsp = (nq && na) ? 2 : 1;
+  int64_t nb_ = nblk(ctx->lat.V, 128);
+  if ((rc = ensure_red(ctx, nb_ * nsp))) return rc;
+  nrq::launch_norms(h->P, ctx->lat.V, sp0, nsp, ctx->d_red, nb_, ctx->stream);
   if ((rc = check_launch(ctx, "k_norms"))) return rc;
-  if ((rc = reduce_to_host(ctx, nb_, 2, 0u))) return rc;
+  if ((rc = reduce_to_host(ctx, nb_, nsp, 0u))) return rc;
   if (nq) *nq = std::sqrt(ctx->h_res[0]);
-  if (na) *na = std::sqrt(ctx->h_res[1]);
+  if (na) *na = std::sqrt(ctx->h_res[nsp - 1]);
   return NRQ_OK;
 }
 

@@ -683,160 +683,102 @@ void launch_single_point(double2 *P, int64_t V, int64_t sq, int64_t sa, cudaStre
   k_single_point<<<(unsigned)((V + 255) / 256), 256, 0, st>>>(P, V, sq, sa);
 }
 
-__global__ void __launch_bounds__(256) k_norms(const double2 *__restrict__ P, int64_t V, double *partials) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double v[2] = {0.0, 0.0};
-  if (s < V)
-    for (int sp = 0; sp < 2; ++sp)
-      for (int k = 0; k < 36; ++k) v[sp] += norm2(ldg(P + (int64_t)(sp * 36 + k) * V + s));
-  __shared__ double sh[8][2];
+// |psi|^2 of species sp0 .. sp0 + nsp - 1 (blockIdx.y picks the species), one
+// partial per (block, species).  One thread per site with its 36 loads
+// unrolled: bound by the 576 B per site and species it reads (64^3, both
+// species: 49 us, 95 % of the copy rate).
+__global__ void __launch_bounds__(128) k_norms(const double2 *__restrict__ P, int64_t V, int sp0, double *partials) {
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  double v = 0.0;
+  if (s < V) {
+    const double2 *p = P + (int64_t)((sp0 + (int)blockIdx.y) * 36) * V + s;
+#pragma unroll
+    for (int k = 0; k < 36; ++k) v += norm2(ldg(p + (int64_t)k * V));
+  }
+  __shared__ double sh[4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = 0; k < 2; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  if (lane == 0) {
-    sh[warp][0] = v[0];
-    sh[warp][1] = v[1];
-  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) sh[warp] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0, b = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
-      a += sh[k][0];
-      b += sh[k][1];
-    }
-    partials[blockIdx.x * 2] = a;
-    partials[blockIdx.x * 2 + 1] = b;
-  }
+  if (threadIdx.x == 0) partials[(int64_t)blockIdx.x * gridDim.y + blockIdx.y] = (sh[0] + sh[1]) + (sh[2] + sh[3]);
 }
-void launch_norms(const double2 *P, int64_t V, double *partials, int64_t &nblk, cudaStream_t st) {
-  nblk = (V + 255) / 256;
-  k_norms<<<(unsigned)nblk, 256, 0, st>>>(P, V, partials);
+void launch_norms(const double2 *P, int64_t V, int sp0, int nsp, double *partials, int64_t &nblk, cudaStream_t st) {
+  nblk = (V + 127) / 128;
+  k_norms<<<dim3((unsigned)nblk, (unsigned)nsp), 128, 0, st>>>(P, V, sp0, partials);
 }
 
-// Sparse Gamma tables for the zero-momentum meson correlators
-// (src/nrqcd.f90:1484-1661): entries (row, col, re, im) of Gamma = T^a x s_k,
-// 1 x s_k or T^a x 1 (index 2*colour + spin), with the reference's matrices.
-struct GamEntry {
-  double re, im;
-  int r, c;
-};
-struct GamTable {
-  int ngam[3];       // O1_3S1, O8_1S0, O8_3S1
-  int start[3][24];  // entry offset per Gamma
-  int count[3][24];
-  GamEntry e[3 * 24 * 8];
-};
-__constant__ GamTable c_gam;
-
+// Zero-momentum meson correlators (src/nrqcd.f90:1484-1661).  With A the
+// antiquark's and Q the quark's 6x6 matrix, each is a weighted sum over a
+// basis of matrices G of i Tr(A^+ G Q G) = i sum conj(A[d1][d0]) G[d1][d2]
+// Q[d2][d3] G[d3][d0], and the sums over the bases close:
+//   sum_k s_k[s1][s2] s_k[s3][s0] = 2 d(s1,s0) d(s2,s3) - d(s1,s2) d(s3,s0)
+//   sum_a T_a[c1][c2] T_a[c3][c0] = (d(c1,c0) d(c2,c3) - d(c1,c2) d(c3,c0)/3)/2
+// (the reference's transposed s_2, T_2, T_5, T_7 enter in pairs and change
+// neither).  So all four follow from S = sum conj(A) Q, the products of the
+// partial traces over spin (3x3) and over colour (2x2), and Tr A, Tr Q:
+//   O1_1S0 = i S                      O1_3S1 = i (2 Ps - S) / 3
+//   O8_1S0 = i (6/8) (Pc - S/3) / 2   O8_3S1 = i (6/24) (Pt - Pc/2 - Ps/3 + S/6)
+// One pass over the 72 planes: bound by the 1152 B per site it reads (64^3:
+// 53 us; the sums over the sparse products of the 35 matrices took 714 us).
+//
 // GCONJ: the _gconjg variants (src/nrqcd.f90:1728-1905), conj(A) in place of
-// A^+, i.e. A's indices swapped in every product below
+// A^+, i.e. A transposed.
 template <bool GCONJ>
 __global__ void __launch_bounds__(128) k_correlators(const double2 *__restrict__ P, int64_t V, double *partials) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  cplx S = {0.0, 0.0}, Ps = {0.0, 0.0}, Pc = {0.0, 0.0}, Pt = {0.0, 0.0};
   if (s < V) {
-    // Q[r][c] = quark (row r, col c), A likewise
-    auto q = [&](int r, int c) { return ldg(P + (int64_t)(c * 6 + r) * V + s); };
-    auto a = [&](int r, int c) {
-      return GCONJ ? ldg(P + (int64_t)(36 + r * 6 + c) * V + s) : ldg(P + (int64_t)(36 + c * 6 + r) * V + s);
-    };
-    // O1_1S0 = i Tr(A^+ Q) = i sum_{rc} conj(A[r][c]) Q[r][c]
-    cplx t = {0.0, 0.0};
-    for (int r = 0; r < 6; ++r)
-      for (int c = 0; c < 6; ++c) cmac_cj(t, a(r, c), q(r, c));
-    cplx o = times_i(t);
-    v[0] = o.re;
-    v[1] = o.im;
-    const double wts[3] = {1.0 / 3.0, 6.0 / 8.0, 6.0 / 24.0};
-    for (int kind = 0; kind < 3; ++kind) {
-      cplx sum = {0.0, 0.0};
-      for (int g = 0; g < c_gam.ngam[kind]; ++g) {
-        const int st0 = c_gam.start[kind][g], n = c_gam.count[kind][g];
-        // Tr(A^+ G Q G) = sum conj(A[d1][d0]) G[d1][d2] Q[d2][d3] G[d3][d0]
-        for (int e1 = 0; e1 < n; ++e1) {
-          const GamEntry ga = c_gam.e[st0 + e1];  // (d1, d2)
-          for (int e2 = 0; e2 < n; ++e2) {
-            const GamEntry gb = c_gam.e[st0 + e2];  // (d3, d0)
-            cplx gg = cplx{ga.re, ga.im} * cplx{gb.re, gb.im};
-            cplx qa = q(ga.c, gb.r);
-            cplx term = {0.0, 0.0};
-            cmac_cj(term, a(ga.r, gb.c), qa);
-            cmac(sum, gg, term);
-          }
-        }
-      }
-      cplx ov = times_i(sum) * wts[kind];
-      v[2 + 2 * kind] = ov.re;
-      v[3 + 2 * kind] = ov.im;
-    }
-  }
-  __shared__ double sh[4][8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int k = 0; k < 8; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  if (lane == 0)
-    for (int k = 0; k < 8; ++k) sh[warp][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x < 8) {
-    double acc = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) acc += sh[k][threadIdx.x];
-    partials[blockIdx.x * 8 + threadIdx.x] = acc;
-  }
-}
-
-static void build_gamma_table(GamTable &T) {
-  // reference generators (row-major) and Pauli matrices (su2.f90 arrays)
-  double Tre[8][9] = {{0}}, Tim[8][9] = {{0}};
-  const double h = 0.5, s8 = 0.5 / 1.7320508075688772, d8 = 1.0 / 1.7320508075688772;
-  Tre[0][1] = Tre[0][3] = h;
-  Tim[1][1] = h; Tim[1][3] = -h;
-  Tre[2][0] = h; Tre[2][4] = -h;
-  Tre[3][2] = Tre[3][6] = h;
-  Tim[4][2] = h; Tim[4][6] = -h;
-  Tre[5][5] = Tre[5][7] = h;
-  Tim[6][5] = h; Tim[6][7] = -h;
-  Tre[7][0] = s8; Tre[7][4] = s8; Tre[7][8] = -d8;
-  double Sre[3][4] = {{0, 1, 1, 0}, {0, 0, 0, 0}, {1, 0, 0, -1}};
-  double Sim[3][4] = {{0, 0, 0, 0}, {0, 1, -1, 0}, {0, 0, 0, 0}};
-  int ne = 0;
-  auto add_gamma = [&](int kind, int g, const double *Are, const double *Aim, const double *Bre,
-                       const double *Bim) {
-    T.start[kind][g] = ne;
-    int cnt = 0;
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c)
-        for (int s = 0; s < 2; ++s)
-          for (int t = 0; t < 2; ++t) {
-            double ar = Are[r * 3 + c], ai = Aim[r * 3 + c], br = Bre[s * 2 + t], bi = Bim[s * 2 + t];
-            double vr = ar * br - ai * bi, vi = ar * bi + ai * br;
-            if (vr != 0.0 || vi != 0.0) {
-              T.e[ne++] = GamEntry{vr, vi, 2 * r + s, 2 * c + t};
-              ++cnt;
+    cplx ca[4], cq[4];  // partial traces over colour, index 2*row spin + column spin
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ca[k] = cq[k] = {0.0, 0.0};
+#pragma unroll
+    for (int c1 = 0; c1 < 3; ++c1)
+#pragma unroll
+      for (int c0 = 0; c0 < 3; ++c0) {
+        cplx sa = {0.0, 0.0}, sq = {0.0, 0.0};
+#pragma unroll
+        for (int s1 = 0; s1 < 2; ++s1)
+#pragma unroll
+          for (int s0 = 0; s0 < 2; ++s0) {
+            const int r = 2 * c1 + s1, c = 2 * c0 + s0;
+            const cplx q = ldg(P + (int64_t)(c * 6 + r) * V + s);
+            const cplx a = ldg(P + (int64_t)(36 + (GCONJ ? r * 6 + c : c * 6 + r)) * V + s);
+            cmac_cj(S, a, q);
+            if (s1 == s0) {
+              sa = sa + a;
+              sq = sq + q;
+            }
+            if (c1 == c0) {
+              ca[2 * s1 + s0] = ca[2 * s1 + s0] + a;
+              cq[2 * s1 + s0] = cq[2 * s1 + s0] + q;
             }
           }
-    T.count[kind][g] = cnt;
-  };
-  double I3re[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, I3im[9] = {0};
-  double I2re[4] = {1, 0, 0, 1}, I2im[4] = {0};
-  T.ngam[0] = 3;
-  for (int k = 0; k < 3; ++k) add_gamma(0, k, I3re, I3im, Sre[k], Sim[k]);
-  T.ngam[1] = 8;
-  for (int a = 0; a < 8; ++a) add_gamma(1, a, Tre[a], Tim[a], I2re, I2im);
-  T.ngam[2] = 24;
-  int g = 0;
-  for (int k = 0; k < 3; ++k)
-    for (int a = 0; a < 8; ++a) add_gamma(2, g++, Tre[a], Tim[a], Sre[k], Sim[k]);
+        cmac_cj(Ps, sa, sq);
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) cmac_cj(Pc, ca[k], cq[k]);
+    Pt = conj(ca[0] + ca[3]) * (cq[0] + cq[3]);
+  }
+  const cplx o[4] = {times_i(S), (1.0 / 3.0) * times_i(2.0 * Ps - S), (3.0 / 8.0) * times_i(Pc - (1.0 / 3.0) * S),
+                     0.25 * times_i(Pt - 0.5 * Pc - (1.0 / 3.0) * Ps + (1.0 / 6.0) * S)};
+  __shared__ double sh[4][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    double v = (k & 1) ? o[k >> 1].im : o[k >> 1].re;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+    if (lane == 0) sh[warp][k] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 8)
+    partials[(int64_t)blockIdx.x * 8 + threadIdx.x] =
+        (sh[0][threadIdx.x] + sh[1][threadIdx.x]) + (sh[2][threadIdx.x] + sh[3][threadIdx.x]);
 }
 
 void launch_correlators(const double2 *P, int64_t V, double *partials, int64_t &nblk, cudaStream_t st,
                         bool gconjg) {
-  static GamTable T;
-  static bool built = false;
-  if (!built) {
-    build_gamma_table(T);
-    built = true;
-  }
-  cudaMemcpyToSymbolAsync(c_gam, &T, sizeof(T), 0, cudaMemcpyHostToDevice, st);
   nblk = (V + 127) / 128;
   if (gconjg) k_correlators<true><<<(unsigned)nblk, 128, 0, st>>>(P, V, partials);
   else k_correlators<false><<<(unsigned)nblk, 128, 0, st>>>(P, V, partials);

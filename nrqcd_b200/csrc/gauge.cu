@@ -435,11 +435,12 @@ __global__ void __launch_bounds__(256) k_gauss(Lat L, const double2 *__restrict_
 }
 
 // Final deterministic reduction: out[q] = op over nblk partials[b*nq+q]
-// (op: 0 sum, 1 max selected by mask bit q).
+// (op: 0 sum, 1 max selected by mask bit q); the blocks of the grid share
+// the values q.
 __global__ void k_reduce_final(const double *__restrict__ partials, int64_t nblk, int nq,
                                unsigned maxmask, double *out) {
   __shared__ double sh[256];
-  for (int q = 0; q < nq; ++q) {
+  for (int q = blockIdx.x; q < nq; q += gridDim.x) {
     const bool isMax = (maxmask >> q) & 1u;
     double acc = 0.0;
     for (int64_t b = threadIdx.x; b < nblk; b += blockDim.x) {

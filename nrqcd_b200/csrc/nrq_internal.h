@@ -15,11 +15,10 @@ struct nrq_ctx {
   nrq::Lat lat{};
   int64_t n[3] = {0, 0, 0};
   double a[4] = {0, 0, 0, 0};
-  // reduction scratch (device + pinned host mirror)
+  // reduction scratch: device partial sums, pinned results
   double *d_red = nullptr;     // partial sums, red_cap doubles
   int64_t red_cap = 0;
-  double *d_res = nullptr;     // final results, 64 doubles
-  double *h_res = nullptr;     // pinned, 64 doubles
+  double *h_res = nullptr;     // final results, pinned, 64 doubles (the last reduction stage stores into it)
   // staging buffer for layout transposes (device), grown on demand
   void *d_stage = nullptr;
   size_t stage_bytes = 0;

@@ -233,16 +233,15 @@ class NRQCDField:
         return self.last_stats
 
     # ------------------------------------------------------------ observables
-    def _norms(self):
-        a, b = ctypes.c_double(), ctypes.c_double()
-        self._call("nrq_heavy_norms", ctypes.byref(a), ctypes.byref(b))
-        return a.value, b.value
-
     def GetNorm_Quark(self) -> float:
-        return self._norms()[0]
+        a = ctypes.c_double()
+        self._call("nrq_heavy_norms", ctypes.byref(a), None)
+        return a.value
 
     def GetNorm_AntiQ(self) -> float:
-        return self._norms()[1]
+        a = ctypes.c_double()
+        self._call("nrq_heavy_norms", None, ctypes.byref(a))
+        return a.value
 
     def _correlators(self):
         out = np.empty(8)
