@@ -50,67 +50,6 @@ __device__ void field_strength_from_plaquette(const m3 &P, double scale_, double
     }
 }
 
-// Same quantity for plaquettes inside the principal branch with small
-// angles, without an eigen-decomposition.  For unitary P = exp(iH) whose
-// eigenphases satisfy |theta| < pi/2, K = (P - P^+)/(2i) = sin(H) and
-// H = asin(K) = sum_n c_n K^(2n+1), c_n = (2n)!/(4^n (n!)^2 (2n+1)).  The
-// powers of K are reduced with Cayley-Hamilton (K^3 = t1 K^2 - t2 K + t3 1
-// with the real invariants of the hermitian K), so the series runs on three
-// real coefficients and H = f0 1 + f1 K + f2 K^2 is assembled once.  Used
-// when |K|_F <= 0.3 and Re Tr P > 2 (all eigenphases then lie within
-// |theta| < 0.31); the Jacobi route handles every other plaquette.  Both
-// return Re(LogU(P)/i) to rounding.
-__device__ bool field_strength_small_angle(const m3 &P, double scale_, double F[9]) {
-  const double trP = P.e[0].re + P.e[4].re + P.e[8].re;
-  m3 K;
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      // (P[r][c] - conj(P[c][r])) / (2i)
-      cplx d = P.e[r * 3 + c] - conj(P.e[c * 3 + r]);
-      K.e[r * 3 + c] = {0.5 * d.im, -0.5 * d.re};
-    }
-  double nf2 = 0.0;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) nf2 += norm2(K.e[k]);
-  if (!(trP > 2.0) || !(nf2 <= 0.09)) return false;
-  const double rho = sqrt(nf2);
-  const m3 K2 = mul(K, K);
-  const double t1 = K.e[0].re + K.e[4].re + K.e[8].re;
-  const double trK2 = K2.e[0].re + K2.e[4].re + K2.e[8].re;
-  const double t2 = 0.5 * (t1 * t1 - trK2);
-  // det K (real for hermitian K)
-  const cplx det = K.e[0] * (K.e[4] * K.e[8] - K.e[5] * K.e[7]) - K.e[1] * (K.e[3] * K.e[8] - K.e[5] * K.e[6]) +
-                   K.e[2] * (K.e[3] * K.e[7] - K.e[4] * K.e[6]);
-  const double t3 = det.re;
-  // K^m = a 1 + b K + d K^2 ; start m = 1
-  double a = 0.0, b = 1.0, d = 0.0;
-  double f0 = 0.0, f1 = 1.0, f2 = 0.0;  // c_0 K
-  double cn = 1.0, pw = rho;            // c_n (n = 0) and rho^(2n+1)
-  for (int n = 1; n <= 40; ++n) {
-    // two multiplications by K: K^(2n+1) from K^(2n-1)
-    for (int rep = 0; rep < 2; ++rep) {
-      const double an = d * t3, bn = a - d * t2, dn = b + d * t1;
-      a = an;
-      b = bn;
-      d = dn;
-    }
-    cn *= (double)(2 * n - 1) * (double)(2 * n - 1) / ((double)(2 * n) * (double)(2 * n + 1));
-    pw *= nf2;
-    f0 += cn * a;
-    f1 += cn * b;
-    f2 += cn * d;
-    if (cn * pw < 1e-19 * rho) break;
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const double h = f1 * K.e[k].re + f2 * K2.e[k].re + ((k % 4 == 0) ? f0 : 0.0);
-    F[k] = h * scale_;
-  }
-  return true;
-}
-
 // E_j(y) entering the CN operator: -Re(sum_a E~^a T^a)/a0/a_j (real symmetric)
 __device__ __forceinline__ m3 efield_cn(const Lat &L, const double *__restrict__ E, int64_t y, int j) {
   const int64_t V = L.V;
@@ -155,8 +94,14 @@ __global__ void __launch_bounds__(128) k_cn_prepare(Lat L, const double2 *__rest
                          load_link(U, V, nb(L, x, k, +1), j)),
                   load_link(U, V, x, k));
     double F[9];
-    if (!field_strength_small_angle(P, 1.0 / L.a[j] / L.a[k], F))
-      field_strength_from_plaquette(P, 1.0 / L.a[j] / L.a[k], F);
+    m3 H;
+    const double scale_ = 1.0 / L.a[j] / L.a[k];
+    if (log_unitary(P, H)) {
+#pragma unroll
+      for (int m = 0; m < 9; ++m) F[m] = H.e[m].re * scale_;
+    } else {
+      field_strength_from_plaquette(P, scale_, F);
+    }
     for (int m = 0; m < 9; ++m) B[m] += F[m];
   }
 #pragma unroll

@@ -164,26 +164,29 @@ __global__ void __launch_bounds__(128) k_gluon_fields(Lat L, const double2 *__re
   if (s >= V) return;
 #pragma unroll 1
   for (int i = 0; i < 3; ++i) {
-    cplx ev[3];
-    m3 S;
-    eigenc3(load_link(U, V, s, i), ev, S);
-    double th[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) th[k] = atan2(ev[k].im, ev[k].re);
-    // ArgLogU = S^+ diag(theta) S
+    const m3 u = load_link(U, V, s, i);
     m3 h;
+    if (!log_unitary(u, h)) {
+      cplx ev[3];
+      m3 S;
+      eigenc3(u, ev, S);
+      double th[3];
 #pragma unroll
-    for (int r = 0; r < 3; ++r)
+      for (int k = 0; k < 3; ++k) th[k] = atan2(ev[k].im, ev[k].re);
+      // ArgLogU = S^+ diag(theta) S
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        cplx acc = {0.0, 0.0};
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const cplx a = conj(S.e[k * 3 + r]), b = S.e[k * 3 + c];
-          acc = acc + th[k] * (a * b);
+        for (int c = 0; c < 3; ++c) {
+          cplx acc = {0.0, 0.0};
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const cplx a = conj(S.e[k * 3 + r]), b = S.e[k * 3 + c];
+            acc = acc + th[k] * (a * b);
+          }
+          h.e[r * 3 + c] = acc;
         }
-        h.e[r * 3 + c] = acc;
-      }
+    }
     cplx tr[8];
     traces_with_generators(h, tr);
 #pragma unroll

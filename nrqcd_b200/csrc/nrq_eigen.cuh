@@ -90,4 +90,68 @@ __device__ inline void eigenc3(const m3 &Ain, cplx d[3], m3 &U) {
   }
 }
 
+// ------------------------------------------------------------ unitary log
+// c_n = 2^2n (n!)^2 / (2n+1)!, the coefficients of the series below
+constexpr int kLogTerms = 144;
+struct LogCoef {
+  double c[kLogTerms];
+};
+constexpr LogCoef make_log_coef() {
+  LogCoef t{};
+  t.c[0] = 1.0;
+  for (int n = 1; n < kLogTerms; ++n) t.c[n] = t.c[n - 1] * (2.0 * n) / (2.0 * n + 1.0);
+  return t;
+}
+static __constant__ LogCoef c_log = make_log_coef();
+
+// H with P = exp(iH) and eigenphases theta in (-pi, pi), for unitary P whose
+// sin^2(theta/2) stay below 3/4, without an eigen-decomposition.  Euler's
+// series of the arctangent at tan(theta/2) reads
+//   theta = sin(theta) sum_n c_n y^n,   y = sin^2(theta/2),
+// so H = K sum_n c_n Y^n with K = (P - P^+)/(2i) = sin H and
+// Y = (2 - P - P^+)/4 = sin^2(H/2), which commute.  The sum is taken by
+// Horner's rule on three real coefficients (Y^3 = t1 Y^2 - t2 Y + t3 by
+// Cayley-Hamilton, Y hermitian), as many terms as the largest eigenvalue,
+// bounded by rho = |Y|_F, needs for 1e-17: about 20 for plaquettes of a
+// thermal field.  The Jacobi route takes any unitary matrix but diverges
+// over a warp and costs 2-3 times the rest of the preparation: false asks
+// for it.  The line rho = 3/4 needs 137 terms, still under the Jacobi
+// sweeps' time; beyond it the terms grow as 1 / (1 - rho).
+__device__ __forceinline__ bool log_unitary(const m3 &P, m3 &H) {
+  m3 K, Y;
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const cplx a = P.e[r * 3 + c], b = conj(P.e[c * 3 + r]);
+      K.e[r * 3 + c] = {0.5 * (a.im - b.im), -0.5 * (a.re - b.re)};
+      Y.e[r * 3 + c] = {(r == c ? 0.5 : 0.0) - 0.25 * (a.re + b.re), -0.25 * (a.im + b.im)};
+    }
+  const m3 Y2 = mul(Y, Y);
+  const double t1 = Y.e[0].re + Y.e[4].re + Y.e[8].re;
+  const double ty2 = Y2.e[0].re + Y2.e[4].re + Y2.e[8].re;
+  if (!(ty2 <= 0.5625)) return false;
+  const double t2 = 0.5 * (t1 * t1 - ty2);
+  const cplx det = Y.e[0] * (Y.e[4] * Y.e[8] - Y.e[5] * Y.e[7]) - Y.e[1] * (Y.e[3] * Y.e[8] - Y.e[5] * Y.e[6]) +
+                   Y.e[2] * (Y.e[3] * Y.e[7] - Y.e[4] * Y.e[6]);
+  const double t3 = det.re;
+  // terms: rho^n < 1e-17, rho = sqrt(ty2) <= 3/4
+  const int n = min(kLogTerms - 1, (int)(78.3f / -__logf(fmaxf((float)ty2, 1e-34f))) + 2);
+  double a = c_log.c[n], b = 0.0, d = 0.0;
+  for (int k = n - 1; k >= 0; --k) {
+    const double an = fma(d, t3, c_log.c[k]), bn = fma(-d, t2, a), dn = fma(d, t1, b);
+    a = an;
+    b = bn;
+    d = dn;
+  }
+  m3 f;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) f.e[k] = b * Y.e[k] + d * Y2.e[k];
+  f.e[0].re += a;
+  f.e[4].re += a;
+  f.e[8].re += a;
+  H = mul(K, f);
+  return true;
+}
+
 }  // namespace nrq
