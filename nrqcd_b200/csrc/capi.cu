@@ -33,7 +33,9 @@ inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 constexpr size_t kScalDoubles = (size_t)nrq::CN_COLS * nrq::SC_STRIDE;
 // after the scalars: 16 ints of the stencils' error record (the flag, and
 // where a bounded wait expired)
-constexpr size_t kScalBytes = sizeof(double) * (kScalDoubles + 8);
+// and 4 doubles of the spectral enclosure (quark lo, hi, antiquark lo, hi)
+constexpr size_t kScalBytes = sizeof(double) * (kScalDoubles + 8 + 4);
+inline double *scal_bounds(double *scal) { return scal + kScalDoubles + 8; }
 inline int *scal_err(double *scal) { return (int *)(scal + kScalDoubles); }
 // the stencils' record of an expired pipeline wait (4 ints after the
 // scalars): the message of the update that reports it, and a reset
@@ -48,12 +50,6 @@ std::string timeout_message(const double *h_scal) {
     m += std::string(" (") + (stencil == 6 ? "k_cheb5f" : "k_cn_mv" + std::to_string(stencil)) + ", " +
          (role >= 0 && role < 5 ? roles[role] : "?") +
          ", load " + std::to_string(e[2]) + ", CTA " + std::to_string(e[3]);
-    if (e[4] != 0) {  // the FMA stencil's detail: the loader's progress and the barrier's word
-      char buf[96];
-      snprintf(buf, sizeof buf, ", loads issued %d, barrier %08x%08x, parity %d", e[4] - 1, (unsigned)e[6],
-               (unsigned)e[5], e[7]);
-      m += buf;
-    }
     m += ")";
   }
   return m;
@@ -1033,7 +1029,6 @@ extern "C" int nrq_cn_init(nrq_ctx *ctx, double mass, const double c[8], double 
     alloc((void **)&cn->D32, sizeof(float2) * 9 * V);
     alloc((void **)&cn->B32, sizeof(float) * 9 * V);
     for (float2 **pp : {&cn->r32, &cn->dA32, &cn->dB32, &cn->e32}) alloc((void **)pp, sizeof(float2) * 72 * V);
-    alloc((void **)&cn->bounds, sizeof(double) * (4 * ((V + 255) / 256) + 8));
     if (ok && cudaMallocHost((void **)&cn->h_bounds, sizeof(double) * 8) != cudaSuccess) ok = false;
   }
   // the TMA-staged stencil needs 16-byte plane strides for the real-valued
@@ -1102,6 +1097,7 @@ extern "C" int nrq_cn_cheb_info(const nrq_cn *cn, int *last, double ms[2]) {
 extern "C" int nrq_cn_set_merged_update(nrq_cn *cn, int on) {
   if (!cn || on < 0 || on > 1) return NRQ_ERR_BAD_ARG;
   cn->merged_update = on != 0;
+  cn->semi_iter = false;  // either BiCGStab update was asked for
   return NRQ_OK;
 }
 
@@ -1136,11 +1132,13 @@ extern "C" int nrq_cn_finalize(nrq_cn *cn) {
   for (void *p : {(void *)cn->Dsum, (void *)cn->Bsum, (void *)cn->DE, (void *)cn->b, (void *)cn->x, (void *)cn->r,
                   (void *)cn->rh, (void *)cn->p, (void *)cn->v, (void *)cn->t, (void *)cn->s, (void *)cn->scal,
                   (void *)cn->partials, (void *)cn->U32, (void *)cn->DE32, (void *)cn->D32, (void *)cn->B32,
-                  (void *)cn->r32, (void *)cn->dA32, (void *)cn->dB32, (void *)cn->e32, (void *)cn->bounds,
-                  (void *)cn->Wblk, (void *)cn->Wblk5, (void *)cn->Wblk5f})
+                  (void *)cn->r32, (void *)cn->dA32, (void *)cn->dB32, (void *)cn->e32,
+                  (void *)cn->Wblk, (void *)cn->Wblk5f, (void *)cn->spin.W, (void *)cn->spin.S0, (void *)cn->spin.S1,
+                  (void *)cn->spin_scratch, (void *)cn->spin_part, (void *)cn->spin_ticket, (void *)cn->cheb_tab})
     if (p) cudaFree(p);
   if (cn->h_scal) cudaFreeHost(cn->h_scal);
   if (cn->h_bounds) cudaFreeHost(cn->h_bounds);
+  if (cn->h_cheb) cudaFreeHost(cn->h_cheb);
   delete cn;
   return NRQ_OK;
 }
@@ -1152,8 +1150,9 @@ namespace {
 // formed.  Derived data a stencil reads instead (the tensor-core stencil's
 // cached blocks) is extra traffic and is not counted.
 double mv_bytes(const nrq_ctx *ctx, int mode) {
-  // PLAIN, RHS, RES, V, T, RESC, T2, RES2, V2 (the FP32 shadow residual half a stream)
-  const double streams[9] = {2, 3, 5, 3, 2, 3, 2.5, 4.5, 2.5};
+  // PLAIN, RHS, RES, V, T, RESC, T2, RES2, V2 (the FP32 shadow residual half
+  // a stream), RESN, CH0, CHK, CHH
+  const double streams[13] = {2, 3, 5, 3, 2, 3, 2.5, 4.5, 2.5, 2, 3, 4, 5.5};
   return (double)ctx->lat.V * (1152.0 * streams[mode] + 2.0 * (432.0 + 192.0));
 }
 // the tensor-core stencil's backward blocks are -W^H of the forward ones,
@@ -1179,7 +1178,7 @@ int ensure_blocks(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *
   nrq_ctx *ctx = cn->ctx;
   *sign = blocks_sign(cn->w_valid, cn->w_coef, C);
   if (*sign != 0.0) return NRQ_OK;
-  const int64_t V = ctx->lat.V;
+  const int64_t V = ctx->lat.V;  // the caller ran ensure_legacy
   if (!cn->Wblk) NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->Wblk, sizeof(double2) * 216 * V));
   {
     ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + 3456.0));
@@ -1197,62 +1196,97 @@ bool use_cheb5f(const nrq_cn *cn) {
   if (cn->form < 1 || cn->cheb_stencil == NRQ_CHEB_REGISTER || !nrq::cheb5f_applicable(cn->ctx->lat)) return false;
   return cn->cheb_stencil == NRQ_CHEB_BLOCKS || !cn->cheb_tuned || cn->cheb_choice == NRQ_CHEB_BLOCKS;
 }
-// The FMA stencil's blocks (FP64, f32 = false) or the FP32 Chebyshev step's
-// (f32 = true), with the coefficients C.  Where the other precision is
-// missing for the same coefficients and the update will need it too, one
-// pass writes both.
-int ensure_blocks5(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *sign, bool f32 = false) {
+// the matrices of the other stencils, on demand after cn_prepare
+int ensure_legacy(nrq_cn *cn, const nrq_gauge *g) {
+  if (cn->legacy_valid) return NRQ_OK;
   nrq_ctx *ctx = cn->ctx;
-  *sign = f32 ? blocks_sign(cn->w5f_valid, cn->w5f_coef, C) : blocks_sign(cn->w5_valid, cn->w5_coef, C);
+  ProfScope ps(ctx, 3, (double)ctx->lat.V * (432.0 + 192.0));
+  nrq::launch_cn_prepare(ctx->lat, g->U, g->E, cn->Dsum, cn->Bsum, cn->DE, ctx->stream);
+  cn->legacy_valid = true;
+  return check_launch(ctx, "k_cn_prepare");
+}
+// The FP32 Chebyshev step's blocks with the coefficients C.
+int ensure_blocks5f(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *sign) {
+  nrq_ctx *ctx = cn->ctx;
+  *sign = blocks_sign(cn->w5f_valid, cn->w5f_coef, C);
   if (*sign != 0.0) return NRQ_OK;
   const int64_t V = ctx->lat.V;
-  const bool want64 = !f32 || (cn->stencil == NRQ_STENCIL_FMA && blocks_sign(cn->w5_valid, cn->w5_coef, C) == 0.0);
-  const bool want32 = f32 || (use_cheb5f(cn) && blocks_sign(cn->w5f_valid, cn->w5f_coef, C) == 0.0);
-  if (want64 && !cn->Wblk5)
-    NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->Wblk5, sizeof(double2) * nrq::cn_mv5_block_entries(V)));
-  if (want32 && !cn->Wblk5f)
+  int rc = ensure_legacy(cn, g);
+  if (rc) return rc;
+  if (!cn->Wblk5f)
     NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->Wblk5f, sizeof(float2) * nrq::cn_mv5_block_entries(V)));
   {
-    ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + (want64 ? 3456.0 : 0.0) + (want32 ? 1728.0 : 0.0)));
-    nrq::launch_cn_blocks5(ctx->lat, C, g->U, cn->DE, want64 ? cn->Wblk5 : nullptr, want32 ? cn->Wblk5f : nullptr,
-                           ctx->stream);
+    ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + 1728.0));
+    nrq::launch_cn_blocks5(ctx->lat, C, g->U, cn->DE, nullptr, cn->Wblk5f, ctx->stream);
   }
-  if (want64) {
-    cn->w5_coef = C;
-    cn->w5_valid = true;
-  }
-  if (want32) {
-    cn->w5f_coef = C;
-    cn->w5f_valid = true;
-  }
+  cn->w5f_coef = C;
+  cn->w5f_valid = true;
   *sign = 1.0;
   return check_launch(ctx, "k_cn_blocks5");
+}
+// The operator in its spin structure for the coefficients C (of A^H, tau =
+// dt a0/2 of that solve); sign -1 where it was built for C negated.
+int ensure_spin(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *sign) {
+  nrq_ctx *ctx = cn->ctx;
+  const int64_t V = ctx->lat.V;
+  *sign = blocks_sign(cn->spin_valid, cn->spin_coef, C);
+  if (*sign != 0.0) {  // the site term as well
+    for (int sp = 0; sp < 2; ++sp)
+      if (cn->spin_coef.mag[sp].im != *sign * C.mag[sp].im || cn->spin_coef.dar[sp].im != *sign * C.dar[sp].im)
+        *sign = 0.0;
+    if (*sign != 0.0) return NRQ_OK;
+  }
+  auto want = [&](auto **p, size_t bytes) { return *p ? cudaSuccess : cudaMalloc((void **)p, bytes); };
+  if (!cn->spin_ticket) {
+    NRQ_CUDA_TRY(ctx, want(&cn->spin_ticket, sizeof(unsigned)));
+    NRQ_CUDA_TRY(ctx, cudaMemsetAsync(cn->spin_ticket, 0, sizeof(unsigned), ctx->stream));
+  }
+  NRQ_CUDA_TRY(ctx, want(&cn->spin_part, sizeof(double) * 4 * ((V + 255) / 256)));
+  NRQ_CUDA_TRY(ctx, want(&cn->spin_scratch, sizeof(double) * 7 * V));
+  NRQ_CUDA_TRY(ctx, want(&cn->spin.S0, sizeof(double2) * 9 * V));
+  NRQ_CUDA_TRY(ctx, want(&cn->spin.S1, sizeof(double) * 9 * V));
+  NRQ_CUDA_TRY(ctx, want(&cn->spin.W, sizeof(double2) * 81 * V));
+  {
+    ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0 + 1296.0 + 216.0));
+    // H = (A^H - 1) / (i tau): any tau with the coefficients' scale serves
+    // the enclosure as long as the solve uses the same one
+    nrq::launch_spin_prepare(ctx->lat, C, nullptr, 1, cn->spin_tau != 0.0 ? cn->spin_tau : 1.0, g->U, g->E, cn->spin,
+                             cn->spin_scratch, ctx->stream);
+  }
+  cn->spin_coef = C;
+  cn->spin_valid = true;
+  *sign = 1.0;
+  return check_launch(ctx, "k_spin_prepare");
 }
 // The stencil launch of one 12-column application.  The tensor-core stencil
 // needs imaginary off-diagonal coefficients and tensor maps; otherwise the
 // TMA-staged stencil runs, and without tensor maps the register-tiled one.
 // cn->last_stencil records which ran (the partial rows it left).
-int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq::MvArgs &a) {
+int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq::MvArgs &a, int *err = nullptr) {
   nrq_ctx *ctx = cn->ctx;
-  if (cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(C)) {
+  if (cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(C) && nrq::cn_spin_applicable(ctx->lat)) {
     double sign = 0.0;
-    int rc = ensure_blocks5(cn, C, g, &sign);
+    int rc = ensure_spin(cn, C, g, &sign);
     if (rc) return rc;
     ProfScope ps(ctx, 0, mv_bytes(ctx, mode));
-    if (nrq::launch_cn_mv5(mode, ctx->lat, C, sign, cn->Wblk5, cn->Dsum, cn->Bsum, a, scal_err(cn->scal),
-                           ctx->sm_count, ctx->stream, cn->wait_cycles, cn->stall_load) == 0) {
-      cn->last_stencil = NRQ_STENCIL_FMA;
-      return NRQ_OK;
+    if (sign < 0.0 && mode != nrq::MV_PLAIN && mode != nrq::MV_RHS) {  // the other modes apply A^H alone
+      cn->spin_valid = false;
+      if ((rc = ensure_spin(cn, C, g, &sign))) return rc;
     }
+    nrq::launch_cn_spin(mode, ctx->lat, cn->spin, sign, a, err ? err : scal_err(cn->scal), ctx->stream,
+                        cn->wait_cycles, cn->stall_load);
+    cn->last_stencil = NRQ_STENCIL_FMA;
+    return NRQ_OK;
   }
-  if (mode == nrq::MV_T2 || mode == nrq::MV_RES2 || mode == nrq::MV_V2) {  // asked for only after an FMA launch
-    ctx->last_error = "cn stencil: the merged update needs the FMA stencil";
+  if (mode >= nrq::MV_T2) {  // asked for only after an FMA launch
+    ctx->last_error = "cn stencil: this mode needs the FMA stencil";
     return NRQ_ERR_BAD_ARG;
   }
+  int rc = ensure_legacy(cn, g);
+  if (rc) return rc;
   if (cn->stencil == NRQ_STENCIL_TENSOR && offdiag_imaginary(C)) {
     double sign = 0.0;
-    int rc = ensure_blocks(cn, C, g, &sign);
-    if (rc) return rc;
+    if ((rc = ensure_blocks(cn, C, g, &sign))) return rc;
     ProfScope ps(ctx, 0, mv_bytes(ctx, mode));
     if (nrq::launch_cn_mv4(mode, ctx->lat, C, sign, cn->Wblk, cn->Dsum, cn->Bsum, a, scal_err(cn->scal),
                            ctx->sm_count, ctx->stream) == 0) {
@@ -1281,17 +1315,15 @@ bool mv_t_needs_s(const nrq_cn *cn, const nrq::CnCoef &CH) {
   if ((cn->stencil == NRQ_STENCIL_TENSOR || cn->stencil == NRQ_STENCIL_FMA) && offdiag_imaginary(CH)) return true;
   return cn->tma_ok && cn->stencil != NRQ_STENCIL_REGISTER;
 }
-void fin(nrq_cn *cn, int stage) {
+void fin(nrq_cn *cn, int stage, double *scal = nullptr) {
   nrq_ctx *ctx = cn->ctx;
-  // partial rows: one per 32-site block (register-tiled), per (unit, colour
-  // warp) (TMA-staged), per CTA (tensor-core)
+  // partial rows: one per 32-site block (register-tiled, FMA), per (unit,
+  // colour warp) (TMA-staged), per CTA (tensor-core)
   int64_t rows = cn->nblocks;
   if (stage <= 2 && cn->last_stencil == NRQ_STENCIL_TMA) rows = 3 * cn->nblocks;
   if (stage <= 2 && cn->last_stencil == NRQ_STENCIL_TENSOR) rows = nrq::cn_mv4_rows(ctx->lat.V, ctx->sm_count);
-  if ((stage <= 2 || stage == 5 || stage == 7) && cn->last_stencil == NRQ_STENCIL_FMA)
-    rows = nrq::cn_mv5_rows(ctx->lat.V, ctx->sm_count);
   ProfScope ps(ctx, 2, (double)rows * 12 * 3 * 8);
-  nrq::launch_cn_finalize(stage, rows, cn->partials, cn->scal, cn->tol, ctx->stream);
+  nrq::launch_cn_finalize(stage, rows, cn->partials, scal ? scal : cn->scal, cn->tol, ctx->stream);
 }
 // Choose the stencil by timing, on this lattice and field, the work each
 // does in the solve: for the plain form t = A^H (r - alpha v) (the
@@ -1309,7 +1341,10 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
     cn->stencil = cn->forced_stencil;
     return NRQ_OK;
   }
-  if (!cn->tma_ok) return NRQ_OK;  // only the register-tiled stencil applies
+  if (!cn->tma_ok) {  // the register-tiled and the FMA stencil apply: the latter where the coefficients allow it
+    if (offdiag_imaginary(CH) && nrq::cn_spin_applicable(ctx->lat)) cn->stencil = NRQ_STENCIL_FMA;
+    return NRQ_OK;
+  }
   cudaStream_t st = ctx->stream;
   const bool prof = ctx->prof;
   ctx->prof = false;
@@ -1362,16 +1397,15 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
     double sign = 0.0;
     // a first, untimed build allocates the block sets (once per solver);
     // the timed one is the rebuild every update makes
-    rc = which == NRQ_STENCIL_TENSOR ? ensure_blocks(cn, CH, g, &sign) : ensure_blocks5(cn, CH, g, &sign);
+    rc = which == NRQ_STENCIL_TENSOR ? ensure_blocks(cn, CH, g, &sign) : ensure_spin(cn, CH, g, &sign);
     if (rc) continue;
     cudaEventRecord(e0, st);
     if (which == NRQ_STENCIL_TENSOR) {
       cn->w_valid = false;
       rc = ensure_blocks(cn, CH, g, &sign);
     } else {
-      cn->w5_valid = false;
-      cn->w5f_valid = false;
-      rc = ensure_blocks5(cn, CH, g, &sign);
+      cn->spin_valid = false;
+      rc = ensure_spin(cn, CH, g, &sign);
     }
     cudaEventRecord(e1, st);
     cudaEventSynchronize(e1);
@@ -1384,24 +1418,37 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   ctx->prof = prof;
   if (rc) return rc;
   if ((rc = check_launch(ctx, "stencil tuning"))) return rc;
-  const double per_update = cn->form == 0 ? 10.0 : 3.0;
-  auto cost = [&](int which) { return per_update * cn->tune_ms[which] + build_ms[which]; };
+  // the FMA stencil's plain solve is the Chebyshev semi-iteration, which
+  // also has no vector passes: about 8 launches
+  auto cost = [&](int which) {
+    const double n = cn->form != 0 ? 3.0 : (which == NRQ_STENCIL_FMA && cn->semi_iter) ? 8.0 : 10.0;
+    return n * cn->tune_ms[which] + build_ms[which];
+  };
   int best = NRQ_STENCIL_REGISTER;
   for (int which = 1; which < 4; ++which)
     if (cn->tune_ms[which] > 0.0 && cost(which) < cost(best)) best = which;
   cn->stencil = best;
   return NRQ_OK;
 }
-int cn_prepare(nrq_cn *cn, const nrq_gauge *g) {
-  nrq_ctx *ctx = cn->ctx;
+// the gauge field of this update: every derived set follows it on demand
+// (tau = dt a0/2 of its solve, for the spectral enclosure)
+int cn_prepare(nrq_cn *cn, const nrq_gauge *g, double dt) {
   int rc = gauge_sync64(g);
   if (rc) return rc;
-  ProfScope ps(ctx, 3, (double)ctx->lat.V * (432.0 + 192.0));
-  nrq::launch_cn_prepare(ctx->lat, g->U, g->E, cn->Dsum, cn->Bsum, cn->DE, ctx->stream);
-  cn->w_valid = false;  // the cached blocks follow the new gauge field on demand
-  cn->w5_valid = false;
+  cn->legacy_valid = false;
+  cn->w_valid = false;
   cn->w5f_valid = false;
-  return check_launch(ctx, "k_cn_prepare");
+  cn->spin_valid = false;
+  cn->spin_tau = dt * cn->ctx->a[0] / 2.0;
+  return NRQ_OK;
+}
+// spectral enclosure of H, A^H = 1 + i spin_tau H, into out (4 doubles of the
+// device); the operator was built for A^H
+int spin_bounds(nrq_cn *cn, double *out) {
+  nrq_ctx *ctx = cn->ctx;
+  ProfScope ps(ctx, 3, (double)ctx->lat.V * 56.0);
+  nrq::launch_spin_bounds(ctx->lat, 1, cn->spin_scratch, cn->spin_part, cn->spin_ticket, out, ctx->stream);
+  return check_launch(ctx, "k_spin_bounds");
 }
 }  // namespace
 
@@ -1411,7 +1458,7 @@ extern "C" int nrq_cn_apply(nrq_cn *cn, const nrq_gauge *g, double mass, const d
   nrq_ctx *ctx = cn->ctx;
   if (g->ctx != ctx || in->ctx != ctx || out->ctx != ctx || mass == 0.0) return NRQ_ERR_BAD_ARG;
   int rc = set_device(ctx);
-  if (!rc) rc = cn_prepare(cn, g);
+  if (!rc) rc = cn_prepare(cn, g, dt);
   if (rc) return rc;
   nrq::CnCoef C = make_coef(ctx, mass, c, dt, herm != 0);
   nrq::MvArgs a{};
@@ -1484,21 +1531,19 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   const nrq::CnCoef CA = make_coef(ctx, mass, c, dt, false);
   const nrq::CnCoef CH = make_coef(ctx, mass, c, dt, true);
   const double tau = std::fabs(dt) * ctx->a[0] / 2.0;
-  int rc = cn_prepare(cn, g);
+  int rc = cn_prepare(cn, g, dt);
+  double spin_sign = 0.0;
+  if (!rc) rc = ensure_legacy(cn, g);
+  if (!rc) rc = ensure_spin(cn, CH, g, &spin_sign);
   if (rc) return rc;
   {
     ProfScope ps(ctx, 3, (double)V * (1080.0 + 540.0));
     nrq::launch_cn_to_f32(V, g->U, cn->DE, cn->Dsum, cn->Bsum, cn->U32, cn->DE32, cn->D32, cn->B32, st);
   }
   // spectral enclosure of H per species
-  {
-    ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + 216.0));
-    const int64_t nblk = (V + 255) / 256;
-    nrq::launch_cn_bounds(L, CH, dt > 0 ? tau : -tau, g->U, cn->Dsum, cn->Bsum, cn->DE, cn->bounds,
-                          cn->bounds + 4 * nblk, st);
-    NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(cn->h_bounds, cn->bounds + 4 * nblk, sizeof(double) * 4,
-                                      cudaMemcpyDeviceToHost, st));
-  }
+  if ((rc = spin_bounds(cn, scal_bounds(cn->scal)))) return rc;
+  NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(cn->h_bounds, scal_bounds(cn->scal), sizeof(double) * 4, cudaMemcpyDeviceToHost,
+                                    st));
   int64_t matvecs = 0, vstreams = 0;
   {  // RHS = A psi ; x0 = 2 RHS - psi
     nrq::MvArgs a{};
@@ -1642,7 +1687,7 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     // FP32 inner Chebyshev solve of A^H e = r, then x += e
     float2 *dcur = cn->dA32, *dnext = cn->dB32;
     double wsign = 0.0;
-    if (use_cheb5f(cn) && (rc = ensure_blocks5(cn, CH, g, &wsign, true))) return rc;
+    if (use_cheb5f(cn) && (rc = ensure_blocks5f(cn, CH, g, &wsign))) return rc;
     if (cn->cheb_stencil < 0 && !cn->cheb_tuned && (rc = tune_cheb(cn, CH, coef[0], wsign))) return rc;
     const bool blk = use_cheb5f(cn);
     for (int k = 0; k < m; ++k) {
@@ -1753,6 +1798,183 @@ static bool accept_recursive(const nrq_cn *cn, const double rel[nrq::CN_COLS]) {
   return true;
 }
 
+// The plain solve A^H x = b by the Chebyshev semi-iteration on the segment
+// 1 + i tau [lo, hi] that holds the spectrum (A^H is normal: real Wilson
+// coefficients), from x0 in cn->x.  A step is one stencil launch with the
+// whole vector work in its epilogue (four vector streams, no inner products,
+// no other launch), where BiCGStab's iteration takes two stencil launches,
+// two vector passes and three scalar stages for the same two orders of
+// application; the step count follows from the first residual and the
+// segment, |r_m| <= |r_0| / |T_m(sigma)| in every column, so the host reads
+// the device once a solve.  64^3: 0.40 ms a step against 1.40 ms an
+// iteration.
+//
+// The bound is rigorous, so a solve ends on it (after m steps max_rel is the
+// bound); the first solve, every 16th after it and, with confirm_always,
+// every one confirm with the true residual.  Returns false, with x0 still in
+// cn->x, where the enclosure is not finite or the segment asks for more than
+// kChebTab or maxits steps (light quarks, large steps): BiCGStab takes those.
+static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const nrq::CnCoef &CH, int64_t matvecs,
+                           int64_t vstreams, nrq_cn_stats *stats, int *status_out) {
+  nrq_ctx *ctx = cn->ctx;
+  cudaStream_t st = ctx->stream;
+  const int64_t V = ctx->lat.V;
+  double *hc = cn->h_cheb;
+  int &status = *status_out;
+  status = NRQ_OK;
+  int64_t its = 0;
+  double initial = -1.0, maxrel = 0.0;
+  bool conv = false, stored = false;
+  double2 *cur = cn->x, *prev = cn->p;  // the iterate and the one before it
+  // confirm on the first solve and every kReconfirm-th unconfirmed one
+  const bool confirm = cn->confirm_always || !cn->semi_confirmed || cn->semi_unconfirmed >= nrq_cn::kReconfirm;
+  // one residual pass of `cur`; MV_CH0 also writes x_1 into prev
+  auto residual = [&](int mode) -> int {
+    nrq::MvArgs a{};
+    a.in = cur;
+    a.bvec = cn->b;
+    a.out = prev;
+    a.partials = cn->partials;
+    a.cheb = cn->cheb_tab;
+    int rc = mv(cn, mode, CH, g, a, scal_err(hc));
+    if (rc) return rc;
+    fin(cn, 0, hc);
+    matvecs += 1;
+    vstreams += mode == nrq::MV_CH0 ? 3 : 2;
+    if ((rc = check_launch(ctx, "cn residual"))) return rc;
+    NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    if (*scal_err(hc) != 0) {
+      ctx->last_error = timeout_message(hc);
+      std::memset(scal_err(hc), 0, 16 * sizeof(int));
+      return NRQ_ERR_TIMEOUT;
+    }
+    return NRQ_OK;
+  };
+  auto rel_of = [&](int k) {
+    const double *sc = hc + k * nrq::SC_STRIDE;
+    return sc[nrq::SC_BB] > 0.0 ? std::sqrt(sc[nrq::SC_RR] / sc[nrq::SC_BB]) : 0.0;
+  };
+  for (;;) {
+    if ((status = residual(nrq::MV_CH0)) != NRQ_OK) break;
+    bool all = true, nonfin = false;
+    maxrel = 0.0;
+    for (int k = 0; k < nrq::CN_COLS; ++k) {
+      const double *sc = hc + k * nrq::SC_STRIDE;
+      all = all && sc[nrq::SC_CONV] != 0.0;
+      nonfin = nonfin || sc[nrq::SC_NONFIN] != 0.0;
+      maxrel = std::max(maxrel, rel_of(k));
+    }
+    if (initial < 0.0) initial = maxrel;
+    if (nonfin) {
+      status = NRQ_ERR_NONFINITE;
+      ctx->last_error = "CN solve: non-finite residual";
+      break;
+    }
+    if (all) {
+      conv = true;
+      cn->last_true = true;
+      break;
+    }
+    // steps: every column's bound within 0.9 of the tolerance, rounding aside
+    ChebSeg seg[2];
+    bool finite = true;
+    for (int sp = 0; sp < 2; ++sp) {
+      const double lo = scal_bounds(hc)[2 * sp], hi = scal_bounds(hc)[2 * sp + 1];
+      finite = finite && std::isfinite(lo) && std::isfinite(hi) && hi >= lo;
+      cn->last_lo[sp] = lo;
+      cn->last_hi[sp] = hi;
+      seg[sp] = cheb_segment(cn->spin_tau, lo, hi);
+    }
+    double worst[2] = {0.0, 0.0}, bound = 0.0;
+    for (int k = 0; k < nrq::CN_COLS; ++k) worst[k / 6] = std::max(worst[k / 6], rel_of(k));
+    int m = 0;
+    if (finite)
+      for (m = 1; m <= nrq::kChebTab; ++m) {
+        bound = std::max(worst[0] / cheb_gain(seg[0].sigma, m), worst[1] / cheb_gain(seg[1].sigma, m)) +
+                8.0 * DBL_EPSILON;
+        if (bound <= 0.9 * cn->tol) break;
+      }
+    if (!finite || m > nrq::kChebTab || its + m > cn->maxits) {
+      if (its == 0) return false;  // x0 is still in cn->x
+      status = NRQ_ERR_NOT_CONVERGED;  // a confirmed residual above the tolerance and no steps left
+      break;
+    }
+    std::swap(cur, prev);  // x_1
+    ++its;
+    stored = false;
+    for (int k = 1; k < m; ++k) {
+      const bool last = k == m - 1 && cn->history_guess;
+      if (last && (status = nrqh::ensure_hist(h, cn->history_depth)) != NRQ_OK) break;
+      nrq::MvArgs a{};
+      a.in = cur;
+      a.in2 = h->P;
+      a.bvec = cn->b;
+      a.out = prev;
+      a.cheb = cn->cheb_tab;
+      a.step = k;
+      a.r32 = last ? hist_next(h) : nullptr;
+      if ((status = mv(cn, last ? nrq::MV_CHH : nrq::MV_CHK, CH, g, a, scal_err(hc))) != NRQ_OK) break;
+      std::swap(cur, prev);
+      matvecs += 1;
+      vstreams += last ? 5 : 4;
+      ++its;
+      stored = last;
+    }
+    if (status != NRQ_OK) break;
+    if ((status = check_launch(ctx, "cn iteration")) != NRQ_OK) break;
+    if (!confirm) {
+      conv = true;
+      maxrel = bound;
+      cn->last_true = false;
+      ++cn->semi_unconfirmed;
+      break;
+    }
+    if ((status = residual(nrq::MV_RESN)) != NRQ_OK) break;
+    conv = true;
+    maxrel = 0.0;
+    for (int k = 0; k < nrq::CN_COLS; ++k) {
+      const double *sc = hc + k * nrq::SC_STRIDE;
+      conv = conv && sc[nrq::SC_CONV] != 0.0;
+      if (sc[nrq::SC_NONFIN] != 0.0) status = NRQ_ERR_NONFINITE;
+      maxrel = std::max(maxrel, rel_of(k));
+    }
+    if (status == NRQ_ERR_NONFINITE) {
+      conv = false;
+      ctx->last_error = "CN solve: non-finite residual";
+      break;
+    }
+    if (conv) {
+      cn->last_true = true;
+      cn->semi_confirmed = true;
+      cn->semi_unconfirmed = 0;
+      break;
+    }
+  }
+  if (cur != cn->x) std::swap(cn->x, cn->p);
+  const bool keep = cn->history_guess && status == NRQ_OK;
+  if (keep && !stored) {
+    if ((status = nrqh::ensure_hist(h, cn->history_depth)) != NRQ_OK) return true;
+    ProfScope ps(ctx, 1, (double)V * (1152.0 * 3 + 576.0));
+    nrq::launch_hist_store(72 * V, cn->x, cn->b, h->P, hist_next(h), st);
+    if ((status = check_launch(ctx, "k_hist_store")) != NRQ_OK) return true;
+  }
+  std::swap(h->P, cn->x);
+  if (keep) hist_push(h);
+  else h->hist_count = 0;
+  cn->last_iterations = its;
+  cn->last_matvecs = matvecs;
+  cn->last_vecstreams = vstreams;
+  if (stats) {
+    stats->iterations = its;
+    stats->matvecs = matvecs;
+    stats->vector_streams = vstreams;
+    stats->max_rel_residual = maxrel;
+    stats->converged = conv ? 1 : 0;
+    stats->initial_rel_residual = std::max(initial, 0.0);
+  }
+  return true;
+}
+
 extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mass, const double c[8],
                                    double dt, nrq_cn_stats *stats) {
   if (!cn || !h || !g || !c) return NRQ_ERR_BAD_ARG;
@@ -1765,25 +1987,49 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
   const nrq::Lat L = ctx->lat;
   const nrq::CnCoef CA = make_coef(ctx, mass, c, dt, false);
   const nrq::CnCoef CH = make_coef(ctx, mass, c, dt, true);
-  if ((rc = cn_prepare(cn, g))) return rc;
+  if ((rc = cn_prepare(cn, g, dt))) return rc;
   if (!cn->stencil_tuned && (rc = tune_stencil(cn, CH, g))) return rc;
   int64_t matvecs = 0, vstreams = 0;
-  // RHS = A psi ; extrapolated start x0 = 2 RHS - psi
+  const bool fma = cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(CH) && nrq::cn_spin_applicable(L);
+  const bool semi = fma && cn->semi_iter;
+  if (fma) {
+    double sign = 0.0;
+    if ((rc = ensure_spin(cn, CH, g, &sign))) return rc;
+  }
+  if (semi) {  // the Chebyshev coefficients, ahead of the right-hand side
+    if (!cn->cheb_tab) NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->cheb_tab, sizeof(nrq::ChebTab)));
+    if (!cn->h_cheb) {
+      NRQ_CUDA_TRY(ctx, cudaMallocHost((void **)&cn->h_cheb, kScalBytes));
+      std::memset(cn->h_cheb, 0, kScalBytes);
+    }
+    if ((rc = spin_bounds(cn, scal_bounds(cn->scal)))) return rc;
+    nrq::launch_cheb_tab(scal_bounds(cn->scal), cn->spin_tau, cn->cheb_tab, scal_bounds(cn->h_cheb), st);
+  }
+  // RHS = A psi ; start x0 = 2 RHS - psi, plus the extrapolated t of the last steps
+  const int hist_d = cn->history_guess ? std::min(cn->history_depth, h->hist_count) : 0;
   {
     nrq::MvArgs a{};
     a.in = h->P;
     a.out = cn->b;
     a.out2 = cn->x;
+    if (fma)
+      for (int k = 0; k < hist_d; ++k) {
+        a.hist[k] = hist_v(h, k + 1);
+        a.hcoef[k] = nrq::hist_coef(hist_d, k);
+      }
     if ((rc = mv(cn, nrq::MV_RHS, CA, g, a))) return rc;
     matvecs += 1;
     vstreams += 1;  // extra write of x0
   }
-  if (cn->history_guess && h->hist_count >= 1) {  // x0 += the extrapolated t of the last steps
-    const int d = std::min(cn->history_depth, h->hist_count);
+  if (!fma && hist_d >= 1) {
     const float2 *t[4] = {hist_v(h, 1), hist_v(h, 2), hist_v(h, 3), hist_v(h, 4)};
-    ProfScope ps(ctx, 1, (double)L.V * (1152.0 * 2 + 576.0 * d));
-    nrq::launch_hist_extrapolate(72 * L.V, cn->x, t, d, st);
+    ProfScope ps(ctx, 1, (double)L.V * (1152.0 * 2 + 576.0 * hist_d));
+    nrq::launch_hist_extrapolate(72 * L.V, cn->x, t, hist_d, st);
     vstreams += 2;
+  }
+  if (semi) {
+    int status = NRQ_OK;
+    if (cn_update_semi(cn, h, g, CH, matvecs, vstreams, stats, &status)) return status;
   }
   // the merged update on the FMA stencil (the right-hand side ran on it)
   // keeps the shadow residual rh in FP32, in the first half of the rh

@@ -324,25 +324,38 @@ void launch_vec_p(Lat L, double2 *p, const double2 *r, const double2 *v, const d
 // ------------------------------------------------------------ scalar stages
 __device__ __forceinline__ cplx cdiv_safe(cplx a, cplx b) { return cdiv(a, b); }
 
-__global__ void k_cn_finalize(int stage, int64_t nblocks, const double *__restrict__ partials,
-                              double *__restrict__ scal, double tol) {
+__global__ void __launch_bounds__(512) k_cn_finalize(int stage, int64_t nblocks, const double *__restrict__ partials,
+                                                     double *__restrict__ scal, double tol) {
   const int col = blockIdx.x;
   const int nq = (stage == 4 || stage == 6) ? 1 : stage == 5 ? 5 : stage == 7 ? 4 : (stage == 0 || stage == 1) ? 2 : 3;
-  __shared__ double sh[5][256];
+  __shared__ double sh[5][16];
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int64_t b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int k = 0; k < nq; ++k) acc[k] += partials[(b * CN_COLS + col) * nq + k];
-  for (int k = 0; k < 5; ++k) sh[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int wd = blockDim.x / 2; wd > 0; wd >>= 1) {
-    if (threadIdx.x < wd)
-      for (int k = 0; k < 5; ++k) sh[k][threadIdx.x] += sh[k][threadIdx.x + wd];
-    __syncthreads();
+  for (int64_t b = threadIdx.x; b < nblocks; b += blockDim.x) {
+    const double *p = partials + (b * CN_COLS + col) * nq;
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+      if (k < nq) acc[k] += p[k];
   }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o);
+    if (lane == 0) sh[k][warp] = acc[k];
+  }
+  __syncthreads();
+  if (warp == 0)
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      double v = lane < 16 ? sh[k][lane] : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) sh[k][0] = v;
+    }
   if (threadIdx.x != 0) return;
   double *sc = scal + col * SC_STRIDE;
   const double q0 = sh[0][0], q1 = sh[1][0], q2 = sh[2][0];
-  const bool conv = sc[SC_CONV] != 0.0;
+  const bool conv = stage != 0 && stage != 7 && sc[SC_CONV] != 0.0;
   if (stage == 0 || stage == 7) {  // rr, bb after a (re)start; rho = rh.r (7: FP32 shadow rh)
     sc[SC_RR] = q0;
     sc[SC_BB] = q1;
@@ -432,7 +445,7 @@ __global__ void k_cn_finalize(int stage, int64_t nblocks, const double *__restri
 
 void launch_cn_finalize(int stage, int64_t nblocks, const double *partials, double *scal, double tol,
                         cudaStream_t st) {
-  k_cn_finalize<<<CN_COLS, 256, 0, st>>>(stage, nblocks, partials, scal, tol);
+  k_cn_finalize<<<CN_COLS, 512, 0, st>>>(stage, nblocks, partials, scal, tol);
 }
 
 // ------------------------------------------------------------ batched scalars
@@ -761,13 +774,16 @@ __global__ void k_hist_store(int64_t n, const double2 *__restrict__ X, const dou
   const double2 x = X[i], b = B[i], p = Psi[i];
   T[i] = make_float2((float)(x.x - (2.0 * b.x - p.x)), (float)(x.y - (2.0 * b.y - p.y)));
 }
-void launch_hist_extrapolate(int64_t n, double2 *X, const float2 *const *t, int d, cudaStream_t st) {
+double hist_coef(int d, int k) {
   static const double kCoef[4][4] = {{1, 0, 0, 0}, {2, -1, 0, 0}, {3, -3, 1, 0}, {4, -6, 4, -1}};
+  return kCoef[d - 1][k];
+}
+void launch_hist_extrapolate(int64_t n, double2 *X, const float2 *const *t, int d, cudaStream_t st) {
   HistExtrap H{};
   d = d < 1 ? 1 : (d > 4 ? 4 : d);
   for (int k = 0; k < 4; ++k) {
     H.t[k] = k < d ? t[k] : nullptr;
-    H.c[k] = kCoef[d - 1][k];
+    H.c[k] = k < d ? hist_coef(d, k) : 0.0;
   }
   k_hist_extrapolate<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, X, H);
 }

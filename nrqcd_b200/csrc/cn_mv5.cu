@@ -409,445 +409,6 @@ __device__ __forceinline__ void exchange_halves(const double (&acc)[6][3][2], do
 
 }  // namespace
 
-// Sum of six doubles over the warp by halving exchanges (8 shuffles where
-// six butterflies take 30): after the exchange across lane bit 4 each half
-// of the warp carries three of the values, across bit 3 two (the third
-// padded), across bit 2 one, then bits 1 and 0 finish the sum.  Lane L ends
-// with value 3 (L >> 4) + 2 ((L >> 3) & 1) + ((L >> 2) & 1) (index 3 of a
-// half is the padding); warp_sum6_slot gives that index, or -1.
-__device__ __forceinline__ double warp_sum6(const double v[6], int lane) {
-  const bool b4 = (lane >> 4) & 1, b3 = (lane >> 3) & 1, b2 = (lane >> 2) & 1;
-  double w[4];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const double mine = b4 ? v[j + 3] : v[j], other = b4 ? v[j] : v[j + 3];
-    w[j] = mine + __shfl_xor_sync(0xffffffffu, other, 16);
-  }
-  w[3] = 0.0;
-  double y[2];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const double mine = b3 ? w[j + 2] : w[j], other = b3 ? w[j] : w[j + 2];
-    y[j] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
-  }
-  double z = (b2 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b2 ? y[0] : y[1], 4);
-  z += __shfl_xor_sync(0xffffffffu, z, 2);
-  z += __shfl_xor_sync(0xffffffffu, z, 1);
-  return z;
-}
-__device__ __forceinline__ int warp_sum6_slot(int lane) {
-  if (lane & 3) return -1;
-  const int idx = 2 * ((lane >> 3) & 1) + ((lane >> 2) & 1);
-  return idx < 3 ? 3 * (lane >> 4) + idx : -1;
-}
-
-template <int MODE>
-__global__ void __maxnreg__(mv5::kMaxReg)
-    k_cn_mv5(Lat L, CnCoef C, double nb_sign, const __grid_constant__ Mv5Maps maps, const double2 *__restrict__ W,
-             MvArgs A, int nunits, int *err, long long wait_cycles, int stall_load) {
-  using namespace mv5;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kBufs][2], empty_bar[kBufs], dfull[2], dempty[2];
-  __shared__ volatile int s_issued;  // loads the producer issued (diagnostics of an expired wait)
-  __shared__ uint32_t s_tmem;        // the exchange's tensor-memory columns
-  __shared__ double red[kWarps][3][MODE == MV_T2 ? 5 : MODE == MV_RES2 ? 4 : 3];
-  unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int V = (int)L.V;  // the launcher admits V < 2^31 only
-
-  if (threadIdx.x == 0) {
-    s_issued = 0;
-    for (int b = 0; b < kBufs; ++b) {
-      mbar_init(&full_bar[b][0], 1);
-      mbar_init(&full_bar[b][1], 1);
-      mbar_init(&empty_bar[b], 4);  // the four consumer warps of the load's species
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&dfull[b], 1);
-      mbar_init(&dempty[b], kWarps);  // every consumer warp
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) tc::tmem_alloc(&s_tmem, kTmemCols);
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t tbase = s_tmem;
-
-  const int my_units = (nunits - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
-  const int total = my_units * kLoads;
-
-  // bounded wait with this launch's limit
-  auto wait = [&](uint64_t *bar, uint32_t parity) -> bool {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-      if (clock64() - t0 > wait_cycles) return false;
-    return true;
-  };
-
-  // ---------------------------------------------------------- producer
-  if (warp >= kWarps) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kProdReg));
-    if (warp == kWarps && lane == 0) {
-      const int stop = stall_load >= 0 ? min(stall_load, total) : total;
-      bool ok = true;
-      int i = 0, ndiag = 0;
-      UnitPos P{0, 0, 0, 0};
-      for (; i < stop && ok; ++i) {
-        const int b = i % kBufs;
-        if (i >= kBufs) {
-          const uint32_t par = (uint32_t)((i / kBufs - 1) & 1);
-          const int j = i - kBufs;  // the buffer's previous load
-          // every consumer warp of the species released the buffer, and its
-          // previous load landed
-          if (!wait(&empty_bar[b], par)) {
-            record_timeout(err, 5, 2, i);
-            ok = false;
-          } else if (!mbar_wait(&full_bar[b][j & 1], (uint32_t)((j / kPer) & 1))) {
-            record_timeout(err, 5, 3, i);
-            ok = false;
-          }
-          if (!ok) break;
-        }
-        const int li = i % kLoads, stg = li >> 1, sp = li & 1;
-        if (li == 0) P = unit_pos_of(L, (int)blockIdx.x + (i / kLoads) * (int)gridDim.x);
-        const int x0 = P.x0;
-        if (li == 0) {  // the unit's diagonal matrices, with its first load
-          const int k = i / kLoads, db = k & 1;
-          if (k >= 2) {
-            const uint32_t dpar = (uint32_t)((k / 2 - 1) & 1);
-            if (!wait(&dempty[db], dpar)) {
-              record_timeout(err, 5, 2, i);
-              ok = false;
-            } else if (!mbar_wait(&dfull[db], dpar)) {
-              record_timeout(err, 5, 3, i);
-              ok = false;
-            }
-            if (!ok) break;
-          }
-          unsigned char *dd = smem + kOffDiag + db * kDiagStride;
-          mbar_expect_tx(&dfull[db], kDiagD + kDiagB);
-          tma_2d(dd, &maps.D, 2 * x0, 0, &dfull[db]);
-          tma_2d(dd + kDiagD, &maps.B, x0, 0, &dfull[db]);
-          ++ndiag;
-        }
-        const int ss = spin_start5(L, P, stg);
-        const int ws = blk_start5(x0, ss, stg);
-        const int I = stg == 0 ? 0 : (stg + 1) / 2;
-        unsigned char *bb = smem + b * kBufBytes;
-        int yl = -1, yr = -1;
-        if (stg == 0) x_wraps5(L, P, yl, yr);
-        uint32_t tx = 2u * kTileBytes;
-        if (stg == 0) tx += (yl >= 0 ? 2u : 0u) * kColBytes + (yr >= 0 ? kColBytes : 0u);
-        uint64_t *fb = &full_bar[b][sp];
-        mbar_expect_tx(fb, tx);
-        tma_2d(bb, &maps.spin, 2 * ss, sp * 36, fb);
-        tma_2d(bb + kOffW, &maps.W, 2 * ws, (I * 2 + sp) * 36, fb);
-        if (stg == 0) {
-          if (yl >= 0) {
-            tma_2d(bb + kOffX, &maps.spin1, 2 * yl, sp * 36, fb);
-            tma_2d(bb + kOffX + kColStride, &maps.W1, 2 * yl, sp * 36, fb);
-          }
-          if (yr >= 0) tma_2d(bb + kOffX + 2 * kColStride, &maps.spin1, 2 * yr, sp * 36, fb);
-        }
-        s_issued = i + 1;
-      }
-      // every issued load lands before the CTA exits: loads before the last
-      // kBufs were waited for above
-      for (int k = max(0, i - kBufs); k < i; ++k)
-        if (!mbar_wait(&full_bar[k % kBufs][k & 1], (uint32_t)((k / kPer) & 1))) {
-          record_timeout(err, 5, 4, k);
-          break;
-        }
-      for (int k = max(0, ndiag - 2); k < ndiag; ++k)
-        if (!mbar_wait(&dfull[k & 1], (uint32_t)((k >> 1) & 1))) {
-          record_timeout(err, 5, 4, -1 - k);
-          break;
-        }
-    }
-    return;
-  }
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsReg));
-
-  // ---------------------------------------------------------- consumers
-  // warp w = 4 kh + 2 sp + h: input-row half kh, species sp, column half h;
-  // lane = site of the 32-site unit.  The thread accumulates all six output
-  // rows of columns 3h .. 3h + 2 over input rows 3 kh .. 3 kh + 2 of its site
-  // and species; after the unit's last stage it keeps rows 3 kh .. 3 kh + 2
-  // of the sum (exchange_halves with warp w ^ 4).
-  const int kh = warp >> 2, sp = (warp >> 1) & 1, h = warp & 1;
-  const int pair_bar = 2 + (warp & 3);  // named barrier of the warp pair (ids 2-5)
-  // the thread's first spinor plane and block entries (see nb_products)
-  const int pofs = 18 * h + 3 * kh, wofs_f = 3 * kh, wofs_b = 18 * kh;
-  const int site_in_unit = lane;
-  constexpr int NQ = MODE == MV_T2 ? 5 : MODE == MV_RES2 ? 4 : (MODE == MV_T) ? 3
-                   : ((MODE == MV_RES || MODE == MV_V || MODE == MV_V2 || MODE == MV_RESC) ? 2 : 0);
-  // the products with the FP32 shadow residual (MV_T2: rh.t, MV_RES2:
-  // rh.r) are summed over the warp after every unit into the warp's own
-  // slots XQ, XQ + 1 of red, which keeps them out of the registers of the
-  // stage loop; the other sums (NR per column) stay in registers
-  constexpr int XQ = MODE == MV_T2 ? 3 : MODE == MV_RES2 ? 2 : -1;
-  constexpr int NR = XQ >= 0 ? XQ : NQ;
-  constexpr bool kShadow = MODE == MV_T2 || MODE == MV_V2;  // reads sh32
-  double qs[3][3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) qs[k][0] = qs[k][1] = qs[k][2] = 0.0;
-  // the lane that ends with value j of the per-unit sums (re and im of the
-  // three columns) owns its slot of red, which it clears here
-  if (XQ >= 0 && warp_sum6_slot(lane) >= 0) {
-    const int j = warp_sum6_slot(lane);
-    red[warp][j >> 1][XQ + (j & 1)] = 0.0;
-  }
-  const cplx ak = C.kin[sp], am = C.mag[sp], ad = C.dar[sp];
-  const cplx dg = C.dkin * ak + cplx{1.0, 0.0};
-  bool dead = false;
-
-  for (int u = 0; u < my_units; ++u) {
-    const UnitPos P = unit_pos_of(L, (int)blockIdx.x + u * (int)gridDim.x);
-    const int x0 = P.x0;
-    const int x = x0 + site_in_unit;
-    const bool act = x < V;
-    const int xs = act ? x : V - 1;  // a valid site for the addresses of idle lanes
-    int nb[6];
-    neighbours5(L, P, xs - x0, nb);
-    int yl = -1, yr = -1;
-    x_wraps5(L, P, yl, yr);
-    double acc[6][3][2];
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) acc[r][k][0] = acc[r][k][1] = 0.0;
-    // the epilogue's operand at the own site: b for the residuals, rh for V,
-    // the input itself for RHS and T; the FP32 shadow residual for V2, T2
-    const double2 *epi_src =
-        (MODE == MV_V) ? A.in2 : (MODE == MV_RES || MODE == MV_RES2 || MODE == MV_RESC) ? A.bvec : A.in;
-    cplx ev[3][3];
-    float2 eh[3][3];
-
-#pragma unroll
-    for (int stg = 0; stg < kStages; ++stg) {
-      const int ld = u * kLoads + stg * 2 + sp;
-      const int b = ld % kBufs;
-      if (stg == kStages - 2 && MODE != MV_PLAIN) {
-        // the epilogue's operands, loaded into registers two stages ahead
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const int64_t o = (int64_t)(sp * 36 + (3 * h + k) * 6 + 3 * kh + i) * V + xs;
-            if (MODE != MV_V2) ev[i][k] = ldg(epi_src + o);
-            if (kShadow) eh[i][k] = __ldg(A.sh32 + o);
-          }
-      }
-      int role = -1;
-      if (!dead && !wait(&full_bar[b][sp], (uint32_t)((ld / kPer) & 1))) role = 0;
-      // stage 0 also reads the unit's diagonal matrices
-      if (stg == 0 && !dead && role < 0 && !wait(&dfull[u & 1], (uint32_t)((u >> 1) & 1))) role = 1;
-      // warp-uniform: the products below use warp votes
-      if (__any_sync(0xffffffffu, role >= 0) && !dead) {
-        dead = true;
-        if (role >= 0) {
-          record_timeout(err, 5, role, ld);
-          if (err[3] == (int)blockIdx.x && err[2] == ld) {  // this thread's record: add the detail
-            const uint64_t word =
-                role == 0 ? *(volatile uint64_t *)&full_bar[b][sp] : *(volatile uint64_t *)&dfull[u & 1];
-            err[4] = s_issued + 1;
-            err[5] = (int)(uint32_t)word;
-            err[6] = (int)(uint32_t)(word >> 32);
-            err[7] = role == 0 ? (ld / kPer) & 1 : (u >> 1) & 1;
-          }
-        }
-      }
-      const unsigned char *bb = smem + b * kBufBytes;
-      const uint32_t s_tile = smem_u32(bb), s_w = smem_u32(bb + kOffW);
-      if (!dead) {
-        const int ss = spin_start5(L, P, stg);
-        const int ws = blk_start5(x0, ss, stg);
-        if (stg == 0) {
-          // diagonal (colour only): row (c, s) takes input rows (j, s);
-          // x - ss = site_in_unit + 1 lies inside the tile for every lane
-          const unsigned char *dd = smem + kOffDiag + (u & 1) * kDiagStride;
-          const uint32_t s_d = smem_u32(dd) + (uint32_t)(site_in_unit * 16);
-          const uint32_t s_b = smem_u32(dd + kDiagD) + (uint32_t)(site_in_unit * 8);
-          const uint32_t s_own = s_tile + (uint32_t)((site_in_unit + 1) * 16);
-          if (kh == 0)
-            diag_products<0>(acc, h, s_d, s_b, s_own, ad, am, dg, nb_sign);
-          else
-            diag_products<1>(acc, h, s_d, s_b, s_own, ad, am, dg, nb_sign);
-        }
-        // neighbours of this stage: stage 0 = +x (forward) and -x (backward)
-#pragma unroll
-        for (int hh = 0; hh < (stg == 0 ? 2 : 1); ++hh) {
-          const bool bwd = stg == 0 ? (hh == 1) : (stg % 2 == 0);
-          const int d = stg == 0 ? hh : stg + 1;  // neighbour index in nb[]
-          const int I = d >> 1;
-          const int y = nb[d];                   // neighbour site
-          const int m = bwd ? y : xs;            // site of the forward block
-          const bool ps = (unsigned)(y - ss) < (unsigned)kTileS;  // spinor in the tile
-          const bool wsh = (unsigned)(m - ws) < (unsigned)kTileS; // block in the tile
-          // stage 0: a wrapped x neighbour in the wrap columns
-          const bool pw = stg == 0 && !ps && y == (bwd ? yl : yr);
-          const bool ww = stg == 0 && bwd && !wsh && m == yl;
-          if (stg == 0 && __any_sync(0xffffffffu, act && (pw || ww)) &&
-              __all_sync(0xffffffffu, ((ps || pw) && (wsh || ww)) || !act)) {
-            // shared memory, a lane's operands in the tile or in a wrap
-            // column (per-lane strides)
-            const uint32_t xc = smem_u32(bb + kOffX);
-            const uint32_t wst = ww ? 16u : (uint32_t)kTileS * 16u, pst = pw ? 16u : (uint32_t)kTileS * 16u;
-            const uint32_t wa = (ww ? xc + kColStride : s_w + (uint32_t)((m - ws) * 16)) +
-                                (uint32_t)(bwd ? wofs_b : wofs_f) * wst;
-            const uint32_t pa =
-                (pw ? xc + (bwd ? 0u : 2u * kColStride) : s_tile + (uint32_t)((y - ss) * 16)) + (uint32_t)pofs * pst;
-            auto lw = [&](int e) { return lds_d2(wa + (uint32_t)e * wst); };
-            auto lp = [&](int e) { return lds_d2(pa + (uint32_t)e * pst); };
-            if (bwd)
-              nb_products<true>(acc, lw, lp);
-            else
-              nb_products<false>(acc, lw, lp);
-          } else if (__all_sync(0xffffffffu, (ps && wsh) || !act)) {
-            // every operand of the warp in shared memory
-            constexpr uint32_t kPl = kTileS * 16u;  // plane stride of the tiles
-            const uint32_t wa = s_w + (uint32_t)((m - ws) * 16) + (uint32_t)(bwd ? wofs_b : wofs_f) * kPl;
-            const uint32_t pa = s_tile + (uint32_t)((y - ss) * 16) + (uint32_t)pofs * kPl;
-            auto lw = [&](int e) { return lds_d2(wa + (uint32_t)e * kPl); };
-            auto lp = [&](int e) { return lds_d2(pa + (uint32_t)e * kPl); };
-            if (bwd)
-              nb_products<true>(acc, lw, lp);
-            else
-              nb_products<false>(acc, lw, lp);
-          } else if (act) {
-            // some lanes' operands outside the tiles (periodic wraps, tile
-            // edges): those lanes read global memory, the others the tiles
-            const int64_t wst = wsh ? kTileS : V, pst = ps ? kTileS : V;
-            const double2 *wp = (wsh ? (const double2 *)(bb + kOffW) + (m - ws)
-                                     : W + (int64_t)((I * 2 + sp) * 36) * V + m) +
-                                (bwd ? wofs_b : wofs_f) * wst;
-            const double2 *pp = (ps ? (const double2 *)bb + (y - ss) : A.in + (int64_t)(sp * 36) * V + y) + pofs * pst;
-            auto lw = [&](int e) { return wp[e * wst]; };
-            auto lp = [&](int e) { return pp[e * pst]; };
-            if (bwd)
-              nb_products<true>(acc, lw, lp);
-            else
-              nb_products<false>(acc, lw, lp);
-          }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&empty_bar[b]);
-        if (stg == 0) mbar_arrive(&dempty[u & 1]);
-      }
-    }
-
-    // ---------------------------------------------------------- epilogue
-    // every warp of the pair takes both barriers of the exchange, dead or
-    // not, active lanes or not
-    cplx ht[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};  // this unit's product with the shadow, per column
-    double res[3][3][2];
-    if (kh == 0)
-      exchange_halves<0>(acc, res, tbase, warp, pair_bar);
-    else
-      exchange_halves<1>(acc, res, tbase, warp, pair_bar);
-    if (!dead && act) {
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const int64_t off = (int64_t)(sp * 36 + (3 * h + k) * 6 + 3 * kh + i) * V + x;
-          // D in + sgn N in = sgn (sgn D in + N in), sgn = +-1: the diagonal
-          // was scaled by sgn and the neighbour sum was not
-          const cplx y_ = {nb_sign * res[i][k][0], nb_sign * res[i][k][1]};
-          const cplx ev_ = ev[i][k];
-          if (MODE == MV_PLAIN) {
-            st(A.out + off, y_);
-          } else if (MODE == MV_RHS) {
-            st(A.out + off, y_);
-            st(A.out2 + off, 2.0 * y_ - ev_);
-          } else if (MODE == MV_RES) {
-            const cplx rv = ev_ - y_;
-            st(A.out + off, rv);
-            st(A.out2 + off, rv);
-            st(A.out3 + off, rv);
-            qs[k][0] += norm2(rv);
-            qs[k][1] += norm2(ev_);
-          } else if (MODE == MV_RES2) {
-            const cplx rv = ev_ - y_;
-            const float2 f = make_float2((float)rv.re, (float)rv.im);
-            st(A.out + off, rv);
-            A.sh32[off] = f;
-            st(A.out3 + off, rv);
-            qs[k][0] += norm2(rv);
-            qs[k][1] += norm2(ev_);
-            cmac_cj(ht[k], cplx{(double)f.x, (double)f.y}, rv);
-          } else if (MODE == MV_V) {
-            st(A.out + off, y_);
-            cplx dd = {0.0, 0.0};
-            cmac_cj(dd, ev_, y_);
-            qs[k][0] += dd.re;
-            qs[k][1] += dd.im;
-          } else if (MODE == MV_V2) {
-            st(A.out + off, y_);
-            cplx dd = {0.0, 0.0};
-            cmac_cj(dd, cplx{(double)eh[i][k].x, (double)eh[i][k].y}, y_);
-            qs[k][0] += dd.re;
-            qs[k][1] += dd.im;
-          } else if (MODE == MV_RESC) {
-            const cplx rv = ev_ - y_;
-            const cplx dv = rv * A.inv_theta[sp];
-            A.r32[off] = make_float2((float)rv.re, (float)rv.im);
-            A.d32[off] = make_float2((float)dv.re, (float)dv.im);
-            qs[k][0] += norm2(rv);
-            qs[k][1] += norm2(ev_);
-          } else {  // MV_T, MV_T2: in = s
-            st(A.out + off, y_);
-            cplx dd = {0.0, 0.0};
-            cmac_cj(dd, y_, ev_);
-            qs[k][0] += dd.re;
-            qs[k][1] += dd.im;
-            qs[k][2] += norm2(y_);
-            if (MODE == MV_T2) cmac_cj(ht[k], cplx{(double)eh[i][k].x, (double)eh[i][k].y}, y_);
-          }
-        }
-    }
-    if (XQ >= 0) {
-      const double hv[6] = {ht[0].re, ht[0].im, ht[1].re, ht[1].im, ht[2].re, ht[2].im};
-      const double z = warp_sum6(hv, lane);
-      const int j = warp_sum6_slot(lane);  // recomputed: a register held across the stages spills
-      if (j >= 0) red[warp][j >> 1][XQ + (j & 1)] += z;
-    }
-  }
-
-  // every consumer warp is done with the tensor memory before warp 0 frees it
-  tc::fence_before_sync();
-  named_bar_sync(1, kWarps * 32);
-  tc::fence_after_sync();
-  if (warp == 0) tc::tmem_dealloc(tbase, kTmemCols);
-
-  // one partial row per CTA: each column summed over the warp's lanes, then
-  // over the two row-half warps of its species and column half in a fixed
-  // order
-  if constexpr (NQ > 0) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-      for (int kk = 0; kk < NR; ++kk) {  // the shadow products are in red already
-        double v = qs[k][kk];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[warp][k][kk] = v;
-      }
-    named_bar_sync(1, kWarps * 32);
-    if (threadIdx.x < CN_COLS * NQ) {
-      const int col12 = threadIdx.x / NQ, kk = threadIdx.x % NQ;
-      const int spc = col12 / 6, n = col12 % 6, hc = n / 3, k = n % 3;
-      // warps 4 kh + 2 spc + hc for kh = 0, 1
-      A.partials[((int64_t)blockIdx.x * CN_COLS + col12) * NQ + kk] =
-          red[2 * spc + hc][k][kk] + red[4 + 2 * spc + hc][k][kk];
-    }
-  }
-}
-
 // The same stencil over every field of a batch (the batching form's
 // right-hand side and refinement residual; k_batch_mv2 in cn_mv.cu is the
 // register-tiled alternative): work items (field, unit), field fastest
@@ -1241,43 +802,7 @@ void launch_cn_blocks5(Lat L, const CnCoef &C, const double2 *U, const double2 *
 }
 
 int64_t cn_mv5_units(int64_t V) { return (V + mv5::kUnit - 1) / mv5::kUnit; }
-int64_t cn_mv5_rows(int64_t V, int sm_count) { return std::min<int64_t>(cn_mv5_units(V), sm_count); }
 int64_t cn_mv5_block_entries(int64_t V) { return 216 * V; }
-
-int launch_cn_mv5(int mode, Lat L, const CnCoef &C, double nb_sign, const double2 *W, const double2 *Dsum,
-                  const double *Bsum, const MvArgs &a, int *err, int sm_count, cudaStream_t st,
-                  long long wait_cycles, int stall_load) {
-  using namespace mv5;
-  const uint64_t V = (uint64_t)L.V;
-  // B tiles start at x0 = 32 u (16-byte aligned rows need an even V as well)
-  if (L.V < kTileS || L.V > 0x7fffffffLL || (L.V & 1)) return -1;
-  Mv5Maps maps;
-  memset(&maps, 0, sizeof(maps));
-  if (!stage::encode(&maps.spin, a.in, 2 * V, 72, 2 * kTileS, 36) ||
-      !stage::encode(&maps.W, W, 2 * V, 216, 2 * kTileS, 36) ||
-      !stage::encode(&maps.spin1, a.in, 2 * V, 72, 2, 36) || !stage::encode(&maps.W1, W, 2 * V, 216, 2, 36) ||
-      !stage::encode(&maps.D, Dsum, 2 * V, 9, 2 * kUnit, 9) || !stage::encode(&maps.B, Bsum, V, 9, kUnit, 9))
-    return -1;
-  const int nunits = (int)cn_mv5_units(L.V);
-  const unsigned grid = (unsigned)cn_mv5_rows(L.V, sm_count);
-  auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    kern<<<grid, kThreads, kSmemBytes, st>>>(L, C, nb_sign, maps, W, a, nunits, err, wait_cycles, stall_load);
-  };
-  switch (mode) {
-    case MV_PLAIN: go(k_cn_mv5<MV_PLAIN>); break;
-    case MV_RHS: go(k_cn_mv5<MV_RHS>); break;
-    case MV_RES: go(k_cn_mv5<MV_RES>); break;
-    case MV_V: go(k_cn_mv5<MV_V>); break;
-    case MV_RESC: go(k_cn_mv5<MV_RESC>); break;
-    case MV_T2: go(k_cn_mv5<MV_T2>); break;
-    case MV_RES2: go(k_cn_mv5<MV_RES2>); break;
-    case MV_V2: go(k_cn_mv5<MV_V2>); break;
-    default: go(k_cn_mv5<MV_T>); break;
-  }
-  return 0;
-}
-
 
 bool batch_mv5_applicable(const Lat &L) { return L.V >= mv5::kTileS && L.V <= 0x7fffffffLL && (L.V & 1) == 0; }
 

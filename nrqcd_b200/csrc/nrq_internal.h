@@ -182,10 +182,27 @@ struct nrq_cn {
   double2 *Wblk = nullptr;
   bool w_valid = false;
   nrq::CnCoef w_coef{};
-  // FP64 FMA stencil: the same blocks as 216 planes
-  double2 *Wblk5 = nullptr;
-  bool w5_valid = false;
-  nrq::CnCoef w5_coef{};
+  // FMA stencil: the operator in its spin structure (real coefficients),
+  // built for spin_coef from the current gauge field on demand, with the
+  // scratch planes and partial rows of the spectral enclosure and its ticket
+  nrq::SpinOp spin{};
+  bool spin_valid = false;
+  nrq::CnCoef spin_coef{};
+  double spin_tau = 0.0;
+  double *spin_scratch = nullptr, *spin_part = nullptr;
+  unsigned *spin_ticket = nullptr;
+  // plain form on the FMA stencil: the Chebyshev semi-iteration (semi_iter;
+  // setting the merged update of BiCGStab selects BiCGStab), its coefficient
+  // table, the pinned block its kernels report into (the layout of h_scal),
+  // whether a solve was confirmed yet and the unconfirmed ones since
+  bool semi_iter = true;
+  nrq::ChebTab *cheb_tab = nullptr;
+  double *h_cheb = nullptr;
+  bool semi_confirmed = false;
+  int semi_unconfirmed = 0;
+  // the other stencils' per-step matrices (Dsum, Bsum, DE) follow the gauge
+  // field on demand
+  bool legacy_valid = false;
   // the FP32 Chebyshev step of the precision forms: the same blocks rounded
   // to FP32, and which step kernel runs (-1: k_cheb5f where it applies, else
   // k_cheb32; NRQ_CHEB_* forces one); last_cheb: the one the last update ran
@@ -207,7 +224,6 @@ struct nrq_cn {
   float2 *U32 = nullptr, *DE32 = nullptr, *D32 = nullptr;
   float *B32 = nullptr;
   float2 *r32 = nullptr, *dA32 = nullptr, *dB32 = nullptr, *e32 = nullptr;
-  double *bounds = nullptr;    // partial blocks, then 4 final values
   double *h_bounds = nullptr;  // pinned
   int64_t last_inner = 0;      // FP32 Chebyshev steps of the last update
   int64_t last_outer = 0;      // FP64 refinement passes of the last update

@@ -76,30 +76,79 @@ struct CnCoef {
 //   MV_V2:   MV_V with rh^H v from sh32;
 //   MV_T2:   MV_T on a materialised s that also reduces rh^H t from sh32,
 //            from which the merged update takes beta
+// Spin-structured stencil only, the Chebyshev semi-iteration of the plain
+// solve (tab: its coefficients, ChebTab below):
+//   MV_RESN: |b - y|^2 and |b|^2 alone;
+//   MV_CH0:  x_1 = x_0 + r_0 / theta, with the sums of MV_RESN;
+//   MV_CHK:  x_{k+1} = x_k + c1 (x_k - x_{k-1}) + c2 (b - y), x_{k-1} in out
+//            and overwritten;
+//   MV_CHH:  MV_CHK that also stores the step's history x - (2b - psi) in FP32
 enum MvMode { MV_PLAIN = 0, MV_RHS = 1, MV_RES = 2, MV_V = 3, MV_T = 4, MV_RESC = 5, MV_T2 = 6, MV_RES2 = 7,
-              MV_V2 = 8 };
+              MV_V2 = 8, MV_RESN = 9, MV_CH0 = 10, MV_CHK = 11, MV_CHH = 12 };
+
+struct ChebTab;
 
 struct MvArgs {
-  const double2 *in;  // operand (PLAIN/RHS: psi, RES: x, V: p, T: r)
-  const double2 *in2; // T: v ; RHS: (unused)
-  double2 *out;       // PLAIN: A in ; RHS: b ; RES: r ; V: v ; T: t
+  const double2 *in;  // operand (PLAIN/RHS: psi, RES, CH*: x, V: p, T: r)
+  const double2 *in2; // T: v ; CHH: psi ; RHS: (unused)
+  double2 *out;       // PLAIN: A in ; RHS: b ; RES: r ; V: v ; T: t ; CH0: x_1 ; CHK, CHH: x_{k-1}, then x_{k+1}
   double2 *out2;      // RHS: x0 = 2b - psi ; RES: rh
   double2 *out3;      // RES: p
-  const double2 *bvec;// RES: b
+  const double2 *bvec;// RES, CH*: b
   const double *scal; // per-column scalars
   double *partials;   // per block, per column, NQ doubles
   // MV_RESC (residual for the FP32 Chebyshev inner solve): r32 = f32(b - A^H x),
-  // d32 = f32((b - A^H x) / theta_species)
+  // d32 = f32((b - A^H x) / theta_species); CHH: r32 = the history slot
   float2 *r32;
   float2 *d32;
   cplx inv_theta[2];
   float2 *sh32;       // RES2: FP32 shadow residual written; V2, T2: read
+  // spin-structured stencil: the Chebyshev table and step; RHS: the history
+  // vectors added to x0 with their coefficients (null: none)
+  const ChebTab *cheb;
+  int step;
+  const float2 *hist[4];
+  double hcoef[4];
 };
 
 // per-species coefficients of one Chebyshev step: d' = c1 d + c2 r
 struct ChebCoef {
   cplx c1[2], c2[2];
 };
+
+// the Chebyshev coefficients of one operator by step (step[0]: c1 = 0, c2 =
+// 1/theta) and the enclosure of its hermitian part they were made for
+// (k_cheb_tab, cn_spin.cu)
+constexpr int kChebTab = 40;
+struct ChebTab {
+  ChebCoef step[kChebTab];
+  cplx inv_theta[2];
+  double lo[2], hi[2];
+};
+
+// The operator in its spin structure (cn_spin.cu), real Wilson coefficients:
+// A^H psi(x) = (1 + i (S0 +- S1)) psi(x) + the six neighbours' blocks from
+// three colour matrices a direction.  Planes of V: W 81 complex ((I*3 + m)*9
+// + row*3 + column), S0 9 complex, S1 9 real, each per coefficient set.
+struct SpinOp {
+  double2 *W, *S0;
+  double *S1;
+};
+// Builds op for nm coefficient sets (device array Cm; null: the one set C),
+// and seven real scratch planes a set for the spectral enclosure (null: none).
+// tau = dt a0 / 2.
+void launch_spin_prepare(Lat L, const CnCoef &C, const CnCoef *Cm, int nm, double tau, const double2 *U,
+                         const double *E, const SpinOp &op, double *scratch, cudaStream_t st);
+// out[4*set] = {lo, hi} of the quark's and the antiquark's H, A^H = 1 + i tau
+// H; partials: 4 doubles per 256 sites and set; ticket: one zero per set
+void launch_spin_bounds(Lat L, int nm, const double *scratch, double *partials, unsigned *ticket, double *out,
+                        cudaStream_t st);
+void launch_cheb_tab(const double *bounds, double tau, ChebTab *tab, double *host_bounds, cudaStream_t st);
+bool cn_spin_applicable(const Lat &L);
+// the stencil over op (sign = -1: A = 2 - A^H, for MV_PLAIN and MV_RHS); one
+// partial row per 32-site block
+void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs &a, int *err, cudaStream_t st,
+                    long long wait_cycles, int stall_load);
 
 constexpr int CN_SITES_PER_BLOCK = 32;
 constexpr int CN_COLS = 12;  // 2 species x 6 propagator columns
@@ -149,21 +198,14 @@ int64_t cn_mv4_units(int64_t V);
 int64_t cn_mv4_rows(int64_t V, int sm_count);
 int launch_cn_mv4(int mode, Lat L, const CnCoef &C, double nb_sign, const double2 *W, const double2 *Dsum,
                   const double *Bsum, const MvArgs &a, int *err, int sm_count, cudaStream_t st);
-// FP64 FMA stencil (cn_mv5.cu) on the same forward blocks, stored as 216
-// planes (direction, species, row, column; cn_mv5_block_entries complex in
-// all); the same conditions as the tensor-core stencil.  wait_cycles bounds
-// every pipeline wait; stall_load >= 0 stops the producer before that load
-// (the test of the timeout path).  One partial row per CTA (cn_mv5_rows).
-// launch_cn_blocks5 writes the blocks in FP64 (W), rounded to FP32 (Wf), or
-// both in one pass; a null pointer skips that precision.
+// launch_cn_blocks5 (cn_mv5.cu) writes the forward blocks as 216 planes
+// (direction, species, row, column; cn_mv5_block_entries complex in all) in
+// FP64 (W), rounded to FP32 (Wf), or both in one pass; a null pointer skips
+// that precision.
 void launch_cn_blocks5(Lat L, const CnCoef &C, const double2 *U, const double2 *DE, double2 *W, float2 *Wf,
                        cudaStream_t st);
 int64_t cn_mv5_units(int64_t V);
-int64_t cn_mv5_rows(int64_t V, int sm_count);
 int64_t cn_mv5_block_entries(int64_t V);
-int launch_cn_mv5(int mode, Lat L, const CnCoef &C, double nb_sign, const double2 *W, const double2 *Dsum,
-                  const double *Bsum, const MvArgs &a, int *err, int sm_count, cudaStream_t st,
-                  long long wait_cycles, int stall_load);
 // finalize stages: 0 = after RES (rr, bb), 1 = alpha (rh.v), 2 = omega (t.s, t.t), 3 = beta (rh.r, r.r)
 void launch_cn_finalize(int stage, int64_t nblocks, const double *partials, double *scal, double tol,
                         cudaStream_t st);
@@ -287,6 +329,8 @@ void launch_prop_soa2f(const double2 *P, double2 *f, int64_t V, cudaStream_t st)
 void launch_single_point(double2 *P, int64_t V, int64_t sq, int64_t sa, cudaStream_t st);
 // |psi|^2 of species sp0 .. sp0 + nsp - 1 (nsp values per partial row)
 void launch_norms(const double2 *P, int64_t V, int sp0, int nsp, double *partials, int64_t &nblk, cudaStream_t st);
+// coefficient of the (k+1)-th newest of d history vectors (degree d - 1 extrapolation)
+double hist_coef(int d, int k);
 // x += sum_k c_k t_k over the d newest history vectors t[0..d-1] (d = 1..4),
 // c the coefficients of the degree d - 1 extrapolation
 void launch_hist_extrapolate(int64_t n, double2 *X, const float2 *const *t, int d, cudaStream_t st);
