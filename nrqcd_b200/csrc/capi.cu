@@ -1427,6 +1427,10 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   int best = NRQ_STENCIL_REGISTER;
   for (int which = 1; which < 4; ++which)
     if (cn->tune_ms[which] > 0.0 && cost(which) < cost(best)) best = which;
+  // the semi-iteration wins by more than the timing's noise at every size (a
+  // coupled step with it against the best of the others: 242 against 374 us
+  // at 12^3, 4.9 against 6.9 ms at 64^3)
+  if (cn->form == 0 && cn->semi_iter && cn->tune_ms[NRQ_STENCIL_FMA] > 0.0) best = NRQ_STENCIL_FMA;
   cn->stencil = best;
   return NRQ_OK;
 }
@@ -1806,7 +1810,7 @@ static bool accept_recursive(const nrq_cn *cn, const double rel[nrq::CN_COLS]) {
 // two vector passes and three scalar stages for the same two orders of
 // application; the step count follows from the first residual and the
 // segment, |r_m| <= |r_0| / |T_m(sigma)| in every column, so the host reads
-// the device once a solve.  64^3: 0.40 ms a step against 1.40 ms an
+// the device once a solve.  64^3: 0.41 ms a step against 1.40 ms an
 // iteration.
 //
 // The bound is rigorous, so a solve ends on it (after m steps max_rel is the

@@ -30,7 +30,10 @@
 //
 // Bound: 64^3, the solver's step (four vector streams, 6.1 KB a site): 0.25 ms
 // at the copy rate, 0.21 ms at the FP64 rate that FMAs with distinct operands
-// reach (49 of 64 a clock and SM); see k_cn_spin below for what it takes.
+// reach (49 of 64 a clock and SM).  It takes 0.41 ms: twelve warps an SM (166
+// registers) hide the loads only in part, a block spends a fifth of its time
+// before its first product and in its epilogue, and the loads alone take 0.31
+// ms (the launch without its products).  24^3: 28 us, 12^3: 12 us.
 //
 // Every mbarrier wait is bounded (wait_cycles); on expiry the thread records
 // NRQ_ERR_TIMEOUT in *err and its warp skips the remaining work.  stall_load
@@ -126,7 +129,7 @@ constexpr int kPrepSites = 32;
 // the site term of the hermitian H (A^H = 1 + i tau H) for quark and
 // antiquark.  One thread per site and direction; the Darwin and magnetic
 // matrices are sums over directions, exchanged through shared memory.  64^3:
-// TODO.
+// 280 us (254 registers, 8 warps an SM; the FP64 pipe 28 % active), 12^3: 10 us.
 __global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C1, const CnCoef *__restrict__ Cm,
                                                                 int nm, double tau, const double2 *__restrict__ U,
                                                                 const double *__restrict__ E, SpinOp op,
@@ -350,8 +353,13 @@ __global__ void __launch_bounds__(256) k_spin_bounds(Lat L, const double *__rest
 namespace {
 constexpr int kUnit = 32;   // sites of a block, one per lane
 constexpr int kWarps = 6;   // one propagator column of both species each
-constexpr int kAhead = 3;   // spinor operands in registers: this step's and the next two's
-constexpr int kWBufs = 3;   // matrix buffers
+// Spinor operands in registers: this step's and the next three's; matrices
+// staged two neighbours ahead.  (64^3, a coupled step: 4.16 ms with the next
+// two and one neighbour, 4.09 with the next three, 3.98 with both.  Prefetches
+// to L2, of the epilogue's operands or of later units', cost 2-20 %; a
+// persistent form with the next unit's first loads issued early 10 %.)
+constexpr int kAhead = 4;
+constexpr int kWBufs = 5;
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
@@ -365,12 +373,39 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// acc += +-(w or conj(w)) p
+// acc += +-(w or conj(w)) p in halves: the products with Re w, then those
+// with Im w, so that consecutive FMAs share an operand register (an FP64 FMA
+// with three fresh operands issues every 2.7 cycles, with one reused 2.3)
+template <int S>
+__device__ __forceinline__ void smac_re(cplx &acc, const double2 w, const double2 p) {
+  const double wr = S > 0 ? w.x : -w.x;
+  acc.re = fma(wr, p.x, acc.re);
+  acc.im = fma(wr, p.y, acc.im);
+}
 template <int S, bool CJ>
-__device__ __forceinline__ void smac(cplx &acc, const double2 w, const double2 p) {
-  const double wr = S > 0 ? w.x : -w.x, wi = (S > 0) == !CJ ? w.y : -w.y;
-  acc.re = fma(wr, p.x, fma(-wi, p.y, acc.re));
-  acc.im = fma(wr, p.y, fma(wi, p.x, acc.im));
+__device__ __forceinline__ void smac_im(cplx &acc, const double2 w, const double2 p) {
+  const double wi = (S > 0) == !CJ ? w.y : -w.y;
+  acc.re = fma(-wi, p.y, acc.re);
+  acc.im = fma(wi, p.x, acc.im);
+}
+template <int SA, int SB, bool CJ>
+__device__ __forceinline__ void smac2(const double2 w, cplx &a, const double2 p, cplx &b, const double2 q) {
+  smac_re<SA>(a, w, p);
+  smac_re<SB>(b, w, q);
+  smac_im<SA, CJ>(a, w, p);
+  smac_im<SB, CJ>(b, w, q);
+}
+template <int SA, int SB, bool CJ>
+__device__ __forceinline__ void smac4(const double2 w, cplx &a, const double2 p, cplx &b, const double2 q, cplx &c,
+                                      const double2 r, cplx &d, const double2 s) {
+  smac_re<SA>(a, w, p);
+  smac_re<SA>(b, w, q);
+  smac_re<SB>(c, w, r);
+  smac_re<SB>(d, w, s);
+  smac_im<SA, CJ>(a, w, p);
+  smac_im<SA, CJ>(b, w, q);
+  smac_im<SB, CJ>(c, w, r);
+  smac_im<SB, CJ>(d, w, s);
 }
 
 // One step: direction I, forward (B = false) or backward, one input colour.
@@ -384,24 +419,17 @@ __device__ __forceinline__ void spin_products(cplx (&a)[4][3], const double2 (&m
   constexpr int S01 = I == 0 ? 1 : S, S10 = I == 0 ? -1 : S;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
+    if (I < 2) smac2<S, -S, B>(m[0][i], a[0][i], q[0], a[3][i], q[3]);
+    if (I < 2) smac2<S, -S, B>(m[1][i], a[1][i], q[1], a[2][i], q[2]);
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
     if (I < 2) {
-      smac<S, B>(a[0][i], m[0][i], q[0]);
-      smac<S, B>(a[1][i], m[1][i], q[1]);
-      smac<-S, B>(a[2][i], m[1][i], q[2]);
-      smac<-S, B>(a[3][i], m[0][i], q[3]);
-      smac<S01, B>(a[0][i], m[2][i], q[1]);
-      smac<S10, B>(a[1][i], m[2][i], q[0]);
-      smac<S01, B>(a[2][i], m[2][i], q[3]);
-      smac<S10, B>(a[3][i], m[2][i], q[2]);
+      smac4<S01, S10, B>(m[2][i], a[0][i], q[1], a[2][i], q[3], a[1][i], q[0], a[3][i], q[2]);
     } else {
-      smac<S, B>(a[0][i], m[0][i], q[0]);
-      smac<S, B>(a[1][i], m[0][i], q[1]);
-      smac<-S, B>(a[2][i], m[0][i], q[2]);
-      smac<-S, B>(a[3][i], m[0][i], q[3]);
-      smac<S, B>(a[0][i], m[B ? 1 : 2][i], q[1]);
-      smac<S, B>(a[1][i], m[B ? 2 : 1][i], q[0]);
-      smac<S, B>(a[2][i], m[B ? 1 : 2][i], q[3]);
-      smac<S, B>(a[3][i], m[B ? 2 : 1][i], q[2]);
+      smac4<S, -S, B>(m[0][i], a[0][i], q[0], a[1][i], q[1], a[2][i], q[2], a[3][i], q[3]);
+      smac2<S, S, B>(m[B ? 1 : 2][i], a[0][i], q[1], a[2][i], q[3]);
+      smac2<S, S, B>(m[B ? 2 : 1][i], a[1][i], q[0], a[3][i], q[2]);
     }
   }
 }
@@ -443,7 +471,6 @@ struct SpinSmem {
   double s1[9][kUnit];
   uint64_t full[6];  // the matrices of neighbour n (and, n = 0, the site term) landed
 };
-static_assert(sizeof(SpinSmem) <= 49152, "static shared memory");
 
 // y = A^H in of the warp's column c at the lane's site x: acc[species*2 +
 // spin][colour]; own[colour] = the input at x itself.  Returns false where a
@@ -481,6 +508,7 @@ __device__ __forceinline__ bool spin_apply(const Lat &L, const double2 *__restri
   stage(0);
 #pragma unroll
   for (int t = 0; t < kAhead - 1; ++t) load(t, own[t]);
+  stage(1);
 #pragma unroll
   for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -494,13 +522,13 @@ __device__ __forceinline__ bool spin_apply(const Lat &L, const double2 *__restri
       if (!ok) record_timeout(err, 5, 0, n);
     }
     if (!__all_sync(0xffffffffu, ok)) return false;
-    // every warp issued its copies of n when it entered neighbour n - 1, so
-    // all have left n - 2, whose buffer n + 1 takes
-    if (n + 1 < 6) stage(n + 1);
+    // every warp issued its copies of n when it entered neighbour n - 2, so
+    // all have left n - 3, whose buffer n + 2 takes
+    if (n + 2 < 6) stage(n + 2);
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const int t = 3 * n + j;
-      load(t + kAhead - 1, own[(t + kAhead - 1) % kAhead]);
+      if (t + kAhead - 1 < 21) load(t + kAhead - 1, own[(t + kAhead - 1) % kAhead]);
       double2 m[3][3];
 #pragma unroll
       for (int t3 = 0; t3 < 3; ++t3)
@@ -515,8 +543,7 @@ __device__ __forceinline__ bool spin_apply(const Lat &L, const double2 *__restri
       if (n == 5) spin_products<2, true>(acc, m, q);
     }
   }
-  // the site term; step 20's operand is still to be loaded
-  load(20, own[20 % kAhead]);
+  // the site term
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const double2 (&q)[4] = own[(18 + j) % kAhead];
@@ -548,7 +575,8 @@ __device__ __forceinline__ bool spin_apply(const Lat &L, const double2 *__restri
 template <int MODE>
 __global__ void __launch_bounds__(kUnit *kWarps, 2)
     k_cn_spin(Lat L, SpinOp op, double sign, MvArgs A, int *err, long long wait_cycles, int stall_load) {
-  __shared__ __align__(16) SpinSmem sm;
+  extern __shared__ __align__(16) unsigned char raw_[];
+  SpinSmem &sm = *reinterpret_cast<SpinSmem *>(raw_);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x < 6) mbar_init(&sm.full[threadIdx.x], kUnit * kWarps);
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -571,35 +599,52 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
   for (int sp = 0; sp < 2; ++sp)
 #pragma unroll
     for (int k = 0; k < 5; ++k) qs[sp][k] = 0.0;
-  const ChebTab *tab = A.cheb;
   if (ok && act) {
+    constexpr bool kB = MODE == MV_RES || MODE == MV_RES2 || MODE == MV_RESC || MODE == MV_RESN || MODE == MV_CH0 ||
+                        MODE == MV_CHK || MODE == MV_CHH;
+    constexpr bool kCheb = MODE == MV_CHK || MODE == MV_CHH;
+    constexpr bool kShadow = MODE == MV_V2 || MODE == MV_T2;
+    cplx c1[2], c2[2];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {  // batches of three rows: their operands, then their results
-      const int sp = h >> 1, r0 = 3 * (h & 1);
-      const int64_t off = (int64_t)(sp * 36 + warp * 6 + r0) * V + x;
-      cplx e1[3], e2[3], e3[3];
-      float2 f[3][4];
+    for (int sp = 0; sp < 2; ++sp) {
+      if (kCheb) c1[sp] = A.cheb->step[A.step].c1[sp];
+      if (kCheb) c2[sp] = A.cheb->step[A.step].c2[sp];
+      if (MODE == MV_CH0) c2[sp] = A.cheb->inv_theta[sp];
+    }
+    // batches of three rows, the operands of the next batch loaded before
+    // this one's results are stored
+    cplx e1[2][3], e2[2][3], e3[2][3];
+    float2 f[2][3][4];
+    auto fetch = [&](int h) {
+      const int64_t off = (int64_t)((h >> 1) * 36 + warp * 6 + 3 * (h & 1)) * V + x;
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         const int64_t o = off + (int64_t)r * V;
-        if (MODE == MV_RES || MODE == MV_RES2 || MODE == MV_RESC || MODE == MV_RESN || MODE == MV_CH0 ||
-            MODE == MV_CHK || MODE == MV_CHH)
-          e1[r] = ldg(A.bvec + o);
-        if (MODE == MV_V) e1[r] = ldg(A.in2 + o);
-        if (MODE == MV_CHK || MODE == MV_CHH) e2[r] = ld(A.out + o);
-        if (MODE == MV_CHH) e3[r] = ldg(A.in2 + o);
-        if (MODE == MV_V2 || MODE == MV_T2) f[r][0] = __ldg(A.sh32 + o);
+        if (kB) e1[h & 1][r] = ldg(A.bvec + o);
+        if (MODE == MV_V) e1[h & 1][r] = ldg(A.in2 + o);
+        if (kCheb) e2[h & 1][r] = ld(A.out + o);
+        if (MODE == MV_CHH) e3[h & 1][r] = ldg(A.in2 + o);
+        if (kShadow) f[h & 1][r][0] = __ldg(A.sh32 + o);
         if (MODE == MV_RHS)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            if (A.hist[k]) f[r][k] = __ldg(A.hist[k] + o);
+            if (A.hist[k]) f[h & 1][r][k] = __ldg(A.hist[k] + o);
       }
+    };
+    fetch(0);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int sp = h >> 1, r0 = 3 * (h & 1);
+      const int64_t off = (int64_t)(sp * 36 + warp * 6 + r0) * V + x;
+      if (h < 3) fetch(h + 1);
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         const int64_t o = off + (int64_t)r * V;
         const int sr = (r0 + r) & 1, i = (r0 + r) >> 1;
         const double2 ow = own[(18 + i) % kAhead][2 * sp + sr];
         const cplx in = {ow.x, ow.y};
+        const cplx ev = e1[h & 1][r];
+        const float2 fv = f[h & 1][r][0];
         cplx y = acc[2 * sp + sr][i];
         if (MODE == MV_PLAIN || MODE == MV_RHS)
           if (sign < 0.0) y = 2.0 * in - y;
@@ -608,17 +653,16 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
         } else if (MODE == MV_RHS) {
           st(A.out + o, y);
           cplx x0 = 2.0 * y - in;
-          cplx dx = {0.0, 0.0};
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             if (A.hist[k]) {
-              dx.re = fma(A.hcoef[k], (double)f[r][k].x, dx.re);
-              dx.im = fma(A.hcoef[k], (double)f[r][k].y, dx.im);
+              x0.re = fma(A.hcoef[k], (double)f[h & 1][r][k].x, x0.re);
+              x0.im = fma(A.hcoef[k], (double)f[h & 1][r][k].y, x0.im);
             }
-          st(A.out2 + o, x0 + dx);
+          st(A.out2 + o, x0);
         } else if (MODE == MV_V || MODE == MV_V2) {
           st(A.out + o, y);
-          const cplx rh = MODE == MV_V ? e1[r] : cplx{(double)f[r][0].x, (double)f[r][0].y};
+          const cplx rh = MODE == MV_V ? ev : cplx{(double)fv.x, (double)fv.y};
           cplx d = {0.0, 0.0};
           cmac_cj(d, rh, y);
           qs[sp][0] += d.re;
@@ -632,12 +676,12 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
           qs[sp][2] += norm2(y);
           if (MODE == MV_T2) {
             cplx t = {0.0, 0.0};
-            cmac_cj(t, cplx{(double)f[r][0].x, (double)f[r][0].y}, y);
+            cmac_cj(t, cplx{(double)fv.x, (double)fv.y}, y);
             qs[sp][3] += t.re;
             qs[sp][4] += t.im;
           }
         } else {
-          const cplx rv = e1[r] - y;
+          const cplx rv = ev - y;
           if (MODE == MV_RES) {
             st(A.out + o, rv);
             st(A.out2 + o, rv);
@@ -658,18 +702,18 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
               A.d32[o] = make_float2((float)dv.re, (float)dv.im);
             }
           } else if (MODE == MV_CH0) {
-            st(A.out + o, in + tab->inv_theta[sp] * rv);
-          } else if (MODE == MV_CHK || MODE == MV_CHH) {
-            const cplx xn = in + tab->step[A.step].c1[sp] * (in - e2[r]) + tab->step[A.step].c2[sp] * rv;
+            st(A.out + o, in + c2[sp] * rv);
+          } else if (kCheb) {
+            const cplx xn = in + c1[sp] * (in - e2[h & 1][r]) + c2[sp] * rv;
             st(A.out + o, xn);
             if (MODE == MV_CHH) {
-              const cplx t = xn - (2.0 * e1[r] - e3[r]);
+              const cplx t = xn - (2.0 * ev - e3[h & 1][r]);
               A.r32[o] = make_float2((float)t.re, (float)t.im);
             }
           }
-          if (MODE != MV_CHK && MODE != MV_CHH) {
+          if (!kCheb) {
             qs[sp][0] += norm2(rv);
-            qs[sp][1] += norm2(e1[r]);
+            qs[sp][1] += norm2(ev);
           }
         }
       }
@@ -741,7 +785,8 @@ void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs
                     long long wait_cycles, int stall_load) {
   const unsigned grid = (unsigned)((L.V + kUnit - 1) / kUnit);
   auto go = [&](auto kern) {
-    kern<<<grid, kUnit * kWarps, 0, st>>>(L, op, sign, a, err, wait_cycles, stall_load);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpinSmem));
+    kern<<<grid, kUnit * kWarps, sizeof(SpinSmem), st>>>(L, op, sign, a, err, wait_cycles, stall_load);
   };
   switch (mode) {
     case MV_PLAIN: go(k_cn_spin<MV_PLAIN>); break;
