@@ -40,13 +40,18 @@ struct nrq_cn_batch {
   std::vector<double> masses;     // distinct masses
   std::vector<int> group_size;    // fields per distinct mass
   std::vector<double2 *> xbuf;    // current iterate buffer of every entry
-  // per-step gauge-derived data (owned copies)
+  // per-step gauge-derived data of the register-tiled kernels (owned copies)
   double2 *U64 = nullptr, *Dsum = nullptr, *DE = nullptr;
   double *Bsum = nullptr;
   float2 *U32 = nullptr, *DE32 = nullptr, *D32 = nullptr;
   float *B32 = nullptr;
   double *bpart = nullptr;   // bounds partial blocks
   double *bounds = nullptr;  // 4 per distinct mass
+  // the spectral enclosure's scratch planes, its tickets, and the masses'
+  // A^H coefficients
+  double *scratch = nullptr;
+  unsigned *tickets = nullptr;
+  nrq::CnCoef *d_coef = nullptr, *h_coef = nullptr;
   // per-field vectors, contiguous over fields
   double2 *b_all = nullptr;
   float2 *r32_all = nullptr, *dA_all = nullptr, *dB_all = nullptr, *e32_all = nullptr;
@@ -72,16 +77,14 @@ struct nrq_cn_batch {
   bool tuned = false;
   int variant = 0, order = 0;  // Chebyshev kernel variant (nrq_kernels.cuh) and block order
   double cand_ms[2 * nrq::BATCH_CHEB_VARIANTS] = {-1, -1, -1, -1, -1, -1, -1, -1};
-  // FP32 blocks of every distinct mass (Chebyshev variant 3; null where the
-  // lattice does not allow it) and the bounded waits' error record
-  float2 *W5f = nullptr;
+  // the operator of every distinct mass in its spin structure, rounded to
+  // FP32 for Chebyshev variant 3 (null where that does not apply) and in
+  // FP64 for the right-hand side and residuals (null for odd V): fp64 = 1
+  // runs the spin-structured stencil, 0 the register-tiled one (timed with
+  // the Chebyshev candidates).  err: the bounded waits' record.
+  nrq::SpinOp spin{};
+  nrq::SpinOp32 spin32{};
   int *err = nullptr, *h_err = nullptr;
-  // the FP64 stencil of the right-hand side and residuals: per-update FP64
-  // blocks of every distinct mass and every field's tensor maps (null where
-  // the lattice does not allow it); fp64 = 1 runs it, 0 the register-tiled
-  // one (timed with the Chebyshev candidates)
-  double2 *W5 = nullptr;
-  nrq::CnBatchMaps *d_fmaps = nullptr, *h_fmaps = nullptr;
   int fp64 = 0;
   double fp64_ms[2] = {-1, -1};
   // generation: changes with every new schedule, tuning or key
@@ -189,7 +192,6 @@ void fill_table(nrq_cn_batch *b, const double c[8], double dt) {
     f.tau = dt * ctx->a[0] / 2.0;
     f.mass = m;
     f.wblk = b->mass_of[i];
-    if (b->h_fmaps && !nrq::batch_mv5_field_maps(b->h_fmaps + i, ctx->lat, f.psi, f.x)) b->fp64 = 0;
     if (learned_on(b)) {
       nrq_heavy *h = b->fields[i];
       f.h1 = hist_v1(h);
@@ -202,63 +204,61 @@ void fill_table(nrq_cn_batch *b, const double c[8], double dt) {
       f.h3 = hist_v(h, 3);
       f.h4 = hist_v(h, 4);
       f.hnew = hist_next(h);
+      f.hstart = 1;
     }
   }
+  for (size_t k = 0; k < b->masses.size(); ++k) b->h_coef[k] = nrqh::make_coef(ctx, b->masses[k], c, dt, true);
 }
 
 int upload_table(nrq_cn_batch *b, cudaStream_t st) {
   NRQ_CUDA_TRY(b->ctx, cudaMemcpyAsync(b->d_tab, b->h_tab, sizeof(nrq::BatchField) * b->nf,
                                        cudaMemcpyHostToDevice, st));
-  if (b->d_fmaps)
-    NRQ_CUDA_TRY(b->ctx, cudaMemcpyAsync(b->d_fmaps, b->h_fmaps, sizeof(nrq::CnBatchMaps) * b->nf,
-                                         cudaMemcpyHostToDevice, st));
+  NRQ_CUDA_TRY(b->ctx, cudaMemcpyAsync(b->d_coef, b->h_coef, sizeof(nrq::CnCoef) * b->masses.size(),
+                                       cudaMemcpyHostToDevice, st));
   return NRQ_OK;
 }
 
 // ---- enqueue helpers (no host synchronisation) ----------------------------
-// the FP64 stencil of every field: MV_RHS or MV_RESC, the FMA stencil on the
-// blocks (fp64 = 1, where it applies) or the register-tiled one
+bool spin64(const nrq_cn_batch *b) { return b->fp64 == 1 && b->spin.W; }
+
+// the FP64 stencil of every field: MV_RHS or MV_RESC, spin-structured (fp64 =
+// 1, where it applies) or register-tiled
 void launch_fp64(nrq_cn_batch *b, int mode, int fp64, int skip_done, cudaStream_t st) {
   nrq_ctx *ctx = b->ctx;
-  if (fp64 == 1 && b->W5 &&
-      nrq::launch_batch_mv5(mode, b->order, ctx->lat, b->W5, (int)b->masses.size(), b->Dsum, b->Bsum, b->d_fmaps,
-                            b->d_tab, b->nf, skip_done, b->err, ctx->sm_count, st, nrq_wait_cycles_default) == 0)
-    return;
-  nrq::launch_batch_mv(mode, b->order, ctx->lat, b->U64, b->Dsum, b->Bsum, b->DE, b->d_tab, b->nf, skip_done, st);
+  if (fp64 == 1 && b->spin.W)
+    nrq::launch_batch_spin(mode, b->order, ctx->lat, b->spin, b->d_tab, b->nf, skip_done,
+                           !b->tuned || b->variant != 3, b->err, st, nrq_wait_cycles_default);
+  else
+    nrq::launch_batch_mv(mode, b->order, ctx->lat, b->U64, b->Dsum, b->Bsum, b->DE, b->d_tab, b->nf, skip_done, st);
 }
 
-// gauge-derived data of this step: link copy, CN blocks, FP32 copies, the
-// spectral enclosure of every mass and the Chebyshev coefficients of every
-// field
-int enq_prepare(nrq_cn_batch *b, const nrq_gauge *g, const double c[8], double dt, cudaStream_t st) {
+// gauge-derived data of this step: the operator of every mass with its
+// spectral enclosure, the Chebyshev coefficients of every field, and where a
+// register-tiled kernel runs (or is timed) its link copy and matrices
+int enq_prepare(nrq_cn_batch *b, const nrq_gauge *g, double dt, cudaStream_t st) {
   nrq_ctx *ctx = b->ctx;
   const nrq::Lat L = ctx->lat;
   const int64_t V = L.V;
-  NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(b->U64, g->U, sizeof(double2) * 27 * V, cudaMemcpyDeviceToDevice, st));
-  {
+  const int nm = (int)b->masses.size();
+  const bool want32 = b->spin32.W && (!b->tuned || b->variant == 3), want64 = b->spin.W && (!b->tuned || b->fp64 == 1);
+  const bool reg32 = !b->tuned || b->variant != 3, reg64 = !b->tuned || !spin64(b);
+  if (reg32 || reg64) {
+    NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(b->U64, g->U, sizeof(double2) * 27 * V, cudaMemcpyDeviceToDevice, st));
     ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0));
     nrq::launch_cn_prepare(L, b->U64, g->E, b->Dsum, b->Bsum, b->DE, st);
   }
-  {
+  if (reg32) {
     ProfScope ps(ctx, 3, (double)V * (1080.0 + 540.0));
     nrq::launch_cn_to_f32(V, b->U64, b->DE, b->Dsum, b->Bsum, b->U32, b->DE32, b->D32, b->B32, st);
   }
-  // per-update blocks of every mass: FP32 for Chebyshev variant 3, FP64 for
-  // the FP64 FMA stencil (the tuner times both before it chooses)
-  const bool want32 = b->W5f && (!b->tuned || b->variant == 3), want64 = b->W5 && (!b->tuned || b->fp64 == 1);
-  if (want32 || want64)
-    for (size_t k = 0; k < b->masses.size(); ++k) {
-      ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + (want32 ? 1728.0 : 0.0) + (want64 ? 3456.0 : 0.0)));
-      const nrq::CnCoef CH = nrqh::make_coef(ctx, b->masses[k], c, dt, true);
-      const int64_t off = (int64_t)k * nrq::cn_mv5_block_entries(V);
-      nrq::launch_cn_blocks5(L, CH, b->U64, b->DE, want64 ? b->W5 + off : nullptr, want32 ? b->W5f + off : nullptr,
-                             st);
-    }
-  const double tau = dt * ctx->a[0] / 2.0;
-  for (size_t k = 0; k < b->masses.size(); ++k) {
-    ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + 216.0));
-    const nrq::CnCoef CH = nrqh::make_coef(ctx, b->masses[k], c, dt, true);
-    nrq::launch_cn_bounds(L, CH, tau, b->U64, b->Dsum, b->Bsum, b->DE, b->bpart, b->bounds + 4 * k, st);
+  {
+    ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0 + nm * ((want64 ? 1512.0 : 0.0) + (want32 ? 756.0 : 0.0) + 56.0)));
+    nrq::launch_spin_prepare(L, nrq::CnCoef{}, b->d_coef, nm, dt * ctx->a[0] / 2.0, g->U, g->E,
+                             want64 ? b->spin : nrq::SpinOp{}, want32 ? b->spin32 : nrq::SpinOp32{}, b->scratch, st);
+  }
+  {
+    ProfScope ps(ctx, 3, (double)V * 56.0 * nm);
+    nrq::launch_spin_bounds(L, nm, b->scratch, b->bpart, b->tickets, b->bounds, st);
   }
   nrq::launch_batch_coef(b->d_tab, b->nf, b->flags, st);
   return check_launch(ctx, "batch prepare");
@@ -269,10 +269,10 @@ int enq_rhs(nrq_cn_batch *b, const nrq_gauge *g, cudaStream_t st) {
   nrq_ctx *ctx = b->ctx;
   {
     ProfScope ps(ctx, 0, (double)ctx->lat.V * (b->nf * 1152.0 * 3 + 432.0 + 192.0));
-    launch_fp64(b, nrq::MV_RHS, b->fp64, 0, st);
+    launch_fp64(b, nrq::MV_RHS, b->fp64, 0, st);  // spin-structured: with the history start
   }
   int rc = check_launch(ctx, "batch rhs");
-  if (!rc && hist_on(b)) {
+  if (!rc && hist_on(b) && !spin64(b)) {
     ProfScope ps(ctx, 1, (double)ctx->lat.V * b->nf * (1152.0 * 2 + 576.0 * (kBatchHistDepth + 1)));
     nrq::launch_batch_hist_start(ctx->lat.V, b->d_tab, b->nf, st);
     rc = check_launch(ctx, "batch history start");
@@ -285,7 +285,7 @@ int enq_rhs(nrq_cn_batch *b, const nrq_gauge *g, cudaStream_t st) {
       NRQ_CUDA_TRY(ctx, cudaEventCreate(&e1));
       cudaEventRecord(e0, st);
     }
-    rc = nrqh::learned_guess_batch(b->learn, ctx, b->d_tab, b->nf, b->U64, g->E, b->lgf, b->lfeat, b->lomega, st);
+    rc = nrqh::learned_guess_batch(b->learn, ctx, b->d_tab, b->nf, g->U, g->E, b->lgf, b->lfeat, b->lomega, st);
     if (b->time_guess) {
       cudaEventRecord(e1, st);
       cudaEventSynchronize(e1);
@@ -316,32 +316,38 @@ int enq_residual(nrq_cn_batch *b, cudaStream_t st, bool first) {
 }
 
 // Chebyshev step `step` of every field with kernel variant / block order
-// (nonzero: the variant does not apply)
-int launch_cheb(nrq_cn_batch *b, int step, int variant, int order, cudaStream_t st) {
+// (nonzero: the variant does not apply); last: the last launch of a pass,
+// which variant 3 ends with the update of x
+int launch_cheb(nrq_cn_batch *b, int step, int variant, int order, bool last, cudaStream_t st) {
   nrq_ctx *ctx = b->ctx;
-  if (variant == 3)
-    return b->W5f ? nrq::launch_batch_cheb5f(step, order, ctx->lat, b->W5f, (int)b->masses.size(), b->D32, b->B32,
-                                             b->dA_all, b->dB_all, b->d_tab, b->nf, b->err, ctx->sm_count, st,
-                                             nrq_wait_cycles_default)
-                  : 1;
-  return nrq::launch_batch_cheb(step, variant, order, ctx->lat, b->U32, b->D32, b->B32, b->DE32, b->d_tab, b->nf,
-                                st);
+  if (variant != 3)
+    return nrq::launch_batch_cheb(step, variant, order, ctx->lat, b->U32, b->D32, b->B32, b->DE32, b->d_tab, b->nf,
+                                  st);
+  if (!b->spin32.W) return 1;
+  nrq::launch_batch_cheb_spin(step, last, order, ctx->lat, b->spin32, b->d_tab, b->nf, b->err, st,
+                              nrq_wait_cycles_default);
+  return 0;
 }
 
-// m FP32 Chebyshev steps on A^H e = r, then x += e
+// m FP32 Chebyshev steps on A^H e = r, and x += e
 int enq_inner(nrq_cn_batch *b, int m, cudaStream_t st) {
   nrq_ctx *ctx = b->ctx;
   const double V = (double)ctx->lat.V;
-  for (int k = 0; k < m; ++k) {
-    ProfScope ps(ctx, 0, V * (b->nf * 576.0 * 6 + 756.0));
-    if (launch_cheb(b, k, b->variant, b->order, st)) {
+  const bool spin = b->variant == 3;
+  const int n = spin ? m - 1 : m;  // launches: the first step of variant 3 needs none
+  for (int k = 0; k < n; ++k) {
+    ProfScope ps(ctx, 0, V * (b->nf * 576.0 * (spin ? 4 : 6) + 756.0));
+    if (launch_cheb(b, k, b->variant, b->order, k == n - 1, st)) {
       ctx->last_error = "batch: unsupported Chebyshev tile";
       return NRQ_ERR_BAD_ARG;
     }
   }
-  {
+  if (!spin || m == 1) {
     ProfScope ps(ctx, 1, V * b->nf * (1152.0 * 2 + 576.0));
-    nrq::launch_batch_add_e(72 * ctx->lat.V, b->d_tab, b->nf, st);
+    if (spin)
+      nrq::launch_batch_cheb_one(72 * ctx->lat.V, b->d_tab, b->nf, st);
+    else
+      nrq::launch_batch_add_e(72 * ctx->lat.V, b->d_tab, b->nf, st);
   }
   return check_launch(ctx, "batch inner solve");
 }
@@ -359,8 +365,8 @@ int enq_readback(nrq_cn_batch *b, cudaStream_t st) {
 // marks the columns it brings within the tolerance (with the measured
 // margin) as converged, so that the final check skips the fields it
 // predicts in full; the check's measured columns then calibrate the margin.
-int enq_scheduled(nrq_cn_batch *b, const nrq_gauge *g, const double c[8], double dt, cudaStream_t st) {
-  int rc = enq_prepare(b, g, c, dt, st);
+int enq_scheduled(nrq_cn_batch *b, const nrq_gauge *g, double dt, cudaStream_t st) {
+  int rc = enq_prepare(b, g, dt, st);
   if (!rc) rc = enq_rhs(b, g, st);
   for (size_t p = 0; !rc && p < b->schedule.size(); ++p) {
     rc = enq_residual(b, st, p == 0);
@@ -403,8 +409,8 @@ Check check(const nrq_cn_batch *b) {
 int steps_for(const nrq_cn_batch *b, double dt, double gain) {
   gain = std::max(gain, 10.0);
   // FP32 arithmetic caps one pass at about 1e6; a pass that can finish the
-  // solve may aim up to 3e7 (the FP64 check decides whether it did)
-  if (gain > 3e7) gain = 1e6;
+  // solve may aim up to 1e7 (the FP64 check decides whether it did)
+  if (gain > 1e7) gain = 1e6;
   const double tau = dt * b->ctx->a[0] / 2.0;
   int m = 1;
   for (; m < nrq::BATCH_MAX_CHEB; ++m) {
@@ -439,11 +445,14 @@ int autotune(nrq_cn_batch *b, cudaStream_t st) {
     for (int order = 0; order < 2; ++order) {
       const int idx = variant * 2 + order;
       b->cand_ms[idx] = -1.0;
-      if ((variant == 2 && !even) || (variant == 3 && !b->W5f)) continue;
+      if ((variant == 2 && !even) || (variant == 3 && !b->spin32.W)) continue;
       // warm-up launch, then timed repetitions
-      int bad = launch_cheb(b, 0, variant, order, st);
+      // (variant 3: its second step, which reads r and d and writes the
+      // second d slot)
+      const int step = variant == 3 ? 1 : 0;
+      int bad = launch_cheb(b, step, variant, order, false, st);
       cudaEventRecord(e0, st);
-      for (int r = 0; r < reps && !bad; ++r) bad = launch_cheb(b, 0, variant, order, st);
+      for (int r = 0; r < reps && !bad; ++r) bad = launch_cheb(b, step, variant, order, false, st);
       cudaEventRecord(e1, st);
       if (bad) continue;
       int rc = check_launch(ctx, "batch autotune");
@@ -469,7 +478,7 @@ int autotune(nrq_cn_batch *b, cudaStream_t st) {
   b->fp64 = 0;
   for (int which = 0; which < 2; ++which) {
     b->fp64_ms[which] = -1.0;
-    if (which == 1 && !b->W5) continue;
+    if (which == 1 && !b->spin.W) continue;
     launch_fp64(b, nrq::MV_RESC, which, 0, st);
     cudaEventRecord(e0, st);
     for (int r = 0; r < reps; ++r) launch_fp64(b, nrq::MV_RESC, which, 0, st);
@@ -498,7 +507,10 @@ int autotune(nrq_cn_batch *b, cudaStream_t st) {
 int refine_adaptive(nrq_cn_batch *b, double dt, cudaStream_t st, int budget, std::vector<int> &used, Check &chk) {
   nrq_ctx *ctx = b->ctx;
   for (int p = 0; p < budget && !chk.conv && !chk.nonfin && !chk.badbounds && !chk.timeout; ++p) {
-    const int m = steps_for(b, dt, chk.worst / (0.3 * b->tol));
+    // to 0.3 tol; deeper where a pass only finishes, and while the histories
+    // fill (the first updates from the sources)
+    const double aim = p > 0 || (hist_on(b) && depth_of(b) < kBatchHistDepth) ? 0.05 : 0.3;
+    const int m = steps_for(b, dt, chk.worst / (aim * b->tol));
     int rc = enq_inner(b, m, st);
     if (!rc) rc = enq_residual(b, st, false);
     if (!rc) rc = enq_readback(b, st);
@@ -521,7 +533,7 @@ int64_t sum(const std::vector<int> &v) {
 int update_calibrate(nrq_cn_batch *b, const nrq_gauge *g, const double c[8], double dt, cudaStream_t st,
                      Check &chk) {
   nrq_ctx *ctx = b->ctx;
-  int rc = enq_prepare(b, g, c, dt, st);
+  int rc = enq_prepare(b, g, dt, st);
   if (rc) return rc;
   NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(b->h_bounds, b->bounds, sizeof(double) * 4 * b->masses.size(),
                                     cudaMemcpyDeviceToHost, st));
@@ -606,7 +618,7 @@ int conclude(nrq_cn_batch *b, const Check &chk, int64_t inner, int64_t passes) {
   b->last_conv = chk.conv;
   if (chk.timeout) {
     b->ctx->last_error = std::string("batch stencil: a bounded pipeline wait expired (") +
-                         (b->h_err[1] / 16 == 7 ? "k_batch_mv5" : "k_cheb5f") + ", load " +
+                         (b->h_err[1] / 16 == 5 ? "k_cn_spin" : "k_cheb_spin") + ", load " +
                          std::to_string(b->h_err[2]) + ", CTA " + std::to_string(b->h_err[3]) + ")";
     cudaMemsetAsync(b->err, 0, sizeof(int) * 16, b->ctx->stream);
     b->h_err[0] = 0;
@@ -660,13 +672,12 @@ int capture(nrq_ctx *ctx, cudaStream_t st, cudaGraph_t *graph, int (*body)(void 
 struct StepArgs {
   nrq_cn_batch *b;
   const nrq_gauge *g;
-  const double *c;
   double dt;
   bool leapfrog;
 };
 int step_body(void *p) {
   StepArgs *a = (StepArgs *)p;
-  int rc = enq_scheduled(a->b, a->g, a->c, a->dt, a->b->ctx->stream);
+  int rc = enq_scheduled(a->b, a->g, a->dt, a->b->ctx->stream);
   if (!rc && a->leapfrog) rc = nrq_gauge_update((nrq_gauge *)a->g, a->dt);
   return rc;
 }
@@ -729,7 +740,7 @@ extern "C" int nrq_cn_batch_create(nrq_ctx *ctx, int nfields, nrq_heavy *const *
   NRQ_B_ALLOC(b->DE32, sizeof(float2) * 54 * V);
   NRQ_B_ALLOC(b->D32, sizeof(float2) * 9 * V);
   NRQ_B_ALLOC(b->B32, sizeof(float) * 9 * V);
-  NRQ_B_ALLOC(b->bpart, sizeof(double) * 4 * nbb);
+  NRQ_B_ALLOC(b->bpart, sizeof(double) * 4 * nbb * b->masses.size());
   NRQ_B_ALLOC(b->bounds, sizeof(double) * 4 * b->masses.size());
   NRQ_B_ALLOC(b->b_all, sizeof(double2) * P * nfields);
   NRQ_B_ALLOC(b->r32_all, sizeof(float2) * P * nfields);
@@ -742,11 +753,19 @@ extern "C" int nrq_cn_batch_create(nrq_ctx *ctx, int nfields, nrq_heavy *const *
   NRQ_B_ALLOC(b->flags, sizeof(int) * nfields);
   NRQ_B_ALLOC(b->d_tab, sizeof(nrq::BatchField) * nfields);
   NRQ_B_ALLOC(b->err, sizeof(int) * 16);
-  if (nrq::cheb5f_applicable(ctx->lat))
-    NRQ_B_ALLOC(b->W5f, sizeof(float2) * nrq::cn_mv5_block_entries(V) * b->masses.size());
-  if (nrq::batch_mv5_applicable(ctx->lat)) {
-    NRQ_B_ALLOC(b->W5, sizeof(double2) * nrq::cn_mv5_block_entries(V) * b->masses.size());
-    NRQ_B_ALLOC(b->d_fmaps, sizeof(nrq::CnBatchMaps) * nfields);
+  const int64_t nm = (int64_t)b->masses.size();
+  NRQ_B_ALLOC(b->scratch, sizeof(double) * 7 * V * nm);
+  NRQ_B_ALLOC(b->tickets, sizeof(unsigned) * nm);
+  NRQ_B_ALLOC(b->d_coef, sizeof(nrq::CnCoef) * nm);
+  if (nrq::cheb_spin_applicable(ctx->lat)) {
+    NRQ_B_ALLOC(b->spin32.W, sizeof(float2) * 81 * V * nm);
+    NRQ_B_ALLOC(b->spin32.S0, sizeof(float2) * 9 * V * nm);
+    NRQ_B_ALLOC(b->spin32.S1, sizeof(float) * 9 * V * nm);
+  }
+  if (V % 2 == 0 && V >= 34 && nrq::cn_spin_applicable(ctx->lat)) {
+    NRQ_B_ALLOC(b->spin.W, sizeof(double2) * 81 * V * nm);
+    NRQ_B_ALLOC(b->spin.S0, sizeof(double2) * 9 * V * nm);
+    NRQ_B_ALLOC(b->spin.S1, sizeof(double) * 9 * V * nm);
   }
   b->xbuf.assign(nfields, nullptr);
   for (int i = 0; i < nfields; ++i) NRQ_B_ALLOC(b->xbuf[i], sizeof(double2) * P);
@@ -756,10 +775,10 @@ extern "C" int nrq_cn_batch_create(nrq_ctx *ctx, int nfields, nrq_heavy *const *
   if ((e = cudaMallocHost(&b->h_flags, sizeof(int) * nfields)) != cudaSuccess) return fail(e);
   if ((e = cudaMallocHost(&b->h_bounds, sizeof(double) * 4 * b->masses.size())) != cudaSuccess) return fail(e);
   if ((e = cudaMallocHost(&b->h_err, sizeof(int) * 16)) != cudaSuccess) return fail(e);
-  if (b->d_fmaps && (e = cudaMallocHost(&b->h_fmaps, sizeof(nrq::CnBatchMaps) * nfields)) != cudaSuccess)
-    return fail(e);
+  if ((e = cudaMallocHost(&b->h_coef, sizeof(nrq::CnCoef) * nm)) != cudaSuccess) return fail(e);
   std::memset(b->h_err, 0, sizeof(int) * 16);
   if ((e = cudaMemsetAsync(b->err, 0, sizeof(int) * 16, ctx->stream)) != cudaSuccess) return fail(e);
+  if ((e = cudaMemsetAsync(b->tickets, 0, sizeof(unsigned) * nm, ctx->stream)) != cudaSuccess) return fail(e);
   // defined contents for the FP32 vectors and flags the tuner's first launches read
   for (float2 *p : {b->r32_all, b->dA_all, b->dB_all, b->e32_all})
     if ((e = cudaMemsetAsync(p, 0, sizeof(float2) * P * nfields, ctx->stream)) != cudaSuccess) return fail(e);
@@ -783,13 +802,14 @@ extern "C" int nrq_cn_batch_destroy(nrq_cn_batch *b) {
                   (void *)b->D32, (void *)b->B32, (void *)b->bpart, (void *)b->bounds, (void *)b->b_all,
                   (void *)b->r32_all, (void *)b->dA_all, (void *)b->dB_all, (void *)b->e32_all, (void *)b->part_all,
                   (void *)b->scal_all, (void *)b->flags, (void *)b->d_tab, (void *)b->lgf, (void *)b->lfeat,
-                  (void *)b->lomega, (void *)b->W5f, (void *)b->err, (void *)b->W5, (void *)b->d_fmaps,
-                  (void *)b->pstate})
+                  (void *)b->lomega, (void *)b->spin32.W, (void *)b->spin32.S0, (void *)b->spin32.S1, (void *)b->err,
+                  (void *)b->spin.W, (void *)b->spin.S0, (void *)b->spin.S1, (void *)b->scratch, (void *)b->tickets,
+                  (void *)b->d_coef, (void *)b->pstate})
     if (p) cudaFree(p);
   for (double2 *p : b->xbuf)
     if (p) cudaFree(p);
   for (void *p : {(void *)b->h_tab, (void *)b->h_scal, (void *)b->h_flags, (void *)b->h_bounds, (void *)b->h_err,
-                  (void *)b->h_fmaps})
+                  (void *)b->h_coef})
     if (p) cudaFreeHost(p);
   delete b;
   return NRQ_OK;
@@ -834,7 +854,7 @@ int batch_update(nrq_cn_batch *b, const nrq_gauge *g, const double c[8], double 
     if (b->exec && (b->exec_gen != b->gen || b->exec_g != g)) free_graph(b->exec);
     if (!b->exec) {
       cudaGraph_t graph = nullptr;
-      StepArgs a{b, g, c, dt, false};
+      StepArgs a{b, g, dt, false};
       if ((rc = capture(ctx, st, &graph, step_body, &a))) return rc;
       cudaError_t e = cudaGraphInstantiate(&b->exec, graph, 0);
       cudaGraphDestroy(graph);
@@ -848,7 +868,7 @@ int batch_update(nrq_cn_batch *b, const nrq_gauge *g, const double c[8], double 
     }
     NRQ_CUDA_TRY(ctx, cudaGraphLaunch(b->exec, st));
   } else {
-    if ((rc = enq_scheduled(b, g, c, dt, st))) return rc;
+    if ((rc = enq_scheduled(b, g, dt, st))) return rc;
   }
   NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   if (learned_on(b) && (rc = nrqh::learned_check(b->learn))) return rc;
@@ -963,7 +983,7 @@ extern "C" int nrq_cn_batch_fp64_info(const nrq_cn_batch *b, int *which, double 
 
 extern "C" int nrq_cn_batch_set_fp64(nrq_cn_batch *b, int which) {
   if (!b || which < 0 || which > 1) return NRQ_ERR_BAD_ARG;
-  if (which == 1 && !b->W5) {
+  if (which == 1 && !b->spin.W) {
     b->ctx->last_error = "batch: the FP64 block stencil needs an even V of at least 34 sites";
     return NRQ_ERR_BAD_ARG;
   }
@@ -982,7 +1002,7 @@ extern "C" int nrq_cn_batch_set_variant(nrq_cn_batch *b, int variant, int order)
         return NRQ_ERR_BAD_ARG;
       }
   }
-  if (variant == 3 && !b->W5f) {
+  if (variant == 3 && !b->spin32.W) {
     b->ctx->last_error = "batch: the FP32 block step needs V a multiple of 4, V >= 36, nx even";
     return NRQ_ERR_BAD_ARG;
   }
@@ -991,7 +1011,7 @@ extern "C" int nrq_cn_batch_set_variant(nrq_cn_batch *b, int variant, int order)
   } else {
     b->variant = variant;
     b->order = order;
-    if (b->fp64 < 0 || !b->tuned) b->fp64 = b->W5 ? 1 : 0;  // untimed: the FMA stencil where it applies
+    if (b->fp64 < 0 || !b->tuned) b->fp64 = b->spin.W ? 1 : 0;  // untimed: the FMA stencil where it applies
     b->tuned = true;
   }
   b->have_key = false;  // recalibrate the schedule with the new kernel
@@ -1076,7 +1096,7 @@ extern "C" int nrq_ensemble_step(nrq_ensemble *e, const double c[8], double dt, 
       cudaGraphNode_t prev = nullptr;
       for (int i = 0; i < n; ++i) {
         cudaGraph_t child = nullptr;
-        StepArgs a{e->batches[i], e->gauges[i], c, dt, true};
+        StepArgs a{e->batches[i], e->gauges[i], dt, true};
         if ((rc = capture(e->batches[i]->ctx, e->batches[i]->ctx->stream, &child, step_body, &a))) {
           cudaGraphDestroy(master);
           if (e->batches[i]->ctx != ctx0) ctx0->last_error = e->batches[i]->ctx->last_error;

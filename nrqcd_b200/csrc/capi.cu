@@ -47,7 +47,7 @@ std::string timeout_message(const double *h_scal) {
   const int stencil = e[1] / 16, role = e[1] % 16;
   std::string m = "CN stencil: a bounded pipeline wait expired";
   if (e[1] != 0) {
-    m += std::string(" (") + (stencil == 6 ? "k_cheb5f" : "k_cn_mv" + std::to_string(stencil)) + ", " +
+    m += std::string(" (") + (stencil == 6 ? "k_cheb_spin" : stencil == 5 ? "k_cn_spin" : "k_cn_mv" + std::to_string(stencil)) + ", " +
          (role >= 0 && role < 5 ? roles[role] : "?") +
          ", load " + std::to_string(e[2]) + ", CTA " + std::to_string(e[3]);
     m += ")";
@@ -1077,7 +1077,7 @@ extern "C" int nrq_cn_set_stencil(nrq_cn *cn, int stencil) {
 
 extern "C" int nrq_cn_set_cheb_stencil(nrq_cn *cn, int which) {
   if (!cn || which < -1 || which > NRQ_CHEB_BLOCKS) return NRQ_ERR_BAD_ARG;
-  if (which == NRQ_CHEB_BLOCKS && !nrq::cheb5f_applicable(cn->ctx->lat)) {
+  if (which == NRQ_CHEB_BLOCKS && !nrq::cheb_spin_applicable(cn->ctx->lat)) {
     cn->ctx->last_error = "nrq_cn_set_cheb_stencil: the FP32 block step needs V a multiple of 4, V >= 36, nx even";
     return NRQ_ERR_BAD_ARG;
   }
@@ -1133,7 +1133,8 @@ extern "C" int nrq_cn_finalize(nrq_cn *cn) {
                   (void *)cn->rh, (void *)cn->p, (void *)cn->v, (void *)cn->t, (void *)cn->s, (void *)cn->scal,
                   (void *)cn->partials, (void *)cn->U32, (void *)cn->DE32, (void *)cn->D32, (void *)cn->B32,
                   (void *)cn->r32, (void *)cn->dA32, (void *)cn->dB32, (void *)cn->e32,
-                  (void *)cn->Wblk, (void *)cn->Wblk5f, (void *)cn->spin.W, (void *)cn->spin.S0, (void *)cn->spin.S1,
+                  (void *)cn->Wblk, (void *)cn->spin.W, (void *)cn->spin.S0, (void *)cn->spin.S1,
+                  (void *)cn->spin32.W, (void *)cn->spin32.S0, (void *)cn->spin32.S1,
                   (void *)cn->spin_scratch, (void *)cn->spin_part, (void *)cn->spin_ticket, (void *)cn->cheb_tab})
     if (p) cudaFree(p);
   if (cn->h_scal) cudaFreeHost(cn->h_scal);
@@ -1189,13 +1190,14 @@ int ensure_blocks(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *
   *sign = 1.0;
   return check_launch(ctx, "k_cn_blocks");
 }
-// whether the precision form's inner steps run on the FP32 blocks: forced,
-// or the faster of the two on the first update (before it, the blocks are
-// built so that the timing can run)
-bool use_cheb5f(const nrq_cn *cn) {
-  if (cn->form < 1 || cn->cheb_stencil == NRQ_CHEB_REGISTER || !nrq::cheb5f_applicable(cn->ctx->lat)) return false;
+// whether the precision form's inner steps may run on the spin-structured
+// operator / register-tiled: forced, or the faster of the two on the first
+// update (before it, both, so that the timing can run)
+bool use_cheb_spin(const nrq_cn *cn) {
+  if (cn->form < 1 || cn->cheb_stencil == NRQ_CHEB_REGISTER || !nrq::cheb_spin_applicable(cn->ctx->lat)) return false;
   return cn->cheb_stencil == NRQ_CHEB_BLOCKS || !cn->cheb_tuned || cn->cheb_choice == NRQ_CHEB_BLOCKS;
 }
+bool use_cheb_reg(const nrq_cn *cn) { return !use_cheb_spin(cn) || (cn->cheb_stencil < 0 && !cn->cheb_tuned); }
 // the matrices of the other stencils, on demand after cn_prepare
 int ensure_legacy(nrq_cn *cn, const nrq_gauge *g) {
   if (cn->legacy_valid) return NRQ_OK;
@@ -1205,24 +1207,17 @@ int ensure_legacy(nrq_cn *cn, const nrq_gauge *g) {
   cn->legacy_valid = true;
   return check_launch(ctx, "k_cn_prepare");
 }
-// The FP32 Chebyshev step's blocks with the coefficients C.
-int ensure_blocks5f(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *sign) {
-  nrq_ctx *ctx = cn->ctx;
-  *sign = blocks_sign(cn->w5f_valid, cn->w5f_coef, C);
-  if (*sign != 0.0) return NRQ_OK;
-  const int64_t V = ctx->lat.V;
+// their FP32 copies, for the register-tiled Chebyshev step
+int ensure_f32(nrq_cn *cn, const nrq_gauge *g) {
+  if (cn->f32_valid) return NRQ_OK;
   int rc = ensure_legacy(cn, g);
   if (rc) return rc;
-  if (!cn->Wblk5f)
-    NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->Wblk5f, sizeof(float2) * nrq::cn_mv5_block_entries(V)));
-  {
-    ProfScope ps(ctx, 3, (double)V * (432.0 + 864.0 + 1728.0));
-    nrq::launch_cn_blocks5(ctx->lat, C, g->U, cn->DE, nullptr, cn->Wblk5f, ctx->stream);
-  }
-  cn->w5f_coef = C;
-  cn->w5f_valid = true;
-  *sign = 1.0;
-  return check_launch(ctx, "k_cn_blocks5");
+  nrq_ctx *ctx = cn->ctx;
+  ProfScope ps(ctx, 3, (double)ctx->lat.V * (1080.0 + 540.0));
+  nrq::launch_cn_to_f32(ctx->lat.V, g->U, cn->DE, cn->Dsum, cn->Bsum, cn->U32, cn->DE32, cn->D32, cn->B32,
+                        ctx->stream);
+  cn->f32_valid = true;
+  return check_launch(ctx, "k_cn_to_f32");
 }
 // The operator in its spin structure for the coefficients C (of A^H, tau =
 // dt a0/2 of that solve); sign -1 where it was built for C negated.
@@ -1246,12 +1241,19 @@ int ensure_spin(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *si
   NRQ_CUDA_TRY(ctx, want(&cn->spin.S0, sizeof(double2) * 9 * V));
   NRQ_CUDA_TRY(ctx, want(&cn->spin.S1, sizeof(double) * 9 * V));
   NRQ_CUDA_TRY(ctx, want(&cn->spin.W, sizeof(double2) * 81 * V));
+  nrq::SpinOp32 op32{};
+  if (use_cheb_spin(cn)) {
+    NRQ_CUDA_TRY(ctx, want(&cn->spin32.S0, sizeof(float2) * 9 * V));
+    NRQ_CUDA_TRY(ctx, want(&cn->spin32.S1, sizeof(float) * 9 * V));
+    NRQ_CUDA_TRY(ctx, want(&cn->spin32.W, sizeof(float2) * 81 * V));
+    op32 = cn->spin32;
+  }
   {
-    ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0 + 1296.0 + 216.0));
+    ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0 + (op32.W ? 1.5 : 1.0) * (1296.0 + 216.0)));
     // H = (A^H - 1) / (i tau): any tau with the coefficients' scale serves
     // the enclosure as long as the solve uses the same one
     nrq::launch_spin_prepare(ctx->lat, C, nullptr, 1, cn->spin_tau != 0.0 ? cn->spin_tau : 1.0, g->U, g->E, cn->spin,
-                             cn->spin_scratch, ctx->stream);
+                             op32, cn->spin_scratch, ctx->stream);
   }
   cn->spin_coef = C;
   cn->spin_valid = true;
@@ -1441,7 +1443,7 @@ int cn_prepare(nrq_cn *cn, const nrq_gauge *g, double dt) {
   if (rc) return rc;
   cn->legacy_valid = false;
   cn->w_valid = false;
-  cn->w5f_valid = false;
+  cn->f32_valid = false;
   cn->spin_valid = false;
   cn->spin_tau = dt * cn->ctx->a[0] / 2.0;
   return NRQ_OK;
@@ -1478,14 +1480,14 @@ using nrqh::cheb_gain;
 using nrqh::cheb_segment;
 namespace {
 // The first update's choice between the two FP32 Chebyshev steps: one warm-up
-// and three timed launches of each as a first step, reading d = dA32 and
-// writing only e32 and dB32 (the r operand pointed at e32 as well), which the
-// solve's real first step rewrites before it reads them.
-int tune_cheb(nrq_cn *cn, const nrq::CnCoef &CH, const nrq::ChebCoef &K, double wsign) {
+// and three timed launches of each, reading dA32 and r32 and writing only
+// e32 and dB32 (the register-tiled step's r operand pointed at e32 as well),
+// which the solve rewrites before it reads them.
+int tune_cheb(nrq_cn *cn, const nrq::CnCoef &CH, const nrq::ChebCoef &K, const nrq::cplx inv_theta[2]) {
   nrq_ctx *ctx = cn->ctx;
   cn->cheb_tuned = true;
   cn->cheb_choice = NRQ_CHEB_REGISTER;
-  if (!nrq::cheb5f_applicable(ctx->lat)) return NRQ_OK;
+  if (!nrq::cheb_spin_applicable(ctx->lat)) return NRQ_OK;
   cudaStream_t st = ctx->stream;
   const bool prof = ctx->prof;
   ctx->prof = false;
@@ -1495,12 +1497,11 @@ int tune_cheb(nrq_cn *cn, const nrq::CnCoef &CH, const nrq::ChebCoef &K, double 
   const int reps = 3;
   for (int which = 0; which < 2; ++which) {
     cn->cheb_ms[which] = -1.0;
-    bool ok = true;
-    for (int r = 0; r < reps + 1 && ok; ++r) {
+    for (int r = 0; r < reps + 1; ++r) {
       if (r == 1) cudaEventRecord(e0, st);
       if (which == NRQ_CHEB_BLOCKS)
-        ok = nrq::launch_cheb5f(true, ctx->lat, CH, wsign, cn->Wblk5f, cn->D32, cn->B32, cn->dA32, cn->dB32, cn->e32,
-                                cn->e32, K, scal_err(cn->scal), ctx->sm_count, st, cn->wait_cycles) == 0;
+        nrq::launch_cheb_spin(1, false, ctx->lat, cn->spin32, cn->r32, cn->dA32, cn->dB32, nullptr, nullptr, K,
+                              inv_theta, scal_err(cn->scal), st, cn->wait_cycles);
       else
         nrq::launch_cheb32(true, ctx->lat, CH, cn->U32, cn->D32, cn->B32, cn->DE32, cn->dA32, cn->dB32, cn->e32,
                            cn->e32, K, st);
@@ -1509,14 +1510,14 @@ int tune_cheb(nrq_cn *cn, const nrq::CnCoef &CH, const nrq::ChebCoef &K, double 
     cudaEventSynchronize(e1);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    if (ok) cn->cheb_ms[which] = ms / reps;
+    cn->cheb_ms[which] = ms / reps;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   ctx->prof = prof;
   int rc = check_launch(ctx, "Chebyshev step timing");
   if (rc) return rc;
-  if (cn->cheb_ms[NRQ_CHEB_BLOCKS] > 0.0 && cn->cheb_ms[NRQ_CHEB_BLOCKS] < cn->cheb_ms[NRQ_CHEB_REGISTER])
+  if (cn->cheb_ms[NRQ_CHEB_BLOCKS] < cn->cheb_ms[NRQ_CHEB_REGISTER])
     cn->cheb_choice = NRQ_CHEB_BLOCKS;
   return NRQ_OK;
 }
@@ -1537,37 +1538,47 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   const double tau = std::fabs(dt) * ctx->a[0] / 2.0;
   int rc = cn_prepare(cn, g, dt);
   double spin_sign = 0.0;
-  if (!rc) rc = ensure_legacy(cn, g);
   if (!rc) rc = ensure_spin(cn, CH, g, &spin_sign);
   if (rc) return rc;
-  {
-    ProfScope ps(ctx, 3, (double)V * (1080.0 + 540.0));
-    nrq::launch_cn_to_f32(V, g->U, cn->DE, cn->Dsum, cn->Bsum, cn->U32, cn->DE32, cn->D32, cn->B32, st);
-  }
   // spectral enclosure of H per species
   if ((rc = spin_bounds(cn, scal_bounds(cn->scal)))) return rc;
   NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(cn->h_bounds, scal_bounds(cn->scal), sizeof(double) * 4, cudaMemcpyDeviceToHost,
                                     st));
   int64_t matvecs = 0, vstreams = 0;
+  // learned form: x = 2 RHS - psi + w1 u + w2 v (network), history restarted
+  // with the network's part; every refinement correction is added to it
+  const bool learned = cn->form == 2 && nrqh::learned_ready(cn->learn);
+  // otherwise the plain solve's extrapolated start from the field's history;
+  // on the FMA stencil the right-hand side's launch adds it and starts the
+  // new history vector with the added part, which every correction then joins
+  const bool hist = !learned && cn->history_guess;
+  const bool fma = cn->stencil == NRQ_STENCIL_FMA && nrq::cn_spin_applicable(L);
+  if (hist && fma && (rc = nrqh::ensure_hist(h, cn->history_depth))) return rc;
+  const int hist_depth = hist ? std::min(cn->history_depth, h->hist_count) : 0;
+  const int hist_count = h->hist_count;
+  float2 *hacc = hist && fma ? hist_next(h) : nullptr;
   {  // RHS = A psi ; x0 = 2 RHS - psi
     nrq::MvArgs a{};
     a.in = h->P;
     a.out = cn->b;
     a.out2 = cn->x;
+    a.r32 = hacc;
+    if (hacc)
+      for (int k = 0; k < hist_depth; ++k) {
+        a.hist[k] = hist_v(h, k + 1);
+        a.hcoef[k] = nrq::hist_coef(hist_depth, k);
+      }
+    // the oldest history vector's slot is overwritten from here on: an
+    // update that ends early leaves the field without a history
+    if (hacc) h->hist_count = 0;
     if ((rc = mv(cn, nrq::MV_RHS, CA, g, a))) return rc;
     matvecs += 1;
     vstreams += 1;
   }
-  // learned form: x = 2 RHS - psi + w1 u + w2 v (network), history restarted
-  // with the network's part; every refinement correction is added to it
-  const bool learned = cn->form == 2 && nrqh::learned_ready(cn->learn);
-  // otherwise the plain solve's extrapolated start from the field's history
-  const bool hist = !learned && cn->history_guess;
-  if (hist && h->hist_count >= 1) {
-    const int d = std::min(cn->history_depth, h->hist_count);
+  if (hist_depth >= 1 && !hacc) {
     const float2 *t[4] = {hist_v(h, 1), hist_v(h, 2), hist_v(h, 3), hist_v(h, 4)};
-    ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * d));
-    nrq::launch_hist_extrapolate(72 * V, cn->x, t, d, st);
+    ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * hist_depth));
+    nrq::launch_hist_extrapolate(72 * V, cn->x, t, hist_depth, st);
     vstreams += 2;
   }
   if (learned) {
@@ -1576,6 +1587,7 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     if ((rc = nrqh::learned_guess(cn->learn, ctx, h->P, cn->b, hist_v1(h), hist_v2(h), hist_next(h), g->U, g->E,
                                   mass, dt, cn->x, st)))
       return rc;
+    hacc = hist_next(h);
   }
   NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   if (learned && (rc = nrqh::learned_check(cn->learn))) return rc;
@@ -1610,10 +1622,10 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   }
   // smallest inner step count whose guaranteed gain reaches `gain` on both
   // species.  FP32 arithmetic caps one pass at about 1e6; a pass that can
-  // finish the solve may aim up to 3e7 (the FP64 check decides whether it did)
+  // finish the solve may aim up to 1e7 (the FP64 check decides whether it did)
   auto inner_steps = [&](double gain) {
     gain = std::max(gain, 10.0);
-    if (gain > 3e7) gain = 1e6;
+    if (gain > 1e7) gain = 1e6;
     int m = 1;
     while (m < kMaxInner && std::min(cheb_gain(seg[0].sigma, m), cheb_gain(seg[1].sigma, m)) < gain) ++m;
     return m;
@@ -1633,7 +1645,9 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     a.in = cn->x;
     a.bvec = cn->b;
     a.r32 = cn->r32;
-    a.d32 = cn->dA32;
+    // d = r / theta starts the register-tiled inner steps only; the other
+    // FP64 stencils write it in any case
+    a.d32 = use_cheb_reg(cn) || cn->stencil != NRQ_STENCIL_FMA ? cn->dA32 : nullptr;
     a.partials = cn->partials;
     for (int sp = 0; sp < 2; ++sp) {
       std::complex<double> it = 1.0 / seg[sp].theta;
@@ -1681,42 +1695,51 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
       break;
     }
     if (outer == 7) break;
-    // gain needed to bring the worst column to 0.3 tol in this pass
+    // gain needed to bring the worst column to 0.3 tol in this pass; deeper
+    // where a pass only finishes, and while the field's history fills: the
+    // first updates from a source, whose error sits on the few sites the
+    // field has reached
     double worst = 0.0;
     for (int kk = 0; kk < nrq::CN_COLS; ++kk) worst = std::max(worst, rel[kk]);
+    const double aim = outer > 0 || (hist && hist_count < cn->history_depth) ? 0.05 : 0.3;
     // maxits bounds the FP32 inner steps of the whole update
-    int m = inner_steps(worst / (0.3 * cn->tol));
+    int m = inner_steps(worst / (aim * cn->tol));
     if (inner + m > cn->maxits) m = (int)(cn->maxits - inner);
     if (m <= 0) break;
-    // FP32 inner Chebyshev solve of A^H e = r, then x += e
-    float2 *dcur = cn->dA32, *dnext = cn->dB32;
-    double wsign = 0.0;
-    if (use_cheb5f(cn) && (rc = ensure_blocks5f(cn, CH, g, &wsign))) return rc;
-    if (cn->cheb_stencil < 0 && !cn->cheb_tuned && (rc = tune_cheb(cn, CH, coef[0], wsign))) return rc;
-    const bool blk = use_cheb5f(cn);
-    for (int k = 0; k < m; ++k) {
-      ProfScope ps(ctx, 0, (double)V * (576.0 * 6 + 756.0));
-      if (blk)
-        rc = nrq::launch_cheb5f(k == 0, L, CH, wsign, cn->Wblk5f, cn->D32, cn->B32, dcur, dnext, cn->r32, cn->e32,
-                                coef[k], scal_err(cn->scal), ctx->sm_count, st, cn->wait_cycles);
-      if (!blk || rc) {
-        rc = NRQ_OK;
+    // FP32 inner Chebyshev solve of A^H e = r, and x += e
+    if (use_cheb_reg(cn) && (rc = ensure_f32(cn, g))) return rc;
+    if (use_cheb_spin(cn) && (rc = ensure_spin(cn, CH, g, &spin_sign))) return rc;
+    if (cn->cheb_stencil < 0 && !cn->cheb_tuned && (rc = tune_cheb(cn, CH, coef[0], a.inv_theta))) return rc;
+    if (use_cheb_spin(cn)) {
+      cn->last_cheb = NRQ_CHEB_BLOCKS;
+      if (m == 1) {
+        ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * (hacc ? 3 : 1)));
+        nrq::launch_cheb_one(72 * V, cn->r32, cn->x, hacc, a.inv_theta, st);
+      }
+      for (int k = 0; k < m - 1; ++k) {
+        const bool last = k == m - 2;
+        ProfScope ps(ctx, 0, (double)V * (576.0 * (k == 0 ? 1 : k == 1 ? 2 : 3) +
+                                          (last ? 1152.0 * 2 + (hacc ? 1152.0 : 0.0) : 576.0) + 756.0));
+        nrq::launch_cheb_spin(k, last, L, cn->spin32, cn->r32, cn->dA32, cn->dB32, cn->x, hacc, coef[k], a.inv_theta,
+                              scal_err(cn->scal), st, cn->wait_cycles);
+      }
+    } else {
+      cn->last_cheb = NRQ_CHEB_REGISTER;
+      float2 *dcur = cn->dA32, *dnext = cn->dB32;
+      for (int k = 0; k < m; ++k) {
+        ProfScope ps(ctx, 0, (double)V * (576.0 * 6 + 756.0));
         nrq::launch_cheb32(k == 0, L, CH, cn->U32, cn->D32, cn->B32, cn->DE32, dcur, dnext, cn->r32, cn->e32,
                            coef[k], st);
-        cn->last_cheb = NRQ_CHEB_REGISTER;
-      } else {
-        cn->last_cheb = NRQ_CHEB_BLOCKS;
+        std::swap(dcur, dnext);
       }
-      std::swap(dcur, dnext);
+      ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * (hacc ? 3 : 1)));
+      if (hacc)
+        nrqh::add_e_hist(72 * V, cn->x, cn->e32, hacc, st);
+      else
+        nrq::launch_add_e(72 * V, cn->x, cn->e32, st);
     }
+    if ((rc = check_launch(ctx, "Chebyshev step"))) return rc;
     inner += m;
-    if (learned) {
-      ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * 3));
-      nrqh::add_e_hist(72 * V, cn->x, cn->e32, hist_next(h), st);
-    } else {
-      ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0));
-      nrq::launch_add_e(72 * V, cn->x, cn->e32, st);
-    }
     matvecs += m;
     vstreams += 3;
     // the pass's guaranteed gain per species (quark columns 0-5, antiquark
@@ -1744,8 +1767,9 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     }
   }
   if (status == NRQ_OK && !conv) status = NRQ_ERR_NOT_CONVERGED;
-  bool keep = learned && status == NRQ_OK;
-  if (hist && status == NRQ_OK) {  // t = x - (2 RHS - psi) into the history
+  bool keep = hacc && status == NRQ_OK;
+  if (keep && !learned) h->hist_count = hist_count;
+  if (hist && !hacc && status == NRQ_OK) {  // t = x - (2 RHS - psi) into the history
     if ((rc = nrqh::ensure_hist(h, cn->history_depth))) return rc;
     ProfScope ps(ctx, 1, (double)V * (1152.0 * 3 + 576.0));
     nrq::launch_hist_store(72 * V, cn->x, cn->b, h->P, hist_next(h), st);
@@ -1880,6 +1904,10 @@ static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const n
       break;
     }
     // steps: every column's bound within 0.9 of the tolerance, rounding aside
+    // (0.1 while the field's history fills: the first updates from a source,
+    // whose error sits on the few sites the field has reached, where the
+    // tolerance leaves it room)
+    const double aim = cn->history_guess && h->hist_count < cn->history_depth && cn->tol > 1e-13 ? 0.1 : 0.9;
     ChebSeg seg[2];
     bool finite = true;
     for (int sp = 0; sp < 2; ++sp) {
@@ -1896,7 +1924,7 @@ static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const n
       for (m = 1; m <= nrq::kChebTab; ++m) {
         bound = std::max(worst[0] / cheb_gain(seg[0].sigma, m), worst[1] / cheb_gain(seg[1].sigma, m)) +
                 8.0 * DBL_EPSILON;
-        if (bound <= 0.9 * cn->tol) break;
+        if (bound <= aim * cn->tol) break;
       }
     if (!finite || m > nrq::kChebTab || its + m > cn->maxits) {
       if (its == 0) return false;  // x0 is still in cn->x

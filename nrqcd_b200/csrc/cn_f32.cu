@@ -5,7 +5,7 @@
 // Inner solver: Chebyshev iteration for A^H e = r.  With real Wilson
 // coefficients A^H = 1 + i tau H, H hermitian (cn.cu), so the spectrum of A^H
 // lies on the segment {1 + i tau lambda : lambda in [lo, hi]}, which
-// k_cn_bounds encloses per step (block Gershgorin).  With centre theta and
+// k_spin_bounds (cn_spin.cu) encloses per step (block Gershgorin).  With centre theta and
 // half-length delta of that segment, sigma = theta/delta, rho_0 = 1/sigma,
 // d_0 = r_0/theta and
 //   e_{k+1} = e_k + d_k,   r_{k+1} = r_k - A^H d_k,
@@ -80,131 +80,6 @@ __global__ void k_cn_to_f32(int64_t V, const double2 *__restrict__ U, const doub
     D32[(int64_t)k * V + s] = make_float2((float)v.x, (float)v.y);
     B32[(int64_t)k * V + s] = (float)B[(int64_t)k * V + s];
   }
-}
-
-// ------------------------------------------------------------------ spectral bounds
-// Per site and species: lower/upper Gershgorin ends of the hermitian H with
-// A^H = 1 + i tau H (real coefficients r_t = Im(conj(alpha_t)) / tau).
-// partials[b*4 + {0,1,2,3}] = {min lo_q, max hi_q, min lo_a, max hi_a}.
-// bound on the spectral norm of a near-unitary link: sqrt of the largest
-// absolute row sum of U^+ U (Gershgorin)
-__device__ __forceinline__ double link_norm(const double2 *M, int64_t V, int64_t y) {
-  cplx u[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) u[k] = ldg(M + (int64_t)k * V + y);
-  double mx = 0.0;
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    double row = 0.0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      cplx a = {0.0, 0.0};
-#pragma unroll
-      for (int k = 0; k < 3; ++k) cmac_cj(a, u[k * 3 + r], u[k * 3 + c]);
-      row += hypot(a.re, a.im);
-    }
-    mx = fmax(mx, row);
-  }
-  return sqrt(mx);
-}
-
-__device__ __forceinline__ double frob(const double2 *M, int64_t V, int64_t y) {
-  double s = 0.0;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    double2 v = __ldg(M + (int64_t)k * V + y);
-    s += v.x * v.x + v.y * v.y;
-  }
-  return sqrt(s);
-}
-
-__global__ void __launch_bounds__(256) k_cn_bounds(Lat L, CnCoef C, double tau, const double2 *__restrict__ U,
-                                                   const double2 *__restrict__ Dsum, const double *__restrict__ Bsum,
-                                                   const double2 *__restrict__ DE, double *partials) {
-  int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double v[4] = {1e300, -1e300, 1e300, -1e300};
-  if (x < L.V) {
-    const int64_t V = L.V;
-    // neighbour block norms are species independent up to the coefficients
-    double nU[6], nDE[6];
-    for (int i = 0; i < 3; ++i) {
-      const int64_t xm = nb(L, x, i, -1);
-      nU[2 * i] = link_norm(U + (int64_t)(i * 9) * V, V, x);
-      nU[2 * i + 1] = link_norm(U + (int64_t)(i * 9) * V, V, xm);
-      nDE[2 * i] = frob(DE + (int64_t)((i * 2) * 9) * V, V, x) + frob(DE + (int64_t)((i * 2 + 1) * 9) * V, V, x);
-      nDE[2 * i + 1] = frob(DE + (int64_t)((i * 2) * 9) * V, V, xm) + frob(DE + (int64_t)((i * 2 + 1) * 9) * V, V, xm);
-    }
-    for (int sp = 0; sp < 2; ++sp) {
-      // conj(alpha) = i tau r  ->  r = Im(conj(alpha)) / tau
-      const double rk = C.kin[sp].im / tau, rm = C.mag[sp].im / tau, rd = C.dar[sp].im / tau,
-                   rs = C.so[sp].im / tau;
-      // diagonal colour block rk*dkin 1 + rd D^T + rm B (hermitian)
-      double M_re[9], M_im[9];
-      for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c) {
-          double2 dv = __ldg(Dsum + (int64_t)(c * 3 + r) * V + x);  // D^T[r][c]
-          double bv = __ldg(Bsum + (int64_t)(c * 3 + r) * V + x);
-          M_re[r * 3 + c] = rd * dv.x + rm * bv + (r == c ? rk * C.dkin : 0.0);
-          M_im[r * 3 + c] = rd * dv.y;
-        }
-      const double cen = (M_re[0] + M_re[4] + M_re[8]) / 3.0;
-      double dev = 0.0;
-      for (int k = 0; k < 9; ++k) {
-        const double re = M_re[k] - ((k % 4 == 0) ? cen : 0.0);
-        dev += re * re + M_im[k] * M_im[k];
-      }
-      double R = sqrt(dev);
-      for (int n = 0; n < 6; ++n) R += fabs(rk) * 0.5 * C.inva2[n / 2] * nU[n] + fabs(rs) * nDE[n];
-      R *= 1.0 + 1e-9;
-      v[2 * sp] = cen - R;
-      v[2 * sp + 1] = cen + R;
-    }
-  }
-  __shared__ double sh[8][4];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    v[0] = fmin(v[0], __shfl_down_sync(0xffffffffu, v[0], o));
-    v[1] = fmax(v[1], __shfl_down_sync(0xffffffffu, v[1], o));
-    v[2] = fmin(v[2], __shfl_down_sync(0xffffffffu, v[2], o));
-    v[3] = fmax(v[3], __shfl_down_sync(0xffffffffu, v[3], o));
-  }
-  if (lane == 0)
-    for (int k = 0; k < 4; ++k) sh[warp][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a[4] = {1e300, -1e300, 1e300, -1e300};
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      a[0] = fmin(a[0], sh[w][0]);
-      a[1] = fmax(a[1], sh[w][1]);
-      a[2] = fmin(a[2], sh[w][2]);
-      a[3] = fmax(a[3], sh[w][3]);
-    }
-    for (int k = 0; k < 4; ++k) partials[blockIdx.x * 4 + k] = a[k];
-  }
-}
-
-__global__ void k_cn_bounds_final(const double *__restrict__ partials, int64_t nblk, double *out) {
-  __shared__ double sh[4][256];
-  double a[4] = {1e300, -1e300, 1e300, -1e300};
-  for (int64_t b = threadIdx.x; b < nblk; b += blockDim.x) {
-    a[0] = fmin(a[0], partials[b * 4]);
-    a[1] = fmax(a[1], partials[b * 4 + 1]);
-    a[2] = fmin(a[2], partials[b * 4 + 2]);
-    a[3] = fmax(a[3], partials[b * 4 + 3]);
-  }
-  for (int k = 0; k < 4; ++k) sh[k][threadIdx.x] = a[k];
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      sh[0][threadIdx.x] = fmin(sh[0][threadIdx.x], sh[0][threadIdx.x + w]);
-      sh[1][threadIdx.x] = fmax(sh[1][threadIdx.x], sh[1][threadIdx.x + w]);
-      sh[2][threadIdx.x] = fmin(sh[2][threadIdx.x], sh[2][threadIdx.x + w]);
-      sh[3][threadIdx.x] = fmax(sh[3][threadIdx.x], sh[3][threadIdx.x + w]);
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x < 4) out[threadIdx.x] = sh[threadIdx.x][0];
 }
 
 // ------------------------------------------------------------------ FP32 Chebyshev step
@@ -448,12 +323,6 @@ __global__ void k_add_e(int64_t n, double2 *__restrict__ X, const float2 *__rest
 void launch_cn_to_f32(int64_t V, const double2 *U, const double2 *DE, const double2 *D, const double *B, float2 *U32,
                       float2 *DE32, float2 *D32, float *B32, cudaStream_t st) {
   k_cn_to_f32<<<(unsigned)((V + 255) / 256), 256, 0, st>>>(V, U, DE, D, B, U32, DE32, D32, B32);
-}
-void launch_cn_bounds(Lat L, const CnCoef &C, double tau, const double2 *U, const double2 *Dsum, const double *Bsum,
-                      const double2 *DE, double *partials, double *out, cudaStream_t st) {
-  const int64_t nblk = (L.V + 255) / 256;
-  k_cn_bounds<<<(unsigned)nblk, 256, 0, st>>>(L, C, tau, U, Dsum, Bsum, DE, partials);
-  k_cn_bounds_final<<<1, 256, 0, st>>>(partials, nblk, out);
 }
 void launch_cheb32(bool first, Lat L, const CnCoef &C, const float2 *U, const float2 *Dsum, const float *Bsum,
                    const float2 *DE, const float2 *D, float2 *Dn, float2 *R, float2 *E, const ChebCoef &K,

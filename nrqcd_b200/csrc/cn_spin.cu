@@ -21,12 +21,14 @@
 // 18 steps (neighbour, input colour) each take nine matrix entries and four
 // spinor entries, 96 FP64 FMAs on 13 16-byte loads; three further steps take
 // the site term.  The matrices of a neighbour are staged in shared memory by
-// all six warps (cp.async, three buffers, one mbarrier per neighbour: a warp
-// that sees the matrices of neighbour n landed knows that every warp has
-// left neighbour n - 2, so the third buffer is free), and the spinors go
-// straight to registers two steps ahead.  Nothing depends on the lattice's
+// all six warps (cp.async, one mbarrier per neighbour, two neighbours ahead:
+// a warp that sees the matrices of neighbour n landed knows that every warp
+// has left neighbour n - 3, so a fifth buffer is free), and the spinors go
+// straight to registers three steps ahead.  Nothing depends on the lattice's
 // shape: each lane reads its own neighbours' addresses, so one kernel serves
-// rows of any length, and small lattices get one block per 32 sites.
+// rows of any length, and small lattices get one block per 32 sites.  In a
+// batch the blocks run over (field, unit).  The device code is in
+// cn_spin.cuh.
 //
 // Bound: 64^3, the solver's step (four vector streams, 6.1 KB a site): 0.25 ms
 // at the copy rate, 0.21 ms at the FP64 rate that FMAs with distinct operands
@@ -44,9 +46,8 @@
 #include <algorithm>
 
 #include "../../include/nrqcd_b200.h"
+#include "cn_spin.cuh"
 #include "nrq_eigen.cuh"
-#include "nrq_kernels.cuh"
-#include "stage.cuh"
 
 namespace nrq {
 
@@ -122,7 +123,8 @@ constexpr int kPrepSites = 32;
 }  // namespace
 
 // Builds the operator of the nm coefficient sets Cm (null: the one set C1),
-// from the links and the electric field: W (81 planes of V complex per set,
+// from the links and the electric field, in FP64 (op) and rounded to FP32
+// (op32), either left out where its pointers are null: W (81 planes of V complex per set,
 // (I*3 + m)*9 + row*3 + column), S0 (9 planes, row*3 + column), S1 (9 real
 // planes) and, for the spectral enclosure, seven real planes per set: the
 // norm bound of the block to x + I (I = 0..2), and centre and deviation of
@@ -133,7 +135,7 @@ constexpr int kPrepSites = 32;
 __global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C1, const CnCoef *__restrict__ Cm,
                                                                 int nm, double tau, const double2 *__restrict__ U,
                                                                 const double *__restrict__ E, SpinOp op,
-                                                                double *__restrict__ scratch) {
+                                                                SpinOp32 op32, double *__restrict__ scratch) {
   __shared__ double sD[3][9][kPrepSites];  // Darwin: 0..2 the diagonal, then 01, 02, 12 as (re, im)
   __shared__ double sB[3][6][kPrepSites];
   const int l = threadIdx.x % kPrepSites, i = threadIdx.x / kPrepSites;
@@ -204,7 +206,9 @@ __global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C
   if (!act) return;
   for (int km = 0; km < nm; ++km) {
     const CnCoef &C = Cm ? Cm[km] : C1;
-    double2 *W = op.W + (int64_t)km * 81 * V + (int64_t)(i * 27) * V + x;
+    const int64_t ow = (int64_t)km * 81 * V + (int64_t)(i * 27) * V + x;
+    double2 *W = op.W + ow;
+    float2 *Wf = op32.W + ow;
     const cplx ck = (-0.5 * C.inva2[i]) * C.kin[0];
     const cplx c0 = times_i(C.so[0]), c1 = -times_i(C.so[0]);
 #pragma unroll
@@ -227,9 +231,16 @@ __global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C
           b = times_i(e0) + e1;
           o = e1 - times_i(e0);
         }
-        st(W + (int64_t)(r * 3 + c) * V, a);
-        st(W + (int64_t)(9 + r * 3 + c) * V, b);
-        st(W + (int64_t)(18 + r * 3 + c) * V, o);
+        if (op.W) {
+          st(W + (int64_t)(r * 3 + c) * V, a);
+          st(W + (int64_t)(9 + r * 3 + c) * V, b);
+          st(W + (int64_t)(18 + r * 3 + c) * V, o);
+        }
+        if (op32.W) {
+          Wf[(int64_t)(r * 3 + c) * V] = make_float2((float)a.re, (float)a.im);
+          Wf[(int64_t)(9 + r * 3 + c) * V] = make_float2((float)b.re, (float)b.im);
+          Wf[(int64_t)(18 + r * 3 + c) * V] = make_float2((float)o.re, (float)o.im);
+        }
       }
     // S0 = Im(dar) D^T, S1 = Im(mag) B + Im(kin) sum 1/a^2
     const double dd = C.dar[0].im, mm = C.mag[0].im, kk = C.kin[0].im * C.dkin;
@@ -247,8 +258,16 @@ __global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C
       double bv = B[0];
 #pragma unroll
       for (int e = 1; e < 6; ++e) bv = q == e ? B[e] : bv;
-      st(op.S0 + (int64_t)km * 9 * V + (int64_t)(i * 3 + c) * V + x, dd * v);
-      op.S1[(int64_t)km * 9 * V + (int64_t)(i * 3 + c) * V + x] = mm * bv + (i == c ? kk : 0.0);
+      const int64_t os = (int64_t)km * 9 * V + (int64_t)(i * 3 + c) * V + x;
+      const double b1 = mm * bv + (i == c ? kk : 0.0);
+      if (op.W) {
+        st(op.S0 + os, dd * v);
+        op.S1[os] = b1;
+      }
+      if (op32.W) {
+        op32.S0[os] = make_float2((float)(dd * v.re), (float)(dd * v.im));
+        op32.S1[os] = (float)b1;
+      }
     }
     if (scratch) {
       double *s = scratch + (int64_t)km * 7 * V + x;
@@ -350,244 +369,73 @@ __global__ void __launch_bounds__(256) k_spin_bounds(Lat L, const double *__rest
 }
 
 // ------------------------------------------------------------------ stencil
-namespace {
-constexpr int kUnit = 32;   // sites of a block, one per lane
-constexpr int kWarps = 6;   // one propagator column of both species each
-// Spinor operands in registers: this step's and the next three's; matrices
-// staged two neighbours ahead.  (64^3, a coupled step: 4.16 ms with the next
-// two and one neighbour, 4.09 with the next three, 3.98 with both.  Prefetches
-// to L2, of the epilogue's operands or of later units', cost 2-20 %; a
-// persistent form with the next unit's first loads issued early 10 %.)
-constexpr int kAhead = 4;
-constexpr int kWBufs = 5;
-
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-// arrives on bar once this thread's copies so far have landed
-__device__ __forceinline__ void cp_async_arrive(uint64_t *bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// acc += +-(w or conj(w)) p in halves: the products with Re w, then those
-// with Im w, so that consecutive FMAs share an operand register (an FP64 FMA
-// with three fresh operands issues every 2.7 cycles, with one reused 2.3)
-template <int S>
-__device__ __forceinline__ void smac_re(cplx &acc, const double2 w, const double2 p) {
-  const double wr = S > 0 ? w.x : -w.x;
-  acc.re = fma(wr, p.x, acc.re);
-  acc.im = fma(wr, p.y, acc.im);
-}
-template <int S, bool CJ>
-__device__ __forceinline__ void smac_im(cplx &acc, const double2 w, const double2 p) {
-  const double wi = (S > 0) == !CJ ? w.y : -w.y;
-  acc.re = fma(-wi, p.y, acc.re);
-  acc.im = fma(wi, p.x, acc.im);
-}
-template <int SA, int SB, bool CJ>
-__device__ __forceinline__ void smac2(const double2 w, cplx &a, const double2 p, cplx &b, const double2 q) {
-  smac_re<SA>(a, w, p);
-  smac_re<SB>(b, w, q);
-  smac_im<SA, CJ>(a, w, p);
-  smac_im<SB, CJ>(b, w, q);
-}
-template <int SA, int SB, bool CJ>
-__device__ __forceinline__ void smac4(const double2 w, cplx &a, const double2 p, cplx &b, const double2 q, cplx &c,
-                                      const double2 r, cplx &d, const double2 s) {
-  smac_re<SA>(a, w, p);
-  smac_re<SA>(b, w, q);
-  smac_re<SB>(c, w, r);
-  smac_re<SB>(d, w, s);
-  smac_im<SA, CJ>(a, w, p);
-  smac_im<SA, CJ>(b, w, q);
-  smac_im<SB, CJ>(c, w, r);
-  smac_im<SB, CJ>(d, w, s);
-}
-
-// One step: direction I, forward (B = false) or backward, one input colour.
-// m[t][i]: entry (i, j) of matrix t, backward entry (j, i) of the
-// neighbour's; q = the input entries (quark spin 0, 1, antiquark spin 0, 1);
-// a[species*2 + spin][i] the output colours.
-template <int I, bool B>
-__device__ __forceinline__ void spin_products(cplx (&a)[4][3], const double2 (&m)[3][3], const double2 (&q)[4]) {
-  constexpr int S = B ? -1 : 1;
-  // signs of the off-diagonal blocks (upper right, lower left), I < 2
-  constexpr int S01 = I == 0 ? 1 : S, S10 = I == 0 ? -1 : S;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (I < 2) smac2<S, -S, B>(m[0][i], a[0][i], q[0], a[3][i], q[3]);
-    if (I < 2) smac2<S, -S, B>(m[1][i], a[1][i], q[1], a[2][i], q[2]);
-  }
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    if (I < 2) {
-      smac4<S01, S10, B>(m[2][i], a[0][i], q[1], a[2][i], q[3], a[1][i], q[0], a[3][i], q[2]);
-    } else {
-      smac4<S, -S, B>(m[0][i], a[0][i], q[0], a[1][i], q[1], a[2][i], q[2], a[3][i], q[3]);
-      smac2<S, S, B>(m[B ? 1 : 2][i], a[0][i], q[1], a[2][i], q[3]);
-      smac2<S, S, B>(m[B ? 2 : 1][i], a[1][i], q[0], a[3][i], q[2]);
-    }
-  }
-}
-
-// First site of work unit u.  Where every row holds whole units (nx a
-// multiple of 32) and ny, nz are multiples of 8, the units are taken in
-// blocks of 8 x 8 rows (x fastest, then y and z within the block), so that
-// the +-y and +-z neighbours of a unit are read within a few hundred units
-// of it, while L2 still holds them (in site order the +-z neighbours are a
-// plane apart: 100 MB of loads at 128^3); otherwise in site order.
-__device__ __forceinline__ int unit_start(const Lat &L, int u) {
-  const int nx = (int)L.nx, ny = (int)L.ny, nz = (int)L.nz;
-  if ((nx & 31) || (ny & 7) || (nz & 7)) return u * kUnit;
-  const int nxu = nx >> 5;
-  int t = u / nxu;
-  const int cx = (u - t * nxu) << 5;
-  const int yi = t & 7, zi = (t >> 3) & 7;
-  t >>= 6;
-  const int nby = ny >> 3;
-  const int bz = t / nby, by = t - bz * nby;
-  return cx + nx * ((by << 3) + yi + ny * ((bz << 3) + zi));
-}
-
-// the six periodic neighbours (+x,-x,+y,-y,+z,-z) of site x (V < 2^31)
-__device__ __forceinline__ void neighbours(const Lat &L, int x, int (&nbr)[6]) {
-  const int nx = (int)L.nx, ny = (int)L.ny, nz = (int)L.nz, nxy = nx * ny, V = (int)L.V;
-  const int t = x / nx, px = x - t * nx, pz = t / ny, py = t - pz * ny;
-  nbr[0] = px + 1 < nx ? x + 1 : x + 1 - nx;
-  nbr[1] = px > 0 ? x - 1 : x - 1 + nx;
-  nbr[2] = py + 1 < ny ? x + nx : x + nx - nxy;
-  nbr[3] = py > 0 ? x - nx : x - nx + nxy;
-  nbr[4] = pz + 1 < nz ? x + nxy : x + nxy - V;
-  nbr[5] = pz > 0 ? x - nxy : x - nxy + V;
-}
-
-struct SpinSmem {
-  double2 w[kWBufs][27][kUnit];
-  double2 s0[9][kUnit];
-  double s1[9][kUnit];
-  uint64_t full[6];  // the matrices of neighbour n (and, n = 0, the site term) landed
-};
-
-// y = A^H in of the warp's column c at the lane's site x: acc[species*2 +
-// spin][colour]; own[colour] = the input at x itself.  Returns false where a
-// wait ran out.
-__device__ __forceinline__ bool spin_apply(const Lat &L, const double2 *__restrict__ W, const double2 *__restrict__ S0,
-                                           const double *__restrict__ S1, const double2 *__restrict__ in, int x, int c,
-                                           SpinSmem &sm, int *err, long long wait_cycles, int stall_load,
-                                           cplx (&acc)[4][3], double2 (&own)[kAhead][4]) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t V = L.V;
-  int nbr[6];
-  neighbours(L, x, nbr);
-  auto stage = [&](int n) {
-    if (stall_load >= 0 && n >= stall_load) return;
-    const double2 *w = W + (int64_t)((n >> 1) * 27) * V + ((n & 1) ? nbr[n] : x);
-    for (int p = warp; p < 27; p += kWarps) cp_async16(smem_u32(&sm.w[n % kWBufs][p][lane]), w + (int64_t)p * V);
-    if (n == 0)
-      for (int p = warp; p < 9; p += kWarps) {
-        cp_async16(smem_u32(&sm.s0[p][lane]), S0 + (int64_t)p * V + x);
-        cp_async8(smem_u32(&sm.s1[p][lane]), S1 + (int64_t)p * V + x);
-      }
-    cp_async_arrive(&sm.full[n]);
-  };
-  // operand of step t: neighbour t / 3 (18 and on: the site itself), input
-  // colour t % 3
-  const double2 *pq = in + (int64_t)(6 * c) * V, *pa = in + (int64_t)(36 + 6 * c) * V;
-  auto load = [&](int t, double2 (&q)[4]) {
-    const int y = t < 18 ? nbr[t / 3] : x;
-    const int64_t o = (int64_t)(2 * (t % 3)) * V + y;
-    q[0] = __ldg(pq + o);
-    q[1] = __ldg(pq + o + V);
-    q[2] = __ldg(pa + o);
-    q[3] = __ldg(pa + o + V);
-  };
-  stage(0);
-#pragma unroll
-  for (int t = 0; t < kAhead - 1; ++t) load(t, own[t]);
-  stage(1);
-#pragma unroll
-  for (int s = 0; s < 4; ++s)
-#pragma unroll
-    for (int i = 0; i < 3; ++i) acc[s][i] = {0.0, 0.0};
-  bool ok = true;
-#pragma unroll
-  for (int n = 0; n < 6; ++n) {
-    if (ok && !mbar_try_wait(&sm.full[n], 0)) {
-      const long long t0 = clock64();
-      while (ok && !mbar_try_wait(&sm.full[n], 0)) ok = clock64() - t0 <= wait_cycles;
-      if (!ok) record_timeout(err, 5, 0, n);
-    }
-    if (!__all_sync(0xffffffffu, ok)) return false;
-    // every warp issued its copies of n when it entered neighbour n - 2, so
-    // all have left n - 3, whose buffer n + 2 takes
-    if (n + 2 < 6) stage(n + 2);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int t = 3 * n + j;
-      if (t + kAhead - 1 < 21) load(t + kAhead - 1, own[(t + kAhead - 1) % kAhead]);
-      double2 m[3][3];
-#pragma unroll
-      for (int t3 = 0; t3 < 3; ++t3)
-#pragma unroll
-        for (int i = 0; i < 3; ++i) m[t3][i] = sm.w[n % kWBufs][t3 * 9 + ((n & 1) ? 3 * j + i : 3 * i + j)][lane];
-      const double2 (&q)[4] = own[t % kAhead];
-      if (n == 0) spin_products<0, false>(acc, m, q);
-      if (n == 1) spin_products<0, true>(acc, m, q);
-      if (n == 2) spin_products<1, false>(acc, m, q);
-      if (n == 3) spin_products<1, true>(acc, m, q);
-      if (n == 4) spin_products<2, false>(acc, m, q);
-      if (n == 5) spin_products<2, true>(acc, m, q);
-    }
-  }
-  // the site term
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const double2 (&q)[4] = own[(18 + j) % kAhead];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      acc[s][j].re += q[s].x;
-      acc[s][j].im += q[s].y;
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double2 d = sm.s0[i * 3 + j][lane];
-      const double b = sm.s1[i * 3 + j][lane];
-      const double gq = d.x + b, ga = d.x - b;
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {  // += i (g + i d.y) q
-        const double g = s < 2 ? gq : ga;
-        acc[s][i].re = fma(-g, q[s].y, fma(-d.y, q[s].x, acc[s][i].re));
-        acc[s][i].im = fma(g, q[s].x, fma(-d.y, q[s].y, acc[s][i].im));
-      }
-    }
-  }
-  return true;
-}
-}  // namespace
-
 // One application of the operator (sign = +1: A^H, -1: A = 2 - A^H) to the 12
 // columns, with the mode's vector work at the own site (MvMode); partial sums
 // in one row per block: partials[(block*12 + column)*NQ + q].
-template <int MODE>
-__global__ void __launch_bounds__(kUnit *kWarps, 2)
-    k_cn_spin(Lat L, SpinOp op, double sign, MvArgs A, int *err, long long wait_cycles, int stall_load) {
-  extern __shared__ __align__(16) unsigned char raw_[];
-  SpinSmem &sm = *reinterpret_cast<SpinSmem *>(raw_);
+//
+// BATCH (MV_RHS, MV_RESC): the fields of the device table, each on its own
+// coefficient set, blocks over (field, unit); MV_RHS adds the field's history
+// to its start and keeps the added part in hnew, MV_RESC skips fields that
+// have converged (skip_done).
+struct SpinBatch {
+  const BatchField *tab;
+  int nf, nunits, order, skip_done, want_d;
+};
+template <int MODE, bool BATCH>
+__global__ void __launch_bounds__(spin::kUnit *spin::kWarps, 2)
+    k_cn_spin(Lat L, SpinOp op, double sign, MvArgs A, SpinBatch Bt, int *err, long long wait_cycles, int stall_load) {
+  using namespace spin;
+  constexpr int kAhead = Num<double>::kAhead;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem<double> &sm = *reinterpret_cast<Smem<double> *>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x < 6) mbar_init(&sm.full[threadIdx.x], kUnit * kWarps);
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  __syncthreads();
   const int V = (int)L.V;
-  const int s = unit_start(L, (int)blockIdx.x) + lane;
+  int u = (int)blockIdx.x;
+  const BatchField *F = nullptr;
+  if (BATCH) {
+    int f;
+    batch_item(Bt.nf, Bt.nunits, Bt.order, f, u);
+    F = Bt.tab + f;
+    if (MODE == MV_RESC && Bt.skip_done && batch_field_done(*F)) return;
+    op.W += (int64_t)F->wblk * 81 * V;
+    op.S0 += (int64_t)F->wblk * 9 * V;
+    op.S1 += (int64_t)F->wblk * 9 * V;
+    if (MODE == MV_RHS) {
+      A.in = F->psi;
+      A.out = F->b;
+      A.out2 = F->x;
+      A.hist[0] = A.hist[1] = A.hist[2] = A.hist[3] = nullptr;
+      A.r32 = nullptr;
+      if (F->hstart) {
+        A.hist[0] = F->h1;
+        A.hist[1] = F->h2;
+        A.hist[2] = F->h3;
+        A.hist[3] = F->h4;
+        A.r32 = F->hnew;
+        // the degree d - 1 extrapolation of d vectors
+        const int d = F->h4 ? 4 : F->h3 ? 3 : F->h2 ? 2 : 1;
+        A.hcoef[0] = d;
+        A.hcoef[1] = d == 4 ? -6.0 : d == 3 ? -3.0 : -1.0;
+        A.hcoef[2] = d == 4 ? 4.0 : 1.0;
+        A.hcoef[3] = -1.0;
+      }
+    } else {
+      A.in = F->x;
+      A.bvec = F->b;
+      A.r32 = F->r32;
+      A.d32 = Bt.want_d ? F->dA : nullptr;
+      A.inv_theta[0] = F->inv_theta[0];
+      A.inv_theta[1] = F->inv_theta[1];
+      A.partials = F->partials;
+    }
+  }
+  init_barriers(sm);
+  const int s = unit_start(L, u) + lane;
   const bool act = s < V;
   const int x = act ? s : V - 1;  // a valid site for the addresses of idle lanes
-  cplx acc[4][3];
+  cx<double> acc[4][3];
   double2 own[kAhead][4];
-  const bool ok = spin_apply(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, stall_load, acc, own);
+  const bool ok = apply<double>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, stall_load, acc, own);
   cp_async_wait_all();
   constexpr int NQ = MODE == MV_T2 ? 5 : MODE == MV_RES2 ? 4 : MODE == MV_T ? 3
                    : (MODE == MV_RES || MODE == MV_V || MODE == MV_V2 || MODE == MV_RESC || MODE == MV_CH0 ||
@@ -628,7 +476,7 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
         if (MODE == MV_RHS)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            if (A.hist[k]) f[h & 1][r][k] = __ldg(A.hist[k] + o);
+            if (A.hist[k]) f[h & 1][r][k] = A.hist[k][o];  // one of them may be r32
       }
     };
     fetch(0);
@@ -645,21 +493,25 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
         const cplx in = {ow.x, ow.y};
         const cplx ev = e1[h & 1][r];
         const float2 fv = f[h & 1][r][0];
-        cplx y = acc[2 * sp + sr][i];
+        // (A^H - 1) in; the residuals subtract the input first, which leaves
+        // the smaller numbers' rounding
+        const cplx nv = {acc[2 * sp + sr][i].re, acc[2 * sp + sr][i].im};
+        cplx y = in + nv;
         if (MODE == MV_PLAIN || MODE == MV_RHS)
-          if (sign < 0.0) y = 2.0 * in - y;
+          if (BATCH || sign < 0.0) y = in - nv;
         if (MODE == MV_PLAIN) {
           st(A.out + o, y);
         } else if (MODE == MV_RHS) {
           st(A.out + o, y);
-          cplx x0 = 2.0 * y - in;
+          cplx dx = {0.0, 0.0};
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             if (A.hist[k]) {
-              x0.re = fma(A.hcoef[k], (double)f[h & 1][r][k].x, x0.re);
-              x0.im = fma(A.hcoef[k], (double)f[h & 1][r][k].y, x0.im);
+              dx.re = fma(A.hcoef[k], (double)f[h & 1][r][k].x, dx.re);
+              dx.im = fma(A.hcoef[k], (double)f[h & 1][r][k].y, dx.im);
             }
-          st(A.out2 + o, x0);
+          st(A.out2 + o, 2.0 * y - in + dx);
+          if (A.r32) A.r32[o] = make_float2((float)dx.re, (float)dx.im);
         } else if (MODE == MV_V || MODE == MV_V2) {
           st(A.out + o, y);
           const cplx rh = MODE == MV_V ? ev : cplx{(double)fv.x, (double)fv.y};
@@ -681,7 +533,7 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
             qs[sp][4] += t.im;
           }
         } else {
-          const cplx rv = ev - y;
+          const cplx rv = (ev - in) - nv;
           if (MODE == MV_RES) {
             st(A.out + o, rv);
             st(A.out2 + o, rv);
@@ -727,7 +579,7 @@ __global__ void __launch_bounds__(kUnit *kWarps, 2)
         double v = qs[sp][k];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) A.partials[((int64_t)blockIdx.x * CN_COLS + sp * 6 + warp) * NQ + k] = v;
+        if (lane == 0) A.partials[((int64_t)u * CN_COLS + sp * 6 + warp) * NQ + k] = v;
       }
   }
 }
@@ -765,9 +617,9 @@ __global__ void k_cheb_tab(const double *__restrict__ bounds, double tau, ChebTa
 
 // ------------------------------------------------------------------ host
 void launch_spin_prepare(Lat L, const CnCoef &C, const CnCoef *Cm, int nm, double tau, const double2 *U,
-                         const double *E, const SpinOp &op, double *scratch, cudaStream_t st) {
+                         const double *E, const SpinOp &op, const SpinOp32 &op32, double *scratch, cudaStream_t st) {
   const unsigned grid = (unsigned)((L.V + kPrepSites - 1) / kPrepSites);
-  k_spin_prepare<<<grid, kPrepSites * 3, 0, st>>>(L, C, Cm, nm, tau, U, E, op, scratch);
+  k_spin_prepare<<<grid, kPrepSites * 3, 0, st>>>(L, C, Cm, nm, tau, U, E, op, op32, scratch);
 }
 
 void launch_spin_bounds(Lat L, int nm, const double *scratch, double *partials, unsigned *ticket, double *out,
@@ -783,26 +635,44 @@ bool cn_spin_applicable(const Lat &L) { return L.V <= 0x7fffffffLL; }
 
 void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs &a, int *err, cudaStream_t st,
                     long long wait_cycles, int stall_load) {
+  using namespace spin;
   const unsigned grid = (unsigned)((L.V + kUnit - 1) / kUnit);
   auto go = [&](auto kern) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SpinSmem));
-    kern<<<grid, kUnit * kWarps, sizeof(SpinSmem), st>>>(L, op, sign, a, err, wait_cycles, stall_load);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<double>));
+    kern<<<grid, kUnit * kWarps, sizeof(Smem<double>), st>>>(L, op, sign, a, SpinBatch{}, err, wait_cycles,
+                                                            stall_load);
   };
   switch (mode) {
-    case MV_PLAIN: go(k_cn_spin<MV_PLAIN>); break;
-    case MV_RHS: go(k_cn_spin<MV_RHS>); break;
-    case MV_RES: go(k_cn_spin<MV_RES>); break;
-    case MV_V: go(k_cn_spin<MV_V>); break;
-    case MV_T: go(k_cn_spin<MV_T>); break;
-    case MV_RESC: go(k_cn_spin<MV_RESC>); break;
-    case MV_T2: go(k_cn_spin<MV_T2>); break;
-    case MV_RES2: go(k_cn_spin<MV_RES2>); break;
-    case MV_V2: go(k_cn_spin<MV_V2>); break;
-    case MV_RESN: go(k_cn_spin<MV_RESN>); break;
-    case MV_CH0: go(k_cn_spin<MV_CH0>); break;
-    case MV_CHK: go(k_cn_spin<MV_CHK>); break;
-    default: go(k_cn_spin<MV_CHH>); break;
+    case MV_PLAIN: go(k_cn_spin<MV_PLAIN, false>); break;
+    case MV_RHS: go(k_cn_spin<MV_RHS, false>); break;
+    case MV_RES: go(k_cn_spin<MV_RES, false>); break;
+    case MV_V: go(k_cn_spin<MV_V, false>); break;
+    case MV_T: go(k_cn_spin<MV_T, false>); break;
+    case MV_RESC: go(k_cn_spin<MV_RESC, false>); break;
+    case MV_T2: go(k_cn_spin<MV_T2, false>); break;
+    case MV_RES2: go(k_cn_spin<MV_RES2, false>); break;
+    case MV_V2: go(k_cn_spin<MV_V2, false>); break;
+    case MV_RESN: go(k_cn_spin<MV_RESN, false>); break;
+    case MV_CH0: go(k_cn_spin<MV_CH0, false>); break;
+    case MV_CHK: go(k_cn_spin<MV_CHK, false>); break;
+    default: go(k_cn_spin<MV_CHH, false>); break;
   }
+}
+
+void launch_batch_spin(int mode, int order, Lat L, const SpinOp &op, const BatchField *tab, int nfields, int skip_done,
+                       bool want_d, int *err, cudaStream_t st, long long wait_cycles) {
+  using namespace spin;
+  const int nunits = (int)((L.V + kUnit - 1) / kUnit);
+  const SpinBatch bt{tab, nfields, nunits, order, skip_done, want_d ? 1 : 0};
+  auto go = [&](auto kern) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<double>));
+    kern<<<(unsigned)nunits * (unsigned)nfields, kUnit * kWarps, sizeof(Smem<double>), st>>>(
+        L, op, 1.0, MvArgs{}, bt, err, wait_cycles, -1);
+  };
+  if (mode == MV_RHS)
+    go(k_cn_spin<MV_RHS, true>);
+  else
+    go(k_cn_spin<MV_RESC, true>);
 }
 
 }  // namespace nrq

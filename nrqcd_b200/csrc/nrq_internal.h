@@ -203,12 +203,10 @@ struct nrq_cn {
   // the other stencils' per-step matrices (Dsum, Bsum, DE) follow the gauge
   // field on demand
   bool legacy_valid = false;
-  // the FP32 Chebyshev step of the precision forms: the same blocks rounded
-  // to FP32, and which step kernel runs (-1: k_cheb5f where it applies, else
-  // k_cheb32; NRQ_CHEB_* forces one); last_cheb: the one the last update ran
-  float2 *Wblk5f = nullptr;
-  bool w5f_valid = false;
-  nrq::CnCoef w5f_coef{};
+  // the FP32 Chebyshev step of the precision forms: the same operator rounded
+  // to FP32, and which step kernel runs (-1: the faster, NRQ_CHEB_* forces
+  // one); last_cheb: the one the last update ran
+  nrq::SpinOp32 spin32{};
   int cheb_stencil = -1;
   int last_cheb = -1;
   // the timed choice between the two steps (per-launch ms; -1 not timed)
@@ -219,8 +217,10 @@ struct nrq_cn {
   // test of the timeout path, the load its producer stops before (-1: none)
   long long wait_cycles = nrq_wait_cycles_default;
   int stall_load = -1;
-  // precision form (form 1): FP32 copies of the per-step matrices and the
-  // FP32 Chebyshev vectors; spectral bounds of the hermitian part
+  // precision form (form 1): FP32 copies of the per-step matrices for the
+  // register-tiled step (f32_valid: of the current gauge field) and the FP32
+  // Chebyshev vectors; spectral bounds of the hermitian part
+  bool f32_valid = false;
   float2 *U32 = nullptr, *DE32 = nullptr, *D32 = nullptr;
   float *B32 = nullptr;
   float2 *r32 = nullptr, *dA32 = nullptr, *dB32 = nullptr, *e32 = nullptr;

@@ -104,7 +104,8 @@ struct MvArgs {
   cplx inv_theta[2];
   float2 *sh32;       // RES2: FP32 shadow residual written; V2, T2: read
   // spin-structured stencil: the Chebyshev table and step; RHS: the history
-  // vectors added to x0 with their coefficients (null: none)
+  // vectors added to x0 with their coefficients (null: none), r32 the FP32
+  // copy of what they add (may be null, may be one of them)
   const ChebTab *cheb;
   int step;
   const float2 *hist[4];
@@ -134,11 +135,16 @@ struct SpinOp {
   double2 *W, *S0;
   double *S1;
 };
-// Builds op for nm coefficient sets (device array Cm; null: the one set C),
-// and seven real scratch planes a set for the spectral enclosure (null: none).
-// tau = dt a0 / 2.
+// the same planes rounded to FP32
+struct SpinOp32 {
+  float2 *W, *S0;
+  float *S1;
+};
+// Builds op and op32 (either left out where its W is null) for nm
+// coefficient sets (device array Cm; null: the one set C), and seven real
+// scratch planes a set for the spectral enclosure (null: none).  tau = dt a0 / 2.
 void launch_spin_prepare(Lat L, const CnCoef &C, const CnCoef *Cm, int nm, double tau, const double2 *U,
-                         const double *E, const SpinOp &op, double *scratch, cudaStream_t st);
+                         const double *E, const SpinOp &op, const SpinOp32 &op32, double *scratch, cudaStream_t st);
 // out[4*set] = {lo, hi} of the quark's and the antiquark's H, A^H = 1 + i tau
 // H; partials: 4 doubles per 256 sites and set; ticket: one zero per set
 void launch_spin_bounds(Lat L, int nm, const double *scratch, double *partials, unsigned *ticket, double *out,
@@ -198,14 +204,6 @@ int64_t cn_mv4_units(int64_t V);
 int64_t cn_mv4_rows(int64_t V, int sm_count);
 int launch_cn_mv4(int mode, Lat L, const CnCoef &C, double nb_sign, const double2 *W, const double2 *Dsum,
                   const double *Bsum, const MvArgs &a, int *err, int sm_count, cudaStream_t st);
-// launch_cn_blocks5 (cn_mv5.cu) writes the forward blocks as 216 planes
-// (direction, species, row, column; cn_mv5_block_entries complex in all) in
-// FP64 (W), rounded to FP32 (Wf), or both in one pass; a null pointer skips
-// that precision.
-void launch_cn_blocks5(Lat L, const CnCoef &C, const double2 *U, const double2 *DE, double2 *W, float2 *Wf,
-                       cudaStream_t st);
-int64_t cn_mv5_units(int64_t V);
-int64_t cn_mv5_block_entries(int64_t V);
 // finalize stages: 0 = after RES (rr, bb), 1 = alpha (rh.v), 2 = omega (t.s, t.t), 3 = beta (rh.r, r.r)
 void launch_cn_finalize(int stage, int64_t nblocks, const double *partials, double *scal, double tol,
                         cudaStream_t st);
@@ -220,7 +218,8 @@ struct BatchField {
   const double *bounds;          // spectral enclosure of this field's mass (lo0, hi0, lo1, hi1)
   double tau;                    // dt a0 / 2 (signed)
   double mass;                   // heavy mass of this field
-  int wblk;                      // the field's FP32 block set (its distinct mass)
+  int wblk;                      // the field's coefficient set (its distinct mass)
+  int hstart;                    // the field starts from the extrapolation of h1..h4
   // learned initial guess: the field's history (v1 newest, v2 older; null
   // when absent) and the slot the new history goes to (null: no learned guess)
   const float2 *h1, *h2;
@@ -245,25 +244,13 @@ __device__ __forceinline__ bool batch_field_done(const BatchField &f) {
 // fields alone (their iterate did not change since their last check)
 void launch_batch_mv(int mode, int order, Lat L, const double2 *U, const double2 *Dsum, const double *Bsum,
                      const double2 *DE, const BatchField *tab, int nfields, int skip_done, cudaStream_t st);
-// The same two modes (MV_RHS, MV_RESC) on the FP64 FMA stencil's blocks
-// (cn_batch_mv5.cu): W holds nblk block sets of 216 planes, one per distinct
-// mass, built with that mass's A^H coefficients (the field's wblk); fmaps[f]
-// the tensor maps of field f's psi and iterate x (written by
-// batch_mv5_field_maps before every step; device memory).  The residual's
-// partials are one row per (field, 32-site unit), the rows of
-// launch_batch_finalize.  Returns nonzero where it does not apply (V even,
-// at least 34 sites, V < 2^31).
-struct CnBatchMaps {
-  struct {
-    CUtensorMap spin;   // 72 planes x 2V doubles, box {68, 36}
-    CUtensorMap spin1;  // one site, box {2, 36}
-  } in[2];              // 0: psi, 1: the iterate x
-};
-bool batch_mv5_applicable(const Lat &L);
-bool batch_mv5_field_maps(CnBatchMaps *m, const Lat &L, const double2 *psi, const double2 *x);
-int launch_batch_mv5(int mode, int order, Lat L, const double2 *W, int nblk, const double2 *Dsum, const double *Bsum,
-                     const CnBatchMaps *fmaps, const BatchField *tab, int nfields, int skip_done, int *err,
-                     int sm_count, cudaStream_t st, long long wait_cycles);
+// The same two modes (MV_RHS, MV_RESC) on the operator in its spin structure
+// (cn_spin.cu), one coefficient set per distinct mass (the field's wblk).
+// MV_RHS adds the fields' history to their start and fills hnew (hstart);
+// MV_RESC writes d = r / theta only where want_d.  The residual's partials
+// are one row per (field, 32-site unit), the rows of launch_batch_finalize.
+void launch_batch_spin(int mode, int order, Lat L, const SpinOp &op, const BatchField *tab, int nfields, int skip_done,
+                       bool want_d, int *err, cudaStream_t st, long long wait_cycles);
 // Chebyshev kernel variants: 0 = one field per tile, 2 blocks/SM (168
 // registers); 1 = one field per tile, 3 blocks/SM (113 registers); 2 = two
 // fields of one mass per tile, 1 block/SM.  Returns nonzero for an
@@ -271,15 +258,13 @@ int launch_batch_mv5(int mode, int order, Lat L, const double2 *W, int nblk, con
 constexpr int BATCH_CHEB_VARIANTS = 4;
 int launch_batch_cheb(int step, int variant, int order, Lat L, const float2 *U, const float2 *Dsum,
                       const float *Bsum, const float2 *DE, const BatchField *tab, int nfields, cudaStream_t st);
-// Variant 3 of the batched Chebyshev step: the FP32 block step of
-// launch_cheb5f over every field (work items (field, unit), field fastest
-// for order 0), on the block sets Wf (nblk of 216 planes, one per distinct
-// mass, built with that mass's A^H coefficients) and the fields' d vectors
-// (dA_all / dB_all by the step's parity, 72 planes per field).  Returns
-// nonzero where it does not apply.
-int launch_batch_cheb5f(int step, int order, Lat L, const float2 *Wf, int nblk, const float2 *Dsum,
-                        const float *Bsum, const float2 *dA_all, const float2 *dB_all, const BatchField *tab,
-                        int nfields, int *err, int sm_count, cudaStream_t st, long long wait_cycles);
+// Variant 3 of the batched Chebyshev step: launch_cheb_spin over every field
+// (blocks over (field, unit), field fastest for order 0), e on the fields'
+// dA and dB; the last launch of a pass updates x and hnew itself.  A pass of
+// one step is launch_batch_cheb_one.
+void launch_batch_cheb_spin(int step, bool last, int order, Lat L, const SpinOp32 &op, const BatchField *tab,
+                            int nfields, int *err, cudaStream_t st, long long wait_cycles);
+void launch_batch_cheb_one(int64_t n, const BatchField *tab, int nfields, cudaStream_t st);
 void launch_batch_add_e(int64_t n, const BatchField *tab, int nfields, cudaStream_t st);
 // Chebyshev coefficients of every field from its mass's bounds; sets
 // flags[f] = 1 for non-finite bounds
@@ -309,20 +294,19 @@ void launch_batch_calibrate(const BatchField *tab, int nfields, double *pstate, 
 void launch_batch_hist_start(int64_t V, const BatchField *tab, int nfields, cudaStream_t st);
 void launch_cn_to_f32(int64_t V, const double2 *U, const double2 *DE, const double2 *D, const double *B, float2 *U32,
                       float2 *DE32, float2 *D32, float *B32, cudaStream_t st);
-void launch_cn_bounds(Lat L, const CnCoef &C, double tau, const double2 *U, const double2 *Dsum, const double *Bsum,
-                      const double2 *DE, double *partials, double *out, cudaStream_t st);
 void launch_cheb32(bool first, Lat L, const CnCoef &C, const float2 *U, const float2 *Dsum, const float *Bsum,
                    const float2 *DE, const float2 *D, float2 *Dn, float2 *R, float2 *E, const ChebCoef &K,
                    cudaStream_t st);
-// The same Chebyshev step on the FP32 blocks of launch_cn_blocks5 (Wf, built
-// with the coefficients C; nb_sign as for the FP64 FMA stencil), staged by
-// TMA (cn_cheb5f.cu).  cheb5f_applicable: the lattices it describes (V a
-// multiple of 4, at least 36 sites, nx even, V < 2^31).  Returns nonzero if
-// the tensor maps cannot be made; wait_cycles bounds every pipeline wait.
-bool cheb5f_applicable(const Lat &L);
-int launch_cheb5f(bool first, Lat L, const CnCoef &C, double nb_sign, const float2 *Wf, const float2 *Dsum,
-                  const float *Bsum, const float2 *D, float2 *Dn, float2 *R, float2 *E, const ChebCoef &K, int *err,
-                  int sm_count, cudaStream_t st, long long wait_cycles);
+// The inner solve A^H e = r on the operator in its spin structure, FP32
+// (cn_spin32.cu): launch `step` = 0, 1, .. makes e_{step+2} with the step's
+// coefficients K, into ea (even steps) or eb (odd ones); the last one adds it
+// to x and, if not null, to hist instead.  m Chebyshev steps take m - 1
+// launches, one step is launch_cheb_one over the n elements.
+bool cheb_spin_applicable(const Lat &L);
+void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const float2 *r, float2 *ea, float2 *eb,
+                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], int *err, cudaStream_t st,
+                      long long wait_cycles);
+void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const cplx inv_theta[2], cudaStream_t st);
 void launch_add_e(int64_t n, double2 *X, const float2 *E, cudaStream_t st);
 void launch_prop_f2soa(const double2 *f, double2 *P, int64_t V, cudaStream_t st);
 void launch_prop_soa2f(const double2 *P, double2 *f, int64_t V, cudaStream_t st);
