@@ -621,6 +621,93 @@ extern "C" int nrq_gauge_gauss(nrq_gauge *g, double *ref_measure, double *max_no
 namespace {
 constexpr int64_t kProjUnbounded = INT64_MAX;
 
+// The projection on a lattice that fits the GPU (k_gauss_run): launches of
+// up to kRunChunk sweeps, each followed by the read-back of its deviations.
+// The launch that crosses the tolerance is repeated from its own start, for
+// the sweeps up to the crossing, so that the field and the count are those of
+// a test after every sweep; its length follows the decay seen so far, which
+// keeps the repeated part short.  Returns false where the cooperative launch
+// is refused (the caller queues single sweeps).
+constexpr int64_t kRunChunk = 512;
+bool gauss_project_run(nrq_gauge *g, double tol, int64_t limit, int64_t *sweeps, double *deviation, int *rc) {
+  nrq_ctx *ctx = g->ctx;
+  const int64_t V = ctx->lat.V, nw = nrq::gauss_run_warps(V);
+  cudaStream_t st = ctx->stream;
+  const size_t mb = (size_t)nrq::gauss_run_message_bytes(V), eb = sizeof(double) * 24 * V;
+  const size_t db = sizeof(double) * (kRunChunk + 1) * (nw + 1);
+  if ((*rc = ensure_stage(ctx, mb + eb + db + sizeof(int)))) return true;
+  char *base = (char *)ctx->d_stage;
+  double *E2 = (double *)(base + mb), *dev = (double *)(base + mb + eb), *devmax = dev + (kRunChunk + 1) * nw;
+  int *err = (int *)(base + mb + eb + db);
+  auto cuda = [&](cudaError_t e) {
+    if (e != cudaSuccess && !*rc) {
+      ctx->last_error = std::string("Gauss projection: ") + cudaGetErrorString(e);
+      *rc = NRQ_ERR_CUDA;
+    }
+    return e == cudaSuccess;
+  };
+  if (!cuda(cudaMemsetAsync(base, 0, mb, st)) || !cuda(cudaMemsetAsync(err, 0, sizeof(int), st))) return true;
+  const double kdt = 0.01 * ctx->a[0];
+  std::vector<double> d(kRunChunk + 2);
+  double *cur = g->E, *next = E2;
+  uint32_t te = 1, ge = 1;
+  auto launch = [&](double *to, int n) {
+    const cudaError_t e = nrq::launch_gauss_run(ctx->lat, g->U, cur, to, base, dev, devmax, n, te, ge, kdt,
+                                                ctx->sm_count, err, st, nrq_wait_cycles_default);
+    te += (uint32_t)n + 1;
+    ge += (uint32_t)n;
+    return e;
+  };
+  int64_t total = 0, batch = 16, found = -1;
+  double last = 0.0;
+  for (;;) {
+    const int n = (int)std::min(batch, limit - total);
+    const cudaError_t e = launch(next, n);
+    if (e != cudaSuccess && total == 0 && cur == g->E) {
+      cudaGetLastError();
+      return false;
+    }
+    if (!cuda(e) || !cuda(cudaMemcpyAsync(d.data(), devmax, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, st)) ||
+        !cuda(cudaMemcpyAsync(&d[kRunChunk + 1], err, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
+        !cuda(cudaStreamSynchronize(st)))
+      return true;
+    int failed;
+    std::memcpy(&failed, &d[kRunChunk + 1], sizeof(int));
+    if (failed) {
+      ctx->last_error = "Gauss projection: a bounded wait expired (k_gauss_run)";
+      *rc = NRQ_ERR_TIMEOUT;
+      return true;
+    }
+    for (int k = 0; k <= n && found < 0; ++k)
+      if (!(d[k] > tol)) found = k;
+    last = d[found >= 0 ? found : n];
+    if (found >= 0 && found < n) {  // again from cur, up to the crossing
+      if (found > 0 || cur != g->E) {
+        if (!cuda(launch(g->E, (int)found))) return true;
+      }
+      total += found;
+      break;
+    }
+    total += n;
+    std::swap(cur, next);
+    if (found >= 0 || total >= limit) {
+      if (cur != g->E && !cuda(cudaMemcpyAsync(g->E, cur, eb, cudaMemcpyDeviceToDevice, st))) return true;
+      break;
+    }
+    batch = std::min<int64_t>(batch * 2, kRunChunk);
+    // the sweeps that remain at this launch's rate of decay, if that is fewer
+    const double rate = std::log(d[0] / d[n]) / n, need = std::log(d[n] / tol) / rate;
+    if (rate > 0.0 && need < (double)batch) batch = std::max<int64_t>(8, (int64_t)need + 1);
+  }
+  if (sweeps) *sweeps = total;
+  if (deviation) *deviation = last;
+  if (found < 0) {
+    ctx->last_error = "Gauss projection: deviation above tolerance after max_sweeps sweeps";
+    *rc = NRQ_ERR_NOT_CONVERGED;
+  }
+  return true;
+}
+
 // Gauss projection sweeps of EquilibriumInit (gauge:455-500) on g's FP64
 // field.  Sweeps are queued in growing batches; the kernels themselves stop
 // at the first sweep whose deviation is at most tol, so the count is exact.
@@ -630,7 +717,11 @@ int gauss_project(nrq_gauge *g, double tol, int64_t max_sweeps, int64_t *sweeps,
   const int64_t V = L.V;
   const unsigned nbg = (unsigned)nblk(V, 128), nbs = (unsigned)nblk(V, 128);
   int rc = gauge_sync64(g);
-  if (!rc) rc = ensure_stage(ctx, sizeof(double2) * 9 * V);
+  if (rc) return rc;
+  const int64_t limit = max_sweeps > 0 ? max_sweeps : kProjUnbounded;
+  if (nrq::gauss_run_applicable(V, ctx->sm_count) && gauss_project_run(g, tol, limit, sweeps, deviation, &rc))
+    return rc;
+  rc = ensure_stage(ctx, sizeof(double2) * 9 * V);
   if (!rc) rc = ensure_red(ctx, nbg);
   if (rc) return rc;
   if (!ctx->d_proj) NRQ_CUDA_TRY(ctx, cudaMalloc(&ctx->d_proj, sizeof(nrq::GaussProjState)));
@@ -640,7 +731,6 @@ int gauss_project(nrq_gauge *g, double tol, int64_t max_sweeps, int64_t *sweeps,
   NRQ_CUDA_TRY(ctx, cudaMemsetAsync(st, 0, sizeof(nrq::GaussProjState), ctx->stream));
   nrq::k_gauss_g<<<nbg, 128, 0, ctx->stream>>>(L, g->U, g->E, G, ctx->d_red, st, tol, 0);
   if ((rc = check_launch(ctx, "k_gauss_g"))) return rc;
-  const int64_t limit = max_sweeps > 0 ? max_sweeps : kProjUnbounded;
   int64_t queued = 0, batch = 16;
   nrq::GaussProjState h{};
   for (;;) {

@@ -48,6 +48,17 @@ __global__ void k_gauss_g(Lat L, const double2 *__restrict__ U, const double *__
                           int count);
 __global__ void k_gauss_sweep(Lat L, const double2 *__restrict__ U, const double2 *__restrict__ G,
                               double *__restrict__ E, const GaussProjState *st, double kdt);
+// nsweeps sweeps in one launch, from Ein into Eout (may be the same), where
+// gauss_run_applicable; devmax[n] = the deviation before sweep n = 0..nsweeps.
+// messages: gauss_run_message_bytes, zero before a projection's first launch;
+// te, ge: the numbers of the launch's first messages (nsweeps + 1 and nsweeps
+// of them), from 1 on; dev: gauss_run_warps doubles per entry of devmax.
+int gauss_run_warps(int64_t V);
+bool gauss_run_applicable(int64_t V, int sm_count);
+int64_t gauss_run_message_bytes(int64_t V);
+cudaError_t launch_gauss_run(Lat L, const double2 *U, const double *Ein, double *Eout, void *messages, double *dev,
+                             double *devmax, int nsweeps, uint32_t te, uint32_t ge, double kdt, int sm_count, int *err,
+                             cudaStream_t st, long long wait_cycles);
 
 // ---------------- gluon.cu
 __global__ void k_cg_divergence(Lat L, const double2 *__restrict__ U, double2 *__restrict__ D,
