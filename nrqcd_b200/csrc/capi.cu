@@ -865,6 +865,54 @@ double max_norm2_momentum(const nrq_ctx *ctx) {
   }
   return std::sqrt(s);
 }
+// The gauge fixing on short extents: batches of iterations without a host
+// synchronisation, decided on the device (k_cg_rows)
+int coulomb_short(nrq_gauge *g, double tol, double alpha, int64_t max_iterations, int64_t *iterations,
+                  double *deviations) {
+  nrq_ctx *ctx = g->ctx;
+  const nrq::Lat L = ctx->lat;
+  const int64_t V = L.V;
+  cudaStream_t st = ctx->stream;
+  constexpr int kBatch = 32;  // most iterations between two read-backs
+  const size_t tabs = 3 * nrq::kCgMaxExtent;
+  int rc = ensure_gluon(ctx, sizeof(double2) * (41 * V + tabs) + sizeof(double) * (tabs + kBatch));
+  if (rc) return rc;
+  double2 *U2 = (double2 *)ctx->d_gluon, *F = U2 + 27 * V, *G = F + 5 * V, *tw = G + 9 * V;
+  double *p2 = (double *)(tw + tabs), *dev = p2 + tabs;
+  nrq::launch_cg_tables(L, tw, p2, st);
+  const double pmax = max_norm2_momentum(ctx), scale = alpha / (double)V;
+  double2 *cur = g->U, *alt = U2;
+  int64_t queued = 0, found = -1;  // found: iterations whose deviation was above the tolerance
+  for (int batch = 8; found < 0 && queued < max_iterations; batch = 2 * batch < kBatch ? 2 * batch : kBatch) {
+    const int64_t first = queued;
+    const int n = (int)std::min<int64_t>(batch, max_iterations - queued);
+    double h[kBatch];
+    NRQ_CUDA_TRY(ctx, cudaMemsetAsync(dev, 0, sizeof(double) * n, st));
+    for (int k = 0; k < n; ++k, ++queued) {
+      nrq::launch_cg_rows(L, cur, queued ? G : nullptr, alt, tw, F, dev, tol, k, st);
+      if (queued) std::swap(cur, alt);
+      nrq::launch_cg_smooth(L, tw, p2, F, G, pmax, scale, dev, tol, k, st);
+    }
+    if ((rc = check_launch(ctx, "Coulomb gauge fixing"))) return rc;
+    NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(h, dev, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    for (int k = 0; k < n && found < 0; ++k) {
+      if (deviations) deviations[first + k] = h[k];
+      if (!(h[k] > tol)) found = first + k;
+    }
+  }
+  // the links of that deviation, or after max_iterations transformations
+  int64_t transforms = found;
+  if (found < 0) {
+    transforms = max_iterations;
+    if (max_iterations > 0) nrq::launch_cg_rows(L, cur, G, alt, tw, nullptr, dev, tol, 0, st);
+    if ((rc = check_launch(ctx, "Coulomb gauge fixing"))) return rc;
+  }
+  if (transforms & 1)
+    NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(g->U, U2, sizeof(double2) * 27 * V, cudaMemcpyDeviceToDevice, st));
+  if (iterations) *iterations = found < 0 ? max_iterations + 1 : found + 1;
+  return NRQ_OK;
+}
 }  // namespace
 
 extern "C" int nrq_gauge_coulomb_gaugefix(nrq_gauge *g, double tol, double alpha, int64_t max_iterations,
@@ -876,6 +924,10 @@ extern "C" int nrq_gauge_coulomb_gaugefix(nrq_gauge *g, double tol, double alpha
   int rc = set_device(ctx);
   if (!rc) rc = gauge_sync64(g);
   if (rc) return rc;
+  if (nrq::cg_short_applicable(L)) {
+    rc = coulomb_short(g, tol, alpha, max_iterations, iterations, deviations);
+    return rc ? rc : gauge_written64(g);
+  }
   const unsigned nb_ = (unsigned)nblk(V, 128);
   if ((rc = ensure_red(ctx, nb_))) return rc;
   if ((rc = ensure_gluon(ctx, sizeof(double2) * 9 * V))) return rc;
@@ -930,7 +982,7 @@ extern "C" int nrq_gauge_transverse_correlators(nrq_gauge *g, double *aa, double
   }
   const unsigned nb_ = (unsigned)nblk(V, 128);
   const double fwd = ctx->a[1] * ctx->a[2] * ctx->a[3];
-  nrq::k_gluon_fields<<<nb_, 128, 0, ctx->stream>>>(L, g->U, g->E, F);
+  nrq::k_gluon_fields<<<dim3(nb_, 3), 128, 0, ctx->stream>>>(L, g->U, g->E, F);
   bool ok = cudaGetLastError() == cudaSuccess &&
             cufftExecZ2Z(plan, (cufftDoubleComplex *)F, (cufftDoubleComplex *)F, CUFFT_FORWARD) == CUFFT_SUCCESS;
   if (ok) {

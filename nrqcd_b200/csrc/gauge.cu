@@ -474,7 +474,7 @@ __global__ void k_ic_pspace(Lat L, const double2 *__restrict__ R, const double *
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= L.V) return;
   const int64_t V = L.V;
-  int64_t pos[3];
+  uint32_t pos[3];
   coords(L, s, pos[0], pos[1], pos[2]);
   const int64_t off[3] = {0, L.nx, L.nx + L.ny};
   cplx p[3];

@@ -256,27 +256,23 @@ struct Lat {
   double a0, a[3];
 };
 
-__device__ __forceinline__ void coords(const Lat &L, int64_t s, int64_t &x, int64_t &y, int64_t &z) {
-  x = s % L.nx;
-  int64_t t = s / L.nx;
-  y = t % L.ny;
-  z = t / L.ny;
+// (32-bit arithmetic: a lattice of 2^32 sites has two terabytes of links, and
+// the 64-bit divisions cost a kernel of a few microseconds one of them)
+__device__ __forceinline__ void coords(const Lat &L, int64_t s, uint32_t &x, uint32_t &y, uint32_t &z) {
+  const uint32_t u = (uint32_t)s, nx = (uint32_t)L.nx, ny = (uint32_t)L.ny, t = u / nx;
+  x = u - t * nx;
+  z = t / ny;
+  y = t - z * ny;
 }
 // neighbour of site s in direction d (0..2) by +1 (sgn>0) or -1
 __device__ __forceinline__ int64_t nb(const Lat &L, int64_t s, int d, int sgn) {
-  int64_t x, y, z;
+  uint32_t x, y, z;
   coords(L, s, x, y, z);
-  if (d == 0) {
-    x += sgn;
-    x = (x < 0) ? x + L.nx : (x >= L.nx ? x - L.nx : x);
-  } else if (d == 1) {
-    y += sgn;
-    y = (y < 0) ? y + L.ny : (y >= L.ny ? y - L.ny : y);
-  } else {
-    z += sgn;
-    z = (z < 0) ? z + L.nz : (z >= L.nz ? z - L.nz : z);
-  }
-  return x + L.nx * (y + L.ny * z);
+  const uint32_t c = d == 0 ? x : d == 1 ? y : z;
+  const int64_t n = d == 0 ? L.nx : d == 1 ? L.ny : L.nz;
+  const int64_t step = d == 0 ? 1 : d == 1 ? L.nx : L.nx * L.ny;
+  if (sgn > 0) return c + 1 == (uint32_t)n ? s - (n - 1) * step : s + step;
+  return c == 0 ? s + (n - 1) * step : s - step;
 }
 
 // link U_d(s) from SoA planes: plane (d*9 + r*3 + c)

@@ -66,6 +66,19 @@ __global__ void k_cg_divergence(Lat L, const double2 *__restrict__ U, double2 *_
 __global__ void k_cg_accelerate(Lat L, double2 *__restrict__ D, double pmax, double scale);
 __global__ void k_cg_expah(int64_t V, double2 *__restrict__ D);
 __global__ void k_cg_transform(Lat L, double2 *__restrict__ U, const double2 *__restrict__ G);
+// gauge fixing on short extents (three launches an iteration)
+constexpr int kCgMaxExtent = 32, kCgRowSites = 64;
+bool cg_short_applicable(const Lat &L);
+void launch_cg_tables(Lat L, double2 *tw, double *p2, cudaStream_t st);  // 3*kCgMaxExtent entries each
+// U' = G U G^+ from Uin to Uout (G null: no transformation), then its
+// deviation into dev[slot] (zero before) and the x transform of its
+// divergence into F (5V; null: neither).  Nothing where dev[slot - 1] (slot >
+// 0) has met tol.
+void launch_cg_rows(Lat L, const double2 *Uin, const double2 *G, double2 *Uout, const double2 *tw, double2 *F,
+                    double *dev, double tol, int slot, cudaStream_t st);
+// G = ExpAH of the accelerated divergence; nothing where dev[slot] has met tol
+void launch_cg_smooth(Lat L, const double2 *tw, const double *p2, double2 *F, double2 *G, double pmax, double scale,
+                      const double *dev, double tol, int slot, cudaStream_t st);
 __global__ void k_gluon_fields(Lat L, const double2 *__restrict__ U, const double *__restrict__ E,
                                double2 *__restrict__ F);
 __global__ void k_transverse_corr(Lat L, const double2 *__restrict__ F, double fwd, double volume,

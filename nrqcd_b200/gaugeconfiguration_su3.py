@@ -152,7 +152,7 @@ class GaugeConfiguration:
         iteration and the final loop counter.  Returns (loop counter,
         deviations)."""
         n = int(MaxIterations_)
-        dev = np.full(max(n, 1), np.nan)
+        dev = np.empty(max(n, 1))  # the entries of the iterations made are filled in
         it = ctypes.c_int64()
         self._call("nrq_gauge_coulomb_gaugefix", float(Tolerance_), float(alpha_), n, ctypes.byref(it),
                    _capi.dptr(dev))
