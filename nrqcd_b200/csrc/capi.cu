@@ -515,7 +515,7 @@ extern "C" int nrq_gauge_update(nrq_gauge *g, double dt) {
       nrq::k_update_links32<<<nb_, 128, 0, ctx->stream>>>(ctx->lat, g->U32, g->E, dt);
     } else {
       ProfScope ps(ctx, 4, V * (192.0 + 432.0 + 432.0));
-      nrq::k_update_links<<<nb_, 128, 0, ctx->stream>>>(ctx->lat, g->U, g->E, dt);
+      nrq::launch_update_links(ctx->lat, g->U, g->E, dt, ctx->stream);
     }
   };
   auto efield = [&]() {
@@ -524,7 +524,7 @@ extern "C" int nrq_gauge_update(nrq_gauge *g, double dt) {
       nrq::k_update_efield32<<<nb_, 128, 0, ctx->stream>>>(ctx->lat, g->U32, g->E, dt);
     } else {
       ProfScope ps(ctx, 5, V * (432.0 + 192.0 + 192.0));
-      nrq::k_update_efield<<<3 * nb_, 128, 0, ctx->stream>>>(ctx->lat, g->U, g->E, dt);
+      nrq::launch_update_efield(ctx->lat, g->U, g->E, dt, ctx->stream);
     }
   };
   // Update_Leapfrog ordering (gauge:2100-2110)

@@ -10,6 +10,7 @@
 // Paths are those of the reference project (src/gaugeconfiguration_su3.f90
 // abbreviated "gauge").
 #include "nrq_kernels.cuh"
+#include "pdl.cuh"
 
 namespace nrq {
 
@@ -64,62 +65,88 @@ __global__ void k_cold(double2 *__restrict__ U, double *__restrict__ E, int64_t 
 }
 
 // ------------------------------------------------------------ leapfrog
-__global__ void __launch_bounds__(128) k_update_links(Lat L, double2 *__restrict__ U,
-                                                      const double *__restrict__ E, double dt) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+constexpr int kLinkSites = 32, kForceSites = 16;  // consecutive sites of a block
+// One thread per link.  64^3: 62 us, of which the traffic takes 43; the
+// exponential's chain of FMAs at 12 warps an SM (154 registers) the rest (128
+// registers with a little spilled: 3 % faster there, 6 % slower at 30x21x14).
+__global__ void __launch_bounds__(3 * kLinkSites) k_update_links(Lat L, double2 *__restrict__ U,
+                                                                const double *__restrict__ E, double dt) {
+  const int d = (int)threadIdx.x / kLinkSites;
+  const int64_t s = (int64_t)blockIdx.x * kLinkSites + threadIdx.x % kLinkSites;
+  pdl_wait();
+  pdl_trigger();
   if (s >= L.V) return;
   const int64_t V = L.V;
-#pragma unroll 1
-  for (int d = 0; d < 3; ++d) {
-    double al[8];
+  double al[8];
 #pragma unroll
-    for (int a = 0; a < 8; ++a) al[a] = __ldg(E + (int64_t)(d * 8 + a) * V + s) * dt;
-    m3 G = expi_herm(algebra_matrix(al));
-    m3 u = load_link(U, V, s, d);
-    store_link(U, V, s, d, mul(G, u));
-  }
+  for (int a = 0; a < 8; ++a) al[a] = __ldca(E + (int64_t)(d * 8 + a) * V + s) * dt;
+  const m3 u = load_link_c(U, V, s, d);
+  const m3 G = expi_herm(algebra_matrix(al));
+  store_link(U, V, s, d, mul(G, u));
 }
 
-// blocks per SM the force kernel's registers are sized for
-#ifndef NRQ_EFIELD_MIN_BLOCKS
-#define NRQ_EFIELD_MIN_BLOCKS 3
-#endif
-
-// One thread per (site, direction i): the force on link (x, i) from its
-// four staples, k != i in ascending order as gauge:2147-2198 sums them.
-// Block b of the grid holds 128 consecutive sites of direction b % 3, so
-// the three directions of a site range run next to each other and share the
-// neighbour links in L2.
-__global__ void __launch_bounds__(128, NRQ_EFIELD_MIN_BLOCKS) k_update_efield(Lat L, const double2 *__restrict__ U,
-                                                       double *__restrict__ E, double dt) {
-  const int i = (int)(blockIdx.x % 3);
-  const int64_t s = (int64_t)(blockIdx.x / 3) * blockDim.x + threadIdx.x;
-  if (s >= L.V) return;
-  const int64_t V = L.V;
-  m3 sum = m3_zero();
-  const int64_t xpi = nb(L, s, i, +1);
+// The force on link (x, i) from its four staples, one thread for each of the
+// two directions k != i: two staples, U_i(x) times their sum, and the traces,
+// which the lane pair adds.  The three directions of a block's sites run side
+// by side and read the links they share through the SM's L1.
+// Bound: latency of the loads (12 matrices a thread, FP64 pipe a third
+// active).  64^3: 137 us at 15 warps an SM (one thread per link, three
+// matrices live, 12 warps: 147; one thread per row of a link, 24 warps, three
+// times the load instructions: 230); a step at 30x21x14 10.1 -> 7 us, with
+// the launch of the second kernel hidden.
+__global__ void __launch_bounds__(6 * kForceSites, 5) k_update_efield(Lat L, const double2 *U, double *E, double dt) {
+  pdl_wait();
+  pdl_trigger();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, kk = lane >> 4;
+  const int i = w % 3;
+  const int64_t V = L.V, x0 = (int64_t)blockIdx.x * kForceSites + (w / 3) * 16 + (lane & 15);
+  const bool act = x0 < V;
+  const int64_t s = act ? x0 : V - 1;
+  const int k = kk + (kk >= i ? 1 : 0);
+  const double r = L.a0 / L.a[k];
+  const double coef = dt * (r * r);
+  const int64_t xpi = nb(L, s, i, +1), xpk = nb(L, s, k, +1), xmk = nb(L, s, k, -1), xpimk = nb(L, xmk, i, +1);
+  // U staple  U_k(x+i) U_i(x+k)^+ U_k(x)^+
+  m3 t = mul_nd(mul_nd(load_link_c(U, V, xpi, k), load_link_c(U, V, xpk, i)), load_link_c(U, V, s, k));
+  {  // D staple  U_k(x+i-k)^+ U_i(x-k)^+ U_k(x-k)
+    const m3 d = mul_dn(mul(load_link_c(U, V, xmk, i), load_link_c(U, V, xpimk, k)), load_link_c(U, V, xmk, k));
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (k == i) continue;
-    const double r = L.a0 / L.a[k];
-    const double coef = dt * (r * r);
-    const int64_t xpk = nb(L, s, k, +1), xmk = nb(L, s, k, -1);
-    const int64_t xpimk = nb(L, xmk, i, +1);
-    // U staple  U_k(x+i) U_i(x+k)^+ U_k(x)^+
-    m3 su = mul_nd(mul_nd(load_link(U, V, xpi, k), load_link(U, V, xpk, i)), load_link(U, V, s, k));
-    // D staple  U_k(x+i-k)^+ U_i(x-k)^+ U_k(x-k)
-    m3 sd = mul(dag(mul(load_link(U, V, xmk, i), load_link(U, V, xpimk, k))), load_link(U, V, xmk, k));
-#pragma unroll
-    for (int m = 0; m < 9; ++m) sum.e[m] = sum.e[m] + coef * (su.e[m] + sd.e[m]);
+    for (int m = 0; m < 9; ++m) t.e[m] = t.e[m] + d.e[m];
   }
-  m3 ls = mul(load_link(U, V, s, i), sum);
+  t = mul(load_link_c(U, V, s, i), t);
   cplx tr[8];
-  traces_with_generators(ls, tr);
+  traces_with_generators(t, tr);
+  double f[8];
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
-    double *e = E + (int64_t)(i * 8 + a) * V + s;
-    *e = *e - 2.0 * tr[a].im;
+    f[a] = coef * tr[a].im;
+    f[a] += __shfl_xor_sync(0xffffffffu, f[a], 16);
   }
+  if (!act) return;
+  double *e = E + (int64_t)(i * 8 + 4 * kk) * V + s;  // four coordinates a lane
+#pragma unroll
+  for (int a = 0; a < 4; ++a) e[(int64_t)a * V] -= 2.0 * (kk ? f[4 + a] : f[a]);
+}
+
+// the two kernels of a leapfrog step, in either order; inside a capture as
+// ordinary launches
+namespace {
+template <typename K, typename... A>
+void launch_leapfrog(K kernel, unsigned block, int sites, Lat L, cudaStream_t st, A... args) {
+  const unsigned grid = (unsigned)((L.V + sites - 1) / sites);
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(st, &capture);
+  if (capture == cudaStreamCaptureStatusNone)
+    launch_pdl(kernel, grid, block, 0, st, L, args...);
+  else
+    kernel<<<grid, block, 0, st>>>(L, args...);
+}
+}  // namespace
+void launch_update_links(Lat L, double2 *U, const double *E, double dt, cudaStream_t st) {
+  launch_leapfrog(k_update_links, 3 * kLinkSites, kLinkSites, L, st, U, E, dt);
+}
+void launch_update_efield(Lat L, const double2 *U, double *E, double dt, cudaStream_t st) {
+  launch_leapfrog(k_update_efield, 6 * kForceSites, kForceSites, L, st, U, E, dt);
 }
 
 // ------------------------------------------------------------ FP32 links

@@ -13,8 +13,8 @@ __global__ void k_links_soa2f(const double2 *__restrict__ U, double2 *__restrict
 __global__ void k_efield_f2soa(const double *__restrict__ f, double *__restrict__ E, int64_t V);
 __global__ void k_efield_soa2f(const double *__restrict__ E, double *__restrict__ f, int64_t V);
 __global__ void k_cold(double2 *__restrict__ U, double *__restrict__ E, int64_t V);
-__global__ void k_update_links(Lat L, double2 *__restrict__ U, const double *__restrict__ E, double dt);
-__global__ void k_update_efield(Lat L, const double2 *__restrict__ U, double *__restrict__ E, double dt);
+void launch_update_links(Lat L, double2 *U, const double *E, double dt, cudaStream_t st);
+void launch_update_efield(Lat L, const double2 *U, double *E, double dt, cudaStream_t st);
 // precision form of the leapfrog: FP32 links, FP64 Ẽ (gauge.cu)
 __global__ void k_update_links32(Lat L, float2 *__restrict__ U, const double *__restrict__ E, double dt);
 __global__ void k_update_efield32(Lat L, const float2 *__restrict__ U, double *__restrict__ E, double dt);
