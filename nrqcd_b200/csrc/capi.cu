@@ -79,7 +79,7 @@ int ensure_red(nrq_ctx *ctx, int64_t doubles) {
 // block per value, which stores it into the pinned host array itself (a
 // separate copy costs a launch as long as the reduction)
 int reduce_to_host(nrq_ctx *ctx, int64_t nb, int nq, unsigned maxmask) {
-  nrq::k_reduce_final<<<nq, 256, 0, ctx->stream>>>(ctx->d_red, nb, nq, maxmask, ctx->h_res);
+  nrq::launch_reduce_final(ctx->d_red, nb, nq, maxmask, ctx->h_res, ctx->stream);
   int rc = check_launch(ctx, "k_reduce_final");
   if (rc) return rc;
   NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1399,6 +1399,7 @@ int ensure_spin(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *si
   }
   cn->spin_coef = C;
   cn->spin_valid = true;
+  cn->spin_fresh = true;
   *sign = 1.0;
   return check_launch(ctx, "k_spin_prepare");
 }
@@ -1417,8 +1418,9 @@ int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq
       cn->spin_valid = false;
       if ((rc = ensure_spin(cn, C, g, &sign))) return rc;
     }
-    nrq::launch_cn_spin(mode, ctx->lat, cn->spin, sign, a, err ? err : scal_err(cn->scal), ctx->stream,
-                        cn->wait_cycles, cn->stall_load);
+    nrq::launch_cn_spin(mode, ctx->lat, cn->spin, sign, a, !cn->spin_fresh, err ? err : scal_err(cn->scal),
+                        ctx->stream, cn->wait_cycles, cn->stall_load);
+    cn->spin_fresh = false;
     cn->last_stencil = NRQ_STENCIL_FMA;
     return NRQ_OK;
   }
@@ -1592,10 +1594,13 @@ int cn_prepare(nrq_cn *cn, const nrq_gauge *g, double dt) {
 }
 // spectral enclosure of H, A^H = 1 + i spin_tau H, into out (4 doubles of the
 // device); the operator was built for A^H
-int spin_bounds(nrq_cn *cn, double *out) {
+// table: with the Chebyshev table of these bounds, and the bounds into h_cheb
+int spin_bounds(nrq_cn *cn, double *out, bool table) {
   nrq_ctx *ctx = cn->ctx;
   ProfScope ps(ctx, 3, (double)ctx->lat.V * 56.0);
-  nrq::launch_spin_bounds(ctx->lat, 1, cn->spin_scratch, cn->spin_part, cn->spin_ticket, out, ctx->stream);
+  nrq::launch_spin_bounds(ctx->lat, 1, cn->spin_scratch, cn->spin_part, cn->spin_ticket, out, ctx->stream,
+                          cn->spin_tau, table ? cn->cheb_tab : nullptr, table ? scal_bounds(cn->h_cheb) : nullptr);
+  cn->spin_fresh = false;  // its writer has completed when this launch starts
   return check_launch(ctx, "k_spin_bounds");
 }
 }  // namespace
@@ -1643,7 +1648,7 @@ int tune_cheb(nrq_cn *cn, const nrq::CnCoef &CH, const nrq::ChebCoef &K, const n
       if (r == 1) cudaEventRecord(e0, st);
       if (which == NRQ_CHEB_BLOCKS)
         nrq::launch_cheb_spin(1, false, ctx->lat, cn->spin32, cn->r32, cn->dA32, cn->dB32, nullptr, nullptr, K,
-                              inv_theta, scal_err(cn->scal), st, cn->wait_cycles);
+                              inv_theta, false, scal_err(cn->scal), st, cn->wait_cycles);
       else
         nrq::launch_cheb32(true, ctx->lat, CH, cn->U32, cn->D32, cn->B32, cn->DE32, cn->dA32, cn->dB32, cn->e32,
                            cn->e32, K, st);
@@ -1683,7 +1688,7 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   if (!rc) rc = ensure_spin(cn, CH, g, &spin_sign);
   if (rc) return rc;
   // spectral enclosure of H per species
-  if ((rc = spin_bounds(cn, scal_bounds(cn->scal)))) return rc;
+  if ((rc = spin_bounds(cn, scal_bounds(cn->scal), false))) return rc;
   NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(cn->h_bounds, scal_bounds(cn->scal), sizeof(double) * 4, cudaMemcpyDeviceToHost,
                                     st));
   int64_t matvecs = 0, vstreams = 0;
@@ -1863,7 +1868,8 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
         ProfScope ps(ctx, 0, (double)V * (576.0 * (k == 0 ? 1 : k == 1 ? 2 : 3) +
                                           (last ? 1152.0 * 2 + (hacc ? 1152.0 : 0.0) : 576.0) + 756.0));
         nrq::launch_cheb_spin(k, last, L, cn->spin32, cn->r32, cn->dA32, cn->dB32, cn->x, hacc, coef[k], a.inv_theta,
-                              scal_err(cn->scal), st, cn->wait_cycles);
+                              !cn->spin_fresh, scal_err(cn->scal), st, cn->wait_cycles);
+        cn->spin_fresh = false;
       }
     } else {
       cn->last_cheb = NRQ_CHEB_REGISTER;
@@ -2176,8 +2182,7 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
       NRQ_CUDA_TRY(ctx, cudaMallocHost((void **)&cn->h_cheb, kScalBytes));
       std::memset(cn->h_cheb, 0, kScalBytes);
     }
-    if ((rc = spin_bounds(cn, scal_bounds(cn->scal)))) return rc;
-    nrq::launch_cheb_tab(scal_bounds(cn->scal), cn->spin_tau, cn->cheb_tab, scal_bounds(cn->h_cheb), st);
+    if ((rc = spin_bounds(cn, scal_bounds(cn->scal), true))) return rc;
   }
   // RHS = A psi ; start x0 = 2 RHS - psi, plus the extrapolated t of the last steps
   const int hist_d = cn->history_guess ? std::min(cn->history_depth, h->hist_count) : 0;

@@ -28,6 +28,7 @@
 
 #include "nrq_eigen.cuh"
 #include "nrq_kernels.cuh"
+#include "pdl.cuh"
 
 namespace nrq {
 
@@ -330,11 +331,13 @@ __global__ void __launch_bounds__(512) k_cn_finalize(int stage, int64_t nblocks,
   const int nq = (stage == 4 || stage == 6) ? 1 : stage == 5 ? 5 : stage == 7 ? 4 : (stage == 0 || stage == 1) ? 2 : 3;
   __shared__ double sh[5][16];
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  pdl_wait();
+  pdl_trigger();
   for (int64_t b = threadIdx.x; b < nblocks; b += blockDim.x) {
     const double *p = partials + (b * CN_COLS + col) * nq;
 #pragma unroll
     for (int k = 0; k < 5; ++k)
-      if (k < nq) acc[k] += p[k];
+      if (k < nq) acc[k] += __ldcg(p + k);
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -445,48 +448,40 @@ __global__ void __launch_bounds__(512) k_cn_finalize(int stage, int64_t nblocks,
 
 void launch_cn_finalize(int stage, int64_t nblocks, const double *partials, double *scal, double tol,
                         cudaStream_t st) {
-  k_cn_finalize<<<CN_COLS, 512, 0, st>>>(stage, nblocks, partials, scal, tol);
+  launch_pdl(k_cn_finalize, CN_COLS, 512, 0, st, stage, nblocks, partials, scal, tol);
 }
 
 // ------------------------------------------------------------ batched scalars
 // Chebyshev coefficients of every field of a batch from the spectral
 // enclosure of its mass (the device-side counterpart of the host recurrence
-// of the single-field precision form): theta = 1 + i tau (lo+hi)/2,
-// delta = i |tau| (hi-lo)/2, sigma = theta/delta, rho_0 = 1/sigma,
-// rho_{k+1} = 1/(2 sigma - rho_k), c1 = rho_{k+1} rho_k, c2 = 2 rho_{k+1}/delta.
-__global__ void k_batch_coef(BatchField *__restrict__ tab, int nfields, int *__restrict__ flags) {
-  const int fi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (fi >= nfields) return;
-  BatchField &f = tab[fi];
+// of the single-field precision form), cheb[k]: c1 = rho_{k+1} rho_k, c2 of
+// rho_{k+1}.
+// A block per field, a thread per species and step.
+__global__ void k_batch_coef(BatchField *__restrict__ tab, int *__restrict__ flags) {
+  BatchField &f = tab[blockIdx.x];
+  const int sp = threadIdx.x / BATCH_MAX_CHEB, k = threadIdx.x % BATCH_MAX_CHEB;
+  double lo[2], hi[2];
   int bad = 0;
-  for (int sp = 0; sp < 2; ++sp) {
-    double lo = f.bounds[2 * sp], hi = f.bounds[2 * sp + 1];
-    if (!(isfinite(lo) && isfinite(hi) && hi >= lo)) {
+  for (int q = 0; q < 2; ++q) {
+    lo[q] = f.bounds[2 * q];
+    hi[q] = f.bounds[2 * q + 1];
+    if (!(isfinite(lo[q]) && isfinite(hi[q]) && hi[q] >= lo[q])) {
       bad = 1;
-      lo = hi = 0.0;
-    }
-    const cplx one = {1.0, 0.0};
-    const cplx theta = {1.0, f.tau * 0.5 * (lo + hi)};
-    const cplx delta = {0.0, fmax(fabs(f.tau) * 0.5 * (hi - lo), 1e-14)};
-    const cplx sigma = cdiv(theta, delta);
-    f.inv_theta[sp] = cdiv(one, theta);
-    cplx rho = cdiv(one, sigma);
-    // rho_k = T_k(sigma) / T_{k+1}(sigma), so m steps gain 1/|rho_0 ... rho_{m-1}|
-    cplx prod = one;
-    f.gain[sp][0] = 1.0;
-    for (int k = 0; k < BATCH_MAX_CHEB; ++k) {
-      prod = prod * rho;
-      f.gain[sp][k + 1] = 1.0 / sqrt(norm2(prod));
-      const cplx rn = cdiv(one, 2.0 * sigma - rho);
-      f.cheb[k].c1[sp] = rn * rho;
-      f.cheb[k].c2[sp] = cdiv(2.0 * rn, delta);
-      rho = rn;
+      lo[q] = hi[q] = 0.0;
     }
   }
-  flags[fi] = bad;
+  const ChebSegment g(f.tau, sp ? lo[1] : lo[0], sp ? hi[1] : hi[0]);
+  const cplx rn = g.rho(k + 1);
+  f.cheb[k].c1[sp] = rn * g.rho(k);
+  f.cheb[k].c2[sp] = g.c2(rn);
+  f.gain[sp][k + 1] = g.gain(k + 1);
+  if (k != 0) return;
+  f.gain[sp][0] = 1.0;
+  f.inv_theta[sp] = g.inv_theta();
+  if (sp == 0) flags[blockIdx.x] = bad;
 }
 void launch_batch_coef(BatchField *tab, int nfields, int *flags, cudaStream_t st) {
-  k_batch_coef<<<(unsigned)((nfields + 63) / 64), 64, 0, st>>>(tab, nfields, flags);
+  k_batch_coef<<<(unsigned)nfields, 2 * BATCH_MAX_CHEB, 0, st>>>(tab, flags);
 }
 
 // (r.r, b.b) of every column of every field from the residual stencil's
@@ -646,6 +641,7 @@ void launch_single_point(double2 *P, int64_t V, int64_t sq, int64_t sa, cudaStre
 // unrolled: bound by the 576 B per site and species it reads (64^3, both
 // species: 49 us, 95 % of the copy rate).
 __global__ void __launch_bounds__(128) k_norms(const double2 *__restrict__ P, int64_t V, int sp0, double *partials) {
+  pdl_trigger();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double v = 0.0;
   if (s < V) {
@@ -684,6 +680,7 @@ void launch_norms(const double2 *P, int64_t V, int sp0, int nsp, double *partial
 // A^+, i.e. A transposed.
 template <bool GCONJ>
 __global__ void __launch_bounds__(128) k_correlators(const double2 *__restrict__ P, int64_t V, double *partials) {
+  pdl_trigger();
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   cplx S = {0.0, 0.0}, Ps = {0.0, 0.0}, Pc = {0.0, 0.0}, Pt = {0.0, 0.0};
   if (s < V) {

@@ -299,10 +299,14 @@ __global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C
 // of k_spin_prepare, per coefficient set (blockIdx.y): out[4*set] = {lo, hi}
 // of the quark, then of the antiquark.  The last block of a set to finish
 // reduces the partial rows (exact, order-independent); ticket[set] is zero
-// between launches.
+// between launches.  With tab (one set) it also makes the Chebyshev
+// coefficients of the segments, a thread for each, and stores the bounds into
+// the pinned host_bounds.  (40 steps of the recurrence by one thread took 18
+// us, more than a stencil launch at 12^3.)
 __global__ void __launch_bounds__(256) k_spin_bounds(Lat L, const double *__restrict__ scratch,
                                                      double *__restrict__ partials, unsigned *__restrict__ ticket,
-                                                     double *__restrict__ out) {
+                                                     double *__restrict__ out, double tau, ChebTab *__restrict__ tab,
+                                                     double *__restrict__ host_bounds) {
   const int64_t V = L.V;
   const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const double *s = scratch + (int64_t)blockIdx.y * 7 * V;
@@ -345,9 +349,9 @@ __global__ void __launch_bounds__(256) k_spin_bounds(Lat L, const double *__rest
       if (pass == 0)
         row[(int64_t)blockIdx.x * 4 + q] = a;
       else
-        out[4 * blockIdx.y + q] = a;
+        out[4 * blockIdx.y + q] = sh[0][q] = a;
     }
-    if (pass == 1) return;
+    if (pass == 1) break;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -366,6 +370,21 @@ __global__ void __launch_bounds__(256) k_spin_bounds(Lat L, const double *__rest
         v[q] = (q & 1) ? fmax(v[q], w) : fmin(v[q], w);
       }
   }
+  if (!tab) return;
+  __syncthreads();
+  const int sp = threadIdx.x / kChebTab, k = threadIdx.x - sp * kChebTab;
+  if (sp >= 2) return;
+  const double lo = sh[0][2 * sp], hi = sh[0][2 * sp + 1];
+  const ChebSegment g(tau, lo, hi);
+  const cplx rho = g.rho(k);
+  tab->step[k].c1[sp] = k == 0 ? cplx{0.0, 0.0} : rho * g.rho(k - 1);
+  tab->step[k].c2[sp] = k == 0 ? g.inv_theta() : g.c2(rho);
+  if (k != 0) return;
+  tab->inv_theta[sp] = g.inv_theta();
+  tab->lo[sp] = lo;
+  tab->hi[sp] = hi;
+  host_bounds[2 * sp] = lo;
+  host_bounds[2 * sp + 1] = hi;
 }
 
 // ------------------------------------------------------------------ stencil
@@ -383,7 +402,8 @@ struct SpinBatch {
 };
 template <int MODE, bool BATCH>
 __global__ void __launch_bounds__(spin::kUnit *spin::kWarps, 2)
-    k_cn_spin(Lat L, SpinOp op, double sign, MvArgs A, SpinBatch Bt, int *err, long long wait_cycles, int stall_load) {
+    k_cn_spin(Lat L, SpinOp op, double sign, MvArgs A, SpinBatch Bt, int *err, long long wait_cycles, int stall_load,
+              bool early) {
   using namespace spin;
   constexpr int kAhead = Num<double>::kAhead;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -435,7 +455,8 @@ __global__ void __launch_bounds__(spin::kUnit *spin::kWarps, 2)
   const int x = act ? s : V - 1;  // a valid site for the addresses of idle lanes
   cx<double> acc[4][3];
   double2 own[kAhead][4];
-  const bool ok = apply<double>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, stall_load, acc, own);
+  const bool ok = apply<double>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, stall_load,
+                                early, acc, own);
   cp_async_wait_all();
   constexpr int NQ = MODE == MV_T2 ? 5 : MODE == MV_RES2 ? 4 : MODE == MV_T ? 3
                    : (MODE == MV_RES || MODE == MV_V || MODE == MV_V2 || MODE == MV_RESC || MODE == MV_CH0 ||
@@ -468,11 +489,11 @@ __global__ void __launch_bounds__(spin::kUnit *spin::kWarps, 2)
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
         const int64_t o = off + (int64_t)r * V;
-        if (kB) e1[h & 1][r] = ldg(A.bvec + o);
-        if (MODE == MV_V) e1[h & 1][r] = ldg(A.in2 + o);
+        if (kB) e1[h & 1][r] = ld_c(A.bvec + o);
+        if (MODE == MV_V) e1[h & 1][r] = ld_c(A.in2 + o);
         if (kCheb) e2[h & 1][r] = ld(A.out + o);
-        if (MODE == MV_CHH) e3[h & 1][r] = ldg(A.in2 + o);
-        if (kShadow) f[h & 1][r][0] = __ldg(A.sh32 + o);
+        if (MODE == MV_CHH) e3[h & 1][r] = ld_c(A.in2 + o);
+        if (kShadow) f[h & 1][r][0] = __ldca(A.sh32 + o);
         if (MODE == MV_RHS)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -584,37 +605,6 @@ __global__ void __launch_bounds__(spin::kUnit *spin::kWarps, 2)
   }
 }
 
-// The Chebyshev coefficients of the segments the bounds give (lo, hi of
-// quark and antiquark), A^H = 1 + i tau H: theta its centre, delta its half
-// length, sigma = theta / delta, rho_0 = 1 / sigma, rho_{k+1} = 1 / (2 sigma
-// - rho_k); x_1 = x_0 + r_0 / theta, then x_{k+1} = x_k + c1 (x_k - x_{k-1})
-// + c2 r_k with c1 = rho_k rho_{k-1}, c2 = 2 rho_k / delta.  One thread per
-// species; the bounds also go to the pinned host_bounds.
-__global__ void k_cheb_tab(const double *__restrict__ bounds, double tau, ChebTab *__restrict__ tab,
-                           double *__restrict__ host_bounds) {
-  const int sp = threadIdx.x;
-  if (sp >= 2) return;
-  const double lo = bounds[2 * sp], hi = bounds[2 * sp + 1];
-  tab->lo[sp] = lo;
-  tab->hi[sp] = hi;
-  host_bounds[2 * sp] = lo;
-  host_bounds[2 * sp + 1] = hi;
-  const cplx one = {1.0, 0.0};
-  const cplx theta = {1.0, tau * 0.5 * (lo + hi)};
-  const cplx delta = {0.0, fmax(fabs(tau) * 0.5 * (hi - lo), 1e-14)};
-  const cplx sigma = cdiv(theta, delta);
-  tab->inv_theta[sp] = cdiv(one, theta);
-  cplx rho = cdiv(one, sigma);
-  tab->step[0].c1[sp] = {0.0, 0.0};
-  tab->step[0].c2[sp] = tab->inv_theta[sp];
-  for (int k = 1; k < kChebTab; ++k) {
-    const cplx rn = cdiv(one, 2.0 * sigma - rho);
-    tab->step[k].c1[sp] = rn * rho;
-    tab->step[k].c2[sp] = cdiv(2.0 * rn, delta);
-    rho = rn;
-  }
-}
-
 // ------------------------------------------------------------------ host
 void launch_spin_prepare(Lat L, const CnCoef &C, const CnCoef *Cm, int nm, double tau, const double2 *U,
                          const double *E, const SpinOp &op, const SpinOp32 &op32, double *scratch, cudaStream_t st) {
@@ -623,24 +613,21 @@ void launch_spin_prepare(Lat L, const CnCoef &C, const CnCoef *Cm, int nm, doubl
 }
 
 void launch_spin_bounds(Lat L, int nm, const double *scratch, double *partials, unsigned *ticket, double *out,
-                        cudaStream_t st) {
-  k_spin_bounds<<<dim3((unsigned)((L.V + 255) / 256), (unsigned)nm), 256, 0, st>>>(L, scratch, partials, ticket, out);
-}
-
-void launch_cheb_tab(const double *bounds, double tau, ChebTab *tab, double *host_bounds, cudaStream_t st) {
-  k_cheb_tab<<<1, 32, 0, st>>>(bounds, tau, tab, host_bounds);
+                        cudaStream_t st, double tau, ChebTab *tab, double *host_bounds) {
+  k_spin_bounds<<<dim3((unsigned)((L.V + 255) / 256), (unsigned)nm), 256, 0, st>>>(L, scratch, partials, ticket, out,
+                                                                                  tau, tab, host_bounds);
 }
 
 bool cn_spin_applicable(const Lat &L) { return L.V <= 0x7fffffffLL; }
 
-void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs &a, int *err, cudaStream_t st,
-                    long long wait_cycles, int stall_load) {
+void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs &a, bool early, int *err,
+                    cudaStream_t st, long long wait_cycles, int stall_load) {
   using namespace spin;
   const unsigned grid = (unsigned)((L.V + kUnit - 1) / kUnit);
   auto go = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<double>));
-    kern<<<grid, kUnit * kWarps, sizeof(Smem<double>), st>>>(L, op, sign, a, SpinBatch{}, err, wait_cycles,
-                                                            stall_load);
+    launch_pdl(kern, grid, kUnit * kWarps, sizeof(Smem<double>), st, L, op, sign, a, SpinBatch{}, err, wait_cycles,
+               stall_load, early);
   };
   switch (mode) {
     case MV_PLAIN: go(k_cn_spin<MV_PLAIN, false>); break;
@@ -667,7 +654,7 @@ void launch_batch_spin(int mode, int order, Lat L, const SpinOp &op, const Batch
   auto go = [&](auto kern) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<double>));
     kern<<<(unsigned)nunits * (unsigned)nfields, kUnit * kWarps, sizeof(Smem<double>), st>>>(
-        L, op, 1.0, MvArgs{}, bt, err, wait_cycles, -1);
+        L, op, 1.0, MvArgs{}, bt, err, wait_cycles, -1, false);
   };
   if (mode == MV_RHS)
     go(k_cn_spin<MV_RHS, true>);

@@ -5,6 +5,7 @@
 // cn_spin.cu.
 #pragma once
 #include "nrq_kernels.cuh"
+#include "pdl.cuh"
 #include "stage.cuh"
 
 namespace nrq {
@@ -167,13 +168,15 @@ __device__ __forceinline__ void init_barriers(Smem<T> &sm) {
 
 // acc = (A^H - 1) in of column c (the warp's) at the lane's site x:
 // acc[species*2 + spin][colour]; the input at x itself is left in
-// own[(18 + colour) % kAhead].  W, S0, S1: the operator's planes.  Returns
-// false where a wait ran out.
+// own[(18 + colour) % kAhead].  W, S0, S1: the operator's planes.  The kernel
+// before this one on the stream may still run (pdl.cuh) until the input is
+// read; early: the operator is none of its results, so that the first matrices
+// are staged before that.  Returns false where a wait ran out.
 template <typename T>
 __device__ __forceinline__ bool apply(const Lat &L, const typename Num<T>::v2 *__restrict__ W,
                                       const typename Num<T>::v2 *__restrict__ S0, const T *__restrict__ S1,
                                       const typename Num<T>::v2 *__restrict__ in, int x, int c, Smem<T> &sm, int *err,
-                                      long long wait_cycles, int stall_load, cx<T> (&acc)[4][3],
+                                      long long wait_cycles, int stall_load, bool early, cx<T> (&acc)[4][3],
                                       typename Num<T>::v2 (&own)[Num<T>::kAhead][4]) {
   using V2 = typename Num<T>::v2;
   constexpr int kAhead = Num<T>::kAhead, kDist = Num<T>::kDist, kBufs = Smem<T>::kBufs;
@@ -198,12 +201,15 @@ __device__ __forceinline__ bool apply(const Lat &L, const typename Num<T>::v2 *_
   auto load = [&](int t, V2(&q)[4]) {
     const int y = t < 18 ? nbr[t / 3] : x;
     const int64_t o = (int64_t)(2 * (t % 3)) * V + y;
-    q[0] = __ldg(pq + o);
-    q[1] = __ldg(pq + o + V);
-    q[2] = __ldg(pa + o);
-    q[3] = __ldg(pa + o + V);
+    q[0] = __ldca(pq + o);
+    q[1] = __ldca(pq + o + V);
+    q[2] = __ldca(pa + o);
+    q[3] = __ldca(pa + o + V);
   };
+  if (!early) pdl_wait();
   stage(0);
+  if (early) pdl_wait();
+  pdl_trigger();
 #pragma unroll
   for (int t = 0; t < kAhead - 1; ++t) load(t, own[t]);
 #pragma unroll

@@ -45,7 +45,7 @@ __device__ __forceinline__ cx<float> cmul(cx<float> a, cx<float> b) {
 // history instead of out.
 template <bool FIRST, bool LAST, bool BATCH>
 __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
-    k_cheb_spin(Lat L, SpinOp32 op, Step32 A, Batch32 Bt, int *err, long long wait_cycles) {
+    k_cheb_spin(Lat L, SpinOp32 op, Step32 A, Batch32 Bt, int *err, long long wait_cycles, bool early) {
   constexpr int kAhead = Num<float>::kAhead;
   __shared__ __align__(16) Smem<float> sm;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
   const int x = act ? s : V - 1;  // a valid site for the addresses of idle lanes
   cx<float> acc[4][3];
   float2 own[kAhead][4];
-  const bool ok = apply<float>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, -1, acc, own);
+  const bool ok = apply<float>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, -1, early, acc, own);
   cp_async_wait_all();
   if (!ok || !act) return;
 #pragma unroll
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const int64_t o = off + (int64_t)q * V;
-        if (!FIRST) rv[q] = __ldg(A.r + o);
+        if (!FIRST) rv[q] = __ldca(A.r + o);
         if (!FIRST && A.prev) pv[q] = A.prev[o];
         if (LAST) xv[q] = A.x[o];
         if (LAST && A.hist) hv[q] = A.hist[o];
@@ -156,9 +156,12 @@ __global__ void k_cheb_one(int64_t n, Step32 A, const BatchField *__restrict__ t
 
 template <bool BATCH>
 void go(bool first, bool last, int64_t blocks, Lat L, const SpinOp32 &op, const Step32 &A, const Batch32 &Bt, int *err,
-        cudaStream_t st, long long wait_cycles) {
+        cudaStream_t st, long long wait_cycles, bool early) {
   auto run = [&](auto kern) {
-    kern<<<(unsigned)blocks, kUnit * kWarps, 0, st>>>(L, op, A, Bt, err, wait_cycles);
+    if (BATCH)  // (captured into graphs)
+      kern<<<(unsigned)blocks, kUnit * kWarps, 0, st>>>(L, op, A, Bt, err, wait_cycles, false);
+    else
+      launch_pdl(kern, (unsigned)blocks, kUnit * kWarps, 0, st, L, op, A, Bt, err, wait_cycles, early);
   };
   if (first && last)
     run(k_cheb_spin<true, true, BATCH>);
@@ -176,8 +179,8 @@ bool cheb_spin_applicable(const Lat &L) {
 }
 
 void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const float2 *r, float2 *ea, float2 *eb,
-                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], int *err, cudaStream_t st,
-                      long long wait_cycles) {
+                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], bool early, int *err,
+                      cudaStream_t st, long long wait_cycles) {
   Step32 A{};
   A.in = step == 0 ? r : (step & 1) ? ea : eb;
   A.r = r;
@@ -190,7 +193,7 @@ void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const floa
     A.c2[sp] = K.c2[sp];
     A.it[sp] = inv_theta[sp];
   }
-  go<false>(step == 0, last, (L.V + kUnit - 1) / kUnit, L, op, A, Batch32{}, err, st, wait_cycles);
+  go<false>(step == 0, last, (L.V + kUnit - 1) / kUnit, L, op, A, Batch32{}, err, st, wait_cycles, early);
 }
 
 void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const cplx inv_theta[2], cudaStream_t st) {
@@ -207,7 +210,7 @@ void launch_batch_cheb_spin(int step, bool last, int order, Lat L, const SpinOp3
                             int nfields, int *err, cudaStream_t st, long long wait_cycles) {
   const int nunits = (int)((L.V + kUnit - 1) / kUnit);
   go<true>(step == 0, last, (int64_t)nunits * nfields, L, op, Step32{}, Batch32{tab, nfields, nunits, order, step},
-           err, st, wait_cycles);
+           err, st, wait_cycles, false);
 }
 
 void launch_batch_cheb_one(int64_t n, const BatchField *tab, int nfields, cudaStream_t st) {

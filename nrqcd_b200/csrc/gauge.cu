@@ -467,11 +467,12 @@ __global__ void __launch_bounds__(256) k_gauss(Lat L, const double2 *__restrict_
 __global__ void k_reduce_final(const double *__restrict__ partials, int64_t nblk, int nq,
                                unsigned maxmask, double *out) {
   __shared__ double sh[256];
+  pdl_wait();
   for (int q = blockIdx.x; q < nq; q += gridDim.x) {
     const bool isMax = (maxmask >> q) & 1u;
     double acc = 0.0;
     for (int64_t b = threadIdx.x; b < nblk; b += blockDim.x) {
-      double v = partials[b * nq + q];
+      double v = __ldcg(partials + b * nq + q);
       acc = isMax ? fmax(acc, v) : acc + v;
     }
     sh[threadIdx.x] = acc;
@@ -484,6 +485,11 @@ __global__ void k_reduce_final(const double *__restrict__ partials, int64_t nblk
     if (threadIdx.x == 0) out[q] = sh[0];
     __syncthreads();
   }
+}
+
+void launch_reduce_final(const double *partials, int64_t nblk, int nq, unsigned maxmask, double *out,
+                         cudaStream_t st) {
+  launch_pdl(k_reduce_final, (unsigned)nq, 256, 0, st, partials, nblk, nq, maxmask, out);
 }
 
 // ------------------------------------------------------------ initial condition

@@ -187,6 +187,7 @@ struct nrq_cn {
   // scratch planes and partial rows of the spectral enclosure and its ticket
   nrq::SpinOp spin{};
   bool spin_valid = false;
+  bool spin_fresh = false;  // written by the latest launch on the stream
   nrq::CnCoef spin_coef{};
   double spin_tau = 0.0;
   double *spin_scratch = nullptr, *spin_part = nullptr;

@@ -26,6 +26,7 @@ __global__ void k_energy(Lat L, const double2 *__restrict__ U, const double *__r
 __global__ void k_gauss(Lat L, const double2 *__restrict__ U, const double *__restrict__ E, double *partials);
 __global__ void k_reduce_final(const double *__restrict__ partials, int64_t nblk, int nq, unsigned maxmask,
                                double *out);
+void launch_reduce_final(const double *partials, int64_t nblk, int nq, unsigned maxmask, double *out, cudaStream_t st);
 __global__ void k_ic_pspace(Lat L, const double2 *__restrict__ R, const double *__restrict__ mtab,
                             double fwd_scale, double Q, double n0, double g, double2 *__restrict__ A,
                             double2 *__restrict__ Ef);
@@ -151,6 +152,52 @@ struct ChebTab {
   double lo[2], hi[2];
 };
 
+// Chebyshev iteration on the segment of A^H = 1 + i tau H, spec(H) in [lo, hi]:
+// theta its centre, delta its half length, sigma = theta / delta.  The ratios
+// rho_k = T_k(sigma) / T_{k+1}(sigma), which the recurrence rho_0 = 1 / sigma,
+// rho_{k+1} = 1 / (2 sigma - rho_k) makes one after another, come here from
+// T_k = (w^k + w^-k) / 2, w = sigma + sqrt(sigma^2 - 1), |w| > 1, each by
+// itself.  x_1 = x_0 + r_0 / theta, x_{k+1} = x_k + rho_k rho_{k-1} (x_k -
+// x_{k-1}) + c2(rho_k) r_k.
+struct ChebSegment {
+  cplx theta, winv, u;  // u = w^-2
+  double half;
+  __device__ ChebSegment(double tau, double lo, double hi) {
+    theta = {1.0, tau * 0.5 * (lo + hi)};
+    half = fmax(fabs(tau) * 0.5 * (hi - lo), 1e-14);
+    const cplx sigma = {theta.im / half, -theta.re / half};  // over i half
+    const cplx z = sigma * sigma - cplx{1.0, 0.0};
+    const double m = sqrt(0.5 * (hypot(z.re, z.im) + fabs(z.re)));
+    cplx r = z.re >= 0.0 ? cplx{m, m > 0.0 ? 0.5 * z.im / m : 0.0} : cplx{0.5 * fabs(z.im) / m, copysign(m, z.im)};
+    if (sigma.re * r.re + sigma.im * r.im < 0.0) r = -1.0 * r;
+    winv = cdiv({1.0, 0.0}, sigma + r);
+    u = winv * winv;
+  }
+  __device__ cplx pow_u(int k) const {
+    cplx p = {1.0, 0.0}, b = u;
+    for (; k > 0; k >>= 1) {
+      if (k & 1) p = p * b;
+      b = b * b;
+    }
+    return p;
+  }
+  __device__ cplx rho(int k) const {
+    const cplx one = {1.0, 0.0}, p = pow_u(k);
+    return cdiv(winv * (one + p), one + p * u);
+  }
+  // |T_m(sigma)|
+  __device__ double gain(int m) const {
+    double g = 0.5 * sqrt(norm2(cplx{1.0, 0.0} + pow_u(m))), b = 1.0 / sqrt(norm2(winv));
+    for (; m > 0; m >>= 1) {
+      if (m & 1) g *= b;
+      b *= b;
+    }
+    return g;
+  }
+  __device__ cplx inv_theta() const { return cdiv({1.0, 0.0}, theta); }
+  __device__ cplx c2(cplx rho) const { return {2.0 * rho.im / half, -2.0 * rho.re / half}; }
+};
+
 // The operator in its spin structure (cn_spin.cu), real Wilson coefficients:
 // A^H psi(x) = (1 + i (S0 +- S1)) psi(x) + the six neighbours' blocks from
 // three colour matrices a direction.  Planes of V: W 81 complex ((I*3 + m)*9
@@ -170,15 +217,17 @@ struct SpinOp32 {
 void launch_spin_prepare(Lat L, const CnCoef &C, const CnCoef *Cm, int nm, double tau, const double2 *U,
                          const double *E, const SpinOp &op, const SpinOp32 &op32, double *scratch, cudaStream_t st);
 // out[4*set] = {lo, hi} of the quark's and the antiquark's H, A^H = 1 + i tau
-// H; partials: 4 doubles per 256 sites and set; ticket: one zero per set
+// H; partials: 4 doubles per 256 sites and set; ticket: one zero per set.  One
+// set and tab: also the Chebyshev table of these bounds, and the bounds into
+// the pinned host_bounds.
 void launch_spin_bounds(Lat L, int nm, const double *scratch, double *partials, unsigned *ticket, double *out,
-                        cudaStream_t st);
-void launch_cheb_tab(const double *bounds, double tau, ChebTab *tab, double *host_bounds, cudaStream_t st);
+                        cudaStream_t st, double tau = 0.0, ChebTab *tab = nullptr, double *host_bounds = nullptr);
 bool cn_spin_applicable(const Lat &L);
 // the stencil over op (sign = -1: A = 2 - A^H, for MV_PLAIN and MV_RHS); one
-// partial row per 32-site block
-void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs &a, int *err, cudaStream_t st,
-                    long long wait_cycles, int stall_load);
+// partial row per 32-site block.  early: the launch before this one on the
+// stream did not write op.
+void launch_cn_spin(int mode, Lat L, const SpinOp &op, double sign, const MvArgs &a, bool early, int *err,
+                    cudaStream_t st, long long wait_cycles, int stall_load);
 
 constexpr int CN_SITES_PER_BLOCK = 32;
 constexpr int CN_COLS = 12;  // 2 species x 6 propagator columns
@@ -328,8 +377,8 @@ void launch_cheb32(bool first, Lat L, const CnCoef &C, const float2 *U, const fl
 // launches, one step is launch_cheb_one over the n elements.
 bool cheb_spin_applicable(const Lat &L);
 void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const float2 *r, float2 *ea, float2 *eb,
-                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], int *err, cudaStream_t st,
-                      long long wait_cycles);
+                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], bool early, int *err,
+                      cudaStream_t st, long long wait_cycles);
 void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const cplx inv_theta[2], cudaStream_t st);
 void launch_add_e(int64_t n, double2 *X, const float2 *E, cudaStream_t st);
 void launch_prop_f2soa(const double2 *f, double2 *P, int64_t V, cudaStream_t st);

@@ -15,15 +15,16 @@ namespace nrq {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+__device__ __forceinline__ cplx ld_c(const double2 *p) {
+  const double2 v = __ldca(p);
+  return {v.x, v.y};
+}
 // link U_d(s), coherently
 __device__ __forceinline__ m3 load_link_c(const double2 *U, int64_t V, int64_t s, int d) {
   m3 m;
   const double2 *p = U + (int64_t)d * 9 * V + s;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const double2 v = __ldca(p + k * V);
-    m.e[k] = {v.x, v.y};
-  }
+  for (int k = 0; k < 9; ++k) m.e[k] = ld_c(p + k * V);
   return m;
 }
 
