@@ -131,8 +131,9 @@ constexpr int kPrepSites = 32;
 // the site term of the hermitian H (A^H = 1 + i tau H) for quark and
 // antiquark.  One thread per site and direction; the Darwin and magnetic
 // matrices are sums over directions, exchanged through shared memory.  64^3:
-// 280 us (254 registers, 8 warps an SM; the FP64 pipe 28 % active), 12^3: 10 us.
-__global__ void __launch_bounds__(kPrepSites * 3) k_spin_prepare(Lat L, CnCoef C1, const CnCoef *__restrict__ Cm,
+// 240 us at 12 warps an SM (168 registers; 255 registers, 8 warps: 315, 136
+// registers, 15 warps: 280), of which the traffic takes 90; 12^3: 10 us.
+__global__ void __launch_bounds__(kPrepSites * 3, 4) k_spin_prepare(Lat L, CnCoef C1, const CnCoef *__restrict__ Cm,
                                                                 int nm, double tau, const double2 *__restrict__ U,
                                                                 const double *__restrict__ E, SpinOp op,
                                                                 SpinOp32 op32, double *__restrict__ scratch) {

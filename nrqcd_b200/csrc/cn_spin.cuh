@@ -25,7 +25,7 @@ struct Num<double> {
   // Prefetches to L2, of the epilogue's operands or of later units', cost
   // 2-20 %; a persistent form with the next unit's first loads issued early
   // 10 %.)
-  static constexpr int kAhead = 4, kDist = 2;
+  static constexpr int kAhead = 4, kDist = 2;  // kAhead >= 3: the input at the site itself stays
 };
 template <>
 struct Num<float> {
