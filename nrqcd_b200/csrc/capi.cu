@@ -980,13 +980,12 @@ extern "C" int nrq_gauge_transverse_correlators(nrq_gauge *g, double *aa, double
     ctx->last_error = "transverse correlators: cufftPlanMany failed";
     return NRQ_ERR_CUDA;
   }
-  const unsigned nb_ = (unsigned)nblk(V, 128);
   const double fwd = ctx->a[1] * ctx->a[2] * ctx->a[3];
-  nrq::k_gluon_fields<<<dim3(nb_, 3), 128, 0, ctx->stream>>>(L, g->U, g->E, F);
+  nrq::k_gluon_fields<<<dim3((unsigned)nblk(V, 128), 3), 128, 0, ctx->stream>>>(L, g->U, g->E, F);
   bool ok = cudaGetLastError() == cudaSuccess &&
             cufftExecZ2Z(plan, (cufftDoubleComplex *)F, (cufftDoubleComplex *)F, CUFFT_FORWARD) == CUFFT_SUCCESS;
   if (ok) {
-    nrq::k_transverse_corr<<<nb_, 128, 0, ctx->stream>>>(L, F, fwd, (double)V * fwd, out);
+    nrq::k_transverse_corr<<<dim3((unsigned)nblk(V, 64), 2), 64, 0, ctx->stream>>>(L, F, fwd, (double)V * fwd, out);
     ok = cudaGetLastError() == cudaSuccess;
   }
   double *dst[3] = {aa, ee, momenta};

@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(128) k_gluon_fields(Lat L, const double2 *__re
   }
 }
 
-// per momentum site: out[0][s] = AA, out[1][s] = EE, out[2][s] = |p|
+// per momentum site and field (blockIdx.y): out[0][s] = AA, out[1][s] = EE, out[2][s] = |p|
 // (F holds the unscaled forward transforms; fwd = a1 a2 a3)
-__global__ void __launch_bounds__(128) k_transverse_corr(Lat L, const double2 *__restrict__ F, double fwd,
+__global__ void __launch_bounds__(64) k_transverse_corr(Lat L, const double2 *__restrict__ F, double fwd,
                                                          double volume, double *__restrict__ out) {
   const int64_t V = L.V;
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -221,27 +221,25 @@ __global__ void __launch_bounds__(128) k_transverse_corr(Lat L, const double2 *_
       const double re = p[i].re * p[j].re + p[i].im * p[j].im;  // Re(conj(p_i) p_j)
       P[i][j] = pn < 1e-12 ? 0.0 : ((i == j ? 1.0 : 0.0) - re / (pn * pn)) / 2.0;
     }
-#pragma unroll 1
-  for (int field = 0; field < 2; ++field) {
-    double acc = 0.0;
-#pragma unroll 1
-    for (int a = 0; a < 8; ++a) {
-      cplx f[3];
+  const int field = blockIdx.y;
+  double acc = 0.0;
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const double2 v = F[(int64_t)(field * 24 + i * 8 + a) * V + s];
-        f[i] = {v.x * fwd, v.y * fwd};
-      }
-      double res = 0.0;  // Re sum_ij f_i P_ij conj(f_j)
+  for (int a = 0; a < 8; ++a) {
+    cplx f[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) res += P[i][j] * (f[i].re * f[j].re + f[i].im * f[j].im);
-      acc += (res / volume) / 8.0;
+    for (int i = 0; i < 3; ++i) {
+      const double2 v = F[(int64_t)(field * 24 + i * 8 + a) * V + s];
+      f[i] = {v.x * fwd, v.y * fwd};
     }
-    out[(int64_t)field * V + s] = acc;
+    double res = 0.0;  // Re sum_ij f_i P_ij conj(f_j)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) res += P[i][j] * (f[i].re * f[j].re + f[i].im * f[j].im);
+    acc += (res / volume) / 8.0;
   }
-  out[2 * V + s] = pn;
+  out[(int64_t)field * V + s] = acc;
+  if (field == 0) out[2 * V + s] = pn;
 }
 
 // ------------------------------------------------------------ short extents
