@@ -627,7 +627,7 @@ constexpr int64_t kProjUnbounded = INT64_MAX;
 // the sweeps up to the crossing, so that the field and the count are those of
 // a test after every sweep; its length follows the decay seen so far, which
 // keeps the repeated part short.  Returns false where the cooperative launch
-// is refused (the caller queues single sweeps).
+// or its workspace is refused (the caller queues single sweeps).
 constexpr int64_t kRunChunk = 512;
 bool gauss_project_run(nrq_gauge *g, double tol, int64_t limit, int64_t *sweeps, double *deviation, int *rc) {
   nrq_ctx *ctx = g->ctx;
@@ -635,7 +635,10 @@ bool gauss_project_run(nrq_gauge *g, double tol, int64_t limit, int64_t *sweeps,
   cudaStream_t st = ctx->stream;
   const size_t mb = (size_t)nrq::gauss_run_message_bytes(V), eb = sizeof(double) * 24 * V;
   const size_t db = sizeof(double) * (kRunChunk + 1) * (nw + 1);
-  if ((*rc = ensure_stage(ctx, mb + eb + db + sizeof(int)))) return true;
+  if (ensure_stage(ctx, mb + eb + db + sizeof(int))) {
+    cudaGetLastError();
+    return false;
+  }
   char *base = (char *)ctx->d_stage;
   double *E2 = (double *)(base + mb), *dev = (double *)(base + mb + eb), *devmax = dev + (kRunChunk + 1) * nw;
   int *err = (int *)(base + mb + eb + db);
@@ -866,9 +869,10 @@ double max_norm2_momentum(const nrq_ctx *ctx) {
   return std::sqrt(s);
 }
 // The gauge fixing on short extents: batches of iterations without a host
-// synchronisation, decided on the device (k_cg_rows)
+// synchronisation, decided on the device (k_cg_rows); *refused: its workspace
+// does not fit the memory
 int coulomb_short(nrq_gauge *g, double tol, double alpha, int64_t max_iterations, int64_t *iterations,
-                  double *deviations) {
+                  double *deviations, bool *refused) {
   nrq_ctx *ctx = g->ctx;
   const nrq::Lat L = ctx->lat;
   const int64_t V = L.V;
@@ -876,7 +880,11 @@ int coulomb_short(nrq_gauge *g, double tol, double alpha, int64_t max_iterations
   constexpr int kBatch = 32;  // most iterations between two read-backs
   const size_t tabs = 3 * nrq::kCgMaxExtent;
   int rc = ensure_gluon(ctx, sizeof(double2) * (41 * V + tabs) + sizeof(double) * (tabs + kBatch));
-  if (rc) return rc;
+  *refused = rc != NRQ_OK;
+  if (rc) {
+    cudaGetLastError();
+    return rc;
+  }
   double2 *U2 = (double2 *)ctx->d_gluon, *F = U2 + 27 * V, *G = F + 5 * V, *tw = G + 9 * V;
   double *p2 = (double *)(tw + tabs), *dev = p2 + tabs;
   nrq::launch_cg_tables(L, tw, p2, st);
@@ -925,8 +933,9 @@ extern "C" int nrq_gauge_coulomb_gaugefix(nrq_gauge *g, double tol, double alpha
   if (!rc) rc = gauge_sync64(g);
   if (rc) return rc;
   if (nrq::cg_short_applicable(L)) {
-    rc = coulomb_short(g, tol, alpha, max_iterations, iterations, deviations);
-    return rc ? rc : gauge_written64(g);
+    bool refused = false;
+    rc = coulomb_short(g, tol, alpha, max_iterations, iterations, deviations, &refused);
+    if (!refused) return rc ? rc : gauge_written64(g);
   }
   const unsigned nb_ = (unsigned)nblk(V, 128);
   if ((rc = ensure_red(ctx, nb_))) return rc;
@@ -1981,14 +1990,16 @@ static bool accept_recursive(const nrq_cn *cn, const double rel[nrq::CN_COLS]) {
 // two vector passes and three scalar stages for the same two orders of
 // application; the step count follows from the first residual and the
 // segment, |r_m| <= |r_0| / |T_m(sigma)| in every column, so the host reads
-// the device once a solve.  64^3: 0.41 ms a step against 1.40 ms an
+// the device once a solve.  64^3: 0.38 ms a step against 1.40 ms an
 // iteration.
 //
 // The bound is rigorous, so a solve ends on it (after m steps max_rel is the
 // bound); the first solve, every 16th after it and, with confirm_always,
 // every one confirm with the true residual.  Returns false, with x0 still in
 // cn->x, where the enclosure is not finite or the segment asks for more than
-// kChebTab or maxits steps (light quarks, large steps): BiCGStab takes those.
+// kChebTab or maxits steps (light quarks, large steps): BiCGStab takes those,
+// with two passes.  (kChebTab = 40 is about where its adaptivity overtakes the
+// bound: the enclosure asks for 3-6 times its iterations.)
 static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const nrq::CnCoef &CH, int64_t matvecs,
                            int64_t vstreams, nrq_cn_stats *stats, int *status_out) {
   nrq_ctx *ctx = cn->ctx;
@@ -2169,12 +2180,20 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
   if ((rc = cn_prepare(cn, g, dt))) return rc;
   if (!cn->stencil_tuned && (rc = tune_stencil(cn, CH, g))) return rc;
   int64_t matvecs = 0, vstreams = 0;
-  const bool fma = cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(CH) && nrq::cn_spin_applicable(L);
-  const bool semi = fma && cn->semi_iter;
+  bool fma = cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(CH) && nrq::cn_spin_applicable(L);
   if (fma) {
     double sign = 0.0;
-    if ((rc = ensure_spin(cn, CH, g, &sign))) return rc;
+    rc = ensure_spin(cn, CH, g, &sign);
+    if (rc && !cn->spin.W && !cn->tma_ok && cn->forced_stencil < 0) {
+      // no memory for the operator: the stencil that needs none
+      cudaGetLastError();
+      cn->stencil = NRQ_STENCIL_REGISTER;
+      fma = false;
+      rc = NRQ_OK;
+    }
+    if (rc) return rc;
   }
+  const bool semi = fma && cn->semi_iter;
   if (semi) {  // the Chebyshev coefficients, ahead of the right-hand side
     if (!cn->cheb_tab) NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->cheb_tab, sizeof(nrq::ChebTab)));
     if (!cn->h_cheb) {
@@ -2213,7 +2232,10 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
   // keeps the shadow residual rh in FP32, in the first half of the rh
   // buffer: any fixed shadow vector serves BiCGStab, and every product
   // with it (rho_0 included) uses the same rounded values
-  const bool merged = cn->merged_update && cn->last_stencil == NRQ_STENCIL_FMA;
+  // (not after the semi-iteration has declined: the steps that need more than
+  // its table are large against the inverse of H, and there the merged beta
+  // and the FP32 shadow stagnate where two passes converge)
+  const bool merged = cn->merged_update && cn->last_stencil == NRQ_STENCIL_FMA && !semi;
   float2 *const sh32 = merged ? reinterpret_cast<float2 *>(cn->rh) : nullptr;
   bool restart = true, just_restarted = false;
   bool half_accept = false;  // ended at a half step on the recursive |s|

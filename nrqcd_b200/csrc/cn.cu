@@ -21,9 +21,10 @@
 //   alpha_so = -kappa c4/(8M^2); antiquark: M -> -M, c -> conj(c).
 //
 // Layout: propagator planes (species*36 + col*6 + row), V complex each.
-// The stencil kernels live in cn_mv3.cu (TMA-staged) and cn_mv.cu
-// (register-tiled); this file holds the per-step preparation, the BiCGStab
-// vector updates and scalar stages, and the propagator I/O and observables.
+// The stencil kernels live in cn_spin.cu (the default), cn_mv4.cu
+// (tensor-core), cn_mv3.cu (TMA-staged) and cn_mv.cu (register-tiled); this
+// file holds the per-step preparation of the last three, the BiCGStab vector
+// updates and scalar stages, and the propagator I/O and observables.
 #include <algorithm>
 
 #include "nrq_eigen.cuh"

@@ -158,7 +158,7 @@ template <bool BATCH>
 void go(bool first, bool last, int64_t blocks, Lat L, const SpinOp32 &op, const Step32 &A, const Batch32 &Bt, int *err,
         cudaStream_t st, long long wait_cycles, bool early) {
   auto run = [&](auto kern) {
-    if (BATCH)  // (captured into graphs)
+    if (BATCH)
       kern<<<(unsigned)blocks, kUnit * kWarps, 0, st>>>(L, op, A, Bt, err, wait_cycles, false);
     else
       launch_pdl(kern, (unsigned)blocks, kUnit * kWarps, 0, st, L, op, A, Bt, err, wait_cycles, early);

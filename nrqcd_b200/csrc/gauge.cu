@@ -128,25 +128,12 @@ __global__ void __launch_bounds__(6 * kForceSites, 5) k_update_efield(Lat L, con
   for (int a = 0; a < 4; ++a) e[(int64_t)a * V] -= 2.0 * (kk ? f[4 + a] : f[a]);
 }
 
-// the two kernels of a leapfrog step, in either order; inside a capture as
-// ordinary launches
-namespace {
-template <typename K, typename... A>
-void launch_leapfrog(K kernel, unsigned block, int sites, Lat L, cudaStream_t st, A... args) {
-  const unsigned grid = (unsigned)((L.V + sites - 1) / sites);
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(st, &capture);
-  if (capture == cudaStreamCaptureStatusNone)
-    launch_pdl(kernel, grid, block, 0, st, L, args...);
-  else
-    kernel<<<grid, block, 0, st>>>(L, args...);
-}
-}  // namespace
+// the two kernels of a leapfrog step, in either order
 void launch_update_links(Lat L, double2 *U, const double *E, double dt, cudaStream_t st) {
-  launch_leapfrog(k_update_links, 3 * kLinkSites, kLinkSites, L, st, U, E, dt);
+  launch_pdl(k_update_links, (unsigned)((L.V + kLinkSites - 1) / kLinkSites), 3 * kLinkSites, 0, st, L, U, E, dt);
 }
 void launch_update_efield(Lat L, const double2 *U, double *E, double dt, cudaStream_t st) {
-  launch_leapfrog(k_update_efield, 6 * kForceSites, kForceSites, L, st, U, E, dt);
+  launch_pdl(k_update_efield, (unsigned)((L.V + kForceSites - 1) / kForceSites), 6 * kForceSites, 0, st, L, U, E, dt);
 }
 
 // ------------------------------------------------------------ FP32 links

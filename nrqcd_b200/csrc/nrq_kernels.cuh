@@ -144,7 +144,7 @@ struct ChebCoef {
 
 // the Chebyshev coefficients of one operator by step (step[0]: c1 = 0, c2 =
 // 1/theta) and the enclosure of its hermitian part they were made for
-// (k_cheb_tab, cn_spin.cu)
+// (k_spin_bounds, cn_spin.cu)
 constexpr int kChebTab = 40;
 struct ChebTab {
   ChebCoef step[kChebTab];

@@ -28,6 +28,7 @@ __device__ __forceinline__ m3 load_link_c(const double2 *U, int64_t V, int64_t s
   return m;
 }
 
+// (inside a capture an ordinary launch: graphs keep full dependencies)
 template <typename... P, typename... A>
 cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchAttribute attr{};
@@ -38,8 +39,10 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(st, &capture);
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = capture == cudaStreamCaptureStatusNone ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
