@@ -54,7 +54,7 @@ STENCIL_DRAM_BYTES_PER_SITE = {2: 7968.0, 3: 7722.0}
 LEAPFROG_FORCE_FLOPS_PER_SITE = 27 * 27 * 4 * 2
 # FP64 stencils of the solver, by NRQ_STENCIL_* index
 STENCIL_NAMES = {0: "k_cn_mv2 (register-tiled)", 1: "k_cn_mv3 (TMA-staged)", 2: "k_cn_mv4 (FP64 tensor cores)",
-                 3: "k_cn_mv5 (FP64 FMA on cached blocks)"}
+                 3: "k_cn_spin (FP64 FMA, spin structure)"}
 
 
 def parse():
@@ -404,11 +404,11 @@ def measure_gluon_distribution(L, cpu=True, steps=10):
 
 # ------------------------------------------------------------------ CN forms
 # name -> (form, history start, merged update, confirm every solve) of the
-# plain form; the speed-ups are against plain_fp64_bicgstab, the library's
-# default plain solve (start extrapolated from the field's history, x, r and
-# p updated in one pass, the recursive residual accepted with the measured
-# margin); beside it the plain solve from 2b - psi alone and the plain solve
-# with two update passes and every solve confirmed by the true residual
+# plain form; the speed-ups are against plain_fp64_bicgstab, the plain solve
+# by BiCGStab (start extrapolated from the field's history, x, r and p updated
+# in one pass, the recursive residual accepted with the measured margin);
+# beside it the same from 2b - psi alone and with two update passes and every
+# solve confirmed by the true residual
 FORMS = {"plain_fp64_bicgstab": (0, 1, 1, 0), "plain_fp64_bicgstab_no_history": (0, 0, 1, 0),
          "plain_fp64_bicgstab_two_pass_confirmed": (0, 1, 0, 1),
          "precision_fp32_chebyshev_fp64_refinement": (1, 1, 1, 0), "learned_guess_precision": (2, 1, 1, 0)}
@@ -995,7 +995,7 @@ def main():
     stencil = {"in_use": nrqcd.STENCIL_NAMES[which],
                "tuning_ms_per_launch": {"k_cn_mv2": float(tune_ms[0]), "k_cn_mv3_with_vec_s": float(tune_ms[1]),
                                         "k_cn_mv4_with_vec_s": float(tune_ms[2]),
-                                        "k_cn_mv5_with_vec_s": float(tune_ms[3])}}
+                                        "k_cn_spin_with_vec_s": float(tune_ms[3])}}
 
     # ---------------- leapfrog-only steps (the long leapfrog phases before the
     # propagators start), CUDA events on the library stream
@@ -1070,10 +1070,11 @@ def main():
         # 12-column launch: U and E once per species (2 x 624 B) plus 1152 B
         # per vector stream; the tensor-core stencil's design reads its cached
         # 6x6 blocks (3456 B) and diagonal matrices (216 B) in place of U and
-        # E, reported beside it and not credited
+        # E, the FMA stencil's the operator in its spin structure (1296 and
+        # 216 B), reported beside it and not credited
         achieved = sten["bytes"] / (sten["ms"] / 1000.0) / 1e9 if sten["ms"] > 0 else None
         tensor = which in (nrqcd.STENCIL_TENSOR, nrqcd.STENCIL_FMA)
-        blk_bytes = 3552.0 if which == nrqcd.STENCIL_FMA else 3456.0
+        blk_bytes = 1296.0 if which == nrqcd.STENCIL_FMA else 3456.0
         design_bytes = sten["bytes"] + (sten["launches"] * V * (blk_bytes + 216.0 - 1248.0) if tensor else 0.0)
         # FP64 arithmetic of one 12-column stencil launch per site: 2 species x
         # (6 neighbours x 6 columns x 36 + 6 columns x 18) complex FMAs (4 DFMA
@@ -1099,7 +1100,7 @@ def main():
             "warmup": max(3, args.warmup), "ms_per_step": ms_per_step, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
             "config": dict(workload_config(L, world),
-                           bicgstab_update="two-pass" if args.two_pass else "merged",
+                           plain_solve="BiCGStab, two-pass update" if args.two_pass else "Chebyshev semi-iteration",
                            history_depth=args.history_depth if args.history_depth is not None else "default"),
             "roofline": {"bound": "hbm", "kernel": "CN 12-column stencil: " + stencil["in_use"],
                          "achieved": achieved, "peak": peak, "unit": "GB/s",

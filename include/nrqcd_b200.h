@@ -185,12 +185,15 @@ int nrq_heavy_correlators_gconjg(nrq_heavy *h, double out[8]);
 
 /* ---- Crank-Nicolson solver module: src/nrqcd.f90:167-212, 619-869 ------ */
 /* InitModule(Mass, WilsonCoeffs, StepWidth, kspTol); c = 4 complex (8 doubles).
- * form: 0 = plain FP64 (BiCGStab, fused stencil/axpy/dot kernels);
+ * form: 0 = plain FP64 (Chebyshev semi-iteration on the FMA stencil, else
+ *           BiCGStab, with fused stencil/axpy/dot kernels);
  *       1 = precision (FP32 Chebyshev inner iterations inside FP64
  *           iterative refinement to the same tol; real Wilson coefficients).
  * maxits bounds the Krylov iterations (the reference's PETSc default 1e4):
- * BiCGStab iterations of the plain form, FP32 Chebyshev inner steps of the
- * precision forms (over all refinement passes of one update).              */
+ * Chebyshev steps or BiCGStab iterations of the plain form (where the steps
+ * the Chebyshev bound asks for exceed it, BiCGStab runs), FP32 Chebyshev
+ * inner steps of the precision forms (over all refinement passes of one
+ * update).                                                                 */
 int nrq_cn_init(nrq_ctx *ctx, double mass, const double c[8], double stepwidth, double tol,
                 int64_t maxits, int form, nrq_cn **cn);
 /* FinalizeModule, src/nrqcd.f90:199-212 */
@@ -198,9 +201,11 @@ int nrq_cn_finalize(nrq_cn *cn);
 /* FP64 stencils of the solver (no reference counterpart: PETSc applies its
  * assembled matrix; these apply the same operator matrix-free).
  * REGISTER: register-tiled; TMA: TMA-staged; TENSOR: FP64 tensor-core MMAs
- * on per-update 6x6 blocks; FMA: FP64 FMAs on the same per-update blocks
+ * on per-update 6x6 blocks; FMA: FP64 FMAs on the per-update operator in
+ * its spin structure, three colour matrices a direction for both species
  * (TENSOR and FMA need real Wilson coefficients; otherwise the TMA or
- * register-tiled stencil runs).                                           */
+ * register-tiled stencil runs).  Lattices that tensor maps cannot describe
+ * (odd volumes) run FMA where the coefficients allow it.                  */
 #define NRQ_STENCIL_REGISTER 0
 #define NRQ_STENCIL_TMA 1
 #define NRQ_STENCIL_TENSOR 2
@@ -211,8 +216,8 @@ int nrq_cn_finalize(nrq_cn *cn);
 int nrq_cn_stencil_info(const nrq_cn *cn, int *stencil, double ms[4]);
 /* Test hook of the FMA stencil's bounded pipeline waits (no reference
  * counterpart).  wait_cycles bounds every wait (0 restores the default,
- * about two seconds); stall_load >= 0 makes the stencil's loader stop
- * before that load of every CTA, so the wait for it runs out: the update
+ * about two seconds); stall_load >= 0 makes every CTA stop staging before
+ * that neighbour's matrices, so the wait for them runs out: the update
  * then returns NRQ_ERR_TIMEOUT, nothing faults, and the context stays
  * usable.  -1 (the default) stops nowhere.                                */
 int nrq_cn_set_wait_test(nrq_cn *cn, int64_t wait_cycles, int stall_load);
@@ -221,8 +226,8 @@ int nrq_cn_set_wait_test(nrq_cn *cn, int64_t wait_cycles, int stall_load);
 int nrq_cn_set_stencil(nrq_cn *cn, int stencil);
 /* The FP32 Chebyshev step of the precision forms (forms 1 and 2; no
  * reference counterpart).  REGISTER: the operator assembled from FP32 links
- * and field strengths per launch; BLOCKS: FP32 FMAs on per-update 6x6
- * blocks staged by TMA (V a multiple of 4, V >= 36, nx even).  -1 (the
+ * and field strengths per launch; BLOCKS: FP32 FMAs on the per-update
+ * operator in its spin structure (V a multiple of 4, V >= 36, nx even).  -1 (the
  * default) times both on the first update where BLOCKS applies and keeps
  * the faster; forcing BLOCKS on a lattice it cannot describe is
  * NRQ_ERR_BAD_ARG.  nrq_cn_cheb_info gives the step the last update ran
@@ -260,8 +265,9 @@ int nrq_cn_set_history_depth(nrq_cn *cn, int depth);
  * the first solve and every 16th after an unconfirmed run confirm.
  * nrq_cn_true_residual_info: whether the last update's max_rel_residual is
  * the true residual (1) or the recursive or predicted one (0).            */
-/* Plain form on the FMA stencil: on = 1 (the default) updates x, r and p of
- * an iteration in one pass, beta taken from rh.t, which the t = A^H s launch
+/* Plain form on the FMA stencil: selects BiCGStab in place of the Chebyshev
+ * semi-iteration (the default).  on = 1 updates x, r and p of an iteration
+ * in one pass, beta taken from rh.t, which the t = A^H s launch
  * reduces (rh.s vanishes by the choice of alpha, so rho_new = -omega rh.t),
  * with the shadow residual rh kept in FP32 (every product with it, rho_0
  * included, uses the same rounded values); 0 keeps two passes (x and r,
@@ -340,8 +346,8 @@ int nrq_cn_batch_info(const nrq_cn_batch *batch, int *variant, int *order, doubl
  * restore the timed choice (variant -1).  The next update recalibrates.    */
 int nrq_cn_batch_set_variant(nrq_cn_batch *batch, int variant, int order);
 /* The FP64 stencil of the batch's right-hand side and residuals: 0 the
- * register-tiled one, 1 FP64 FMAs on per-update blocks of every mass staged
- * by TMA (V even, V >= 34).  The batch times both with its Chebyshev
+ * register-tiled one, 1 FP64 FMAs on the per-update operator of every mass
+ * in its spin structure (V even, V >= 34).  The batch times both with its Chebyshev
  * candidates on the first update (ms, index = which; -1 where not timed);
  * nrq_cn_batch_set_fp64 forces one (the next update recalibrates).        */
 int nrq_cn_batch_fp64_info(const nrq_cn_batch *batch, int *which, double ms[2]);

@@ -68,9 +68,9 @@ def solver_handle():
 STENCIL_REGISTER = 0  # register-tiled FP64 stencil (k_cn_mv2)
 STENCIL_TMA = 1       # TMA-staged FP64 stencil (k_cn_mv3)
 STENCIL_TENSOR = 2    # FP64 tensor-core stencil on per-update 6x6 blocks (k_cn_mv4)
-STENCIL_FMA = 3       # FP64 FMA stencil on the same per-update blocks (k_cn_mv5)
+STENCIL_FMA = 3       # FP64 FMA stencil on the operator in its spin structure (k_cn_spin)
 STENCIL_NAMES = {STENCIL_REGISTER: "k_cn_mv2 (register-tiled)", STENCIL_TMA: "k_cn_mv3 (TMA-staged)",
-                 STENCIL_TENSOR: "k_cn_mv4 (FP64 tensor cores)", STENCIL_FMA: "k_cn_mv5 (FP64 FMA on cached blocks)"}
+                 STENCIL_TENSOR: "k_cn_mv4 (FP64 tensor cores)", STENCIL_FMA: "k_cn_spin (FP64 FMA, spin structure)"}
 
 
 def SetStencil(stencil=None):
@@ -86,8 +86,8 @@ CHEB_REGISTER, CHEB_BLOCKS = 0, 1
 
 def SetChebStencil(which=None):
     """Precision forms: force the FP32 Chebyshev step (CHEB_REGISTER: the
-    operator assembled per launch; CHEB_BLOCKS: FP32 blocks staged by TMA);
-    None restores the default (blocks where the lattice allows)."""
+    operator assembled per launch; CHEB_BLOCKS: the per-update operator in
+    its spin structure); None restores the choice timed on the next update."""
     _capi.check(_capi.load().nrq_cn_set_cheb_stencil(solver_handle(), -1 if which is None else int(which)),
                 lattice.context(), f"Error in {modulename}: Chebyshev stencil")
 
@@ -104,8 +104,9 @@ def ChebInfo(with_times=False):
 
 
 def SetMergedUpdate(on=True):
-    """Plain form on the FMA stencil: update x, r and p of an iteration in one
-    pass (on=True, the default) or in two (x and r, then p)."""
+    """Plain form on the FMA stencil: BiCGStab in place of the Chebyshev
+    semi-iteration, with the update of x, r and p in one pass (on=True) or in
+    two (x and r, then p)."""
     _capi.check(_capi.load().nrq_cn_set_merged_update(solver_handle(), int(bool(on))), lattice.context(),
                 f"Error in {modulename}: merged update")
 
