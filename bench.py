@@ -43,11 +43,11 @@ A = (0.05, 1.0, 1.0, 1.0)
 TOL = 1e-12
 # DRAM bytes per site of an average stencil launch of a plain 64^3 update
 # (dram__bytes_read.sum + dram__bytes_write.sum, one ncu capture of the
-# update's 9 launches), by NRQ_STENCIL_* index: the tensor-core stencil (2
+# update's launches), by NRQ_STENCIL_* index: the tensor-core stencil (2
 # residual, 4 v and 3 t launches: 10,773, 7,760 and 6,377 B/site) and the
-# FMA stencil (1 right-hand side, 2 residual, 3 v and 3 t launches: 7,573,
-# 10,413, 7,500 and 6,199 B/site)
-STENCIL_DRAM_BYTES_PER_SITE = {2: 7968.0, 3: 7722.0}
+# FMA stencil (right-hand side with the history start 7,545, first residual
+# 5,272, 5 Chebyshev steps 6,421, the last one with the history 8,298 B/site)
+STENCIL_DRAM_BYTES_PER_SITE = {2: 7968.0, 3: 6653.0}
 # FP64 arithmetic of the leapfrog force per site: 3 directions x (4 staples
 # of 2 products + the product with the link) = 27 complex 3x3 products of
 # 27 complex multiply-adds, 4 real FMAs each, 2 flops per FMA

@@ -32,10 +32,11 @@
 //
 // Bound: 64^3, the solver's step (four vector streams, 6.1 KB a site): 0.25 ms
 // at the copy rate, 0.21 ms at the FP64 rate that FMAs with distinct operands
-// reach (49 of 64 a clock and SM).  It takes 0.41 ms: twelve warps an SM (166
-// registers) hide the loads only in part, a block spends a fifth of its time
-// before its first product and in its epilogue, and the loads alone take 0.31
-// ms (the launch without its products).  24^3: 28 us, 12^3: 12 us.
+// reach (49 of 64 a clock and SM).  It takes 0.37 ms (the TMA stencil on dense
+// 6x6 blocks before it 0.47): 70 % of the copy rate, of the shared-memory
+// path's wavefronts and half of the FP64 pipe at twelve warps an SM (166
+// registers); the loads alone take 0.31 ms (the launch without its products).
+// 24^3: 28 us, 12^3: 9 us.
 //
 // Every mbarrier wait is bounded (wait_cycles); on expiry the thread records
 // NRQ_ERR_TIMEOUT in *err and its warp skips the remaining work.  stall_load
@@ -131,8 +132,9 @@ constexpr int kPrepSites = 32;
 // the site term of the hermitian H (A^H = 1 + i tau H) for quark and
 // antiquark.  One thread per site and direction; the Darwin and magnetic
 // matrices are sums over directions, exchanged through shared memory.  64^3:
-// 240 us at 12 warps an SM (168 registers; 255 registers, 8 warps: 315, 136
-// registers, 15 warps: 280), of which the traffic takes 90; 12^3: 10 us.
+// 211 us, with the FP32 copy 240, at 12 warps an SM (168 registers; 255
+// registers, 8 warps: 286 and 315; 136 registers, 15 warps: 280 with the
+// copy), of which the traffic takes 90; 12^3: 10 us.
 __global__ void __launch_bounds__(kPrepSites * 3, 4) k_spin_prepare(Lat L, CnCoef C1, const CnCoef *__restrict__ Cm,
                                                                 int nm, double tau, const double2 *__restrict__ U,
                                                                 const double *__restrict__ E, SpinOp op,

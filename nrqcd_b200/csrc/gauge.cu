@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(3 * kLinkSites) k_update_links(Lat L, double2 
 // which the lane pair adds.  The three directions of a block's sites run side
 // by side and read the links they share through the SM's L1.
 // Bound: latency of the loads (12 matrices a thread, FP64 pipe a third
-// active).  64^3: 137 us at 15 warps an SM (one thread per link, three
+// active).  64^3: 142 us at 15 warps an SM (one thread per link, three
 // matrices live, 12 warps: 147; one thread per row of a link, 24 warps, three
 // times the load instructions: 230); a step at 30x21x14 10.1 -> 7 us, with
 // the launch of the second kernel hidden.
