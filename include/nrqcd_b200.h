@@ -331,8 +331,8 @@ int nrq_cn_batch_attach_learned(nrq_cn_batch *batch, struct nrq_learn *net);
 int nrq_cn_batch_residuals(const nrq_cn_batch *batch, double *rel);
 /* Tuning and schedule: the chosen Chebyshev kernel variant (0: one field
  * per tile, 2 blocks per SM; 1: one field per tile, 3 blocks per SM; 2: two
- * fields of one mass per tile; 3: the FP32 block step, per-update blocks of
- * every mass staged by TMA with the fields' vectors, where the lattice
+ * fields of one mass per tile; 3: the FP32 step on the per-update operator of
+ * every mass in its spin structure, where the lattice
  * allows it: V a multiple of 4, V >= 36, nx even) and block order (0: field
  * fastest, 1: site block fastest), the measured milliseconds per launch of
  * every candidate (NRQ_BATCH_CANDIDATES entries, index variant*2 + order;

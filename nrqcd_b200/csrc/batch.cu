@@ -11,9 +11,10 @@
 // so once the per-pass inner step counts (the schedule) are known a whole step
 // enqueues without host synchronisation and is captured as a CUDA graph.
 //
-// The batch keeps its own FP64 copy of the links, so its solve reads nothing
-// that the leapfrog writes: an ensemble member's step (CN, then leapfrog, as
-// src/main.f90:346-348) is one child graph, and a field that misses the
+// The batch keeps its own operator (and, for the register-tiled kernels, its
+// own copy of the links), so its solve reads nothing that the leapfrog writes:
+// an ensemble member's step (CN, then leapfrog, as src/main.f90:346-348) is one
+// child graph, and a field that misses the
 // tolerance after the scheduled passes can still be refined after the
 // leapfrog has run.
 #include <algorithm>
@@ -1088,9 +1089,8 @@ extern "C" int nrq_ensemble_step(nrq_ensemble *e, const double c[8], double dt, 
       cudaGraph_t master = nullptr;
       NRQ_CUDA_TRY(ctx0, cudaGraphCreate(&master, 0));
       // members run as concurrent branches, except where a member uses the
-      // persistent block stencils: those size their grids to every SM and
-      // hold most of an SM's shared memory, so concurrent members only
-      // fragment the GPU, and the members' steps are chained instead
+      // spin-structured stencils: their launches fill every SM, so concurrent
+      // members would only compete, and the members' steps are chained instead
       bool chain = false;
       for (nrq_cn_batch *b : e->batches) chain = chain || b->variant == 3 || b->fp64 == 1;
       cudaGraphNode_t prev = nullptr;

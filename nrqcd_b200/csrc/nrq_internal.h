@@ -140,7 +140,7 @@ struct nrq_cn {
   double2 *b = nullptr, *x = nullptr, *r = nullptr, *rh = nullptr, *p = nullptr, *v = nullptr,
           *t = nullptr, *s = nullptr;
   // FP64 stencil (NRQ_STENCIL_*): register-tiled, TMA-staged, tensor-core
-  // or FMA on cached blocks.
+  // or FMA in the spin structure.
   // Chosen by timing the applicable ones on the first update (tune_ms, per
   // launch) unless forced; tma_ok: tensor maps can describe the lattice.
   // last_stencil: the stencil of the latest launch (its partial-row count).
