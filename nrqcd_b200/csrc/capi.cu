@@ -1776,11 +1776,14 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
       }
   }
   // smallest inner step count whose guaranteed gain reaches `gain` on both
-  // species.  FP32 arithmetic caps one pass at about 1e6; a pass that can
-  // finish the solve may aim up to 1e7 (the FP64 check decides whether it did)
+  // species.  A pass in FP32 cannot gain more than about 3e7 (its rounding
+  // leaves 4e-8 of the residual it starts from): up to there one pass makes
+  // the whole gain, a larger one is shared by two passes of at most 1e6 each
+  // (shared evenly, so that the first does not end just below the tolerance,
+  // where the solve would stop)
   auto inner_steps = [&](double gain) {
     gain = std::max(gain, 10.0);
-    if (gain > 1e7) gain = 1e6;
+    if (gain > 3e7) gain = std::min(std::sqrt(gain), 1e6);
     int m = 1;
     while (m < kMaxInner && std::min(cheb_gain(seg[0].sigma, m), cheb_gain(seg[1].sigma, m)) < gain) ++m;
     return m;
@@ -1850,15 +1853,15 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
       break;
     }
     if (outer == 7) break;
-    // gain needed to bring the worst column to 0.3 tol in this pass; deeper
-    // where a pass only finishes, and while the field's history fills: the
-    // first updates from a source, whose error sits on the few sites the
-    // field has reached
+    // gain needed to bring the worst column to 0.1 tol: the error of a point
+    // source sits on the few sites the field has reached, so that the worst
+    // element stands well above the norm, and updates that end anywhere below
+    // tol add up (96^3, tol 1e-10, error of the propagator after eight: 8e-11
+    // in norm and 3e-8 of its rms at the worst element with passes to 0.3 tol)
     double worst = 0.0;
     for (int kk = 0; kk < nrq::CN_COLS; ++kk) worst = std::max(worst, rel[kk]);
-    const double aim = outer > 0 || (hist && hist_count < cn->history_depth) ? 0.05 : 0.3;
     // maxits bounds the FP32 inner steps of the whole update
-    int m = inner_steps(worst / (aim * cn->tol));
+    int m = inner_steps(worst / (0.1 * cn->tol));
     if (inner + m > cn->maxits) m = (int)(cn->maxits - inner);
     if (m <= 0) break;
     // FP32 inner Chebyshev solve of A^H e = r, and x += e
