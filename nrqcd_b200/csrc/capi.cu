@@ -1314,6 +1314,18 @@ bool offdiag_imaginary(const nrq::CnCoef &C) {
     if (C.kin[sp].re != 0.0 || C.so[sp].re != 0.0) return false;
   return true;
 }
+// The spin-structured stencil keeps one hermitian site term a species on top:
+// every coefficient imaginary (all four Wilson coefficients real), so that
+// A^H is normal and A = 2 - A^H.  The tensor-core stencil applies the site
+// term in full and needs the weaker condition alone.
+bool spin_coefficients(const nrq::CnCoef &C) {
+  for (int sp = 0; sp < 2; ++sp)
+    if (C.mag[sp].re != 0.0 || C.dar[sp].re != 0.0) return false;
+  return offdiag_imaginary(C);
+}
+bool spin_stencil_applies(const nrq_ctx *ctx, const nrq::CnCoef &C) {
+  return spin_coefficients(C) && nrq::cn_spin_applicable(ctx->lat);
+}
 // +1 / -1 when the current blocks were built for C / for the coefficients
 // whose off-diagonal terms are those of C negated (A vs A^H), 0 otherwise
 double blocks_sign(bool valid, const nrq::CnCoef &w, const nrq::CnCoef &C) {
@@ -1417,7 +1429,7 @@ int ensure_spin(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *si
 // cn->last_stencil records which ran (the partial rows it left).
 int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq::MvArgs &a, int *err = nullptr) {
   nrq_ctx *ctx = cn->ctx;
-  if (cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(C) && nrq::cn_spin_applicable(ctx->lat)) {
+  if (cn->stencil == NRQ_STENCIL_FMA && spin_stencil_applies(ctx, C)) {
     double sign = 0.0;
     int rc = ensure_spin(cn, C, g, &sign);
     if (rc) return rc;
@@ -1457,7 +1469,8 @@ int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq
   }
   if (cn->stencil != NRQ_STENCIL_REGISTER) {  // tensor maps unavailable
     cn->tma_ok = false;
-    cn->stencil = NRQ_STENCIL_REGISTER;
+    // (the FMA stencil waits for coefficients that it takes)
+    if (cn->stencil != NRQ_STENCIL_FMA) cn->stencil = NRQ_STENCIL_REGISTER;
   }
   nrq::launch_cn_mv(mode, ctx->lat, C, g->U, cn->Dsum, cn->Bsum, cn->DE, a, ctx->stream);
   cn->last_stencil = NRQ_STENCIL_REGISTER;
@@ -1466,7 +1479,8 @@ int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq
 // the MV_T input: the register-tiled stencil forms s = r - alpha v on the
 // fly, the staged ones read a materialised s
 bool mv_t_needs_s(const nrq_cn *cn, const nrq::CnCoef &CH) {
-  if ((cn->stencil == NRQ_STENCIL_TENSOR || cn->stencil == NRQ_STENCIL_FMA) && offdiag_imaginary(CH)) return true;
+  if (cn->stencil == NRQ_STENCIL_TENSOR && offdiag_imaginary(CH)) return true;
+  if (cn->stencil == NRQ_STENCIL_FMA && spin_stencil_applies(cn->ctx, CH)) return true;
   return cn->tma_ok && cn->stencil != NRQ_STENCIL_REGISTER;
 }
 void fin(nrq_cn *cn, int stage, double *scal = nullptr) {
@@ -1496,21 +1510,21 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
     return NRQ_OK;
   }
   if (!cn->tma_ok) {  // the register-tiled and the FMA stencil apply: the latter where the coefficients allow it
-    if (offdiag_imaginary(CH) && nrq::cn_spin_applicable(ctx->lat)) cn->stencil = NRQ_STENCIL_FMA;
+    if (spin_stencil_applies(ctx, CH)) cn->stencil = NRQ_STENCIL_FMA;
     return NRQ_OK;
   }
   cudaStream_t st = ctx->stream;
   const bool prof = ctx->prof;
   ctx->prof = false;
   const int reps = 3;
-  const bool tensor = offdiag_imaginary(CH);
+  const bool tensor = offdiag_imaginary(CH), spin = spin_stencil_applies(ctx, CH);
   cudaEvent_t e0, e1;
   NRQ_CUDA_TRY(ctx, cudaEventCreate(&e0));
   NRQ_CUDA_TRY(ctx, cudaEventCreate(&e1));
   int rc = NRQ_OK;
   for (int which = 0; which < 4 && !rc; ++which) {
     cn->tune_ms[which] = -1.0;
-    if ((which == NRQ_STENCIL_TENSOR || which == NRQ_STENCIL_FMA) && !tensor) continue;
+    if ((which == NRQ_STENCIL_TENSOR && !tensor) || (which == NRQ_STENCIL_FMA && !spin)) continue;
     cn->stencil = which;
     for (int r = 0; r < reps + 1 && !rc; ++r) {
       if (r == 1) cudaEventRecord(e0, st);
@@ -2183,7 +2197,7 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
   if ((rc = cn_prepare(cn, g, dt))) return rc;
   if (!cn->stencil_tuned && (rc = tune_stencil(cn, CH, g))) return rc;
   int64_t matvecs = 0, vstreams = 0;
-  bool fma = cn->stencil == NRQ_STENCIL_FMA && offdiag_imaginary(CH) && nrq::cn_spin_applicable(L);
+  bool fma = cn->stencil == NRQ_STENCIL_FMA && spin_stencil_applies(ctx, CH);
   if (fma) {
     double sign = 0.0;
     rc = ensure_spin(cn, CH, g, &sign);
