@@ -1209,7 +1209,8 @@ extern "C" int nrq_cn_stencil_info(const nrq_cn *cn, int *stencil, double ms[4])
 extern "C" int nrq_cn_set_wait_test(nrq_cn *cn, int64_t wait_cycles, int stall_load) {
   if (!cn || wait_cycles < 0 || stall_load < -1) return NRQ_ERR_BAD_ARG;
   cn->wait_cycles = wait_cycles > 0 ? (long long)wait_cycles : nrq_wait_cycles_default;
-  cn->stall_load = stall_load;
+  cn->stall_load = stall_load < 0 ? -1 : stall_load % 16;
+  cn->stall_launch = stall_load < 0 ? -1 : stall_load / 16 - 1;
   return NRQ_OK;
 }
 
@@ -1438,8 +1439,9 @@ int mv(nrq_cn *cn, int mode, const nrq::CnCoef &C, const nrq_gauge *g, const nrq
       cn->spin_valid = false;
       if ((rc = ensure_spin(cn, C, g, &sign))) return rc;
     }
+    const bool stall = cn->stall_launch < 0 || cn->stall_launch == cn->spin_launches++;
     nrq::launch_cn_spin(mode, ctx->lat, cn->spin, sign, a, !cn->spin_fresh, err ? err : scal_err(cn->scal),
-                        ctx->stream, cn->wait_cycles, cn->stall_load);
+                        ctx->stream, cn->wait_cycles, stall ? cn->stall_load : -1);
     cn->spin_fresh = false;
     cn->last_stencil = NRQ_STENCIL_FMA;
     return NRQ_OK;
@@ -1612,6 +1614,7 @@ int cn_prepare(nrq_cn *cn, const nrq_gauge *g, double dt) {
   cn->f32_valid = false;
   cn->spin_valid = false;
   cn->spin_tau = dt * cn->ctx->a[0] / 2.0;
+  cn->spin_launches = 0;
   return NRQ_OK;
 }
 // spectral enclosure of H, A^H = 1 + i spin_tau H, into out (4 doubles of the
@@ -2231,7 +2234,9 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
         a.hist[k] = hist_v(h, k + 1);
         a.hcoef[k] = nrq::hist_coef(hist_d, k);
       }
-    if ((rc = mv(cn, nrq::MV_RHS, CA, g, a))) return rc;
+    // the semi-iteration reads its own record, at the synchronisation after
+    // its first residual
+    if ((rc = mv(cn, nrq::MV_RHS, CA, g, a, semi ? scal_err(cn->h_cheb) : nullptr))) return rc;
     matvecs += 1;
     vstreams += 1;  // extra write of x0
   }

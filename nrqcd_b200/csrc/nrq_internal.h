@@ -216,8 +216,9 @@ struct nrq_cn {
   double cheb_ms[2] = {-1.0, -1.0};
   // bound of the FMA stencil's pipeline waits (clock cycles) and, for the
   // test of the timeout path, the load its producer stops before (-1: none)
+  // in the spin-structured launch number stall_launch of an update (-1: all)
   long long wait_cycles = nrq_wait_cycles_default;
-  int stall_load = -1;
+  int stall_load = -1, stall_launch = -1, spin_launches = 0;
   // precision form (form 1): FP32 copies of the per-step matrices for the
   // register-tiled step (f32_valid: of the current gauge field) and the FP32
   // Chebyshev vectors; spectral bounds of the hermitian part

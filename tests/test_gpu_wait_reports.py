@@ -1,0 +1,56 @@
+"""A bounded wait that runs out in one launch of an update is reported by that
+update, whichever launch it is: the right-hand side (whose record the plain
+solve's semi-iteration reads with its first residual).  The launch's loader
+stops before its fourth load, the waits are bounded at about a millisecond,
+nothing faults, and the context then runs a clean step."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from nrqcd_b200 import GaugeConfiguration, NRQCDField, _capi, nrqcd
+from tests.gpu_util import lattice_ctx
+
+pytestmark = pytest.mark.gpu
+
+A = (0.05, 1.0, 1.0, 1.0)
+M, C = 1.0, [1.0, 1.0, 1.0, 1.0]
+
+
+def update(h, g):
+    st = _capi.CnStats()
+    c = _capi.coeffs(C)
+    rc = _capi.load().nrq_heavy_update_cn(nrqcd.solver_handle(), h.handle, g.handle, M, _capi.dptr(c), 1.0,
+                                          ctypes.byref(st))
+    return rc, st.as_dict()
+
+
+def check_one_launch(oracle, form, tol, launch, before):
+    """`before` clean updates, one with launch number `launch` stalled, then clean fields on the same solver."""
+    n = (8, 6, 4)
+    links, ef = oracle.transverse_box(n, A, 3.0, 1.0, 0.0, 5, identity_links=False)
+    with lattice_ctx(n, A, cn=(M, C, 1.0, tol, 10000, form)):
+        nrqcd.SetStencil(nrqcd.STENCIL_FMA)
+        g = GaugeConfiguration()
+        g.upload(links, ef)
+        h = NRQCDField()
+        h.InitSinglePoint(1, 1)
+        for _ in range(before):
+            rc, st = update(h, g)
+            assert rc == _capi.NRQ_OK and st["converged"] == 1
+        nrqcd.SetWaitTest(wait_cycles=2_000_000, stall_load=3, launch=launch)
+        rc, st = update(h, g)
+        nrqcd.SetWaitTest()
+        assert rc == _capi.NRQ_ERR_TIMEOUT and st["converged"] == 0, (rc, st)
+        q, an = oracle.single_point(n, 1), oracle.single_point(n, 1)
+        h.upload(q, an)
+        rc, st = update(h, g)
+        assert rc == _capi.NRQ_OK and st["converged"] == 1
+        gq, ga = h.download()
+        oracle.cn_update(n, A, links, ef, M, C, 1.0, q, an, tol=1e-14)
+        assert np.abs(gq - q).max() < 50 * tol and np.abs(ga - an).max() < 50 * tol
+
+
+@pytest.mark.parametrize("before", [0, 1, 3])
+def test_right_hand_side(oracle, before):
+    check_one_launch(oracle, nrqcd.FORM_PLAIN_FP64, 1e-12, 0, before)
