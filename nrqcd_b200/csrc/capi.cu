@@ -2010,7 +2010,7 @@ static bool accept_recursive(const nrq_cn *cn, const double rel[nrq::CN_COLS]) {
 // two vector passes and three scalar stages for the same two orders of
 // application; the step count follows from the first residual and the
 // segment, |r_m| <= |r_0| / |T_m(sigma)| in every column, so the host reads
-// the device once a solve.  64^3: 0.38 ms a step against 1.40 ms an
+// the device once before the steps and their error record after them.  64^3: 0.38 ms a step against 1.40 ms an
 // iteration.
 //
 // The bound is rigorous, so a solve ends on it (after m steps max_rel is the
@@ -2034,6 +2034,16 @@ static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const n
   double2 *cur = cn->x, *prev = cn->p;  // the iterate and the one before it
   // confirm on the first solve and every kReconfirm-th unconfirmed one
   const bool confirm = cn->confirm_always || !cn->semi_confirmed || cn->semi_unconfirmed >= nrq_cn::kReconfirm;
+  // waits for the launches so far: NRQ_ERR_TIMEOUT if a bounded wait ran out in one
+  auto finished = [&]() -> int {
+    NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    if (*scal_err(hc) != 0) {
+      ctx->last_error = timeout_message(hc);
+      std::memset(scal_err(hc), 0, 16 * sizeof(int));
+      return NRQ_ERR_TIMEOUT;
+    }
+    return NRQ_OK;
+  };
   // one residual pass of `cur`; MV_CH0 also writes x_1 into prev
   auto residual = [&](int mode) -> int {
     nrq::MvArgs a{};
@@ -2048,13 +2058,7 @@ static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const n
     matvecs += 1;
     vstreams += mode == nrq::MV_CH0 ? 3 : 2;
     if ((rc = check_launch(ctx, "cn residual"))) return rc;
-    NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if (*scal_err(hc) != 0) {
-      ctx->last_error = timeout_message(hc);
-      std::memset(scal_err(hc), 0, 16 * sizeof(int));
-      return NRQ_ERR_TIMEOUT;
-    }
-    return NRQ_OK;
+    return finished();
   };
   auto rel_of = [&](int k) {
     const double *sc = hc + k * nrq::SC_STRIDE;
@@ -2133,6 +2137,8 @@ static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const n
     if (status != NRQ_OK) break;
     if ((status = check_launch(ctx, "cn iteration")) != NRQ_OK) break;
     if (!confirm) {
+      // the field is handed out only once its last launch is known to be whole
+      if ((status = finished()) != NRQ_OK) break;
       conv = true;
       maxrel = bound;
       cn->last_true = false;

@@ -1,6 +1,7 @@
 """A bounded wait that runs out in one launch of an update is reported by that
 update, whichever launch it is: the right-hand side (whose record the plain
-solve's semi-iteration reads with its first residual).  The launch's loader
+solve's semi-iteration reads with its first residual), or a step of a solve
+that ends on its bound, with no residual pass after it.  The launch's loader
 stops before its fourth load, the waits are bounded at about a millisecond,
 nothing faults, and the context then runs a clean step."""
 import ctypes
@@ -54,3 +55,9 @@ def check_one_launch(oracle, form, tol, launch, before):
 @pytest.mark.parametrize("before", [0, 1, 3])
 def test_right_hand_side(oracle, before):
     check_one_launch(oracle, nrqcd.FORM_PLAIN_FP64, 1e-12, 0, before)
+
+
+# launch 0 the right-hand side, 1 the first residual, then the steps
+@pytest.mark.parametrize("launch", [2, 4])
+def test_step_of_an_unconfirmed_solve(oracle, launch):
+    check_one_launch(oracle, nrqcd.FORM_PLAIN_FP64, 1e-12, launch, 2)
