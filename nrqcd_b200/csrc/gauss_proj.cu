@@ -207,8 +207,11 @@ constexpr int kRegRows = 6;        // rows of R in registers, the others in shar
 constexpr double kT8 = 0x1.35cf5e19f6cf7p-52;
 
 struct Msg {
-  uint4 q[5];
+  ulonglong2 q[5];
 };
+__device__ __forceinline__ unsigned long long word(uint32_t lo, uint32_t hi) {
+  return (unsigned long long)hi << 32 | lo;
+}
 __device__ __forceinline__ Msg pack(const double (&v)[8], uint32_t tag) {
   uint32_t lo[8], hi[8];
 #pragma unroll
@@ -223,36 +226,39 @@ __device__ __forceinline__ Msg pack(const double (&v)[8], uint32_t tag) {
   Msg m;
 #pragma unroll
   for (int j = 0; j < 4; ++j)
-    m.q[j] = make_uint4((lo[2 * j] & ~0xffu) | tag, hi[2 * j], (lo[2 * j + 1] & ~0xffu) | tag, hi[2 * j + 1]);
-  m.q[4] = make_uint4(w8l, w8h, w9l, 0u);
+    m.q[j] = make_ulonglong2(word((lo[2 * j] & ~0xffu) | tag, hi[2 * j]),
+                             word((lo[2 * j + 1] & ~0xffu) | tag, hi[2 * j + 1]));
+  m.q[4] = make_ulonglong2(word(w8l, w8h), word(w9l, 0u));
   return m;
 }
 __device__ __forceinline__ void unpack(const Msg &m, double (&v)[8]) {
+  const uint32_t w8l = (uint32_t)m.q[4].x, w8h = (uint32_t)(m.q[4].x >> 32), w9l = (uint32_t)m.q[4].y;
 #pragma unroll
   for (int a = 0; a < 8; ++a) {
-    const uint32_t w = (a & 1) ? m.q[a >> 1].z : m.q[a >> 1].x, h = (a & 1) ? m.q[a >> 1].w : m.q[a >> 1].y;
-    const uint32_t b = a < 3 ? m.q[4].x >> (8 * (a + 1)) : a < 7 ? m.q[4].y >> (8 * (a - 3)) : m.q[4].z >> 8;
-    v[a] = __hiloint2double((int)h, (int)((w & ~0xffu) | (b & 0xffu)));
+    const unsigned long long w = (a & 1) ? m.q[a >> 1].y : m.q[a >> 1].x;
+    const uint32_t b = a < 3 ? w8l >> (8 * (a + 1)) : a < 7 ? w8h >> (8 * (a - 3)) : w9l >> 8;
+    v[a] = __hiloint2double((int)(w >> 32), (int)(((uint32_t)w & ~0xffu) | (b & 0xffu)));
   }
 }
-__device__ __forceinline__ void send(uint4 *p, const uint4 &q) {
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w)
-               : "memory");
+// (vector accesses are as many accesses of their element's type: 8-byte
+// elements, so that a word is never seen in part)
+__device__ __forceinline__ void send(ulonglong2 *p, const ulonglong2 &q) {
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(q.x), "l"(q.y) : "memory");
 }
 // the warp's lanes wait for the message `tag` in their slots p[j*stride]
-__device__ __forceinline__ bool receive(const uint4 *p, int64_t stride, uint32_t tag, Msg &m, int *err,
+__device__ __forceinline__ bool receive(const ulonglong2 *p, int64_t stride, uint32_t tag, Msg &m, int *err,
                                         long long wait_cycles) {
   long long t0 = 0;
   for (int spins = 0;; ++spins) {
 #pragma unroll
     for (int j = 0; j < 5; ++j)
-      asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                   : "=r"(m.q[j].x), "=r"(m.q[j].y), "=r"(m.q[j].z), "=r"(m.q[j].w)
+      asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+                   : "=l"(m.q[j].x), "=l"(m.q[j].y)
                    : "l"(p + j * stride)
                    : "memory");
     uint32_t off = 0;
 #pragma unroll
-    for (int j = 0; j < 5; ++j) off |= (m.q[j].x ^ tag) | (m.q[j].z ^ tag);
+    for (int j = 0; j < 5; ++j) off |= ((uint32_t)m.q[j].x ^ tag) | ((uint32_t)m.q[j].y ^ tag);
     if (__all_sync(0xffffffffu, (off & 0xffu) == 0)) return true;
     if ((spins & 63) == 63) {
       if (t0 == 0) t0 = clock64();
@@ -281,7 +287,7 @@ __device__ __forceinline__ void half_d(const double (&x)[8], const double (&y)[8
 // dev[n*nwarps + w]: the deviation before sweep n = 0..nsweeps over warp w's
 // sites; Eout may be Ein.  Messages are numbered from te (T) and ge (G).
 __global__ void __launch_bounds__(32 * kRunWarps, 1)
-    k_gauss_run(Lat L, const double2 *__restrict__ U, const double *Ein, double *Eout, uint4 *T, uint4 *G,
+    k_gauss_run(Lat L, const double2 *__restrict__ U, const double *Ein, double *Eout, ulonglong2 *T, ulonglong2 *G,
                 double *__restrict__ dev, int nwarps, int nsweeps, uint32_t te, uint32_t ge, double kdt, int *err,
                 long long wait_cycles) {
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -318,8 +324,8 @@ __global__ void __launch_bounds__(32 * kRunWarps, 1)
     for (int a = 0; a < 8; ++a) e[a] = Ein[(int64_t)(k * 8 + a) * V + x];
   }
   const double c = 1.0 / (L.a[k] * L.a0);
-  uint4 *const Tw = T + (int64_t)k * V + x, *const Gw = G + x;
-  const uint4 *const Tr = T + (int64_t)k * V + xm, *const Gr = G + xp;
+  ulonglong2 *const Tw = T + (int64_t)k * V + x, *const Gw = G + x;
+  const ulonglong2 *const Tr = T + (int64_t)k * V + xm, *const Gr = G + xp;
   for (int n = 0;; ++n) {
     Msg m;
     double v[8], g[8];
@@ -405,7 +411,7 @@ cudaError_t launch_gauss_run(Lat L, const double2 *U, const double *Ein, double 
   int nwarps = gauss_run_warps(L.V);
   const int per = (nwarps + sm_count - 1) / sm_count;  // warps a block: spread over the SMs
   const unsigned grid = (unsigned)((nwarps + per - 1) / per);
-  uint4 *T = (uint4 *)messages, *G = T + 15 * L.V;
+  ulonglong2 *T = (ulonglong2 *)messages, *G = T + 15 * L.V;
   void *args[] = {&L, &U, &Ein, &Eout, &T, &G, &dev, &nwarps, &nsweeps, &te, &ge, &kdt, &err, &wait_cycles};
   const cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_gauss_run, dim3(grid), dim3(32 * per), args, 0, st);
   if (e != cudaSuccess) return e;
