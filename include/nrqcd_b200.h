@@ -220,7 +220,10 @@ int nrq_cn_stencil_info(const nrq_cn *cn, int *stencil, double ms[4]);
  * that neighbour's matrices, so the wait for them runs out: the update
  * then returns NRQ_ERR_TIMEOUT, nothing faults, and the context stays
  * usable.  -1 (the default) stops nowhere; load + 16 (k + 1) stops the k-th
- * of an update's stencil launches alone (0: the right-hand side).          */
+ * of an update's stencil launches alone (0: the right-hand side); 4096 + k
+ * instead withholds messages in the k-th launch of a Gauss projection on
+ * this solver's context (lattices that run many sweeps a launch), whose
+ * waits wait_cycles then bounds.                                           */
 int nrq_cn_set_wait_test(nrq_cn *cn, int64_t wait_cycles, int stall_load);
 /* Force a stencil (NRQ_STENCIL_*) or restore the timed choice (-1).
  * NRQ_ERR_BAD_ARG if the stencil cannot describe this lattice.            */

@@ -626,8 +626,10 @@ constexpr int64_t kProjUnbounded = INT64_MAX;
 // The launch that crosses the tolerance is repeated from its own start, for
 // the sweeps up to the crossing, so that the field and the count are those of
 // a test after every sweep; its length follows the decay seen so far, which
-// keeps the repeated part short.  Returns false where the cooperative launch
-// or its workspace is refused (the caller queues single sweeps).
+// keeps the repeated part short.  The sweeps run between two buffers and the
+// field is written once the last launch is known to be whole, so that an
+// expired wait leaves it as it was.  Returns false where the cooperative
+// launch or its workspace is refused (the caller queues single sweeps).
 constexpr int64_t kRunChunk = 512;
 bool gauss_project_run(nrq_gauge *g, double tol, int64_t limit, int64_t *sweeps, double *deviation, int *rc) {
   nrq_ctx *ctx = g->ctx;
@@ -635,13 +637,14 @@ bool gauss_project_run(nrq_gauge *g, double tol, int64_t limit, int64_t *sweeps,
   cudaStream_t st = ctx->stream;
   const size_t mb = (size_t)nrq::gauss_run_message_bytes(V), eb = sizeof(double) * 24 * V;
   const size_t db = sizeof(double) * (kRunChunk + 1) * (nw + 1);
-  if (ensure_stage(ctx, mb + eb + db + sizeof(int))) {
+  if (ensure_stage(ctx, mb + 2 * eb + db + sizeof(int))) {
     cudaGetLastError();
     return false;
   }
   char *base = (char *)ctx->d_stage;
-  double *E2 = (double *)(base + mb), *dev = (double *)(base + mb + eb), *devmax = dev + (kRunChunk + 1) * nw;
-  int *err = (int *)(base + mb + eb + db);
+  double *buf[2] = {(double *)(base + mb), (double *)(base + mb + eb)};
+  double *dev = (double *)(base + mb + 2 * eb), *devmax = dev + (kRunChunk + 1) * nw;
+  int *err = (int *)(base + mb + 2 * eb + db);
   auto cuda = [&](cudaError_t e) {
     if (e != cudaSuccess && !*rc) {
       ctx->last_error = std::string("Gauss projection: ") + cudaGetErrorString(e);
@@ -652,56 +655,57 @@ bool gauss_project_run(nrq_gauge *g, double tol, int64_t limit, int64_t *sweeps,
   if (!cuda(cudaMemsetAsync(base, 0, mb, st)) || !cuda(cudaMemsetAsync(err, 0, sizeof(int), st))) return true;
   const double kdt = 0.01 * ctx->a[0];
   std::vector<double> d(kRunChunk + 2);
-  double *cur = g->E, *next = E2;
+  const double *cur = g->E;
+  double *next = buf[0];
   uint32_t te = 1, ge = 1;
-  auto launch = [&](double *to, int n) {
-    const cudaError_t e = nrq::launch_gauss_run(ctx->lat, g->U, cur, to, base, dev, devmax, n, te, ge, kdt,
-                                                ctx->sm_count, err, st, nrq_wait_cycles_default);
+  int launches = 0;
+  // n sweeps from cur into next
+  auto launch = [&](int n) {
+    const bool stall = ctx->proj_stall == launches++;
+    const cudaError_t e = nrq::launch_gauss_run(ctx->lat, g->U, cur, next, base, dev, devmax, n, te, ge, kdt,
+                                                ctx->sm_count, err, st, ctx->proj_wait, stall);
     te += (uint32_t)n + 1;
     ge += (uint32_t)n;
     return e;
+  };
+  // its deviations; false: *rc says why
+  auto finished = [&](int n) {
+    if (!cuda(cudaMemcpyAsync(d.data(), devmax, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, st)) ||
+        !cuda(cudaMemcpyAsync(&d[kRunChunk + 1], err, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
+        !cuda(cudaStreamSynchronize(st)))
+      return false;
+    int failed;
+    std::memcpy(&failed, &d[kRunChunk + 1], sizeof(int));
+    if (!failed) return true;
+    ctx->last_error = "Gauss projection: a bounded wait expired (k_gauss_run)";
+    *rc = NRQ_ERR_TIMEOUT;
+    return false;
   };
   int64_t total = 0, batch = 16, found = -1;
   double last = 0.0;
   for (;;) {
     const int n = (int)std::min(batch, limit - total);
-    const cudaError_t e = launch(next, n);
-    if (e != cudaSuccess && total == 0 && cur == g->E) {
+    const cudaError_t e = launch(n);
+    if (e != cudaSuccess && cur == g->E) {
       cudaGetLastError();
       return false;
     }
-    if (!cuda(e) || !cuda(cudaMemcpyAsync(d.data(), devmax, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, st)) ||
-        !cuda(cudaMemcpyAsync(&d[kRunChunk + 1], err, sizeof(int), cudaMemcpyDeviceToHost, st)) ||
-        !cuda(cudaStreamSynchronize(st)))
-      return true;
-    int failed;
-    std::memcpy(&failed, &d[kRunChunk + 1], sizeof(int));
-    if (failed) {
-      ctx->last_error = "Gauss projection: a bounded wait expired (k_gauss_run)";
-      *rc = NRQ_ERR_TIMEOUT;
-      return true;
-    }
+    if (!cuda(e) || !finished(n)) return true;
     for (int k = 0; k <= n && found < 0; ++k)
       if (!(d[k] > tol)) found = k;
     last = d[found >= 0 ? found : n];
-    if (found >= 0 && found < n) {  // again from cur, up to the crossing
-      if (found > 0 || cur != g->E) {
-        if (!cuda(launch(g->E, (int)found))) return true;
-      }
-      total += found;
-      break;
-    }
-    total += n;
-    std::swap(cur, next);
-    if (found >= 0 || total >= limit) {
-      if (cur != g->E && !cuda(cudaMemcpyAsync(g->E, cur, eb, cudaMemcpyDeviceToDevice, st))) return true;
-      break;
-    }
+    if (found == 0) break;
+    if (found > 0 && found < n && (!cuda(launch((int)found)) || !finished((int)found))) return true;
+    total += found > 0 ? found : n;
+    cur = next;
+    next = cur == buf[0] ? buf[1] : buf[0];
+    if (found >= 0 || total >= limit) break;
     batch = std::min<int64_t>(batch * 2, kRunChunk);
     // the sweeps that remain at this launch's rate of decay, if that is fewer
     const double rate = std::log(d[0] / d[n]) / n, need = std::log(d[n] / tol) / rate;
     if (rate > 0.0 && need < (double)batch) batch = std::max<int64_t>(8, (int64_t)need + 1);
   }
+  if (cur != g->E && !cuda(cudaMemcpyAsync(g->E, cur, eb, cudaMemcpyDeviceToDevice, st))) return true;
   if (sweeps) *sweeps = total;
   if (deviation) *deviation = last;
   if (found < 0) {
@@ -1209,8 +1213,12 @@ extern "C" int nrq_cn_stencil_info(const nrq_cn *cn, int *stencil, double ms[4])
 extern "C" int nrq_cn_set_wait_test(nrq_cn *cn, int64_t wait_cycles, int stall_load) {
   if (!cn || wait_cycles < 0 || stall_load < -1) return NRQ_ERR_BAD_ARG;
   cn->wait_cycles = wait_cycles > 0 ? (long long)wait_cycles : nrq_wait_cycles_default;
-  cn->stall_load = stall_load < 0 ? -1 : stall_load % 16;
-  cn->stall_launch = stall_load < 0 ? -1 : stall_load / 16 - 1;
+  // from 4096 on: the launches of the context's Gauss projections instead
+  const bool proj = stall_load >= 4096;
+  cn->ctx->proj_wait = proj ? cn->wait_cycles : nrq_wait_cycles_default;
+  cn->ctx->proj_stall = proj ? stall_load - 4096 : -1;
+  cn->stall_load = stall_load < 0 || proj ? -1 : stall_load % 16;
+  cn->stall_launch = stall_load < 0 || proj ? -1 : stall_load / 16 - 1;
   return NRQ_OK;
 }
 

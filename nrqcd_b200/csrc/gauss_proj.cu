@@ -407,8 +407,9 @@ int64_t gauss_run_message_bytes(int64_t V) { return 80 * 4 * V; }
 
 cudaError_t launch_gauss_run(Lat L, const double2 *U, const double *Ein, double *Eout, void *messages, double *dev,
                              double *devmax, int nsweeps, uint32_t te, uint32_t ge, double kdt, int sm_count, int *err,
-                             cudaStream_t st, long long wait_cycles) {
+                             cudaStream_t st, long long wait_cycles, bool stall) {
   int nwarps = gauss_run_warps(L.V);
+  if (stall && nwarps > 1) --nwarps;
   const int per = (nwarps + sm_count - 1) / sm_count;  // warps a block: spread over the SMs
   const unsigned grid = (unsigned)((nwarps + per - 1) / per);
   ulonglong2 *T = (ulonglong2 *)messages, *G = T + 15 * L.V;

@@ -9,6 +9,9 @@
 
 #include "nrq_kernels.cuh"
 
+// about two seconds at 2 GHz: the default bound of a kernel's waits
+constexpr long long nrq_wait_cycles_default = 4000000000LL;
+
 struct nrq_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -24,6 +27,10 @@ struct nrq_ctx {
   size_t stage_bytes = 0;
   // state of a Gauss projection (nrq::GaussProjState), allocated on first use
   void *d_proj = nullptr;
+  // bound of its waits and, for the test of the timeout path, the launch of a
+  // projection that withholds messages (-1: none)
+  long long proj_wait = nrq_wait_cycles_default;
+  int proj_stall = -1;
   // gluon observables: cuFFT plans over 9 and 48 complex planes and their
   // device buffer, created on first use and kept (as the reference keeps its
   // FFT descriptor, src/xpfft.f90:129-139); cufftHandle is an int
@@ -120,9 +127,6 @@ inline void hist_push(nrq_heavy *h) {
 struct nrq_learn;
 
 struct nrq_cn_stats_internal;
-// about two seconds at 2 GHz: the default bound of a pipeline wait
-constexpr long long nrq_wait_cycles_default = 4000000000LL;
-
 struct nrq_cn {
   nrq_ctx *ctx = nullptr;
   double mass = 1.0;

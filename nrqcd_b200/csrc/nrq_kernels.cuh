@@ -54,12 +54,14 @@ __global__ void k_gauss_sweep(Lat L, const double2 *__restrict__ U, const double
 // messages: gauss_run_message_bytes, zero before a projection's first launch;
 // te, ge: the numbers of the launch's first messages (nsweeps + 1 and nsweeps
 // of them), from 1 on; dev: gauss_run_warps doubles per entry of devmax.
+// stall: the last warp is left out, so that the waits for its messages run out
+// (the host's test of the timeout path).
 int gauss_run_warps(int64_t V);
 bool gauss_run_applicable(int64_t V, int sm_count);
 int64_t gauss_run_message_bytes(int64_t V);
 cudaError_t launch_gauss_run(Lat L, const double2 *U, const double *Ein, double *Eout, void *messages, double *dev,
                              double *devmax, int nsweeps, uint32_t te, uint32_t ge, double kdt, int sm_count, int *err,
-                             cudaStream_t st, long long wait_cycles);
+                             cudaStream_t st, long long wait_cycles, bool stall);
 
 // ---------------- gluon.cu
 __global__ void k_cg_divergence(Lat L, const double2 *__restrict__ U, double2 *__restrict__ D,

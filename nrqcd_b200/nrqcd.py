@@ -142,12 +142,14 @@ def SetHistoryGuess(on=True):
                 f"Error in {modulename}: history guess")
 
 
-def SetWaitTest(wait_cycles=0, stall_load=-1, launch=None):
+def SetWaitTest(wait_cycles=0, stall_load=-1, launch=None, projection=None):
     """Test hook of the FMA stencil's bounded pipeline waits: the bound in
     clock cycles (0: the default, about two seconds) and the load its loader
     stops before (-1: none), so that the wait for it runs out; launch: in that
-    one of an update's stencil launches alone (0: the right-hand side)."""
-    load = int(stall_load) + (0 if launch is None or stall_load < 0 else 16 * (int(launch) + 1))
+    one of an update's stencil launches alone (0: the right-hand side);
+    projection: in that launch of a Gauss projection instead."""
+    load = 4096 + int(projection) if projection is not None else int(stall_load) + \
+        (0 if launch is None or stall_load < 0 else 16 * (int(launch) + 1))
     _capi.check(_capi.load().nrq_cn_set_wait_test(solver_handle(), int(wait_cycles), load),
                 lattice.context(), f"Error in {modulename}: wait test")
 

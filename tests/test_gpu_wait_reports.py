@@ -3,7 +3,11 @@ update, whichever launch it is: the right-hand side (whose record the plain
 solve's semi-iteration reads with its first residual), or a step of a solve
 that ends on its bound, with no residual pass after it.  The launch's loader
 stops before its fourth load, the waits are bounded at about a millisecond,
-nothing faults, and the context then runs a clean step."""
+nothing faults, and the context then runs a clean step.
+
+The same of a Gauss projection, whose second launch here repeats the first one
+up to the sweep that met the tolerance: messages withheld in either are an
+error, with the field as it was."""
 import ctypes
 
 import numpy as np
@@ -61,3 +65,32 @@ def test_right_hand_side(oracle, before):
 @pytest.mark.parametrize("launch", [2, 4])
 def test_step_of_an_unconfirmed_solve(oracle, launch):
     check_one_launch(oracle, nrqcd.FORM_PLAIN_FP64, 1e-12, launch, 2)
+
+
+@pytest.mark.parametrize("launch", [0, 1])
+def test_gauss_projection(oracle, launch):
+    n, a = (5, 4, 3), (0.1, 1.0, 1.0, 1.0)
+    links, ef = oracle.transverse_box(n, a, 2.0, 1.0, 0.0, 9, identity_links=False)
+    ef = ef + 0.02 * np.random.default_rng(4).standard_normal(ef.shape)
+    with lattice_ctx(n, a, cn=(M, C, 1.0, 1e-12)):
+        g = GaugeConfiguration()
+
+        def project(tol, limit):
+            sweeps, dev = ctypes.c_int64(), ctypes.c_double()
+            g.upload(links, ef)
+            rc = _capi.load().nrq_gauge_gauss_project(g.handle, tol, limit, ctypes.byref(sweeps), ctypes.byref(dev))
+            return rc, sweeps.value, dev.value
+
+        rc, sweeps, dev = project(1e-9, 5)
+        assert rc == _capi.NRQ_ERR_NOT_CONVERGED and sweeps == 5
+        tol = dev * (1 + 1e-9)  # met after the fifth sweep
+        nrqcd.SetWaitTest(wait_cycles=2_000_000, projection=launch)
+        rc, _, _ = project(tol, 0)
+        nrqcd.SetWaitTest()
+        assert rc == _capi.NRQ_ERR_TIMEOUT
+        assert np.array_equal(g.download()[1], ef)
+        assert project(tol, 0)[:2] == (_capi.NRQ_OK, 5)
+        got = g.download()[1]
+    want, l = ef.copy(), links.copy()
+    oracle.gauss_project(n, a, l, want, tol=1e-9, max_sweeps=5)
+    assert np.abs(got - want).max() < 1e-13 * np.abs(want).max()
