@@ -269,14 +269,16 @@ int nrq_cn_set_history_depth(nrq_cn *cn, int depth);
  * the first solve and every 16th after an unconfirmed run confirm.
  * nrq_cn_true_residual_info: whether the last update's max_rel_residual is
  * the true residual (1) or the recursive or predicted one (0).            */
-/* Plain form on the FMA stencil: selects BiCGStab in place of the Chebyshev
- * semi-iteration (the default).  on = 1 updates x, r and p of an iteration
- * in one pass, beta taken from rh.t, which the t = A^H s launch
- * reduces (rh.s vanishes by the choice of alpha, so rho_new = -omega rh.t),
- * with the shadow residual rh kept in FP32 (every product with it, rho_0
- * included, uses the same rounded values); 0 keeps two passes (x and r,
- * then p) with rho_new = rh.r reduced and rh in FP64.  No reference
- * counterpart (PETSc's KSPBCGS, src/nrqcd.f90:803).                       */
+/* Plain form on the FMA stencil, whose default solver is the Chebyshev
+ * semi-iteration.  0 selects BiCGStab with two update passes an iteration (x
+ * and r, then p), rho_new = rh.r reduced and rh in FP64.  1, the default,
+ * updates x, r and p in one pass where BiCGStab runs: beta from rh.t, which
+ * the t = A^H s launch reduces (rh.s vanishes by the choice of alpha, so
+ * rho_new = -omega rh.t), with the shadow residual rh kept in FP32 (every
+ * product with it, rho_0 included, uses the same rounded values).  A call
+ * with 1 leaves the default solver in place and comes back to it from 0;
+ * beside nrq_cn_set_stencil(cn, NRQ_STENCIL_FMA) it selects that BiCGStab.
+ * No reference counterpart (PETSc's KSPBCGS, src/nrqcd.f90:803).          */
 int nrq_cn_set_merged_update(nrq_cn *cn, int on);
 int nrq_cn_set_true_residual(nrq_cn *cn, int always);
 int nrq_cn_true_residual_info(const nrq_cn *cn, int *last_true);

@@ -1255,8 +1255,11 @@ extern "C" int nrq_cn_cheb_info(const nrq_cn *cn, int *last, double ms[2]) {
 
 extern "C" int nrq_cn_set_merged_update(nrq_cn *cn, int on) {
   if (!cn || on < 0 || on > 1) return NRQ_ERR_BAD_ARG;
+  const bool before = cn->semi_iteration();
   cn->merged_update = on != 0;
-  cn->semi_iter = false;  // either BiCGStab update was asked for
+  cn->merged_asked = on != 0;
+  // the stencil is chosen for the solver
+  if (cn->semi_iteration() != before && cn->forced_stencil < 0) cn->stencil_tuned = false;
   return NRQ_OK;
 }
 
@@ -1599,7 +1602,7 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   // the FMA stencil's plain solve is the Chebyshev semi-iteration, which
   // also has no vector passes: about 8 launches
   auto cost = [&](int which) {
-    const double n = cn->form != 0 ? 3.0 : (which == NRQ_STENCIL_FMA && cn->semi_iter) ? 8.0 : 10.0;
+    const double n = cn->form != 0 ? 3.0 : (which == NRQ_STENCIL_FMA && cn->semi_iteration()) ? 8.0 : 10.0;
     return n * cn->tune_ms[which] + build_ms[which];
   };
   int best = NRQ_STENCIL_REGISTER;
@@ -1608,7 +1611,7 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   // the semi-iteration wins by more than the timing's noise at every size (a
   // coupled step with it against the best of the others: 242 against 374 us
   // at 12^3, 4.9 against 6.9 ms at 64^3)
-  if (cn->form == 0 && cn->semi_iter && cn->tune_ms[NRQ_STENCIL_FMA] > 0.0) best = NRQ_STENCIL_FMA;
+  if (cn->form == 0 && cn->semi_iteration() && cn->tune_ms[NRQ_STENCIL_FMA] > 0.0) best = NRQ_STENCIL_FMA;
   cn->stencil = best;
   return NRQ_OK;
 }
@@ -2227,7 +2230,7 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
     }
     if (rc) return rc;
   }
-  const bool semi = fma && cn->semi_iter;
+  const bool semi = fma && cn->semi_iteration();
   if (semi) {  // the Chebyshev coefficients, ahead of the right-hand side
     if (!cn->cheb_tab) NRQ_CUDA_TRY(ctx, cudaMalloc((void **)&cn->cheb_tab, sizeof(nrq::ChebTab)));
     if (!cn->h_cheb) {

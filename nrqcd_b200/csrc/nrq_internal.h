@@ -196,11 +196,15 @@ struct nrq_cn {
   double spin_tau = 0.0;
   double *spin_scratch = nullptr, *spin_part = nullptr;
   unsigned *spin_ticket = nullptr;
-  // plain form on the FMA stencil: the Chebyshev semi-iteration (semi_iter;
-  // setting the merged update of BiCGStab selects BiCGStab), its coefficient
-  // table, the pinned block its kernels report into (the layout of h_scal),
-  // whether a solve was confirmed yet and the unconfirmed ones since
-  bool semi_iter = true;
+  // plain form on the FMA stencil: the Chebyshev semi-iteration unless
+  // BiCGStab was asked for, by its two-pass update or by its merged one
+  // beside that stencil; its coefficient table, the pinned block its kernels
+  // report into (the layout of h_scal), whether a solve was confirmed yet and
+  // the unconfirmed ones since
+  bool merged_asked = false;
+  bool semi_iteration() const {
+    return merged_update && !(merged_asked && forced_stencil == NRQ_STENCIL_FMA);
+  }
   nrq::ChebTab *cheb_tab = nullptr;
   double *h_cheb = nullptr;
   bool semi_confirmed = false;

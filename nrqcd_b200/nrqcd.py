@@ -104,9 +104,10 @@ def ChebInfo(with_times=False):
 
 
 def SetMergedUpdate(on=True):
-    """Plain form on the FMA stencil: BiCGStab in place of the Chebyshev
-    semi-iteration, with the update of x, r and p in one pass (on=True) or in
-    two (x and r, then p)."""
+    """Plain form on the FMA stencil: on=False selects BiCGStab with two update
+    passes (x and r, then p) in place of the Chebyshev semi-iteration; on=True,
+    the default, comes back to it, or beside SetStencil(STENCIL_FMA) selects
+    BiCGStab with x, r and p updated in one pass."""
     _capi.check(_capi.load().nrq_cn_set_merged_update(solver_handle(), int(bool(on))), lattice.context(),
                 f"Error in {modulename}: merged update")
 
