@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128) k_cn_prepare(Lat L, const double2 *__rest
     double F[9];
     m3 H;
     const double scale_ = 1.0 / L.a[j] / L.a[k];
-    if (log_unitary(P, H)) {
+    if (log_unitary(P, H, true)) {
 #pragma unroll
       for (int m = 0; m < 9; ++m) F[m] = H.e[m].re * scale_;
     } else {

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kPrepSites * 3, 4) k_spin_prepare(Lat L, CnCoe
                                load_link(U, V, nb(L, x, k, +1), j)),
                         load_link(U, V, x, k));
     m3 H;
-    if (!log_unitary(P, H)) log_jacobi(P, H);
+    if (!log_unitary(P, H, true)) log_jacobi(P, H);
     const double s = 1.0 / L.a[j] / L.a[k];
 #pragma unroll
     for (int r = 0; r < 3; ++r)

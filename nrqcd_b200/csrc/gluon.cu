@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128) k_gluon_fields(Lat L, const double2 *__re
   {
     const m3 u = load_link(U, V, s, i);
     m3 h;
-    if (!log_unitary(u, h)) {
+    if (!log_unitary(u, h, false)) {
       cplx ev[3];
       m3 S;
       eigenc3(u, ev, S);

@@ -117,7 +117,22 @@ static __constant__ LogCoef c_log = make_log_coef();
 // over a warp and costs 2-3 times the rest of the preparation: false asks
 // for it.  The line rho = 3/4 needs 137 terms, still under the Jacobi
 // sweeps' time; beyond it the terms grow as 1 / (1 - rho).
-__device__ __forceinline__ bool log_unitary(const m3 &P, m3 &H) {
+// The Jacobi route takes the phases of the eigenvalues, whatever their moduli;
+// the series sees a defect |P^+ P - 1| as an error of up to three times that,
+// so it takes what is unitary to 1e-12, and with small_angle also plaquettes
+// of FP32 links (defects of some 1e-7) below |sin H| = 0.3, where the error
+// stays below the defect times the angle.
+__device__ __forceinline__ bool log_unitary(const m3 &P, m3 &H, bool small_angle) {
+  double defect = 0.0;
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = r; c < 3; ++c) {
+      cplx q = {r == c ? -1.0 : 0.0, 0.0};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) cmac_cj(q, P.e[k * 3 + r], P.e[k * 3 + c]);
+      defect = fma(r == c ? 1.0 : 2.0, norm2(q), defect);
+    }
   m3 K, Y;
 #pragma unroll
   for (int r = 0; r < 3; ++r)
@@ -130,7 +145,7 @@ __device__ __forceinline__ bool log_unitary(const m3 &P, m3 &H) {
   const m3 Y2 = mul(Y, Y);
   const double t1 = Y.e[0].re + Y.e[4].re + Y.e[8].re;
   const double ty2 = Y2.e[0].re + Y2.e[4].re + Y2.e[8].re;
-  if (!(ty2 <= 0.5625)) return false;
+  if (!(ty2 <= 0.5625) || !(defect <= (small_angle && ty2 <= 5.5e-4 ? 1e-10 : 1e-24))) return false;
   const double t2 = 0.5 * (t1 * t1 - ty2);
   const cplx det = Y.e[0] * (Y.e[4] * Y.e[8] - Y.e[5] * Y.e[7]) - Y.e[1] * (Y.e[3] * Y.e[8] - Y.e[5] * Y.e[6]) +
                    Y.e[2] * (Y.e[3] * Y.e[7] - Y.e[4] * Y.e[6]);
