@@ -570,17 +570,26 @@ extern "C" int nrq_gauge_set_precision(nrq_gauge *g, int prec, int reunit_every)
   return NRQ_OK;
 }
 
+namespace {
+// h_res[0] = max |U U^+ - 1|, h_res[1] = max |det U - 1| over the FP64 links
+int links_unitarity(nrq_gauge *g) {
+  nrq_ctx *ctx = g->ctx;
+  const int64_t nb_ = nblk(ctx->lat.V, 256);
+  int rc = ensure_red(ctx, nb_ * 2);
+  if (rc) return rc;
+  nrq::k_unitarity<<<(unsigned)nb_, 256, 0, ctx->stream>>>(ctx->lat, g->U, ctx->d_red);
+  if ((rc = check_launch(ctx, "k_unitarity"))) return rc;
+  return reduce_to_host(ctx, nb_, 2, 3u);
+}
+}  // namespace
+
 extern "C" int nrq_gauge_unitarity(nrq_gauge *g, double *max_dev, double *max_det_dev) {
   if (!g) return NRQ_ERR_BAD_ARG;
   nrq_ctx *ctx = g->ctx;
   int rc = set_device(ctx);
   if (!rc) rc = gauge_sync64(g);
+  if (!rc) rc = links_unitarity(g);
   if (rc) return rc;
-  const int64_t nb_ = nblk(ctx->lat.V, 256);
-  if ((rc = ensure_red(ctx, nb_ * 2))) return rc;
-  nrq::k_unitarity<<<(unsigned)nb_, 256, 0, ctx->stream>>>(ctx->lat, g->U, ctx->d_red);
-  if ((rc = check_launch(ctx, "k_unitarity"))) return rc;
-  if ((rc = reduce_to_host(ctx, nb_, 2, 3u))) return rc;
   if (max_dev) *max_dev = ctx->h_res[0];
   if (max_det_dev) *max_det_dev = ctx->h_res[1];
   return NRQ_OK;
@@ -726,8 +735,12 @@ int gauss_project(nrq_gauge *g, double tol, int64_t max_sweeps, int64_t *sweeps,
   int rc = gauge_sync64(g);
   if (rc) return rc;
   const int64_t limit = max_sweeps > 0 ? max_sweeps : kProjUnbounded;
-  if (nrq::gauss_run_applicable(V, ctx->sm_count) && gauss_project_run(g, tol, limit, sweeps, deviation, &rc))
-    return rc;
+  // many sweeps a launch work in the generators' coordinates, which holds for
+  // unitary links (the matrix form keeps the trace that U^+ E U has for others)
+  if (nrq::gauss_run_applicable(V, ctx->sm_count)) {
+    if ((rc = links_unitarity(g))) return rc;
+    if (ctx->h_res[0] <= 1e-12 && gauss_project_run(g, tol, limit, sweeps, deviation, &rc)) return rc;
+  }
   rc = ensure_stage(ctx, sizeof(double2) * 9 * V);
   if (!rc) rc = ensure_red(ctx, nbg);
   if (rc) return rc;

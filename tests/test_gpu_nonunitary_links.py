@@ -6,12 +6,16 @@ operator with links times 1.001, smooth and rough (a plaquette that is not
 normal gives another logarithm in the other orientation, which the reference
 takes for one of the three planes).
 
-Tolerances as in the other tests of both: 1e-13 of the field's scale and 1e-11
+The Gauss projection in the generators' coordinates drops the trace of U^+ E U,
+so that links that are not unitary take its matrix form.
+
+Tolerances as in the other tests of these: 1e-13 of the field's scale and 1e-11
 of the largest correlator."""
 import numpy as np
 import pytest
 
 from nrqcd_b200 import GaugeConfiguration, NRQCDField, nrqcd
+from nrqcd_b200._capi import NrqcdError
 from tests.gpu_util import lattice_ctx
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +68,18 @@ def test_transverse_correlators(oracle, defect):
     raa, ree, _ = oracle.transverse_correlators(N, A, links, ef)
     assert np.abs(aa - raa).max() < 1e-11 * np.abs(raa).max()
     assert np.abs(ee - ree).max() < 1e-11 * np.abs(ree).max()
+
+
+@pytest.mark.parametrize("defect,factor", [(1e-3, 1.0), (None, 1.0), (0.0, 1.001)])
+def test_gauss_projection(oracle, defect, factor):
+    links, ef = links_off_by(0.2, defect, factor)
+    a = (0.1, 1.0, 0.9, 1.1)
+    with lattice_ctx(N, a):
+        g = GaugeConfiguration()
+        g.upload(links, ef)
+        with pytest.raises(NrqcdError):
+            g.GaussProjection(1e-9, max_sweeps=20)
+        _, got = g.download()
+    want, l = ef.copy(), links.copy()
+    assert oracle.gauss_project(N, a, l, want, tol=1e-9, max_sweeps=20) == 20
+    assert np.abs(got - want).max() < 1e-13 * np.abs(want).max()
