@@ -1407,11 +1407,14 @@ int ensure_f32(nrq_cn *cn, const nrq_gauge *g) {
   return check_launch(ctx, "k_cn_to_f32");
 }
 // The operator in its spin structure for the coefficients C (of A^H, tau =
-// dt a0/2 of that solve); sign -1 where it was built for C negated.
+// dt a0/2 of that solve), in FP64 where the FMA stencil runs, rounded to FP32
+// where the Chebyshev step on it may, and the planes of its spectral
+// enclosure in any case; sign -1 where it was built for C negated.
 int ensure_spin(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *sign) {
   nrq_ctx *ctx = cn->ctx;
   const int64_t V = ctx->lat.V;
-  *sign = blocks_sign(cn->spin_valid, cn->spin_coef, C);
+  const bool want64 = cn->stencil == NRQ_STENCIL_FMA, want32 = use_cheb_spin(cn);
+  *sign = blocks_sign(cn->spin_valid && (cn->spin_has64 || !want64) && (cn->spin_has32 || !want32), cn->spin_coef, C);
   if (*sign != 0.0) {  // the site term as well
     for (int sp = 0; sp < 2; ++sp)
       if (cn->spin_coef.mag[sp].im != *sign * C.mag[sp].im || cn->spin_coef.dar[sp].im != *sign * C.dar[sp].im)
@@ -1425,28 +1428,53 @@ int ensure_spin(nrq_cn *cn, const nrq::CnCoef &C, const nrq_gauge *g, double *si
   }
   NRQ_CUDA_TRY(ctx, want(&cn->spin_part, sizeof(double) * 4 * ((V + 255) / 256)));
   NRQ_CUDA_TRY(ctx, want(&cn->spin_scratch, sizeof(double) * 7 * V));
-  NRQ_CUDA_TRY(ctx, want(&cn->spin.S0, sizeof(double2) * 9 * V));
-  NRQ_CUDA_TRY(ctx, want(&cn->spin.S1, sizeof(double) * 9 * V));
-  NRQ_CUDA_TRY(ctx, want(&cn->spin.W, sizeof(double2) * 81 * V));
+  nrq::SpinOp op{};
+  if (want64) {
+    NRQ_CUDA_TRY(ctx, want(&cn->spin.S0, sizeof(double2) * 9 * V));
+    NRQ_CUDA_TRY(ctx, want(&cn->spin.S1, sizeof(double) * 9 * V));
+    NRQ_CUDA_TRY(ctx, want(&cn->spin.W, sizeof(double2) * 81 * V));
+    op = cn->spin;
+  }
   nrq::SpinOp32 op32{};
-  if (use_cheb_spin(cn)) {
+  if (want32) {
     NRQ_CUDA_TRY(ctx, want(&cn->spin32.S0, sizeof(float2) * 9 * V));
     NRQ_CUDA_TRY(ctx, want(&cn->spin32.S1, sizeof(float) * 9 * V));
     NRQ_CUDA_TRY(ctx, want(&cn->spin32.W, sizeof(float2) * 81 * V));
     op32 = cn->spin32;
   }
   {
-    ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0 + (op32.W ? 1.5 : 1.0) * (1296.0 + 216.0)));
+    ProfScope ps(ctx, 3, (double)V * (432.0 + 192.0 + ((op32.W ? 0.5 : 0.0) + (op.W ? 1.0 : 0.0)) * (1296.0 + 216.0)));
     // H = (A^H - 1) / (i tau): any tau with the coefficients' scale serves
     // the enclosure as long as the solve uses the same one
-    nrq::launch_spin_prepare(ctx->lat, C, nullptr, 1, cn->spin_tau != 0.0 ? cn->spin_tau : 1.0, g->U, g->E, cn->spin,
-                             op32, cn->spin_scratch, ctx->stream);
+    nrq::launch_spin_prepare(ctx->lat, C, nullptr, 1, cn->spin_tau != 0.0 ? cn->spin_tau : 1.0, g->U, g->E, op, op32,
+                             cn->spin_scratch, ctx->stream);
   }
   cn->spin_coef = C;
   cn->spin_valid = true;
+  cn->spin_has64 = want64;
+  cn->spin_has32 = want32;
   cn->spin_fresh = true;
   *sign = 1.0;
   return check_launch(ctx, "k_spin_prepare");
+}
+// ensure_spin for A^H at the head of an update.  Where memory lacks for it and
+// nobody asked for the kernels that read it, the update runs on the ones that
+// need none.
+int ensure_spin_or_less(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
+  double sign = 0.0;
+  int rc = ensure_spin(cn, CH, g, &sign);
+  if (rc && cn->stencil == NRQ_STENCIL_FMA && cn->forced_stencil < 0 && !cn->spin.W) {
+    cudaGetLastError();
+    cn->stencil = cn->tma_ok ? NRQ_STENCIL_TMA : NRQ_STENCIL_REGISTER;
+    rc = cn->form >= 1 ? ensure_spin(cn, CH, g, &sign) : NRQ_OK;
+  }
+  if (rc && use_cheb_spin(cn) && cn->cheb_stencil < 0 && !cn->spin32.W) {
+    cudaGetLastError();
+    cn->cheb_tuned = true;
+    cn->cheb_choice = NRQ_CHEB_REGISTER;
+    rc = ensure_spin(cn, CH, g, &sign);
+  }
+  return rc;
 }
 // The stencil launch of one 12-column application.  The tensor-core stencil
 // needs imaginary off-diagonal coefficients and tensor maps; otherwise the
@@ -1734,7 +1762,7 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   const double tau = std::fabs(dt) * ctx->a[0] / 2.0;
   int rc = cn_prepare(cn, g, dt);
   double spin_sign = 0.0;
-  if (!rc) rc = ensure_spin(cn, CH, g, &spin_sign);
+  if (!rc) rc = ensure_spin_or_less(cn, CH, g);
   if (rc) return rc;
   // spectral enclosure of H per species
   if ((rc = spin_bounds(cn, scal_bounds(cn->scal), false))) return rc;
@@ -2232,16 +2260,8 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
   int64_t matvecs = 0, vstreams = 0;
   bool fma = cn->stencil == NRQ_STENCIL_FMA && spin_stencil_applies(ctx, CH);
   if (fma) {
-    double sign = 0.0;
-    rc = ensure_spin(cn, CH, g, &sign);
-    if (rc && !cn->spin.W && !cn->tma_ok && cn->forced_stencil < 0) {
-      // no memory for the operator: the stencil that needs none
-      cudaGetLastError();
-      cn->stencil = NRQ_STENCIL_REGISTER;
-      fma = false;
-      rc = NRQ_OK;
-    }
-    if (rc) return rc;
+    if ((rc = ensure_spin_or_less(cn, CH, g))) return rc;
+    fma = cn->stencil == NRQ_STENCIL_FMA;
   }
   const bool semi = fma && cn->semi_iteration();
   if (semi) {  // the Chebyshev coefficients, ahead of the right-hand side

@@ -191,6 +191,7 @@ struct nrq_cn {
   // scratch planes and partial rows of the spectral enclosure and its ticket
   nrq::SpinOp spin{};
   bool spin_valid = false;
+  bool spin_has64 = false, spin_has32 = false;  // which of spin, spin32 it was built into
   bool spin_fresh = false;  // written by the latest launch on the stream
   nrq::CnCoef spin_coef{};
   double spin_tau = 0.0;
