@@ -211,8 +211,9 @@ int nrq_cn_finalize(nrq_cn *cn);
 #define NRQ_STENCIL_TENSOR 2
 #define NRQ_STENCIL_FMA 3
 /* The stencil the solver uses and the per-launch milliseconds of each one
- * measured on its first update (index = NRQ_STENCIL_*; -1 before it, or for
- * one that does not apply to the lattice or coefficients).               */
+ * that its choice measured (index = NRQ_STENCIL_*; -1 before it, where the
+ * choice needed no timing, or for one that does not apply to the lattice or
+ * coefficients).                                                           */
 int nrq_cn_stencil_info(const nrq_cn *cn, int *stencil, double ms[4]);
 /* Test hook of the FMA stencil's bounded pipeline waits (no reference
  * counterpart).  wait_cycles bounds every wait (0 restores the default,
@@ -225,8 +226,10 @@ int nrq_cn_stencil_info(const nrq_cn *cn, int *stencil, double ms[4]);
  * this solver's context (lattices that run many sweeps a launch), whose
  * waits wait_cycles then bounds.                                           */
 int nrq_cn_set_wait_test(nrq_cn *cn, int64_t wait_cycles, int stall_load);
-/* Force a stencil (NRQ_STENCIL_*) or restore the timed choice (-1).
- * NRQ_ERR_BAD_ARG if the stencil cannot describe this lattice.            */
+/* Force a stencil (NRQ_STENCIL_*) or have the next update time the applicable
+ * ones and choose (-1).  By default a solver takes FMA where it applies to the
+ * coefficients, and times where BiCGStab runs.  NRQ_ERR_BAD_ARG if the stencil
+ * cannot describe this lattice.                                            */
 int nrq_cn_set_stencil(nrq_cn *cn, int stencil);
 /* The FP32 Chebyshev step of the precision forms (forms 1 and 2; no
  * reference counterpart).  REGISTER: the operator assembled from FP32 links

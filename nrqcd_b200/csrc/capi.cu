@@ -1242,6 +1242,7 @@ extern "C" int nrq_cn_set_stencil(nrq_cn *cn, int stencil) {
     return NRQ_ERR_BAD_ARG;
   }
   cn->forced_stencil = stencil;
+  cn->timing_asked = stencil < 0;
   cn->stencil_tuned = false;
   cn->stencil = stencil >= 0 ? stencil : (cn->tma_ok ? NRQ_STENCIL_TMA : NRQ_STENCIL_REGISTER);
   return NRQ_OK;
@@ -1547,15 +1548,19 @@ void fin(nrq_cn *cn, int stage, double *scal = nullptr) {
   ProfScope ps(ctx, 2, (double)rows * 12 * 3 * 8);
   nrq::launch_cn_finalize(stage, rows, cn->partials, scal ? scal : cn->scal, cn->tol, ctx->stream);
 }
-// Choose the stencil by timing, on this lattice and field, the work each
-// does in the solve: for the plain form t = A^H (r - alpha v) (the
-// register-tiled stencil forms s on the fly, the staged ones need s
-// materialised first); for the precision forms the FP64 refinement
+// The stencil of a solver that forces none.  Where the FMA stencil takes the
+// coefficients, the semi-iteration and the precision forms run on it: it was
+// the fastest at every size (a launch at 12^3 9 us, register-tiled 40; a
+// coupled step at 12^3 242 us against 374 with the best of the others, 64^3
+// 4.9 ms against 6.9).  BiCGStab, and a solver whose caller asked for the
+// timed choice (nrq_cn_set_stencil with -1), time, on this lattice and field,
+// the work each stencil does in the solve: for the plain form t = A^H (r -
+// alpha v) (the register-tiled stencil forms s on the fly, the staged ones
+// need s materialised first); for the precision forms the FP64 refinement
 // residual.  Every buffer written here (s, t, the partials, r32, d32) is
 // rewritten by the solve before it is read.  The choice minimises the time
 // of an update's stencil work (launches per update x time per launch, plus
-// the per-update block build of the tensor-core stencil).  A forced stencil
-// skips this.
+// the per-update block build of the tensor-core stencil).
 int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   nrq_ctx *ctx = cn->ctx;
   cn->stencil_tuned = true;
@@ -1563,15 +1568,18 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
     cn->stencil = cn->forced_stencil;
     return NRQ_OK;
   }
-  if (!cn->tma_ok) {  // the register-tiled and the FMA stencil apply: the latter where the coefficients allow it
-    if (spin_stencil_applies(ctx, CH)) cn->stencil = NRQ_STENCIL_FMA;
+  const bool spin = spin_stencil_applies(ctx, CH);
+  // (odd volumes: the register-tiled and the FMA stencil apply)
+  if (spin && (!cn->tma_ok || (!cn->timing_asked && (cn->form != 0 || cn->semi_iteration())))) {
+    cn->stencil = NRQ_STENCIL_FMA;
     return NRQ_OK;
   }
+  if (!cn->tma_ok) return NRQ_OK;
   cudaStream_t st = ctx->stream;
   const bool prof = ctx->prof;
   ctx->prof = false;
   const int reps = 3;
-  const bool tensor = offdiag_imaginary(CH), spin = spin_stencil_applies(ctx, CH);
+  const bool tensor = offdiag_imaginary(CH);
   cudaEvent_t e0, e1;
   NRQ_CUDA_TRY(ctx, cudaEventCreate(&e0));
   NRQ_CUDA_TRY(ctx, cudaEventCreate(&e1));
@@ -1579,6 +1587,12 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   for (int which = 0; which < 4 && !rc; ++which) {
     cn->tune_ms[which] = -1.0;
     if ((which == NRQ_STENCIL_TENSOR && !tensor) || (which == NRQ_STENCIL_FMA && !spin)) continue;
+    // no memory for the tensor-core stencil's blocks: not a candidate
+    if (which == NRQ_STENCIL_TENSOR && !cn->Wblk &&
+        cudaMalloc((void **)&cn->Wblk, sizeof(double2) * 216 * ctx->lat.V) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
     cn->stencil = which;
     for (int r = 0; r < reps + 1 && !rc; ++r) {
       if (r == 1) cudaEventRecord(e0, st);
@@ -1649,11 +1663,14 @@ int tune_stencil(nrq_cn *cn, const nrq::CnCoef &CH, const nrq_gauge *g) {
   int best = NRQ_STENCIL_REGISTER;
   for (int which = 1; which < 4; ++which)
     if (cn->tune_ms[which] > 0.0 && cost(which) < cost(best)) best = which;
-  // the semi-iteration wins by more than the timing's noise at every size (a
-  // coupled step with it against the best of the others: 242 against 374 us
-  // at 12^3, 4.9 against 6.9 ms at 64^3)
+  // (the semi-iteration by more than the timing's noise)
   if (cn->form == 0 && cn->semi_iteration() && cn->tune_ms[NRQ_STENCIL_FMA] > 0.0) best = NRQ_STENCIL_FMA;
   cn->stencil = best;
+  if (best != NRQ_STENCIL_TENSOR && cn->Wblk) {  // 3.4 KB a site that nothing reads from here on
+    cudaFree(cn->Wblk);
+    cn->Wblk = nullptr;
+    cn->w_valid = false;
+  }
   return NRQ_OK;
 }
 // the gauge field of this update: every derived set follows it on demand
@@ -1762,6 +1779,8 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   const double tau = std::fabs(dt) * ctx->a[0] / 2.0;
   int rc = cn_prepare(cn, g, dt);
   double spin_sign = 0.0;
+  // (before the right-hand side, which then runs on the chosen stencil)
+  if (!rc && !cn->stencil_tuned) rc = tune_stencil(cn, CH, g);
   if (!rc) rc = ensure_spin_or_less(cn, CH, g);
   if (rc) return rc;
   // spectral enclosure of H per species
@@ -1815,7 +1834,6 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   }
   NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   if (learned && (rc = nrqh::learned_check(cn->learn))) return rc;
-  if (!cn->stencil_tuned && (rc = tune_stencil(cn, CH, g))) return rc;
   ChebSeg seg[2];
   for (int sp = 0; sp < 2; ++sp) {
     double lo = cn->h_bounds[2 * sp], hi = cn->h_bounds[2 * sp + 1];

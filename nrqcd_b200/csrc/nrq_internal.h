@@ -145,14 +145,15 @@ struct nrq_cn {
           *t = nullptr, *s = nullptr;
   // FP64 stencil (NRQ_STENCIL_*): register-tiled, TMA-staged, tensor-core
   // or FMA in the spin structure.
-  // Chosen by timing the applicable ones on the first update (tune_ms, per
-  // launch) unless forced; tma_ok: tensor maps can describe the lattice.
+  // Chosen on the first update unless forced, by timing the applicable ones
+  // (tune_ms, per launch) where that was asked for (timing_asked) or BiCGStab
+  // runs; tma_ok: tensor maps can describe the lattice.
   // last_stencil: the stencil of the latest launch (its partial-row count).
   int stencil = 0;
   int forced_stencil = -1;
   int last_stencil = 0;
   bool tma_ok = false;
-  bool stencil_tuned = false;
+  bool stencil_tuned = false, timing_asked = false;
   double tune_ms[4] = {-1.0, -1.0, -1.0, -1.0};
   // plain form: start from 2b - psi + 2 t1 - t2 with the field's history of
   // corrections (FP32); on by default

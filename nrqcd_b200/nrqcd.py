@@ -74,8 +74,8 @@ STENCIL_NAMES = {STENCIL_REGISTER: "k_cn_mv2 (register-tiled)", STENCIL_TMA: "k_
 
 
 def SetStencil(stencil=None):
-    """Force the solver's FP64 stencil (STENCIL_*); None restores the choice
-    timed on the next update."""
+    """Force the solver's FP64 stencil (STENCIL_*); None has the next update
+    time the applicable ones and choose."""
     ctx = lattice.context()
     _capi.check(_capi.load().nrq_cn_set_stencil(solver_handle(), -1 if stencil is None else int(stencil)), ctx,
                 f"Error in {modulename}: stencil")
@@ -156,8 +156,8 @@ def SetWaitTest(wait_cycles=0, stall_load=-1, launch=None, projection=None):
 
 
 def StencilInfo():
-    """(stencil in use, per-launch ms of each stencil timed on the first
-    update; -1 where not timed)."""
+    """(stencil in use, per-launch ms of each stencil that its choice timed;
+    -1 where not timed)."""
     which = ctypes.c_int()
     ms = np.zeros(4)
     _capi.check(_capi.load().nrq_cn_stencil_info(solver_handle(), ctypes.byref(which), _capi.dptr(ms)),
