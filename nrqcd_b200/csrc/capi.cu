@@ -1940,15 +1940,16 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
       break;
     }
     if (outer == 7) break;
-    // gain needed to bring the worst column to 0.1 tol: the error of a point
+    // gain needed to bring the worst column to 0.05 tol: the error of a point
     // source sits on the few sites the field has reached, so that the worst
     // element stands well above the norm, and updates that end anywhere below
     // tol add up (96^3, tol 1e-10, error of the propagator after eight: 8e-11
-    // in norm and 3e-8 of its rms at the worst element with passes to 0.3 tol)
+    // in norm and 3e-8 of its rms at the worst element with passes to 0.3 tol,
+    // 5e-12 and 1e-9 with these)
     double worst = 0.0;
     for (int kk = 0; kk < nrq::CN_COLS; ++kk) worst = std::max(worst, rel[kk]);
     // maxits bounds the FP32 inner steps of the whole update
-    int m = inner_steps(worst / (0.1 * cn->tol));
+    int m = inner_steps(worst / (0.05 * cn->tol));
     if (inner + m > cn->maxits) m = (int)(cn->maxits - inner);
     if (m <= 0) break;
     // FP32 inner Chebyshev solve of A^H e = r, and x += e
