@@ -1741,8 +1741,8 @@ int tune_cheb(nrq_cn *cn, const nrq::CnCoef &CH, const nrq::ChebCoef &K, const n
     for (int r = 0; r < reps + 1; ++r) {
       if (r == 1) cudaEventRecord(e0, st);
       if (which == NRQ_CHEB_BLOCKS)
-        nrq::launch_cheb_spin(1, false, ctx->lat, cn->spin32, cn->r32, cn->dA32, cn->dB32, nullptr, nullptr, K,
-                              inv_theta, false, scal_err(cn->scal), st, cn->wait_cycles);
+        nrq::launch_cheb_spin(1, false, ctx->lat, cn->spin32, cn->r32, cn->dA32, cn->dB32, nullptr, nullptr, nullptr,
+                              nullptr, K, inv_theta, false, scal_err(cn->scal), st, cn->wait_cycles);
       else
         nrq::launch_cheb32(true, ctx->lat, CH, cn->U32, cn->D32, cn->B32, cn->DE32, cn->dA32, cn->dB32, cn->e32,
                            cn->e32, K, st);
@@ -1791,34 +1791,32 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   // learned form: x = 2 RHS - psi + w1 u + w2 v (network), history restarted
   // with the network's part; every refinement correction is added to it
   const bool learned = cn->form == 2 && nrqh::learned_ready(cn->learn);
-  // otherwise the plain solve's extrapolated start from the field's history;
-  // on the FMA stencil the right-hand side's launch adds it and starts the
-  // new history vector with the added part, which every correction then joins
+  // otherwise the plain solve's extrapolated start from the field's history,
+  // which on the FMA stencil the right-hand side's launch adds
   const bool hist = !learned && cn->history_guess;
   const bool fma = cn->stencil == NRQ_STENCIL_FMA && nrq::cn_spin_applicable(L);
-  if (hist && fma && (rc = nrqh::ensure_hist(h, cn->history_depth))) return rc;
-  const int hist_depth = hist ? std::min(cn->history_depth, h->hist_count) : 0;
-  const int hist_count = h->hist_count;
-  float2 *hacc = hist && fma ? hist_next(h) : nullptr;
+  if (hist && (rc = nrqh::ensure_hist(h, cn->history_depth))) return rc;
+  const int hist_count = h->hist_count, hist_depth = hist ? std::min(cn->history_depth, hist_count) : 0;
+  // the vector that the passes update with x: the learned form's part of the
+  // start, which every correction joins; otherwise the new history vector,
+  // stored anew by each pass of the spin-structured step (stored: it is)
+  float2 *hacc = hist ? hist_next(h) : nullptr;
+  bool stored = false;
   {  // RHS = A psi ; x0 = 2 RHS - psi
     nrq::MvArgs a{};
     a.in = h->P;
     a.out = cn->b;
     a.out2 = cn->x;
-    a.r32 = hacc;
-    if (hacc)
+    if (fma)
       for (int k = 0; k < hist_depth; ++k) {
         a.hist[k] = hist_v(h, k + 1);
         a.hcoef[k] = nrq::hist_coef(hist_depth, k);
       }
-    // the oldest history vector's slot is overwritten from here on: an
-    // update that ends early leaves the field without a history
-    if (hacc) h->hist_count = 0;
     if ((rc = mv(cn, nrq::MV_RHS, CA, g, a))) return rc;
     matvecs += 1;
     vstreams += 1;
   }
-  if (hist_depth >= 1 && !hacc) {
+  if (hist_depth >= 1 && !fma) {
     const float2 *t[4] = {hist_v(h, 1), hist_v(h, 2), hist_v(h, 3), hist_v(h, 4)};
     ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * hist_depth));
     nrq::launch_hist_extrapolate(72 * V, cn->x, t, hist_depth, st);
@@ -1958,20 +1956,27 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     if (cn->cheb_stencil < 0 && !cn->cheb_tuned && (rc = tune_cheb(cn, CH, coef[0], a.inv_theta))) return rc;
     if (use_cheb_spin(cn)) {
       cn->last_cheb = NRQ_CHEB_BLOCKS;
+      const double2 *hb = hist ? cn->b : nullptr, *hpsi = hist ? h->P : nullptr;
+      const double hbytes = hist ? 1152.0 * 2 + 576.0 : hacc ? 1152.0 : 0.0;
+      // the oldest history vector's slot is overwritten from here on: an
+      // update that ends early leaves the field without a history
+      if (hist) h->hist_count = 0;
+      stored = hist;
       if (m == 1) {
-        ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * (hacc ? 3 : 1)));
-        nrq::launch_cheb_one(72 * V, cn->r32, cn->x, hacc, a.inv_theta, st);
+        ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 + hbytes));
+        nrq::launch_cheb_one(72 * V, cn->r32, cn->x, hacc, hb, hpsi, a.inv_theta, st);
       }
       for (int k = 0; k < m - 1; ++k) {
         const bool last = k == m - 2;
         ProfScope ps(ctx, 0, (double)V * (576.0 * (k == 0 ? 1 : k == 1 ? 2 : 3) +
-                                          (last ? 1152.0 * 2 + (hacc ? 1152.0 : 0.0) : 576.0) + 756.0));
-        nrq::launch_cheb_spin(k, last, L, cn->spin32, cn->r32, cn->dA32, cn->dB32, cn->x, hacc, coef[k], a.inv_theta,
-                              !cn->spin_fresh, scal_err(cn->scal), st, cn->wait_cycles);
+                                          (last ? 1152.0 * 2 + hbytes : 576.0) + 756.0));
+        nrq::launch_cheb_spin(k, last, L, cn->spin32, cn->r32, cn->dA32, cn->dB32, cn->x, hacc, hb, hpsi, coef[k],
+                              a.inv_theta, !cn->spin_fresh, scal_err(cn->scal), st, cn->wait_cycles);
         cn->spin_fresh = false;
       }
     } else {
       cn->last_cheb = NRQ_CHEB_REGISTER;
+      stored = false;
       float2 *dcur = cn->dA32, *dnext = cn->dB32;
       for (int k = 0; k < m; ++k) {
         ProfScope ps(ctx, 0, (double)V * (576.0 * 6 + 756.0));
@@ -1979,8 +1984,8 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
                            coef[k], st);
         std::swap(dcur, dnext);
       }
-      ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * (hacc ? 3 : 1)));
-      if (hacc)
+      ProfScope ps(ctx, 1, (double)V * (1152.0 * 2 + 576.0 * (learned ? 3 : 1)));
+      if (learned)
         nrqh::add_e_hist(72 * V, cn->x, cn->e32, hacc, st);
       else
         nrq::launch_add_e(72 * V, cn->x, cn->e32, st);
@@ -2014,14 +2019,14 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     }
   }
   if (status == NRQ_OK && !conv) status = NRQ_ERR_NOT_CONVERGED;
-  bool keep = hacc && status == NRQ_OK;
-  if (keep && !learned) h->hist_count = hist_count;
-  if (hist && !hacc && status == NRQ_OK) {  // t = x - (2 RHS - psi) into the history
-    if ((rc = nrqh::ensure_hist(h, cn->history_depth))) return rc;
-    ProfScope ps(ctx, 1, (double)V * (1152.0 * 3 + 576.0));
-    nrq::launch_hist_store(72 * V, cn->x, cn->b, h->P, hist_next(h), st);
-    if ((rc = check_launch(ctx, "k_hist_store"))) return rc;
-    keep = true;
+  const bool keep = (hist || learned) && status == NRQ_OK;
+  if (hist && keep) {
+    h->hist_count = hist_count;
+    if (!stored) {  // t = x - (2 RHS - psi) into the history
+      ProfScope ps(ctx, 1, (double)V * (1152.0 * 3 + 576.0));
+      nrq::launch_hist_store(72 * V, cn->x, cn->b, h->P, hacc, st);
+      if ((rc = check_launch(ctx, "k_hist_store"))) return rc;
+    }
   }
   std::swap(h->P, cn->x);
   if (keep) hist_push(h);

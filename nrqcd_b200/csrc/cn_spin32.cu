@@ -8,8 +8,10 @@
 // vectors (e_k, r, e_{k-1} read; e_{k+1} over e_{k-1}) where the recurrence
 // on (d, r, e) moved seven and its last launch only added d.  r - A^H e is
 // formed as (r - e) - (A^H - 1) e, whose rounding is that of the small part.
-// The last launch adds e_{k+1} to the FP64 iterate (and to the step's
-// history) in place of a pass of its own.
+// The last launch adds e_{k+1} to the FP64 iterate in place of a pass of its
+// own, and stores the step's history x - (2b - psi) from it, the FP64
+// difference rounded once (the learned form and the batch add e_{k+1} to what
+// their start put there instead).
 //
 // Bound: 64^3, 3.1 KB a site: 0.12 ms at the copy rate, 0.08 ms of FP32
 // FMAs; it takes 0.24 ms (the (d, r, e) recurrence on dense 6x6 blocks 0.36,
@@ -29,7 +31,8 @@ struct Step32 {
   const float2 *prev;    // e_{k-1}; null: r / theta
   float2 *out;           // e_{k+1}
   double2 *x;            // last: x += e_{k+1}
-  float2 *hist;          // last: history += e_{k+1} (may be null)
+  float2 *hist;          // last: history += e_{k+1} (may be null), or with b
+  const double2 *b, *psi;  //   history = x - (2b - psi)
   cplx c1[2], c2[2], it[2];
 };
 struct Batch32 {
@@ -42,8 +45,8 @@ __device__ __forceinline__ cx<float> cmul(cx<float> a, cx<float> b) {
 }
 
 // FIRST: e_2 from r alone (A^H e_1 = A^H r / theta); LAST: into x and the
-// history instead of out.
-template <bool FIRST, bool LAST, bool BATCH>
+// history instead of out, 2: the history anew from b and psi.
+template <bool FIRST, int LAST, bool BATCH>
 __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
     k_cheb_spin(Lat L, SpinOp32 op, Step32 A, Batch32 Bt, int *err, long long wait_cycles, bool early) {
   constexpr int kAhead = Num<float>::kAhead;
@@ -90,14 +93,16 @@ __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
     for (int h = 0; h < 2; ++h) {  // three rows at a time
       const int64_t off = (int64_t)(sp * 36 + warp * 6 + 3 * h) * V + x;
       float2 rv[3], pv[3], hv[3];
-      double2 xv[3];
+      double2 xv[3], bv[3], sv[3];
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         const int64_t o = off + (int64_t)q * V;
         if (!FIRST) rv[q] = __ldca(A.r + o);
         if (!FIRST && A.prev) pv[q] = A.prev[o];
         if (LAST) xv[q] = A.x[o];
-        if (LAST && A.hist) hv[q] = A.hist[o];
+        if (LAST == 1 && A.hist) hv[q] = A.hist[o];
+        if (LAST == 2) bv[q] = __ldca(A.b + o);
+        if (LAST == 2) sv[q] = __ldca(A.psi + o);
       }
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
@@ -120,8 +125,12 @@ __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
         const cx<float> a = cmul(c1, d), b = cmul(c2, res);
         const float2 en = make_float2(e.re + (a.re + b.re), e.im + (a.im + b.im));
         if (LAST) {
-          A.x[o] = make_double2(xv[q].x + (double)en.x, xv[q].y + (double)en.y);
-          if (A.hist) A.hist[o] = make_float2(hv[q].x + en.x, hv[q].y + en.y);
+          const double2 xn = make_double2(xv[q].x + (double)en.x, xv[q].y + (double)en.y);
+          A.x[o] = xn;
+          if (LAST == 2)
+            A.hist[o] = make_float2((float)(xn.x - (2.0 * bv[q].x - sv[q].x)), (float)(xn.y - (2.0 * bv[q].y - sv[q].y)));
+          else if (A.hist)
+            A.hist[o] = make_float2(hv[q].x + en.x, hv[q].y + en.y);
         } else {
           A.out[o] = en;
         }
@@ -130,7 +139,7 @@ __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
   }
 }
 
-// m = 1: x += r / theta, history += the same (n elements a field)
+// m = 1: x += r / theta, and the history as above (n elements a field)
 template <bool BATCH>
 __global__ void k_cheb_one(int64_t n, Step32 A, const BatchField *__restrict__ tab) {
   if (BATCH) {
@@ -146,8 +155,12 @@ __global__ void k_cheb_one(int64_t n, Step32 A, const BatchField *__restrict__ t
     const float2 r = A.r[i];
     const cx<float> e = cmul(f2(i >= n / 2 ? A.it[1] : A.it[0]), {r.x, r.y});
     const double2 x = A.x[i];
-    A.x[i] = make_double2(x.x + (double)e.re, x.y + (double)e.im);
-    if (A.hist) {
+    const double2 xn = make_double2(x.x + (double)e.re, x.y + (double)e.im);
+    A.x[i] = xn;
+    if (!BATCH && A.b) {
+      const double2 b = A.b[i], p = A.psi[i];
+      A.hist[i] = make_float2((float)(xn.x - (2.0 * b.x - p.x)), (float)(xn.y - (2.0 * b.y - p.y)));
+    } else if (A.hist) {
       const float2 h = A.hist[i];
       A.hist[i] = make_float2(h.x + e.re, h.y + e.im);
     }
@@ -163,14 +176,24 @@ void go(bool first, bool last, int64_t blocks, Lat L, const SpinOp32 &op, const 
     else
       launch_pdl(kern, (unsigned)blocks, kUnit * kWarps, 0, st, L, op, A, Bt, err, wait_cycles, early);
   };
-  if (first && last)
-    run(k_cheb_spin<true, true, BATCH>);
-  else if (first)
-    run(k_cheb_spin<true, false, BATCH>);
-  else if (last)
-    run(k_cheb_spin<false, true, BATCH>);
-  else
-    run(k_cheb_spin<false, false, BATCH>);
+  // (a batch's fields carry no b and psi here)
+  const bool store = !BATCH && A.b != nullptr;
+  if (!last) {
+    if (first)
+      run(k_cheb_spin<true, 0, BATCH>);
+    else
+      run(k_cheb_spin<false, 0, BATCH>);
+  } else if (store) {
+    if (first)
+      run(k_cheb_spin<true, BATCH ? 1 : 2, BATCH>);
+    else
+      run(k_cheb_spin<false, BATCH ? 1 : 2, BATCH>);
+  } else {
+    if (first)
+      run(k_cheb_spin<true, 1, BATCH>);
+    else
+      run(k_cheb_spin<false, 1, BATCH>);
+  }
 }
 }  // namespace
 
@@ -179,8 +202,8 @@ bool cheb_spin_applicable(const Lat &L) {
 }
 
 void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const float2 *r, float2 *ea, float2 *eb,
-                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], bool early, int *err,
-                      cudaStream_t st, long long wait_cycles) {
+                      double2 *x, float2 *hist, const double2 *b, const double2 *psi, const ChebCoef &K,
+                      const cplx inv_theta[2], bool early, int *err, cudaStream_t st, long long wait_cycles) {
   Step32 A{};
   A.in = step == 0 ? r : (step & 1) ? ea : eb;
   A.r = r;
@@ -188,6 +211,8 @@ void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const floa
   A.out = (step & 1) ? eb : ea;
   A.x = x;
   A.hist = hist;
+  A.b = b;
+  A.psi = psi;
   for (int sp = 0; sp < 2; ++sp) {
     A.c1[sp] = K.c1[sp];
     A.c2[sp] = K.c2[sp];
@@ -196,11 +221,14 @@ void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const floa
   go<false>(step == 0, last, (L.V + kUnit - 1) / kUnit, L, op, A, Batch32{}, err, st, wait_cycles, early);
 }
 
-void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const cplx inv_theta[2], cudaStream_t st) {
+void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const double2 *b, const double2 *psi,
+                     const cplx inv_theta[2], cudaStream_t st) {
   Step32 A{};
   A.r = r;
   A.x = x;
   A.hist = hist;
+  A.b = b;
+  A.psi = psi;
   A.it[0] = inv_theta[0];
   A.it[1] = inv_theta[1];
   k_cheb_one<false><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, A, nullptr);

@@ -375,13 +375,15 @@ void launch_cheb32(bool first, Lat L, const CnCoef &C, const float2 *U, const fl
 // The inner solve A^H e = r on the operator in its spin structure, FP32
 // (cn_spin32.cu): launch `step` = 0, 1, .. makes e_{step+2} with the step's
 // coefficients K, into ea (even steps) or eb (odd ones); the last one adds it
-// to x and, if not null, to hist instead.  m Chebyshev steps take m - 1
+// to x instead and, if not null, to hist, or with b and psi stores hist = x -
+// (2b - psi).  m Chebyshev steps take m - 1
 // launches, one step is launch_cheb_one over the n elements.
 bool cheb_spin_applicable(const Lat &L);
 void launch_cheb_spin(int step, bool last, Lat L, const SpinOp32 &op, const float2 *r, float2 *ea, float2 *eb,
-                      double2 *x, float2 *hist, const ChebCoef &K, const cplx inv_theta[2], bool early, int *err,
-                      cudaStream_t st, long long wait_cycles);
-void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const cplx inv_theta[2], cudaStream_t st);
+                      double2 *x, float2 *hist, const double2 *b, const double2 *psi, const ChebCoef &K,
+                      const cplx inv_theta[2], bool early, int *err, cudaStream_t st, long long wait_cycles);
+void launch_cheb_one(int64_t n, const float2 *r, double2 *x, float2 *hist, const double2 *b, const double2 *psi,
+                     const cplx inv_theta[2], cudaStream_t st);
 void launch_add_e(int64_t n, double2 *X, const float2 *E, cudaStream_t st);
 void launch_prop_f2soa(const double2 *f, double2 *P, int64_t V, cudaStream_t st);
 void launch_prop_soa2f(const double2 *P, double2 *f, int64_t V, cudaStream_t st);
