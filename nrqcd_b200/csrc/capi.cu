@@ -37,10 +37,9 @@ constexpr size_t kScalDoubles = (size_t)nrq::CN_COLS * nrq::SC_STRIDE;
 constexpr size_t kScalBytes = sizeof(double) * (kScalDoubles + 8 + 4);
 inline double *scal_bounds(double *scal) { return scal + kScalDoubles + 8; }
 inline int *scal_err(double *scal) { return (int *)(scal + kScalDoubles); }
-// the stencils' record of an expired pipeline wait (4 ints after the
-// scalars): the message of the update that reports it, and a reset
-std::string timeout_message(const double *h_scal) {
-  const int *e = (const int *)(h_scal + kScalDoubles);
+// the stencils' record of an expired pipeline wait (4 ints): the message of
+// the update that reports it
+std::string timeout_message(const int *e) {
   static const char *roles[] = {"a consumer's wait for a load", "a consumer's wait for the diagonal matrices",
                                 "the loader's wait for a released buffer", "the loader's wait for a landed load",
                                 "the loader's final drain"};
@@ -1196,7 +1195,8 @@ extern "C" int nrq_cn_init(nrq_ctx *ctx, double mass, const double c[8], double 
     alloc((void **)&cn->D32, sizeof(float2) * 9 * V);
     alloc((void **)&cn->B32, sizeof(float) * 9 * V);
     for (float2 **pp : {&cn->r32, &cn->dA32, &cn->dB32, &cn->e32}) alloc((void **)pp, sizeof(float2) * 72 * V);
-    if (ok && cudaMallocHost((void **)&cn->h_bounds, sizeof(double) * 8) != cudaSuccess) ok = false;
+    if (ok && cudaMallocHost((void **)&cn->h_bounds, sizeof(double) * 16) != cudaSuccess) ok = false;
+    if (ok) std::memset(cn->h_bounds, 0, sizeof(double) * 16);
   }
   // the TMA-staged stencil needs 16-byte plane strides for the real-valued
   // magnetic planes (V even) and tiles no wider than the lattice
@@ -1787,6 +1787,9 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   if ((rc = spin_bounds(cn, scal_bounds(cn->scal), false))) return rc;
   NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(cn->h_bounds, scal_bounds(cn->scal), sizeof(double) * 4, cudaMemcpyDeviceToHost,
                                     st));
+  // the spin-structured kernels' record of an expired wait: pinned, read
+  // after a synchronisation without a copy
+  int *const perr = (int *)(cn->h_bounds + 8);
   int64_t matvecs = 0, vstreams = 0;
   // learned form: x = 2 RHS - psi + w1 u + w2 v (network), history restarted
   // with the network's part; every refinement correction is added to it
@@ -1812,7 +1815,7 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
         a.hist[k] = hist_v(h, k + 1);
         a.hcoef[k] = nrq::hist_coef(hist_depth, k);
       }
-    if ((rc = mv(cn, nrq::MV_RHS, CA, g, a))) return rc;
+    if ((rc = mv(cn, nrq::MV_RHS, CA, g, a, perr))) return rc;
     matvecs += 1;
     vstreams += 1;
   }
@@ -1883,6 +1886,18 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
   double pred[nrq::CN_COLS];
   bool pending = false, on_prediction = false;
   cn->last_true = true;
+  // waits for the stream and looks at both records of an expired wait
+  auto timed_out = [&]() -> int {
+    NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+    for (int *e : {perr, scal_err(hs)}) {
+      if (*e == 0) continue;
+      ctx->last_error = timeout_message(e);
+      std::memset(e, 0, 16 * sizeof(int));
+      NRQ_CUDA_TRY(ctx, cudaMemsetAsync(scal_err(cn->scal), 0, 16 * sizeof(int), st));
+      return NRQ_ERR_TIMEOUT;
+    }
+    return NRQ_OK;
+  };
   for (outer = 0; outer < 8; ++outer) {
     nrq::MvArgs a{};
     a.in = cn->x;
@@ -1896,18 +1911,13 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
       std::complex<double> it = 1.0 / seg[sp].theta;
       a.inv_theta[sp] = {it.real(), it.imag()};
     }
-    if ((rc = mv(cn, nrq::MV_RESC, CH, g, a))) return rc;
+    if ((rc = mv(cn, nrq::MV_RESC, CH, g, a, perr))) return rc;
     fin(cn, 0);
     matvecs += 1;
     vstreams += 3;
     if ((rc = check_launch(ctx, "cn residual"))) return rc;
     NRQ_CUDA_TRY(ctx, cudaMemcpyAsync(hs, cn->scal, kScalBytes, cudaMemcpyDeviceToHost, st));
-    NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if (*scal_err(hs) != 0) {
-      NRQ_CUDA_TRY(ctx, cudaMemsetAsync(scal_err(cn->scal), 0, 16 * sizeof(int), st));
-      ctx->last_error = timeout_message(hs);
-      return NRQ_ERR_TIMEOUT;
-    }
+    if ((rc = timed_out())) return rc;
     bool all = true, nonfin = false;
     for (int k = 0; k < nrq::CN_COLS; ++k) {
       all = all && hs[k * nrq::SC_STRIDE + nrq::SC_CONV] != 0.0;
@@ -1970,8 +1980,10 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
         const bool last = k == m - 2;
         ProfScope ps(ctx, 0, (double)V * (576.0 * (k == 0 ? 1 : k == 1 ? 2 : 3) +
                                           (last ? 1152.0 * 2 + hbytes : 576.0) + 756.0));
+        // (a negative bound: the wait test's launch)
+        const bool stall = cn->stall_launch >= 0 && cn->stall_launch == cn->spin_launches++;
         nrq::launch_cheb_spin(k, last, L, cn->spin32, cn->r32, cn->dA32, cn->dB32, cn->x, hacc, hb, hpsi, coef[k],
-                              a.inv_theta, !cn->spin_fresh, scal_err(cn->scal), st, cn->wait_cycles);
+                              a.inv_theta, !cn->spin_fresh, perr, st, stall ? -cn->wait_cycles : cn->wait_cycles);
         cn->spin_fresh = false;
       }
     } else {
@@ -2009,6 +2021,8 @@ int cn_update_precision(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, double mas
     }
     pending = true;
     if (predicted) {
+      // the field is handed out only once its last launch is known to be whole
+      if ((rc = timed_out())) return rc;
       for (int kk = 0; kk < nrq::CN_COLS; ++kk) pred[kk] *= std::max(1.0, cn->cheb_ratio);
       ++cn->cheb_unconfirmed;
       cn->last_true = false;
@@ -2114,7 +2128,7 @@ static bool cn_update_semi(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g, const n
   auto finished = [&]() -> int {
     NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     if (*scal_err(hc) != 0) {
-      ctx->last_error = timeout_message(hc);
+      ctx->last_error = timeout_message(scal_err(hc));
       std::memset(scal_err(hc), 0, 16 * sizeof(int));
       return NRQ_ERR_TIMEOUT;
     }
@@ -2471,7 +2485,7 @@ extern "C" int nrq_heavy_update_cn(nrq_cn *cn, nrq_heavy *h, const nrq_gauge *g,
     NRQ_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     if (*scal_err(hs) != 0) {
       status = NRQ_ERR_TIMEOUT;
-      ctx->last_error = timeout_message(hs);
+      ctx->last_error = timeout_message(scal_err(hs));
       NRQ_CUDA_TRY(ctx, cudaMemsetAsync(scal_err(cn->scal), 0, 16 * sizeof(int), st));
       break;
     }

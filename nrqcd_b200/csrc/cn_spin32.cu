@@ -83,7 +83,10 @@ __global__ void __launch_bounds__(kUnit *kWarps, LAST ? 3 : 4)
   const int x = act ? s : V - 1;  // a valid site for the addresses of idle lanes
   cx<float> acc[4][3];
   float2 own[kAhead][4];
-  const bool ok = apply<float>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, wait_cycles, -1, early, acc, own);
+  // a negative bound: the test of the timeout path, which stages no matrices
+  // from the fourth neighbour on
+  const bool ok = apply<float>(L, op.W, op.S0, op.S1, A.in, x, warp, sm, err, llabs(wait_cycles),
+                               wait_cycles < 0 ? 3 : -1, early, acc, own);
   cp_async_wait_all();
   if (!ok || !act) return;
 #pragma unroll

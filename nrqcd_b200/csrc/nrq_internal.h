@@ -236,7 +236,7 @@ struct nrq_cn {
   float2 *U32 = nullptr, *DE32 = nullptr, *D32 = nullptr;
   float *B32 = nullptr;
   float2 *r32 = nullptr, *dA32 = nullptr, *dB32 = nullptr, *e32 = nullptr;
-  double *h_bounds = nullptr;  // pinned
+  double *h_bounds = nullptr;  // pinned; behind them 16 ints, the record of an expired wait
   int64_t last_inner = 0;      // FP32 Chebyshev steps of the last update
   int64_t last_outer = 0;      // FP64 refinement passes of the last update
   double last_lo[2] = {0, 0}, last_hi[2] = {0, 0};

@@ -3,7 +3,8 @@ update, whichever launch it is: the right-hand side (whose record the plain
 solve's semi-iteration reads with its first residual), or a step of a solve
 that ends on its bound, with no residual pass after it.  The launch's loader
 stops before its fourth load, the waits are bounded at about a millisecond,
-nothing faults, and the context then runs a clean step.
+nothing faults, and the context then runs a clean step.  In the precision form
+a Chebyshev step of an update that ends on its prediction.
 
 The same of a Gauss projection, whose second launch here repeats the first one
 up to the sweep that met the tolerance: messages withheld in either are an
@@ -13,7 +14,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from nrqcd_b200 import GaugeConfiguration, NRQCDField, _capi, nrqcd
+from nrqcd_b200 import GaugeConfiguration, NRQCDField, _capi, lattice, nrqcd
 from tests.gpu_util import lattice_ctx
 
 pytestmark = pytest.mark.gpu
@@ -36,6 +37,8 @@ def check_one_launch(oracle, form, tol, launch, before):
     links, ef = oracle.transverse_box(n, A, 3.0, 1.0, 0.0, 5, identity_links=False)
     with lattice_ctx(n, A, cn=(M, C, 1.0, tol, 10000, form)):
         nrqcd.SetStencil(nrqcd.STENCIL_FMA)
+        if form == nrqcd.FORM_PRECISION:
+            nrqcd.SetChebStencil(nrqcd.CHEB_BLOCKS)
         g = GaugeConfiguration()
         g.upload(links, ef)
         h = NRQCDField()
@@ -47,6 +50,7 @@ def check_one_launch(oracle, form, tol, launch, before):
         rc, st = update(h, g)
         nrqcd.SetWaitTest()
         assert rc == _capi.NRQ_ERR_TIMEOUT and st["converged"] == 0, (rc, st)
+        assert b"wait" in _capi.load().nrq_last_error(lattice.context())
         q, an = oracle.single_point(n, 1), oracle.single_point(n, 1)
         h.upload(q, an)
         rc, st = update(h, g)
@@ -65,6 +69,12 @@ def test_right_hand_side(oracle, before):
 @pytest.mark.parametrize("launch", [2, 4])
 def test_step_of_an_unconfirmed_solve(oracle, launch):
     check_one_launch(oracle, nrqcd.FORM_PLAIN_FP64, 1e-12, launch, 2)
+
+
+# launch 0 the right-hand side, 1 the residual, then the steps
+@pytest.mark.parametrize("launch", [2, 4])
+def test_step_of_a_predicted_update(oracle, launch):
+    check_one_launch(oracle, nrqcd.FORM_PRECISION, 1e-10, launch, 6)
 
 
 @pytest.mark.parametrize("launch", [0, 1])
