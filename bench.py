@@ -403,15 +403,16 @@ def measure_gluon_distribution(L, cpu=True, steps=10):
 
 
 # ------------------------------------------------------------------ CN forms
-# name -> (form, history start, merged update, confirm every solve) of the
-# plain form; the speed-ups are against plain_fp64_bicgstab, the plain solve
-# by BiCGStab (start extrapolated from the field's history, x, r and p updated
-# in one pass, the recursive residual accepted with the measured margin);
-# beside it the same from 2b - psi alone and with two update passes and every
-# solve confirmed by the true residual
-FORMS = {"plain_fp64_bicgstab": (0, 1, 1, 0), "plain_fp64_bicgstab_no_history": (0, 0, 1, 0),
-         "plain_fp64_bicgstab_two_pass_confirmed": (0, 1, 0, 1),
-         "precision_fp32_chebyshev_fp64_refinement": (1, 1, 1, 0), "learned_guess_precision": (2, 1, 1, 0)}
+# name -> (form, history start, BiCGStab's update or none, confirm every solve);
+# the speed-ups are against plain_fp64, the plain form as a program gets it (the
+# Chebyshev semi-iteration from the start extrapolated from the field's
+# history); beside it BiCGStab with x, r and p updated in one pass, the same
+# from 2b - psi alone, and with two update passes and every solve confirmed by
+# the true residual
+FORMS = {"plain_fp64": (0, 1, None, 0), "plain_fp64_bicgstab": (0, 1, "merged", 0),
+         "plain_fp64_bicgstab_no_history": (0, 0, "merged", 0),
+         "plain_fp64_bicgstab_two_pass_confirmed": (0, 1, "two-pass", 1),
+         "precision_fp32_chebyshev_fp64_refinement": (1, 1, None, 0), "learned_guess_precision": (2, 1, None, 0)}
 FORMS_SIZES = (64, 96, 128)
 # lattices of the precision form's drift (the precision configuration names 64^3 and 96^3)
 DRIFT_SIZES = (64, 96)
@@ -448,12 +449,15 @@ def measure_cn_forms(L, steps, params, tol=1e-10, seed=1):
         g.TransversePolarisedOccupiedInit_Box(0.5, 1.0, 0.0, RandomSeed=seed, identity_links=True)
         stream = torch.cuda.ExternalStream(lib.nrq_cuda_stream(lat.ctx))
         cw = _capi.coeffs(WILSON)
-        for name, (form, hist, merged, confirm) in FORMS.items():
+        for name, (form, hist, bicgstab, confirm) in FORMS.items():
             cn = ctypes.c_void_p()
             _capi.check(lib.nrq_cn_init(lat.ctx, MASS, _capi.dptr(cw), 1.0, tol, 10000, form, ctypes.byref(cn)),
                         lat.ctx, "nrq_cn_init")
             _capi.check(lib.nrq_cn_set_history_guess(cn, hist), lat.ctx, "history guess")
-            _capi.check(lib.nrq_cn_set_merged_update(cn, merged), lat.ctx, "merged update")
+            if bicgstab:
+                if bicgstab == "merged":  # beside the FMA stencil
+                    _capi.check(lib.nrq_cn_set_stencil(cn, 3), lat.ctx, "stencil")
+                _capi.check(lib.nrq_cn_set_merged_update(cn, int(bicgstab == "merged")), lat.ctx, "merged update")
             _capi.check(lib.nrq_cn_set_true_residual(cn, confirm), lat.ctx, "true residual")
             net = None
             if form == 2:
@@ -499,7 +503,7 @@ def measure_cn_forms(L, steps, params, tol=1e-10, seed=1):
         g.Deallocate()
     finally:
         lat.close()
-    base = out["plain_fp64_bicgstab"]["s_per_step"]
+    base = out["plain_fp64"]["s_per_step"]
     for v in out.values():
         v["speedup_vs_plain_fp64"] = base / v["s_per_step"]
     return out
