@@ -14,7 +14,9 @@ exceeds the 126 MB L2, so no flush is needed between steps.
 
 For N > 1 (launched with torch.distributed.run) every rank evolves its own
 independent lattice (an ensemble member, seed 1 + rank); there is no
-data-path collective.  Rank 0 prints one JSON line.
+data-path collective.  Rank 0 prints one JSON line of the headline; the
+sections beside it (the solver forms, the ensemble, the precision drift, the
+thermal and gluon workloads, every kernel class) go to the file of --sections.
 """
 from __future__ import annotations
 
@@ -82,8 +84,10 @@ def parse():
     p.add_argument("--no-gluon", action="store_true")
     p.add_argument("--only-gluon", action="store_true", help="print only the gluon-distribution JSON")
     p.add_argument("--only-thermal", action="store_true", help="print only the thermal initial-condition JSON")
-    p.add_argument("--stencil", default="timed", choices=["timed", "register", "tma", "tensor", "fma"],
-                   help="FP64 stencil of the headline step (default: the solver's timed choice)")
+    p.add_argument("--sections", default=os.path.join(ROOT, "bench_sections.json"),
+                   help="file of the full record, headline and sections")
+    p.add_argument("--stencil", default="default", choices=["default", "timed", "register", "tma", "tensor", "fma"],
+                   help="FP64 stencil of the headline step (default: the solver's own choice; timed: the fastest)")
     p.add_argument("--only-drift", action="store_true", help="print only the precision-drift JSON")
     p.add_argument("--two-pass", action="store_true",
                    help="headline step: the two-pass BiCGStab update in place of the merged one")
@@ -863,6 +867,37 @@ def max_over_ranks(x, dist=None):
     return float(t.item())
 
 
+def headline(line, path):
+    """The record's headline: its contract keys and one number or two of each
+    section, short enough to survive wherever only a line's end is kept."""
+    keep = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "clocks", "gpu_launches")
+    out = {k: line[k] for k in keep}
+    cfg = line["config"]
+    out["config"] = {k: cfg[k] for k in ("workload", "lattice", "mass", "krylov_tol", "l2", "parallelism", "plain_solve")}
+    roof = line["roofline"]
+    out["roofline"] = {k: roof[k] for k in ("bound", "kernel", "achieved", "peak", "unit", "frac", "peak_source",
+                                            "avg_launch_ms")}
+    out["cn"] = {k: line["cn"][k] for k in ("iterations_per_step", "matvecs_per_step", "max_rel_residual")}
+    if line["e2e"]:
+        out["e2e"] = {k: line["e2e"][k] for k in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")}
+    if line["cn_forms_at_1e-10"]:
+        short = {"plain_fp64": "plain_fp64", "plain_fp64_bicgstab": "plain_bicgstab",
+                 "precision_fp32_chebyshev_fp64_refinement": "precision", "learned_guess_precision": "learned"}
+        out["cn_s_per_step_at_1e-10"] = {size: {v: float("%.4g" % rows[k]["s_per_step"]) for k, v in short.items()}
+                                         for size, rows in line["cn_forms_at_1e-10"].items() if size.endswith("^3")}
+    if line["batching_ensemble"]:
+        out["ensemble_s_per_step"] = float("%.4g" % line["batching_ensemble"]["graph"]["s_per_step"])
+    if line["thermal_initial_condition"]:
+        out["thermal_projection_ms"] = line["thermal_initial_condition"]["projection_ms"]
+    if line["gluon_distribution"]:
+        out["gaugefix_ms"] = line["gluon_distribution"]["gaugefix_ms"]
+    if line.get("cpu_baseline"):
+        out["cpu_baseline"] = {k: line["cpu_baseline"][k] for k in ("value", "unit", "cores", "kind")}
+    out["sections"] = os.path.basename(path)
+    return out
+
+
 def free_port():
     import socket
     with socket.socket() as sk:
@@ -932,8 +967,8 @@ def main():
     lattice.InitModule([L, L, L], list(A), device=local)
     ctx = lattice.context()
     nrqcd.InitModule(MASS, WILSON, 1.0, TOL)
-    if args.stencil != "timed":
-        nrqcd.SetStencil({"register": nrqcd.STENCIL_REGISTER, "tma": nrqcd.STENCIL_TMA,
+    if args.stencil != "default":
+        nrqcd.SetStencil({"timed": None, "register": nrqcd.STENCIL_REGISTER, "tma": nrqcd.STENCIL_TMA,
                           "tensor": nrqcd.STENCIL_TENSOR, "fma": nrqcd.STENCIL_FMA}[args.stencil])
     if args.two_pass:
         nrqcd.SetMergedUpdate(False)
@@ -1141,7 +1176,9 @@ def main():
         }
         if world == 1 and not args.no_cpu_baseline:
             line["cpu_baseline"] = cpu_baseline_sample(min(L, 64))
-        print(json.dumps(line), flush=True)
+        with open(args.sections, "w") as f:
+            json.dump(line, f, indent=1)
+        print(json.dumps(headline(line, args.sections)), flush=True)
     del h, g
     nrqcd.FinalizeModule()
     lattice.FinalizeModule()
