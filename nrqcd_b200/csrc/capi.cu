@@ -907,7 +907,8 @@ int coulomb_short(nrq_gauge *g, double tol, double alpha, int64_t max_iterations
   const double pmax = max_norm2_momentum(ctx), scale = alpha / (double)V;
   double2 *cur = g->U, *alt = U2;
   int64_t queued = 0, found = -1;  // found: iterations whose deviation was above the tolerance
-  for (int batch = 8; found < 0 && queued < max_iterations; batch = 2 * batch < kBatch ? 2 * batch : kBatch) {
+  // (one iteration first: links that are fixed already end with it)
+  for (int batch = 1; found < 0 && queued < max_iterations;) {
     const int64_t first = queued;
     const int n = (int)std::min<int64_t>(batch, max_iterations - queued);
     double h[kBatch];
@@ -923,6 +924,13 @@ int coulomb_short(nrq_gauge *g, double tol, double alpha, int64_t max_iterations
     for (int k = 0; k < n && found < 0; ++k) {
       if (deviations) deviations[first + k] = h[k];
       if (!(h[k] > tol)) found = first + k;
+    }
+    // then as many as the last decay asks for: each one too many is three
+    // launches that return at entry (2 us apiece), each batch a read-back
+    batch = first == 0 ? 8 : kBatch;
+    if (n > 1) {
+      const double need = std::log(h[n - 1] / tol) / std::log(h[n - 2] / h[n - 1]);
+      if (need >= 0.0 && need < (double)(kBatch - 2)) batch = std::max(4, (int)need + 2);
     }
   }
   // the links of that deviation, or after max_iterations transformations
