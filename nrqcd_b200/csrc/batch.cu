@@ -409,9 +409,10 @@ Check check(const nrq_cn_batch *b) {
 // and species
 int steps_for(const nrq_cn_batch *b, double dt, double gain) {
   gain = std::max(gain, 10.0);
-  // FP32 arithmetic caps one pass at about 1e6; a pass that can finish the
-  // solve may aim up to 1e7 (the FP64 check decides whether it did)
-  if (gain > 1e7) gain = 1e6;
+  // An FP32 pass cannot gain more than about 3e7; a larger gain is shared
+  // evenly by two passes of at most 1e6, so that the first does not end just
+  // below the tolerance, where the update would stop
+  if (gain > 3e7) gain = std::min(std::sqrt(gain), 1e6);
   const double tau = dt * b->ctx->a[0] / 2.0;
   int m = 1;
   for (; m < nrq::BATCH_MAX_CHEB; ++m) {
