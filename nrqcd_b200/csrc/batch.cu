@@ -524,13 +524,13 @@ int refine_adaptive(nrq_cn_batch *b, double dt, cudaStream_t st, int budget, std
   return NRQ_OK;
 }
 
-// calibration step: adaptive passes with host synchronisation; records the
 int64_t sum(const std::vector<int> &v) {
   int64_t s = 0;
   for (int x : v) s += x;
   return s;
 }
 
+// calibration step: adaptive passes with host synchronisation; records the
 // schedule and tunes the kernels on the first call
 int update_calibrate(nrq_cn_batch *b, const nrq_gauge *g, const double c[8], double dt, cudaStream_t st,
                      Check &chk) {

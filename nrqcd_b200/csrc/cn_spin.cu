@@ -132,9 +132,10 @@ constexpr int kPrepSites = 32;
 // the site term of the hermitian H (A^H = 1 + i tau H) for quark and
 // antiquark.  One thread per site and direction; the Darwin and magnetic
 // matrices are sums over directions, exchanged through shared memory.  64^3:
-// 211 us, with the FP32 copy 240, at 12 warps an SM (168 registers; 255
-// registers, 8 warps: 286 and 315; 136 registers, 15 warps: 280 with the
-// copy), of which the traffic takes 90; 12^3: 10 us.
+// 217 us, with the FP32 copy 248, at 12 warps an SM (168 registers; without
+// the test that the plaquettes are unitary 211 and 240; 255 registers, 8
+// warps: 286 and 315; 136 registers, 15 warps: 280 with the copy), of which
+// the traffic takes 90; 12^3: 14 us.
 __global__ void __launch_bounds__(kPrepSites * 3, 4) k_spin_prepare(Lat L, CnCoef C1, const CnCoef *__restrict__ Cm,
                                                                 int nm, double tau, const double2 *__restrict__ U,
                                                                 const double *__restrict__ E, SpinOp op,

@@ -20,8 +20,8 @@ template <>
 struct Num<double> {
   using v2 = double2;
   // Spinor operands in registers: this step's and the next three's; matrices
-  // staged two neighbours ahead.  (64^3, a coupled step: 4.16 ms with the
-  // next two and one neighbour, 4.09 with the next three, 3.98 with both.
+  // staged two neighbours ahead.  (64^3, a coupled step: 4.24 ms with the
+  // next two and one neighbour, 4.09 with the next three, 4.02 with both.
   // Prefetches to L2, of the epilogue's operands or of later units', cost
   // 2-20 %; a persistent form with the next unit's first loads issued early
   // 10 %.)

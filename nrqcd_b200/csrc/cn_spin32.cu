@@ -15,7 +15,9 @@
 //
 // Bound: 64^3, 3.1 KB a site: 0.12 ms at the copy rate, 0.08 ms of FP32
 // FMAs; it takes 0.24 ms (the (d, r, e) recurrence on dense 6x6 blocks 0.36,
-// and 0.10 more for the final addition), 32 fields at 24^3 0.43 ms (0.74).
+// and 0.10 more for the final addition), 32 fields at 24^3 0.43 ms (0.74).  The
+// last launch, 6.1 KB a site with the history, takes 0.37 ms (0.31 adding to an
+// FP32 history; two blocks an SM, 131 registers and no spill: 0.42).
 // Four blocks an SM (80 registers) hide the latency of the loads only in
 // part.
 #include "cn_spin.cuh"
@@ -200,6 +202,8 @@ void go(bool first, bool last, int64_t blocks, Lat L, const SpinOp32 &op, const 
 }
 }  // namespace
 
+// The kernel serves any lattice; the line is the one that callers who force the
+// step were given (nrq_cn_set_cheb_stencil), and the default choice keeps to it.
 bool cheb_spin_applicable(const Lat &L) {
   return L.V >= 36 && L.V <= 0x7fffffffLL && (L.V % 4) == 0 && (L.nx % 2) == 0;
 }
